@@ -40,7 +40,7 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--fmad=false", "-Xcompiler", "-
               "--expt-relaxed-constexpr", "-I", str(INCLUDE), "-I", str(CSRC)]
 # The contracted FP64 build: the compiler may fuse a multiply and an add into
 # one FMA (one rounding instead of two).
-NVCC_FMA_FLAGS = [f if f != "--fmad=false" else "--fmad=true" for f in NVCC_FLAGS]
+NVCC_FMA_FLAGS = [f if f != "--fmad=false" else "--fmad=true" for f in NVCC_FLAGS] + ["-DUNS_FP64_CONTRACT"]
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-Wall", "-Wno-unused-function",
              "-I", str(INCLUDE), "-I", str(CSRC / "host")]
 

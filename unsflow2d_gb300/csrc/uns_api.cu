@@ -18,6 +18,27 @@ __global__ void k_selftest_ratio(const double* a, const double* b, const double*
     if (i >= n) return;
     lt[i] = (uns::ratio_ok(a[i], b[i]) && uns::ratio_ok(c[i], d[i])) ? (uns::ratio_less(a[i], b[i], c[i], d[i]) ? 1 : 0) : -1;
 }
+// The operations of uns_fp64.cuh by number, in the order of uns_selftest_fp64.
+__global__ void k_selftest_fp64(int op, const double* a, const double* b, double* out, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double x = a[i], y = b[i];
+    double r = 0.0;
+    switch (op) {
+        case 0: r = uns::add64(x, y); break;
+        case 1: r = uns::sub64(x, y); break;
+        case 2: r = uns::mul64(x, y); break;
+        case 3: r = uns::div_digits(x, y); break;
+        case 4: r = uns::sqrt_digits(x); break;
+        case 5: r = uns::dhalf(x); break;
+        case 6: r = uns::dtwice(x); break;
+        case 7: r = uns::dlt(x, y) ? 1.0 : 0.0; break;
+        case 8: r = uns::dle(x, y) ? 1.0 : 0.0; break;
+        case 10: r = uns::mul_digits(x, y); break;
+        case 9: r = uns::dpos(x) ? 1.0 : (uns::dneg(x) ? -1.0 : 0.0); break;
+    }
+    out[i] = r;
+}
 
 // Copies n values of each host array in, runs launch, copies out.
 template <class T, class L>
@@ -58,6 +79,12 @@ const char* uns_version(void) { return "unsflow_gpu 0.1 (sm_103a)"; }
 int uns_selftest_div(const double* a, const double* b, double* out, int n) {
     return run_selftest("uns_selftest_div", n, {a, b}, out, [&](std::vector<double*>& d, double* o, int nb) {
         k_selftest_div<<<nb, 256>>>(d[0], d[1], o, n);
+    });
+}
+
+int uns_selftest_fp64(int op, const double* a, const double* b, double* out, int n) {
+    return run_selftest("uns_selftest_fp64", n, {a, b}, out, [&](std::vector<double*>& d, double* o, int nb) {
+        k_selftest_fp64<<<nb, 256>>>(op, d[0], d[1], o, n);
     });
 }
 

@@ -314,6 +314,9 @@ __global__ void __launch_bounds__(kBlock) k_face_ggfc(CCView v) {
 
 __device__ __forceinline__ void d4get(const double4& q, double o[4]) { o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w; }
 __device__ __forceinline__ double4 d4(const double o[4]) { return make_double4(o[0], o[1], o[2], o[3]); }
+__device__ __forceinline__ void f4get(const double4& q, F64 o[4]) { o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w; }
+__device__ __forceinline__ void f4get(const double4& q, F64I o[4]) { o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w; }
+__device__ __forceinline__ double4 f4(const F64 o[4]) { return make_double4(o[0].v, o[1].v, o[2].v, o[3].v); }
 
 // Per-cell gather over the index-sorted face list: spectral radius + dt
 // (timestep.F90:40-49, 101-103), the cell gradient (Gradient_GG
@@ -738,7 +741,7 @@ __device__ __forceinline__ double4 bnd_face_flux(const CCView& v, const Gas& g, 
     const double area = v.farea[f];
     const double2 fc = v.fcen[f];
     const double2 ci = v.cen[in];
-    double qi[4], gxi[4], gyi[4], phi_i[4];
+    F64 qi[4], gxi[4], gyi[4], phi_i[4];
     if constexpr (std::is_same<R, float>::value) {
         const float4* A = v.packf + 4 * (size_t)in;
         const float4 a0 = A[0], a1 = A[1], a2 = A[2], a3 = A[3];
@@ -747,26 +750,26 @@ __device__ __forceinline__ double4 bnd_face_flux(const CCView& v, const Gas& g, 
         gyi[0] = a2.x; gyi[1] = a2.y; gyi[2] = a2.z; gyi[3] = a2.w;
         phi_i[0] = a3.x; phi_i[1] = a3.y; phi_i[2] = a3.z; phi_i[3] = a3.w;
     } else {
-        d4get(v.qp[in], qi);
-        d4get(v.gx[in], gxi);
-        d4get(v.gy[in], gyi);
-        d4get(v.phi[in], phi_i);
+        f4get(v.qp[in], qi);
+        f4get(v.gx[in], gxi);
+        f4get(v.gy[in], gyi);
+        f4get(v.phi[in], phi_i);
     }
     const int bc = v.fbc[f];
-    const double d0 = fc.x - ci.x, d1 = fc.y - ci.y;
-    V4<double> qcl;
+    const F64 d0 = F64(fc.x) - ci.x, d1 = F64(fc.y) - ci.y;
+    V4<F64> qcl;
 #pragma unroll
     for (int j = 0; j < 4; ++j) qcl[j] = qi[j] + phi_i[j] * (gxi[j] * d0 + gyi[j] * d1);
     double4 Fd = make_double4(0.0, 0.0, 0.0, 0.0);
     if (bc == 2001 || bc == 1001) {
-        const V4<double> cin = {cin4[0], cin4[1], cin4[2], cin4[3]};
-        CCBnd<double> b = cc_boundary<double, R>(g, bc, n.x, n.y, area, qcl, cin, g.u_inf, g.v_inf);
+        const V4<F64> cin = {cin4[0], cin4[1], cin4[2], cin4[3]};
+        CCBnd<F64> b = cc_boundary<F64, typename Arith<R>::type, F64>(g, bc, n.x, n.y, area, qcl, cin, g.u_inf, g.v_inf);
         if (!b.ok) set_err(v.err, UNS_ERR_NEG_SOUND_SPEED, f);
-        Fd = make_double4(b.F[0], b.F[1], b.F[2], b.F[3]);
+        Fd = make_double4(b.F[0].v, b.F[1].v, b.F[2].v, b.F[3].v);
         const int out = v.fnb[f].y;
-        v.qc[out] = make_double4(b.gq[0], b.gq[1], b.gq[2], b.gq[3]);
-        v.qp[out] = make_double4(b.gp[0], b.gp[1], b.gp[2], b.gp[3]);
-        v.qT[out] = b.gT;
+        v.qc[out] = make_double4(b.gq[0].v, b.gq[1].v, b.gq[2].v, b.gq[3].v);
+        v.qp[out] = make_double4(b.gp[0].v, b.gp[1].v, b.gp[2].v, b.gp[3].v);
+        v.qT[out] = b.gT.v;
         v.qpf[out] = make_float4((float)b.gp[0], (float)b.gp[1], (float)b.gp[2], (float)b.gp[3]);
         if (bc == 1001) v.fwall[f - v.nfi] = make_double2(Fd.z, Fd.w);
     }
@@ -774,6 +777,12 @@ __device__ __forceinline__ double4 bnd_face_flux(const CCView& v, const Gas& g, 
     return Fd;
 }
 
+// FP64 form, 4.2 M cells: 3.85 -> 1.79 ms.  It was bound by the FP64 unit
+// (228 operations and 14 divisions and square roots per face); now its sums
+// alone are there (6.0 k cycles per warp) and its products, divisions, square
+// roots and halvings on the integer pipe (about 8 k), and what remains above
+// the longer of the two is instruction fetch (4 900 instructions per face,
+// each run once per warp; ncu: 3.2 of 12 stall cycles per issue).
 // One thread per face; the first blocks take the boundary faces, whose FP64
 // ghost arithmetic is the longest per thread, so that they run beside the
 // interior faces instead of after them.
@@ -821,31 +830,30 @@ __global__ void __launch_bounds__(512, std::is_same<R, float>::value ? 2 : 1) k_
         const double area = v.farea[f];
         const double2 fc = v.fcen[f];
         const double2 ci = v.cen[in], co = v.cen[out];
-        double qi[4], gxi[4], gyi[4], phi_i[4], qo[4], gxo[4], gyo[4], phi_o[4];
-        d4get(v.qp[in], qi);
-        d4get(v.gx[in], gxi);
-        d4get(v.gy[in], gyi);
-        d4get(v.phi[in], phi_i);
-        d4get(v.qp[out], qo);
-        d4get(v.gx[out], gxo);
-        d4get(v.gy[out], gyo);
-        d4get(v.phi[out], phi_o);
-        const double zhi = 1.0 / 3.0;
-        double dl0 = fc.x - ci.x, dl1 = fc.y - ci.y;
-        double dr0 = fc.x - co.x, dr1 = fc.y - co.y;
-        V4<double> ql, qr, F;
+        F64I qi[4], gxi[4], gyi[4], phi_i[4], qo[4], gxo[4], gyo[4], phi_o[4];
+        f4get(v.qp[in], qi);
+        f4get(v.gx[in], gxi);
+        f4get(v.gy[in], gyi);
+        f4get(v.phi[in], phi_i);
+        f4get(v.qp[out], qo);
+        f4get(v.gx[out], gxo);
+        f4get(v.gy[out], gyo);
+        f4get(v.phi[out], phi_o);
+        const F64I zhi = 1.0 / 3.0, zlo = 1.0 - 1.0 / 3.0;
+        const F64I dl0 = F64I(fc.x) - ci.x, dl1 = F64I(fc.y) - ci.y;
+        const F64I dr0 = F64I(fc.x) - co.x, dr1 = F64I(fc.y) - co.y;
+        V4<F64I> ql, qr, F;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {  // recon (fvresidual.F90:235-247)
-            double alfa = gxi[j] * dl0 + gyi[j] * dl1;
-            double beta = qo[j] - qi[j];
-            ql[j] = qi[j] + 0.5 * phi_i[j] * (zhi * beta + (1.0 - zhi) * alfa);
+        for (int j = 0; j < 4; ++j) {  // recon (fvresidual.F90:235-247); the two sides' beta differ in sign alone
+            const F64I zb = zhi * (qo[j] - qi[j]);
+            F64I alfa = gxi[j] * dl0 + gyi[j] * dl1;
+            ql[j] = qi[j] + half(phi_i[j]) * (zb + zlo * alfa);
             alfa = gxo[j] * dr0 + gyo[j] * dr1;
-            beta = qi[j] - qo[j];
-            qr[j] = qo[j] + 0.5 * phi_o[j] * (zhi * beta + (1.0 - zhi) * alfa);
+            qr[j] = qo[j] + half(phi_o[j]) * (zlo * alfa - zb);
         }
-        bool ok = flux_dispatch<double>(g, n.x, n.y, area, ql, qr, F);
+        bool ok = flux_dispatch<F64I>(g, n.x, n.y, area, ql, qr, F);
         if (!ok) set_err(v.err, UNS_ERR_NEG_SOUND_SPEED, f);
-        v.fF[f] = make_double4(F[0], F[1], F[2], F[3]);
+        v.fF[f] = make_double4(F[0].v, F[1].v, F[2].v, F[3].v);
     }
 }
 
@@ -1831,17 +1839,9 @@ int enqueue_minmax(uns_cc_handle* h, CCView& v) {
 // k_face_conv's grid: the boundary faces' blocks, then the interior faces'.
 #define LAUNCH_FACE_CONV(R, v)                                                                     \
     do {                                                                                           \
-        const int bs_ = (v).blk_face;                                                              \
+        const int bs_ = face_bs<R>(h, (v));                                                        \
         const int nb_ = std::max(1, ((v).nbf + bs_ - 1) / bs_ + ((v).nfi + bs_ - 1) / bs_);        \
         k_face_conv<R><<<nb_, bs_, 0, h->stream>>>(v);                                             \
-        UNS_CUDA(cudaGetLastError());                                                              \
-    } while (0)
-
-// A launch over n items with block size bs.
-#define LAUNCH_BS(kern, n, bs, ...)                                                                \
-    do {                                                                                           \
-        const int bs_ = (bs);                                                                      \
-        kern<<<std::max(1, (int)(((n) + bs_ - 1) / bs_)), bs_, 0, h->stream>>>(__VA_ARGS__);       \
         UNS_CUDA(cudaGetLastError());                                                              \
     } while (0)
 
@@ -1856,6 +1856,25 @@ inline int spread_bs(const uns_cc_handle* h, int n) {
     while (bs > 32 && (n + bs - 1) / bs < 2 * h->nsm) bs >>= 1;
     return bs;
 }
+
+// Block size of k_face_conv: blk_face in the mixed form and where a caller or
+// the autotuner has set one; in the FP64 form else spread_bs, because that
+// form's code is longer than the instruction cache and the warps of a large
+// block run through it together (4.2 M cells: 1.79 ms at 256 threads, 2.14 at
+// 64; 16 384 cells, where spread_bs gives 64: 33 us, 40 at 256).
+template <class R>
+inline int face_bs(const uns_cc_handle* h, const CCView& v) {
+    return std::is_same<R, float>::value || h->blk_face_set ? v.blk_face : spread_bs(h, v.nof);
+}
+
+// A launch over n items with block size bs.
+#define LAUNCH_BS(kern, n, bs, ...)                                                                \
+    do {                                                                                           \
+        const int bs_ = (bs);                                                                      \
+        kern<<<std::max(1, (int)(((n) + bs_ - 1) / bs_)), bs_, 0, h->stream>>>(__VA_ARGS__);       \
+        UNS_CUDA(cudaGetLastError());                                                              \
+    } while (0)
+
 #define LAUNCH_SPREAD(kern, n, ...) LAUNCH_BS(kern, (n), spread_bs(h, (n)), __VA_ARGS__)
 
 #define LAUNCH_CELL_GRAD(v, flags, cfl)                                                 \
@@ -1899,10 +1918,11 @@ bool grad_by_sides(const uns_cc_handle* h, const CCView& v) {
 // reference main loop's RK stages 2 and 3): the boundary faces' fluxes and
 // the wall cells' residuals; every other cell keeps the residual it has.
 int enqueue_wall_res(uns_cc_handle* h, CCView& v) {
-    const int nbb = (v.nbf + v.blk_face - 1) / v.blk_face;  // k_face_conv's boundary blocks come first
+    const int bs = v.mixed ? face_bs<float>(h, v) : face_bs<double>(h, v);
+    const int nbb = (v.nbf + bs - 1) / bs;  // k_face_conv's boundary blocks come first
     if (nbb == 0) return UNS_OK;
-    if (v.mixed) k_face_conv<float><<<nbb, v.blk_face, 0, h->stream>>>(v);
-    else k_face_conv<double><<<nbb, v.blk_face, 0, h->stream>>>(v);
+    if (v.mixed) k_face_conv<float><<<nbb, bs, 0, h->stream>>>(v);
+    else k_face_conv<double><<<nbb, bs, 0, h->stream>>>(v);
     UNS_CUDA(cudaGetLastError());
     if (v.nwcell > 0) {
         const int nb = (v.nwcell + 31) / 32;
@@ -2270,6 +2290,7 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
         const int b = e ? std::atoi(e) : def;
         return (b == 64 || b == 128 || b == 256 || b == 512) && b <= hi ? b : def;
     };
+    h->blk_face_set = std::getenv("UNS_CC_BLOCK_FACE") != nullptr;
     v.blk_face = block_env("UNS_CC_BLOCK_FACE", 64, 512);
     v.blk_vert = block_env("UNS_CC_BLOCK_VERTEX", kBlock, 512);
     v.blk_grad = block_env("UNS_CC_BLOCK_GRAD", 128, kBlock);
@@ -3031,7 +3052,7 @@ int uns_cc_autotune(uns_cc_handle* h, int reps, int* blocks) {
     cudaStreamSynchronize(h->stream);
     release();
     if (rc) return rc;
-    if (bf) h->v.blk_face = bf;
+    if (bf) { h->v.blk_face = bf; h->blk_face_set = true; }
     if (bv) h->v.blk_vert = bv;
     if (bg) h->v.blk_grad = bg;
     if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }

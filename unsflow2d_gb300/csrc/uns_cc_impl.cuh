@@ -150,6 +150,7 @@ struct uns_cc_handle {
     // LU-SGS levels
     int* woff = nullptr;   // LU-SGS warp schedule: per-warp ranges of v.sched
     int coop_blocks = 0;
+    bool blk_face_set = false;  // v.blk_face was chosen (environment, autotuner), not the default
     int nsm = 1;           // SMs of the device (launch widths of small meshes)
     double4 qinf;
     // graph fast path

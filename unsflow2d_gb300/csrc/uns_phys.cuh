@@ -6,6 +6,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "uns_fp64.cuh"
 #include "unsflow_types.h"
 
 namespace uns {
@@ -52,7 +53,7 @@ template <class R>
 __device__ __forceinline__ V4<R> prim2con(R gamma, const V4<R>& pr) {
     V4<R> c;
     R rho = pr[0], u = pr[1], v = pr[2], p = pr[3];
-    c[0] = p / (gamma - R(1)) + R(0.5) * rho * (u * u + v * v);
+    c[0] = p / (gamma - R(1)) + half(rho) * (u * u + v * v);
     c[1] = rho;
     c[2] = rho * u;
     c[3] = rho * v;
@@ -60,22 +61,37 @@ __device__ __forceinline__ V4<R> prim2con(R gamma, const V4<R>& pr) {
 }
 
 // Mach-number polynomials (CCFVM/solution.F90:265-359)
-template <class R> __device__ __forceinline__ R m1p(R m) { return R(0.5) * (m + fabs(m)); }
-template <class R> __device__ __forceinline__ R m1m(R m) { return R(0.5) * (m - fabs(m)); }
-template <class R> __device__ __forceinline__ R m2p(R m) { return R(0.25) * (m + R(1)) * (m + R(1)); }
-template <class R> __device__ __forceinline__ R m2m(R m) { return R(-0.25) * (m - R(1)) * (m - R(1)); }
-template <class R> __device__ __forceinline__ R m4p(R m, R beta) {
-    return fabs(m) >= R(1) ? R(0.5) * (m + fabs(m)) : m2p(m) * (R(1) - R(16) * beta * m2m(m));
+template <class R> __device__ __forceinline__ R m1p(R m) { return half(m + fabs(m)); }
+template <class R> __device__ __forceinline__ R m1m(R m) { return half(m - fabs(m)); }
+template <class R> __device__ __forceinline__ R m2p(R m) { return quarter(m + R(1)) * (m + R(1)); }
+template <class R> __device__ __forceinline__ R m2m(R m) { return -quarter(m - R(1)) * (m - R(1)); }
+// Fourth- and fifth-degree splittings; beta and al come as 16 beta, 16 al
+// (exact), and kPlain is the case of both zero (van Leer), where the
+// correction factor is one or (+-2 - m) itself.
+template <bool kPlain, class R> __device__ __forceinline__ R m4p(R m, R beta16) {
+    if (fabs(m) >= R(1)) return half(m + fabs(m));
+    if (kPlain) return m2p(m);
+    return m2p(m) * (R(1) - beta16 * m2m(m));
 }
-template <class R> __device__ __forceinline__ R m4m(R m, R beta) {
-    return fabs(m) >= R(1) ? R(0.5) * (m - fabs(m)) : m2m(m) * (R(1) + R(16) * beta * m2p(m));
+template <bool kPlain, class R> __device__ __forceinline__ R m4m(R m, R beta16) {
+    if (fabs(m) >= R(1)) return half(m - fabs(m));
+    if (kPlain) return m2m(m);
+    return m2m(m) * (R(1) + beta16 * m2p(m));
 }
-template <class R> __device__ __forceinline__ R p5p(R m, R al) {
-    return fabs(m) >= R(1) ? R(0.5) * (m + fabs(m)) / m : m2p(m) * ((R(2) - m) - R(16) * al * m * m2m(m));
+template <bool kPlain, class R> __device__ __forceinline__ R p5p(R m, R al16) {
+    if (fabs(m) >= R(1)) return half(m + fabs(m)) / m;
+    if (kPlain) return m2p(m) * (R(2) - m);
+    return m2p(m) * ((R(2) - m) - al16 * m * m2m(m));
 }
-template <class R> __device__ __forceinline__ R p5m(R m, R al) {
-    return fabs(m) >= R(1) ? R(0.5) * (m - fabs(m)) / m : m2m(m) * ((R(-2) - m) + R(16) * al * m * m2p(m));
+template <bool kPlain, class R> __device__ __forceinline__ R p5m(R m, R al16) {
+    if (fabs(m) >= R(1)) return half(m - fabs(m)) / m;
+    if (kPlain) return m2m(m) * (R(-2) - m);
+    return m2m(m) * ((R(-2) - m) + al16 * m * m2p(m));
 }
+// gamma - 1 formed from gamma in R; in 64 bits that is gamma1 itself.
+template <class R> __device__ __forceinline__ R less_one(R G, R) { return G - R(1); }
+__device__ __forceinline__ F64 less_one(F64, F64 G1) { return G1; }
+__device__ __forceinline__ F64I less_one(F64I, F64I G1) { return G1; }
 
 // Roe flux with Harten entropy fix (CCFVM/roe_flux.F90:1-155).  Returns
 // false where the Roe-averaged a^2 <= 0 (the reference stops there).
@@ -85,10 +101,10 @@ __device__ __forceinline__ bool roe_flux(R G, R G1, R nx, R ny, R area, const V4
     R rr = qr[0], ur = qr[1], vr = qr[2], pr = qr[3];
     R ql2 = ul * ul + vl * vl;
     R al2 = G * pl / rl;
-    R hl = al2 / G1 + R(0.5) * ql2;
+    R hl = al2 / G1 + half(ql2);
     R qr2 = ur * ur + vr * vr;
     R ar2 = G * pr / rr;
-    R hr = ar2 / G1 + R(0.5) * qr2;
+    R hr = ar2 / G1 + half(qr2);
     R unl = ul * nx + vl * ny;
     R unr = ur * nx + vr * ny;
     R fc0 = rl * hl * unl + rr * hr * unr;
@@ -101,34 +117,34 @@ __device__ __forceinline__ bool roe_flux(R G, R G1, R nx, R ny, R area, const V4
     R va = (vl * rl12 + vr * rr12) * rd;
     R ha = (hl * rl12 + hr * rr12) * rd;
     R qa2 = ua * ua + va * va;
-    R aa2 = G1 * (ha - R(0.5) * qa2);
+    R aa2 = G1 * (ha - half(qa2));
     bool ok = !(aa2 <= R(0));  // roe_flux.F90:73: `if (aa2 .le. 0)` -- a NaN goes on, as there
     R aa = sqrt(aa2);
     R una = ua * nx + va * ny;
     R vna = -ua * ny + va * nx;
     R e1 = fabs(una - aa), e2 = fabs(una), e4 = fabs(una + aa);
     R del = R(0.1) * aa;
-    R l1 = (e1 < del) ? R(0.5) * (del + e1 * e1 / del) : e1;
-    R l2 = (e2 < del) ? R(0.5) * (del + e2 * e2 / del) : e2;
+    R l1 = (e1 < del) ? half(del + e1 * e1 / del) : e1;
+    R l2 = (e2 < del) ? half(del + e2 * e2 / del) : e2;
     R l3 = l2;
-    R l4 = (e4 < del) ? R(0.5) * (del + e4 * e4 / del) : e4;
+    R l4 = (e4 < del) ? half(del + e4 * e4 / del) : e4;
     R du1 = rr - rl;
     R du2 = rr * ur - rl * ul;
     R du3 = rr * vr - rl * vl;
     R du4 = (rr * hr - pr) - (rl * hl - pl);
     R m1 = (nx * du2 + ny * du3 - una * du1) / aa;
     R m2 = G1 * (du4 - ua * du2 - va * du3 + qa2 * du1) / (aa * aa);
-    R a1 = R(0.5) * (m2 - m1);
+    R a1 = half(m2 - m1);
     R a2 = (ny * du2 - nx * du3 + vna * du1) / aa;
-    R a4 = R(0.5) * (m1 + m2);
+    R a4 = half(m1 + m2);
     R a3 = du1 - a1 - a4;
     R a1l1 = a1 * l1, a2l2 = a2 * l2, a3l3 = a3 * l3, a4l4 = a4 * l4;
     R aact = aa * nx, aast = aa * ny;
-    R Fd0 = a1l1 * (ha - una * aa) + a2l2 * aa * vna + a3l3 * R(0.5) * qa2 + a4l4 * (ha + una * aa);
+    R Fd0 = a1l1 * (ha - una * aa) + a2l2 * aa * vna + half(a3l3) * qa2 + a4l4 * (ha + una * aa);
     R Fd1 = a1l1 + a3l3 + a4l4;
     R Fd2 = a1l1 * (ua - aact) + a2l2 * aa * ny + a3l3 * ua + a4l4 * (ua + aact);
     R Fd3 = a1l1 * (va - aast) - a2l2 * aa * nx + a3l3 * va + a4l4 * (va + aast);
-    R h = R(0.5) * area;
+    R h = half(area);
     flux[0] = h * (fc0 - Fd0);
     flux[1] = h * (fc1 - Fd1);
     flux[2] = h * (fc2 - Fd2);
@@ -143,12 +159,12 @@ __device__ __forceinline__ void rusanov_flux(R G, R G1, R nx, R ny, R area, V4<R
     R rol = ql[0], ul = ql[1], vl = ql[2], pl = ql[3];
     R ql2 = ul * ul + vl * vl;
     R al2 = G * pl / rol;
-    R hl = al2 / G1 + R(0.5) * ql2;
+    R hl = al2 / G1 + half(ql2);
     R cl = sqrt(G * pl / rol);
     R ror = qr[0], ur = qr[1], vr = qr[2], pr = qr[3];
     R qr2 = ur * ur + vr * vr;
     R ar2 = G * pr / ror;
-    R hr = ar2 / G1 + R(0.5) * qr2;
+    R hr = ar2 / G1 + half(qr2);
     R cr = sqrt(G * pr / ror);
     R unl = ul * nx + vl * ny;
     R unr = ur * nx + vr * ny;
@@ -161,7 +177,7 @@ __device__ __forceinline__ void rusanov_flux(R G, R G1, R nx, R ny, R area, V4<R
     for (int i = 0; i < 4; ++i) {
         R f = fl[i] + fr[i];
         f = f + eigen * (ql[i] - qr[i]);
-        flux[i] = R(0.5) * area * f;
+        flux[i] = half(area) * f;
     }
 }
 
@@ -174,29 +190,30 @@ __device__ __forceinline__ void vanleer_core(R G, R G1, R nx, R ny, const V4<R>&
     R unl = ul * nx + vl * ny;
     R ql2 = ul * ul + vl * vl;
     R al2 = G * pl / rl;
-    R hl = al2 / G1 + R(0.5) * ql2;
+    R hl = al2 / G1 + half(ql2);
     R cl = sqrt(al2);
     R ml = unl / cl;
     R rr = qr[0], ur = qr[1], vr = qr[2], pr = qr[3];
     R unr = ur * nx + vr * ny;
     R qr2 = ur * ur + vr * vr;
     R ar2 = G * pr / rr;
-    R hr = ar2 / G1 + R(0.5) * qr2;
+    R hr = ar2 / G1 + half(qr2);
     R cr = sqrt(ar2);
     R mr = unr / cr;
     const R zero = R(0);
-    R plp = p5p(ml, zero), prm = p5m(mr, zero);
-    R mlp = m4p(ml, zero), mlm = m4m(ml, zero), mrp = m4p(mr, zero), mrm = m4m(mr, zero);
+    R plp = p5p<true>(ml, zero), prm = p5m<true>(mr, zero);
+    R mlp = m4p<true>(ml, zero), mlm = m4m<true>(ml, zero), mrp = m4p<true>(mr, zero), mrm = m4m<true>(mr, zero);
     R p12 = plp * pl + prm * pr;
     R fmass_p = rl * cl * mlp;
     R fmass_m = rr * cr * mrm;
     R fmass12 = fmass_p + fmass_m;
-    R delta = -(G * (cr * mrp * mrm * pr - cl * mlp * mlm * pl) / (G - R(1)));
+    R delta = -(G * (cr * mrp * mrm * pr - cl * mlp * mlm * pl) / less_one(G, G1));
     R dissi = fmass_p - fmass_m;
-    R fL[4] = {hl, R(1), ul, vl}, fR[4] = {hr, R(1), ur, vr};
-    R fP[4] = {delta, R(0), nx * p12, ny * p12};
-    for (int i = 0; i < 4; ++i)
-        flux[i] = R(0.5) * fmass12 * (fL[i] + fR[i]) - R(0.5) * dissi * (fR[i] - fL[i]) + fP[i];
+    const R hm = half(fmass12), hd = half(dissi);
+    flux[0] = hm * (hl + hr) - hd * (hr - hl) + delta;
+    flux[1] = hm * R(2) - hd * R(0) + R(0);
+    flux[2] = hm * (ul + ur) - hd * (ur - ul) + nx * p12;
+    flux[3] = hm * (vl + vr) - hd * (vr - vl) + ny * p12;
     hl_o = hl;
     hr_o = hr;
 }
@@ -206,24 +223,25 @@ __device__ __forceinline__ void vanleer_core(R G, R G1, R nx, R ny, const V4<R>&
 template <class R>
 __device__ __forceinline__ void ausm_core(R G, R G1, R nx, R ny, R mref, const V4<R>& ql, const V4<R>& qr, V4<R>& flux,
                                           R& hl_o, R& hr_o) {
-    const R sigma = R(1), ku = R(0.75), kp = R(0.25);
+    const R ku = R(0.75), kp = R(0.25);  // and sigma = 1
     R rl = ql[0], ul = ql[1], vl = ql[2], pl = ql[3];
     R unl = ul * nx + vl * ny;
     R ql2 = ul * ul + vl * vl;
     R al2 = G * pl / rl;
-    R hl = al2 / G1 + R(0.5) * ql2;
+    R hl = al2 / G1 + half(ql2);
     R rr = qr[0], ur = qr[1], vr = qr[2], pr = qr[3];
     R unr = ur * nx + vr * ny;
     R qr2 = ur * ur + vr * vr;
     R ar2 = G * pr / rr;
-    R hr = ar2 / G1 + R(0.5) * qr2;
-    R aL_star = sqrt(R(2) * (G - R(1)) * hl / (G + R(1)));
-    R aR_star = sqrt(R(2) * (G - R(1)) * hr / (G + R(1)));
+    R hr = ar2 / G1 + half(qr2);
+    const R gp1 = G + R(1), gm1 = less_one(G, G1);
+    R aL_star = sqrt(twice(gm1) * hl / gp1);
+    R aR_star = sqrt(twice(gm1) * hr / gp1);
     R aL_hat = aL_star * aL_star / rmax(aL_star, fabs(unl));
-    R aR_hat = aR_star * aR_star / rmax(aR_star, R(-1) * fabs(unr));
+    R aR_hat = aR_star * aR_star / rmax(aR_star, -fabs(unr));
     R c12 = rmin(aL_hat, aR_hat);
     R ml = unl / c12, mr = unr / c12;
-    R mbar2 = R(0.5) * (unl * unl + unr * unr) / (c12 * c12);
+    R mbar2 = half(unl * unl + unr * unr) / (c12 * c12);
     R fa;
     if (mbar2 >= R(1)) {
         fa = R(1);
@@ -232,20 +250,20 @@ __device__ __forceinline__ void ausm_core(R G, R G1, R nx, R ny, R mref, const V
         R Mo = mstar2;
         fa = Mo * (R(2) - Mo);
     }
-    R beta = R(1) / R(8);
-    R alpha = R(3) / R(16) * (R(-4) + R(5) * fa * fa);
-    R plp = p5p(ml, alpha), prm = p5m(mr, alpha);
-    R mlp = m4p(ml, beta), mrm = m4m(mr, beta);
-    R ro12 = R(0.5) * (rl + rr);
-    R mp = -((kp / fa) * rmax((R(1) - sigma * mbar2), R(0)) * (pr - pl) / (ro12 * c12 * c12));
+    const R beta16 = R(2);  // beta = 1/8
+    const R alpha16 = R(16) * (R(0.1875) * (R(-4) + R(5) * fa * fa));
+    R plp = p5p<false>(ml, alpha16), prm = p5m<false>(mr, alpha16);
+    R mlp = m4p<false>(ml, beta16), mrm = m4m<false>(mr, beta16);
+    R ro12 = half(rl + rr);
+    R mp = -((kp / fa) * rmax(R(1) - mbar2, R(0)) * (pr - pl) / (ro12 * c12 * c12));
     R m12 = mlp + mrm + mp;
-    R pu = -(ku * plp * prm * R(2) * ro12 * fa * c12 * (unr - unl));
+    R pu = -(twice(ku * plp * prm) * ro12 * fa * c12 * (unr - unl));
     R p12 = plp * pl + prm * pr + pu;
-    R fl[4] = {hl, R(1), ul, vl}, fr[4] = {hr, R(1), ur, vr};
     R a = m1p(m12) * rl, b = m1m(m12) * rr;
-    for (int i = 0; i < 4; ++i) flux[i] = c12 * (a * fl[i] + b * fr[i]);
-    flux[2] = flux[2] + nx * p12;
-    flux[3] = flux[3] + ny * p12;
+    flux[0] = c12 * (a * hl + b * hr);
+    flux[1] = c12 * (a + b);
+    flux[2] = c12 * (a * ul + b * ur) + nx * p12;
+    flux[3] = c12 * (a * vl + b * vr) + ny * p12;
     hl_o = hl;
     hr_o = hr;
 }
@@ -265,23 +283,23 @@ __device__ __forceinline__ V4<R> farfield_state(R G, R G1, R nx, R ny, R rinf, R
         qb[0] = rho; qb[1] = un * nx + tn * tx; qb[2] = un * ny + tn * ty; qb[3] = p;
     } else if (R(0) <= mach && mach < R(1)) {
         R Vninf = uinf * nx + vinf * ny;
-        R Rp = un + R(2) * a / G1;
-        R Rm = Vninf - R(2) * ainf / G1;
+        R Rp = un + twice(a) / G1;
+        R Rm = Vninf - twice(ainf) / G1;
         R Sb = p / pow(rho, G);
-        R Vnrm = R(0.5) * (Rp + Rm);
+        R Vnrm = half(Rp + Rm);
         qb[1] = Vnrm * nx + tn * tx; qb[2] = Vnrm * ny + tn * ty;
-        R ab = R(0.25) * (Rp - Rm) * G1;
+        R ab = quarter(Rp - Rm) * G1;
         qb[0] = pow(ab * ab / G / Sb, R(1) / G1);
         qb[3] = qb[0] * ab * ab / G;
     } else if (R(-1) < mach && mach < R(0)) {
         R Vninf = uinf * nx + vinf * ny;
         R Vtinf = uinf * tx + vinf * ty;
-        R Rp = un + R(2) * a / G1;
-        R Rm = Vninf - R(2) * ainf / G1;
+        R Rp = un + twice(a) / G1;
+        R Rm = Vninf - twice(ainf) / G1;
         R Sb = pinf / pow(rinf, G);
-        R Vnrm = R(0.5) * (Rp + Rm);
+        R Vnrm = half(Rp + Rm);
         qb[1] = Vnrm * nx + Vtinf * tx; qb[2] = Vnrm * ny + Vtinf * ty;
-        R ab = R(0.25) * (Rp - Rm) * G1;
+        R ab = quarter(Rp - Rm) * G1;
         qb[0] = pow(ab * ab / G / Sb, R(1) / G1);
         qb[3] = qb[0] * ab * ab / G;
     }
@@ -302,7 +320,7 @@ __device__ __forceinline__ PrimT<S> con2prim_t(const Gas& g, S E, S r, S ru, S r
     o.v = rv / r;
     o.e = E / o.rho;
     S q = o.u * o.u + o.v * o.v;
-    o.p = (g.gamma - 1.0) * (E - 0.5 * o.rho * q);
+    o.p = (g.gamma - 1.0) * (E - half(o.rho) * q);
     o.t = o.p / (o.rho * g.znd);
     return o;
 }
@@ -316,6 +334,10 @@ struct Cvt {
 template <class T>
 struct Cvt<T, T> {
     __device__ __forceinline__ static T f(T x) { return x; }
+};
+template <>
+struct Cvt<F64, float> {
+    __device__ __forceinline__ static F64 f(float x) { return F64((double)x); }
 };
 
 // Convective flux of the selected scheme (fvresidual.F90 flux selection).

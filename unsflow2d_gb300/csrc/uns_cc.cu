@@ -316,6 +316,7 @@ __device__ __forceinline__ void d4get(const double4& q, double o[4]) { o[0] = q.
 __device__ __forceinline__ double4 d4(const double o[4]) { return make_double4(o[0], o[1], o[2], o[3]); }
 __device__ __forceinline__ void f4get(const double4& q, F64 o[4]) { o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w; }
 __device__ __forceinline__ void f4get(const double4& q, F64I o[4]) { o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w; }
+__device__ __forceinline__ double4 f4(const F64I o[4]) { return make_double4(o[0].v, o[1].v, o[2].v, o[3].v); }
 __device__ __forceinline__ double4 f4(const F64 o[4]) { return make_double4(o[0].v, o[1].v, o[2].v, o[3].v); }
 
 // Per-cell gather over the index-sorted face list: spectral radius + dt
@@ -337,119 +338,105 @@ __device__ __forceinline__ void warp_atomic_min_u64(const CCView& v, int inst, u
     if ((int)(threadIdx.x & 31) == __ffs(mask) - 1) atomicMin(&v.dtmin[inst], m);
 }
 
+// Arithmetic: F64I, sums on the FP64 unit and products, divisions and tests
+// on the integer pipe.  The unit bounded this kernel (520 instructions and 14
+// divisions per cell, 86 % busy).
 __global__ void __launch_bounds__(kBlock) k_cell_grad(CCView v, int flags, double cfl_in) {
+    // the limiter tolerances of the block's instance (blocks of cells are
+    // instance-pure), formed once per block
+    __shared__ double stol[4], stol2[4];
+    if ((flags & CG_LIM) && threadIdx.x < 4) {
+        const int b = block_inst(v), j = threadIdx.x;
+        const double t = 0.05 * (dec_ord(v.minmax[8 * b + j]) - dec_ord(v.minmax[8 * b + 4 + j]));
+        stol[j] = t;
+        stol2[j] = t * t;
+    }
+    __syncthreads();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= v.noc) return;
     const int inst = cell_inst(v, i);
     if (inst < 0 || stopped(v, inst)) return;
     const int k0 = v.cf_off[i], k1 = v.cf_off[i + 1];
-    const double cvi = v.cv[i];
-    const double rcv = (flags & (CG_DT | CG_GRAD)) ? 1.0 / cvi : 0.0;  // shared by dt/cv and the gradient
+    const F64I cvi = v.cv[i];
     if (flags & CG_DT) {
-        double la = 0.0;
+        F64I la = 0.0;
         for (int k = k0; k < k1; ++k) la = la + v.fla[v.cf[k] & FACE_MASK];
-        v.la[i] = la;
-        double cfl = cur_cfl(v, inst, cfl_in);
-        double dt = cfl * cvi / la;
-        v.dt[i] = dt;
-        v.dcv[i] = div_rn_recip(dt, cvi, rcv);
+        v.la[i] = la.v;
+        const F64I dt = F64I(cur_cfl(v, inst, cfl_in)) * cvi / la;
+        v.dt[i] = dt.v;
+        v.dcv[i] = (dt / cvi).v;
         if (flags & CG_DIAG) {
-            v.diag[i] = v.cv[i] / dt + 0.5 * 1.5 * la;
-            v.diaginv[i] = 1.0 / v.diag[i];
+            const F64I diag = cvi / dt + F64I(0.5 * 1.5) * la;
+            v.diag[i] = diag.v;
+            v.diaginv[i] = (F64I(1.0) / diag).v;
         }
-        warp_atomic_min_u64(v, inst, enc_ord(dt));
+        warp_atomic_min_u64(v, inst, enc_ord(dt.v));
     }
-    double gx[4], gy[4];
+    F64I gx[4], gy[4];
     if (flags & CG_GRAD) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) { gx[j] = 0.0; gy[j] = 0.0; }
+        F64I den = 1.0;
         if (v.grad_type == UNS_GRAD_GG) {
             for (int k = k0; k < k1; ++k) {
                 int e = v.cf[k], f = e & FACE_MASK;
                 double2 n = v.fn[f];
-                double area = v.farea[f];
-                double q[4];
-                d4get(v.fq[f], q);
-                if (f < v.nfi) {
-                    double dx = n.x * area, dy = n.y * area;
-                    if (e & SIDE_BIT) {
+                const F64I area = v.farea[f];
+                F64I q[4];
+                f4get(v.fq[f], q);
+                // + on the `in` side of an interior face, - on the other and on a boundary face
+                const bool minus = f >= v.nfi || (e & SIDE_BIT);
+                const F64I dx = F64I(minus ? -n.x : n.x) * area, dy = F64I(minus ? -n.y : n.y) * area;
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) { gx[j] = gx[j] - q[j] * dx; gy[j] = gy[j] - q[j] * dy; }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) { gx[j] = gx[j] + q[j] * dx; gy[j] = gy[j] + q[j] * dy; }
-                    }
-                } else {
-                    double dx = -n.x * area, dy = -n.y * area;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) { gx[j] = gx[j] + q[j] * dx; gy[j] = gy[j] + q[j] * dy; }
-                }
+                for (int j = 0; j < 4; ++j) { gx[j] = gx[j] + q[j] * dx; gy[j] = gy[j] + q[j] * dy; }
             }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {  // eight quotients by cv through its reciprocal (Markstein)
-                gx[j] = div_rn_recip(gx[j], cvi, rcv);
-                gy[j] = div_rn_recip(gy[j], cvi, rcv);
-            }
+            den = cvi;
         } else if (v.grad_type == UNS_GRAD_GGFC) {
             for (int k = k0; k < k1; ++k) {
                 int f = v.cf[k] & FACE_MASK;
-                double s = v.fasum[f];
-                double a[4], b[4];
-                d4get(v.fgx[f], a);
-                d4get(v.fgy[f], b);
+                const F64I s = v.fasum[f];
+                F64I a[4], b[4];
+                f4get(v.fgx[f], a);
+                f4get(v.fgy[f], b);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) { gx[j] = gx[j] + a[j] * s; gy[j] = gy[j] + b[j] * s; }
             }
-            const double var = v.cov[i], rv = 1.0 / var;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) { gx[j] = div_rn_recip(gx[j], var, rv); gy[j] = div_rn_recip(gy[j], var, rv); }
+            den = v.cov[i];
         } else {  // LSQR
-            double qi[4];
-            d4get(v.qp[i], qi);
             for (int k = k0; k < k1; ++k) {
                 int e = v.cf[k], f = e & FACE_MASK;
-                double4 w = v.lsw[f];
+                const double4 w = v.lsw[f];
                 int2 nb = v.fnb[f];
-                double qa[4], qb[4];
-                d4get(v.qp[nb.x], qa);
-                d4get(v.qp[nb.y], qb);
-                if (f < v.nfi && (e & SIDE_BIT)) {
+                F64I qa[4], qb[4];
+                f4get(v.qp[nb.x], qa);
+                f4get(v.qp[nb.y], qb);
+                const bool out = f < v.nfi && (e & SIDE_BIT);
+                const F64I wx = out ? -w.z : w.x, wy = out ? -w.w : w.y;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        double var = qb[j] - qa[j];
-                        gx[j] = gx[j] - var * w.z;
-                        gy[j] = gy[j] - var * w.w;
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        double var = qb[j] - qa[j];
-                        gx[j] = gx[j] + var * w.x;
-                        gy[j] = gy[j] + var * w.y;
-                    }
+                for (int j = 0; j < 4; ++j) {
+                    const F64I var = qb[j] - qa[j];
+                    gx[j] = gx[j] + var * wx;
+                    gy[j] = gy[j] + var * wy;
                 }
             }
-            (void)qi;
         }
-        v.gx[i] = d4(gx);
-        v.gy[i] = d4(gy);
+        if (v.grad_type != UNS_GRAD_LSQR) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { gx[j] = gx[j] / den; gy[j] = gy[j] / den; }
+        }
+        v.gx[i] = f4(gx);
+        v.gy[i] = f4(gy);
     } else {
-        d4get(v.gx[i], gx);
-        d4get(v.gy[i], gy);
+        f4get(v.gx[i], gx);
+        f4get(v.gy[i], gy);
     }
     if (flags & CG_LIM) {
-        double qmax[4], qmin[4], tol[4];
+        double umax[4], umin[4];
+        F64I qi[4], ph[4];
+        f4get(v.qp[i], qi);
+        f4get(v.phi[i], ph);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            qmax[j] = dec_ord(v.minmax[8 * inst + j]);
-            qmin[j] = dec_ord(v.minmax[8 * inst + 4 + j]);
-            tol[j] = 0.05 * (qmax[j] - qmin[j]);
-        }
-        double qi[4], umax[4], umin[4], ph[4];
-        d4get(v.qp[i], qi);
-        d4get(v.phi[i], ph);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) { umax[j] = qi[j]; umin[j] = qi[j]; }
+        for (int j = 0; j < 4; ++j) { umax[j] = qi[j].v; umin[j] = qi[j].v; }
         for (int k = k0; k < k1; ++k) {
             int e = v.cf[k], f = e & FACE_MASK;
             double u[4];
@@ -461,40 +448,50 @@ __global__ void __launch_bounds__(kBlock) k_cell_grad(CCView v, int flags, doubl
                 double4 a = v.pp[p.x], b = v.pp[p.y];
                 u[0] = 0.5 * (a.x + b.x); u[1] = 0.5 * (a.y + b.y); u[2] = 0.5 * (a.z + b.z); u[3] = 0.5 * (a.w + b.w);
             }
+            // fmax / fmin (19 cycles) are rmax / rmin here: they differ for a
+            // NaN in the cell itself, whose differences below are NaN either
+            // way, and in the sign of a zero, which the differences drop
 #pragma unroll
-            for (int j = 0; j < 4; ++j) { umax[j] = rmax(umax[j], u[j]); umin[j] = rmin(umin[j], u[j]); }
+            for (int j = 0; j < 4; ++j) { umax[j] = fmax(umax[j], u[j]); umin[j] = fmin(umin[j], u[j]); }
         }
         // phi = min(phi, phi0 of every face): the faces' ratios nr/dr are
         // compared exactly and only the smallest is divided (the minimum of
-        // correctly rounded quotients is the rounded minimum), so one IEEE
+        // correctly rounded quotients is the rounded minimum), so one
         // division per variable instead of one per face and variable.
-        double bn[4], bd[4];
+        F64I bn[4], bd[4];
         bool have[4] = {false, false, false, false};
-        double2 c = v.cen[i];
+        const double2 c = v.cen[i];
         for (int k = k0; k < k1; ++k) {
             int f = v.cf[k] & FACE_MASK;
             double2 fc = v.fcen[f];
-            double d0 = fc.x - c.x, d1 = fc.y - c.y;
+            const F64I d0 = F64I(fc.x) - c.x, d1 = F64I(fc.y) - c.y;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                double D_L = gx[j] * d0 + gy[j] * d1;
-                if (D_L > 0.0 || D_L < 0.0) {
-                    double nr, dr;
-                    vk_terms((D_L > 0.0 ? umax[j] : umin[j]) - qi[j], D_L, tol[j], nr, dr);
-                    if (!ratio_ok(nr, dr)) {
-                        ph[j] = rmin(ph[j], nr / dr);
+                const F64I D_L = gx[j] * d0 + gy[j] * d1;
+                const bool pos = dpos(D_L.v);
+                if (pos || dneg(D_L.v)) {
+                    // vk_terms with 2 a b and 2 b b scaled after the product
+                    // (the same bits unless the product is subnormal, which
+                    // terms that ratio_ok accepts do not show)
+                    const F64I a = F64I(pos ? umax[j] : umin[j]) - qi[j];
+                    const F64I aa = a * a, ab = a * D_L, t2 = stol2[j];
+                    const F64I nr = aa + twice(ab) + t2, dr = aa + twice(D_L * D_L) + ab + t2;
+                    if (!ratio_ok(nr.v, dr.v)) {
+                        double n, d;
+                        vk_terms(a.v, D_L.v, stol[j], n, d);
+                        ph[j] = rmin(ph[j], F64I(n / d));
                     } else if (!have[j] || ratio_less(nr, dr, bn[j], bd[j])) {
                         bn[j] = nr; bd[j] = dr; have[j] = true;
                     }
                 } else {
-                    ph[j] = rmin(ph[j], 1.0);
+                    ph[j] = rmin(ph[j], F64I(1.0));
                 }
             }
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
             if (have[j]) ph[j] = rmin(ph[j], bn[j] / bd[j]);
-        v.phi[i] = d4(ph);
+        v.phi[i] = f4(ph);
     }
 }
 

@@ -480,13 +480,21 @@ __device__ __forceinline__ bool ratio_less(double n1, double d1, double n2, doub
     return __fma_rn(n1, d2, -p1) < __fma_rn(n2, d1, -p2);
 }
 
+// The same on F64 or F64I (their products and comparison are the same bits).
+template <class S>
+__device__ __forceinline__ bool ratio_less(S n1, S d1, S n2, S d2) {
+    const S p1 = n1 * d2, p2 = n2 * d1;
+    if (__double_as_longlong(p1.v) != __double_as_longlong(p2.v)) return p1 < p2;
+    return __fma_rn(n1.v, d2.v, -p1.v) < __fma_rn(n2.v, d1.v, -p2.v);
+}
+
 // Whether the ratio test above is exact for these operands: d positive,
 // both with binary exponents within [-463, 457] (n may be zero), so that
 // every cross product and its error term stay normal.
 __device__ __forceinline__ bool ratio_ok(double n, double d) {
     const int en = dexp_field(n), ed = dexp_field(d);
     const bool nz = (__double_as_longlong(n) & 0x7fffffffffffffffLL) == 0;
-    return (nz || (en >= 560 && en <= 1480)) && ed >= 560 && ed <= 1480 && d > 0.0;
+    return (nz || (en >= 560 && en <= 1480)) && ed >= 560 && ed <= 1480 && __double_as_longlong(d) > 0;
 }
 
 // Order-preserving 64-bit encoding of a double for atomicMax/atomicMin.

@@ -73,6 +73,14 @@ __device__ __forceinline__ unsigned long long grp_max_u64(unsigned grp, unsigned
     return ((unsigned long long)mh << 32) | ml;
 }
 
+static __device__ __noinline__ double mean_rare(double a, double b) { return 0.5 * (a + b); }
+__device__ __forceinline__ void d4get(const double4& q, double o[4]) { o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w; }
+__device__ __forceinline__ double4 d4(const double o[4]) { return make_double4(o[0], o[1], o[2], o[3]); }
+__device__ __forceinline__ void f4get(const double4& q, F64 o[4]) { o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w; }
+__device__ __forceinline__ void f4get(const double4& q, F64I o[4]) { o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w; }
+__device__ __forceinline__ double4 f4(const F64I o[4]) { return make_double4(o[0].v, o[1].v, o[2].v, o[3].v); }
+__device__ __forceinline__ double4 f4(const F64 o[4]) { return make_double4(o[0].v, o[1].v, o[2].v, o[3].v); }
+
 // ---------------------------------------------------------------- kernels
 // con2prim (main.F90:62-67) + save_old (solution.F90:118-132) + the global
 // min/max of every cell's primitives incl. ghosts (limiter.F90:146-149) +
@@ -102,12 +110,12 @@ __global__ void __launch_bounds__(kBlock) k_begin(CCView v, int flags) {
             if (v.laminar || v.grad_type == UNS_GRAD_GGFC) v.qT[i] = (double)(p / (r * (float)gi.znd));
             if ((flags & BEGIN_POS) && (r <= 0.f || p <= 0.f)) set_err(v.err, UNS_ERR_NONPOSITIVE, i);
         } else if (flags & BEGIN_PRIM) {
-            Prim P = con2prim(gi, q.x, q.y, q.z, q.w);
-            v.qp[i] = make_double4(P.rho, P.u, P.v, P.p);
-            v.qT[i] = P.t;
-            pr[0] = P.rho; pr[1] = P.u; pr[2] = P.v; pr[3] = P.p;
+            const PrimT<F64I> P = con2prim_t<F64I>(gi, q.x, q.y, q.z, q.w);
+            v.qp[i] = make_double4(q.y, P.u.v, P.v.v, P.p.v);
+            v.qT[i] = P.t.v;
+            pr[0] = q.y; pr[1] = P.u.v; pr[2] = P.v.v; pr[3] = P.p.v;
             have = true;
-            if ((flags & BEGIN_POS) && (P.rho <= 0.0 || P.p <= 0.0)) set_err(v.err, UNS_ERR_NONPOSITIVE, i);
+            if ((flags & BEGIN_POS) && (P.rho <= F64I(0.0) || P.p <= F64I(0.0))) set_err(v.err, UNS_ERR_NONPOSITIVE, i);
         }
         if (flags & BEGIN_OLD) v.qold[i] = q;
     }
@@ -159,6 +167,8 @@ __global__ void __launch_bounds__(kBlock) k_begin(CCView v, int flags) {
 }
 
 // avg_c2v vertex part (average.F90:11-29): pseudo-Laplacian weighted mean.
+// FP64 form: 0.42 -> 0.18 ms at 4.2 M cells with the products and the five
+// divisions on the integer pipe (106 FP64 instructions per vertex -> 36).
 __global__ void __launch_bounds__(512) k_vertex_avg(CCView v) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= v.nop || stopped(v, vert_inst(v, i))) return;
@@ -197,25 +207,25 @@ __global__ void __launch_bounds__(512) k_vertex_avg(CCView v) {
         }
         return;
     }
-    double wt = 0.0, c0 = 0.0, c1 = 0.0, c2 = 0.0, c3 = 0.0, c4 = 0.0;
-#pragma unroll 4
+    F64I wt = 0.0, c0 = 0.0, c1 = 0.0, c2 = 0.0, c3 = 0.0, c4 = 0.0;
     for (int k = v.v2c_off[i]; k < v.v2c_off[i + 1]; ++k) {
         int c = __ldg(&v.v2c[k]);
-        double w = __ldg(&v.v2c_wt[k]);
+        const F64I w = __ldg(&v.v2c_wt[k]);
         wt = wt + w;
-        double4 q = v.qp[c];
-        c0 = c0 + q.x * w;
-        c1 = c1 + q.y * w;
-        c2 = c2 + q.z * w;
-        c3 = c3 + q.w * w;
-        c4 = c4 + v.qT[c] * w;
+        const double4 q = v.qp[c];
+        c0 = c0 + F64I(q.x) * w;
+        c1 = c1 + F64I(q.y) * w;
+        c2 = c2 + F64I(q.z) * w;
+        c3 = c3 + F64I(q.w) * w;
+        c4 = c4 + F64I(v.qT[c]) * w;
     }
-    v.pp[i] = make_double4(c0 / wt, c1 / wt, c2 / wt, c3 / wt);
-    v.ppT[i] = c4 / wt;
+    v.pp[i] = make_double4((c0 / wt).v, (c1 / wt).v, (c2 / wt).v, (c3 / wt).v);
+    v.ppT[i] = (c4 / wt).v;
 }
 
 // avg_c2v face part (average.F90:31-36) + spectral02 face radius
-// (timestep.F90:77-104).
+// (timestep.F90:77-104).  FP64 form: 0.62 -> 0.14 ms at 4.2 M cells (54 FP64
+// instructions per face -> 8; now half HBM-bound, 106 B per face).
 __global__ void __launch_bounds__(kBlock) k_face_prim_spec(CCView v) {
     int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= v.nof) return;
@@ -239,16 +249,20 @@ __global__ void __launch_bounds__(kBlock) k_face_prim_spec(CCView v) {
         return;
     }
     int2 p = v.fpt[f];
-    double4 a = v.pp[p.x], b = v.pp[p.y];
-    double4 q = make_double4(0.5 * (a.x + b.x), 0.5 * (a.y + b.y), 0.5 * (a.z + b.z), 0.5 * (a.w + b.w));
-    v.fq[f] = q;
-    v.fqT[f] = 0.5 * (v.ppT[p.x] + v.ppT[p.y]);
-    double2 n = v.fn[f];
-    double a0 = sqrt(g.gamma * q.w / q.x);
-    double un = q.y * n.x + q.z * n.y;
-    double ll = v.farea[f] * (fabs(un) + a0);
-    ll = ll + g.vll * v.fmu[f] / q.x;
-    v.fla[f] = ll;
+    F64I a[4], b[4], q[4];
+    f4get(v.pp[p.x], a);
+    f4get(v.pp[p.y], b);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) q[j] = half(a[j] + b[j]);
+    v.fq[f] = f4(q);
+    v.fqT[f] = half(F64I(v.ppT[p.x]) + F64I(v.ppT[p.y])).v;
+    const double2 n = v.fn[f];
+    const F64I a0 = sqrt(F64I(g.gamma) * q[3] / q[0]);
+    const F64I un = q[1] * n.x + q[2] * n.y;
+    F64I ll = F64I(v.farea[f]) * (fabs(un) + a0);
+    // the viscous term of an inviscid flow is 0 / q[0]: +0 unless q[0] is 0 or NaN
+    if (v.laminar || !dpos(fabs(q[0]).v)) ll = ll + F64I(g.vll) * F64I(v.fmu[f]) / q[0];
+    v.fla[f] = ll.v;
 }
 
 // Diamond-path face gradient (gradient.F90:183-261, gradtrixy :281-321).
@@ -312,13 +326,6 @@ __global__ void __launch_bounds__(kBlock) k_face_ggfc(CCView v) {
     v.fasum[f] = s;
 }
 
-__device__ __forceinline__ void d4get(const double4& q, double o[4]) { o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w; }
-__device__ __forceinline__ double4 d4(const double o[4]) { return make_double4(o[0], o[1], o[2], o[3]); }
-__device__ __forceinline__ void f4get(const double4& q, F64 o[4]) { o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w; }
-__device__ __forceinline__ void f4get(const double4& q, F64I o[4]) { o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w; }
-__device__ __forceinline__ double4 f4(const F64I o[4]) { return make_double4(o[0].v, o[1].v, o[2].v, o[3].v); }
-__device__ __forceinline__ double4 f4(const F64 o[4]) { return make_double4(o[0].v, o[1].v, o[2].v, o[3].v); }
-
 // Per-cell gather over the index-sorted face list: spectral radius + dt
 // (timestep.F90:40-49, 101-103), the cell gradient (Gradient_GG
 // gradient.F90:95-156, Gradient_GG_FC :159-323, Gradient_LSQR :2-93) and
@@ -338,10 +345,16 @@ __device__ __forceinline__ void warp_atomic_min_u64(const CCView& v, int inst, u
     if ((int)(threadIdx.x & 31) == __ffs(mask) - 1) atomicMin(&v.dtmin[inst], m);
 }
 
-// Arithmetic: F64I, sums on the FP64 unit and products, divisions and tests
-// on the integer pipe.  The unit bounded this kernel (520 instructions and 14
-// divisions per cell, 86 % busy).
-__global__ void __launch_bounds__(kBlock) k_cell_grad(CCView v, int flags, double cfl_in) {
+// The FP64 unit bounded this kernel (520 instructions and 14 divisions per
+// cell, 86 % busy; 4.25 ms at 4.2 M cells).  S = F64I leaves the sums alone
+// there and takes 1.70 ms; its products' latency (138 cycles against 64) is in
+// the way where an SM sub-partition has a warp or two, so small meshes take
+// S = F64 (16 384 cells: 25-29 us against 33).  80 registers for three blocks
+// per SM rather than two: 1.96 -> 1.93 ms; what is rare (a tie of two ratios, a
+// boundary face's average, the native operations) is called, because predicated
+// off it would hold the FP64 unit all the same: 1.93 -> 1.70 ms.
+template <class S>
+__global__ void __launch_bounds__(kBlock, std::is_same<S, F64I>::value ? 3 : 1) k_cell_grad(CCView v, int flags, double cfl_in) {
     // the limiter tolerances of the block's instance (blocks of cells are
     // instance-pure), formed once per block
     __shared__ double stol[4], stol2[4];
@@ -357,36 +370,36 @@ __global__ void __launch_bounds__(kBlock) k_cell_grad(CCView v, int flags, doubl
     const int inst = cell_inst(v, i);
     if (inst < 0 || stopped(v, inst)) return;
     const int k0 = v.cf_off[i], k1 = v.cf_off[i + 1];
-    const F64I cvi = v.cv[i];
+    const S cvi = v.cv[i];
     if (flags & CG_DT) {
-        F64I la = 0.0;
+        S la = 0.0;
         for (int k = k0; k < k1; ++k) la = la + v.fla[v.cf[k] & FACE_MASK];
         v.la[i] = la.v;
-        const F64I dt = F64I(cur_cfl(v, inst, cfl_in)) * cvi / la;
+        const S dt = S(cur_cfl(v, inst, cfl_in)) * cvi / la;
         v.dt[i] = dt.v;
         v.dcv[i] = (dt / cvi).v;
         if (flags & CG_DIAG) {
-            const F64I diag = cvi / dt + F64I(0.5 * 1.5) * la;
+            const S diag = cvi / dt + S(0.5 * 1.5) * la;
             v.diag[i] = diag.v;
-            v.diaginv[i] = (F64I(1.0) / diag).v;
+            v.diaginv[i] = (S(1.0) / diag).v;
         }
         warp_atomic_min_u64(v, inst, enc_ord(dt.v));
     }
-    F64I gx[4], gy[4];
+    S gx[4], gy[4];
     if (flags & CG_GRAD) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) { gx[j] = 0.0; gy[j] = 0.0; }
-        F64I den = 1.0;
+        S den = 1.0;
         if (v.grad_type == UNS_GRAD_GG) {
             for (int k = k0; k < k1; ++k) {
                 int e = v.cf[k], f = e & FACE_MASK;
                 double2 n = v.fn[f];
-                const F64I area = v.farea[f];
-                F64I q[4];
+                const S area = v.farea[f];
+                S q[4];
                 f4get(v.fq[f], q);
                 // + on the `in` side of an interior face, - on the other and on a boundary face
                 const bool minus = f >= v.nfi || (e & SIDE_BIT);
-                const F64I dx = F64I(minus ? -n.x : n.x) * area, dy = F64I(minus ? -n.y : n.y) * area;
+                const S dx = S(minus ? -n.x : n.x) * area, dy = S(minus ? -n.y : n.y) * area;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) { gx[j] = gx[j] + q[j] * dx; gy[j] = gy[j] + q[j] * dy; }
             }
@@ -394,8 +407,8 @@ __global__ void __launch_bounds__(kBlock) k_cell_grad(CCView v, int flags, doubl
         } else if (v.grad_type == UNS_GRAD_GGFC) {
             for (int k = k0; k < k1; ++k) {
                 int f = v.cf[k] & FACE_MASK;
-                const F64I s = v.fasum[f];
-                F64I a[4], b[4];
+                const S s = v.fasum[f];
+                S a[4], b[4];
                 f4get(v.fgx[f], a);
                 f4get(v.fgy[f], b);
 #pragma unroll
@@ -407,14 +420,14 @@ __global__ void __launch_bounds__(kBlock) k_cell_grad(CCView v, int flags, doubl
                 int e = v.cf[k], f = e & FACE_MASK;
                 const double4 w = v.lsw[f];
                 int2 nb = v.fnb[f];
-                F64I qa[4], qb[4];
+                S qa[4], qb[4];
                 f4get(v.qp[nb.x], qa);
                 f4get(v.qp[nb.y], qb);
                 const bool out = f < v.nfi && (e & SIDE_BIT);
-                const F64I wx = out ? -w.z : w.x, wy = out ? -w.w : w.y;
+                const S wx = out ? -w.z : w.x, wy = out ? -w.w : w.y;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const F64I var = qb[j] - qa[j];
+                    const S var = qb[j] - qa[j];
                     gx[j] = gx[j] + var * wx;
                     gy[j] = gy[j] + var * wy;
                 }
@@ -431,12 +444,12 @@ __global__ void __launch_bounds__(kBlock) k_cell_grad(CCView v, int flags, doubl
         f4get(v.gy[i], gy);
     }
     if (flags & CG_LIM) {
-        double umax[4], umin[4];
-        F64I qi[4], ph[4];
+        long long umax[4], umin[4];  // order keys
+        S qi[4], ph[4];
         f4get(v.qp[i], qi);
         f4get(v.phi[i], ph);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) { umax[j] = qi[j].v; umin[j] = qi[j].v; }
+        for (int j = 0; j < 4; ++j) { umax[j] = order_key(qi[j].v); umin[j] = umax[j]; }
         for (int k = k0; k < k1; ++k) {
             int e = v.cf[k], f = e & FACE_MASK;
             double u[4];
@@ -446,45 +459,42 @@ __global__ void __launch_bounds__(kBlock) k_cell_grad(CCView v, int flags, doubl
             } else {
                 int2 p = v.fpt[f];
                 double4 a = v.pp[p.x], b = v.pp[p.y];
-                u[0] = 0.5 * (a.x + b.x); u[1] = 0.5 * (a.y + b.y); u[2] = 0.5 * (a.z + b.z); u[3] = 0.5 * (a.w + b.w);
+                u[0] = mean_rare(a.x, b.x); u[1] = mean_rare(a.y, b.y); u[2] = mean_rare(a.z, b.z); u[3] = mean_rare(a.w, b.w);
             }
-            // fmax / fmin (19 cycles) are rmax / rmin here: they differ for a
-            // NaN in the cell itself, whose differences below are NaN either
-            // way, and in the sign of a zero, which the differences drop
+            // (of two zeros the keys prefer the positive, rmax / rmin the first:
+            // the differences from the cell's value drop the sign)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) { umax[j] = fmax(umax[j], u[j]); umin[j] = fmin(umin[j], u[j]); }
+            for (int j = 0; j < 4; ++j) extend(u[j], umin[j], umax[j]);
         }
         // phi = min(phi, phi0 of every face): the faces' ratios nr/dr are
         // compared exactly and only the smallest is divided (the minimum of
         // correctly rounded quotients is the rounded minimum), so one
         // division per variable instead of one per face and variable.
-        F64I bn[4], bd[4];
+        S bn[4], bd[4];
         bool have[4] = {false, false, false, false};
         const double2 c = v.cen[i];
         for (int k = k0; k < k1; ++k) {
             int f = v.cf[k] & FACE_MASK;
             double2 fc = v.fcen[f];
-            const F64I d0 = F64I(fc.x) - c.x, d1 = F64I(fc.y) - c.y;
+            const S d0 = S(fc.x) - c.x, d1 = S(fc.y) - c.y;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const F64I D_L = gx[j] * d0 + gy[j] * d1;
+                const S D_L = gx[j] * d0 + gy[j] * d1;
                 const bool pos = dpos(D_L.v);
                 if (pos || dneg(D_L.v)) {
                     // vk_terms with 2 a b and 2 b b scaled after the product
                     // (the same bits unless the product is subnormal, which
                     // terms that ratio_ok accepts do not show)
-                    const F64I a = F64I(pos ? umax[j] : umin[j]) - qi[j];
-                    const F64I aa = a * a, ab = a * D_L, t2 = stol2[j];
-                    const F64I nr = aa + twice(ab) + t2, dr = aa + twice(D_L * D_L) + ab + t2;
+                    const S a = S(from_key(pos ? umax[j] : umin[j])) - qi[j];
+                    const S aa = a * a, ab = a * D_L, t2 = stol2[j];
+                    const S nr = aa + twice(ab) + t2, dr = aa + twice(D_L * D_L) + ab + t2;
                     if (!ratio_ok(nr.v, dr.v)) {
-                        double n, d;
-                        vk_terms(a.v, D_L.v, stol[j], n, d);
-                        ph[j] = rmin(ph[j], F64I(n / d));
+                        ph[j] = rmin(ph[j], S(vk_limit_rare(a.v, D_L.v, stol[j])));
                     } else if (!have[j] || ratio_less(nr, dr, bn[j], bd[j])) {
                         bn[j] = nr; bd[j] = dr; have[j] = true;
                     }
                 } else {
-                    ph[j] = rmin(ph[j], F64I(1.0));
+                    ph[j] = rmin(ph[j], S(1.0));
                 }
             }
         }
@@ -774,17 +784,19 @@ __device__ __forceinline__ double4 bnd_face_flux(const CCView& v, const Gas& g, 
     return Fd;
 }
 
-// FP64 form, 4.2 M cells: 3.85 -> 1.79 ms.  It was bound by the FP64 unit
+// FP64 form, 4.2 M cells: 3.85 -> 1.67 ms.  It was bound by the FP64 unit
 // (228 operations and 14 divisions and square roots per face); now its sums
-// alone are there (6.0 k cycles per warp) and its products, divisions, square
-// roots and halvings on the integer pipe (about 8 k), and what remains above
-// the longer of the two is instruction fetch (4 900 instructions per face,
-// each run once per warp; ncu: 3.2 of 12 stall cycles per issue).
+// alone are there (100 instructions, 6.4 k cycles per warp) and its products,
+// divisions, square roots and halvings on the integer pipe (3 400 instructions,
+// 6.8 k cycles).  What remains above the longer of the two is instruction fetch
+// (6 200 instructions per face, each run once per warp; ncu: 3.2 of 12 stall
+// cycles per issue) and latency at six warps per sub-partition (80 registers;
+// at 124 and four warps 1.79 ms).
 // One thread per face; the first blocks take the boundary faces, whose FP64
 // ghost arithmetic is the longest per thread, so that they run beside the
 // interior faces instead of after them.
 template <class R>
-__global__ void __launch_bounds__(512, std::is_same<R, float>::value ? 2 : 1) k_face_conv(CCView v) {
+__global__ void __launch_bounds__(std::is_same<R, float>::value ? 512 : kBlock, std::is_same<R, float>::value ? 2 : 3) k_face_conv(CCView v) {
     const int bs = blockDim.x;
     const int nbb = (v.nbf + bs - 1) / bs;
     const bool bnd = (int)blockIdx.x < nbb;
@@ -901,8 +913,46 @@ __global__ void __launch_bounds__(kBlock) k_face_visc(CCView v) {
 
 // Residual gather in the reference's accumulation order, optionally fused
 // with one RK3 stage (main.F90:92-101) and the block partials of the norm.
+// FP64 form, 4.2 M cells: 0.48 -> 0.20 ms (60 FP64 instructions per cell -> 25:
+// products on the integer pipe, the sum's first term and stage 1's weights 0
+// and 1 dropped); k_cell_rk23 0.45 -> 0.25 ms and k_begin 0.32 -> 0.13 ms alike.
 __device__ __forceinline__ void add4(double r[4], const double4& a) { r[0] = r[0] + a.x; r[1] = r[1] + a.y; r[2] = r[2] + a.z; r[3] = r[3] + a.w; }
 __device__ __forceinline__ void sub4(double r[4], const double4& a) { r[0] = r[0] - a.x; r[1] = r[1] - a.y; r[2] = r[2] - a.z; r[3] = r[3] - a.w; }
+
+// The same on F64 or F64I, the sign by a flip of the operand's sign bit.
+template <class S>
+__device__ __forceinline__ void signed_add4(S r[4], const double4& a, bool minus) {
+    r[0] = r[0] + S(minus ? -a.x : a.x);
+    r[1] = r[1] + S(minus ? -a.y : a.y);
+    r[2] = r[2] + S(minus ? -a.z : a.z);
+    r[3] = r[3] + S(minus ? -a.w : a.w);
+}
+// The face fluxes of a cell in the reference's order, boundary faces first;
+// the sum's first term (0.0 + F) costs no FP64 instruction.
+template <class S>
+__device__ __forceinline__ void gather_res(const CCView& v, int k0, int k1, S r[4]) {
+    bool first = true;
+    auto take = [&](const double4& F, bool minus) {
+        if (first) {
+            r[0] = zero_plus(minus ? -F.x : F.x);
+            r[1] = zero_plus(minus ? -F.y : F.y);
+            r[2] = zero_plus(minus ? -F.z : F.z);
+            r[3] = zero_plus(minus ? -F.w : F.w);
+            first = false;
+        } else {
+            signed_add4(r, F, minus);
+        }
+    };
+    r[0] = r[1] = r[2] = r[3] = 0.0;
+    for (int k = k0; k < k1; ++k) {
+        int f = v.cf[k] & FACE_MASK;
+        if (f >= v.nfi) take(v.fF[f], false);
+    }
+    for (int k = k0; k < k1; ++k) {
+        int e = v.cf[k], f = e & FACE_MASK;
+        if (f < v.nfi) take(v.fF[f], (e & SIDE_BIT) != 0);
+    }
+}
 
 __global__ void __launch_bounds__(kBlock) k_cell_res(CCView v, int irk, int partial) {
     if (stopped(v, block_inst(v))) return;  // blocks of cells are instance-pure
@@ -910,38 +960,30 @@ __global__ void __launch_bounds__(kBlock) k_cell_res(CCView v, int irk, int part
     double rr = 0.0;
     if (i < v.noc && cell_inst(v, i) >= 0) {
         const int k0 = v.cf_off[i], k1 = v.cf_off[i + 1];
-        double r[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int k = k0; k < k1; ++k) {  // boundary faces first
-            int f = v.cf[k] & FACE_MASK;
-            if (f >= v.nfi) add4(r, v.fF[f]);
-        }
-        for (int k = k0; k < k1; ++k) {  // then interior faces
-            int e = v.cf[k], f = e & FACE_MASK;
-            if (f < v.nfi) { if (e & SIDE_BIT) sub4(r, v.fF[f]); else add4(r, v.fF[f]); }
-        }
+        F64I r[4];
+        gather_res(v, k0, k1, r);
         if (v.laminar) {
             for (int k = k0; k < k1; ++k) {
                 int e = v.cf[k], f = e & FACE_MASK;
-                if (f < v.nfi && (e & SIDE_BIT)) add4(r, v.fV[f]); else sub4(r, v.fV[f]);
+                signed_add4(r, v.fV[f], !(f < v.nfi && (e & SIDE_BIT)));
             }
         }
-        v.res[i] = d4(r);
+        v.res[i] = f4(r);
         if (irk > 0) {
-            double a = rk3_a(irk), b = rk3_b(irk);
-            double dtbyarea = v.dcv[i];  // dt / cv, formed once per time step
-            double o[4], c[4], q[4];
-            d4get(v.qc[i], c);
-            if (v.mixed && irk == 1) {  // a = 0, b = 1
+            const F64I dtbyarea = v.dcv[i];  // dt / cv, formed once per time step
+            F64I o[4], c[4], q[4];
+            f4get(v.qc[i], c);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) q[j] = c[j] - dtbyarea * r[j];
-            } else {
-                d4get(v.qold[i], o);
+            for (int j = 0; j < 4; ++j) q[j] = c[j] - dtbyarea * r[j];
+            if (irk > 1) {  // stage 1: a = 0, b = 1
+                const F64I a = rk3_a(irk), b = rk3_b(irk);
+                f4get(v.qold[i], o);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) q[j] = a * o[j] + b * (c[j] - dtbyarea * r[j]);
+                for (int j = 0; j < 4; ++j) q[j] = a * o[j] + b * q[j];
             }
-            v.qc[i] = d4(q);
+            v.qc[i] = f4(q);
         }
-        if (partial) rr = r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3];
+        if (partial) rr = (r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3]).v;
     }
     if (partial) {
         __shared__ double s[kBlock / 32];
@@ -1057,8 +1099,12 @@ __device__ __forceinline__ void rk_update(int irk, double D, const double o[4], 
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         if (kMixed) q[j] = __fma_rn(a, o[j], b * __fma_rn(-D, r[j], q[j]));
-        else q[j] = a * o[j] + b * (q[j] - D * r[j]);
+        else if (irk == 2) q[j] = (F64I(a) * F64I(o[j]) + quarter(F64I(q[j]) - F64I(D) * F64I(r[j]))).v;  // b = 1/4
+        else q[j] = (F64I(a) * F64I(o[j]) + F64I(b) * (F64I(q[j]) - F64I(D) * F64I(r[j]))).v;
     }
+}
+__device__ __forceinline__ double norm2(const double r[4]) {
+    return (F64I(r[0]) * F64I(r[0]) + F64I(r[1]) * F64I(r[1]) + F64I(r[2]) * F64I(r[2]) + F64I(r[3]) * F64I(r[3])).v;
 }
 
 // The residual of wall cell i at stage state q: its wall faces' fluxes
@@ -1080,15 +1126,16 @@ __device__ __forceinline__ void wall_cell_res(const CCView& v, const Gas& g, int
             else { r[0] = __fma_rn(s, F.x, r[0]); r[1] = __fma_rn(s, F.y, r[1]); r[2] = __fma_rn(s, F.z, r[2]); r[3] = __fma_rn(s, F.w, r[3]); }
         }
     } else {  // k_cell_res's order: boundary faces first
-        r[0] = r[1] = r[2] = r[3] = 0.0;
+        F64 t[4] = {0.0, 0.0, 0.0, 0.0};
         for (int k = k0; k < k1; ++k) {
             const int f = v.cf[k] & FACE_MASK;
-            if (f >= v.nfi) add4(r, flux(f));
+            if (f >= v.nfi) signed_add4(t, flux(f), false);
         }
         for (int k = k0; k < k1; ++k) {
             const int e = v.cf[k], f = e & FACE_MASK;
-            if (f < v.nfi) { if (e & SIDE_BIT) sub4(r, v.fF[f]); else add4(r, v.fF[f]); }
+            if (f < v.nfi) signed_add4(t, v.fF[f], (e & SIDE_BIT) != 0);
         }
+        r[0] = t[0].v; r[1] = t[1].v; r[2] = t[2].v; r[3] = t[3].v;
     }
 }
 
@@ -1100,6 +1147,7 @@ __device__ __forceinline__ void wall_cell_res(const CCView& v, const Gas& g, int
 template <class R, bool kWall, bool kFrom1 = false>
 __device__ __forceinline__ double rk23_cell(const CCView& v, int i, int inst) {
     constexpr bool kMixed = std::is_same<R, float>::value;
+    constexpr int kRkUnroll = kWall ? 1 : 2;  // one copy of a wall cell's long body
     double r[4], q[4], o[4];
     d4get(v.qc[i], q);
     d4get(v.qold[i], o);
@@ -1112,6 +1160,7 @@ __device__ __forceinline__ double rk23_cell(const CCView& v, int i, int inst) {
     } else {
         d4get(v.res[i], r);
     }
+#pragma unroll kRkUnroll
     for (int irk = 2; irk <= 3; ++irk) {
         if (kWall) wall_cell_res<R>(v, gas_of(v, inst), i, q, r);
         rk_update<kMixed>(irk, D, o, r, q);
@@ -1119,7 +1168,7 @@ __device__ __forceinline__ double rk23_cell(const CCView& v, int i, int inst) {
     if (kWall) v.res[i] = d4(r);
     v.qc[i] = d4(q);
     if (kMixed) return __fma_rn(r[3], r[3], __fma_rn(r[2], r[2], __fma_rn(r[1], r[1], r[0] * r[0])));
-    return r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3];
+    return norm2(r);
 }
 
 // The wall cells (v.wcell), one per thread in one-warp blocks so that their
@@ -1165,7 +1214,7 @@ __global__ void __launch_bounds__(kBlock) k_cell_rk23(CCView v) {
             double r[4];
             d4get(v.res[i], r);
             if (kMixed) rr = __fma_rn(r[3], r[3], __fma_rn(r[2], r[2], __fma_rn(r[1], r[1], r[0] * r[0])));
-            else rr = r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3];
+            else rr = norm2(r);
         } else {
             rr = rk23_cell<R, false>(v, i, inst);
         }
@@ -1855,13 +1904,18 @@ inline int spread_bs(const uns_cc_handle* h, int n) {
 }
 
 // Block size of k_face_conv: blk_face in the mixed form and where a caller or
-// the autotuner has set one; in the FP64 form else spread_bs, because that
-// form's code is longer than the instruction cache and the warps of a large
-// block run through it together (4.2 M cells: 1.79 ms at 256 threads, 2.14 at
-// 64; 16 384 cells, where spread_bs gives 64: 33 us, 40 at 256).
+// the autotuner has set one.  The FP64 form's code is longer than the
+// instruction cache, and the warps of a large block run through it together:
+// 256 threads on large meshes (4.2 M cells: 1.67 ms, 1.95 at 64 and 128; 262 k
+// cells: 146 us, 156 at 64), 64 where that leaves fewer than four blocks per SM
+// and the last of them idle (102 k cells: 74 us, 76 at 256; 16 k: 33, 39).
 template <class R>
 inline int face_bs(const uns_cc_handle* h, const CCView& v) {
-    return std::is_same<R, float>::value || h->blk_face_set ? v.blk_face : spread_bs(h, v.nof);
+    if (std::is_same<R, float>::value) return v.blk_face;
+    if (h->blk_face_set) return std::min(v.blk_face, kBlock);
+    int bs = kBlock;
+    while (bs > 64 && nblocks(v.nof, bs) < 4 * h->nsm) bs >>= 1;
+    return bs;
 }
 
 // A launch over n items with block size bs.
@@ -1874,10 +1928,15 @@ inline int face_bs(const uns_cc_handle* h, const CCView& v) {
 
 #define LAUNCH_SPREAD(kern, n, ...) LAUNCH_BS(kern, (n), spread_bs(h, (n)), __VA_ARGS__)
 
+#define LAUNCH_FP64_GRAD(v, flags, cfl)                                                          \
+    do {                                                                                       \
+        if (spread_bs(h, (v).noc) < kBlock) LAUNCH_SPREAD(k_cell_grad<F64>, (v).noc, (v), (int)(flags), (cfl)); \
+        else LAUNCH_SPREAD(k_cell_grad<F64I>, (v).noc, (v), (int)(flags), (cfl));              \
+    } while (0)
 #define LAUNCH_CELL_GRAD(v, flags, cfl)                                                 \
     do {                                                                               \
         if ((v).mixed) LAUNCH(k_cell_grad_mixed, (v).noc, (v), (int)(flags), (cfl));   \
-        else LAUNCH_SPREAD(k_cell_grad, (v).noc, (v), (int)(flags), (cfl));            \
+        else LAUNCH_FP64_GRAD(v, flags, cfl);                                          \
     } while (0)
 
 int enqueue_gradient(uns_cc_handle* h, CCView& v, int extra_flags, double cfl, bool do_reduce) {
@@ -2103,7 +2162,7 @@ int cc_record_iteration(uns_cc_handle* h, double cfl, CCRecHook hook, void* ctx)
     LAUNCH_BS(k_vertex_avg, v.nop, v.blk_vert, v);
     LAUNCH_SPREAD(k_face_prim_spec, v.nof, v);
     if (v.grad_type == UNS_GRAD_GGFC) LAUNCH(k_face_ggfc, v.nof, v);
-    LAUNCH_SPREAD(k_cell_grad, v.noc, v, (int)(CG_DT | CG_GRAD), cfl);
+    LAUNCH_FP64_GRAD(v, CG_DT | CG_GRAD, cfl);
     if ((rc = hook(h, REC_AFTER_START, 0, ctx))) return rc;
     for (int irk = 1; irk <= 3; ++irk) {
         if ((rc = hook(h, REC_BEFORE_FACE_CONV, irk, ctx))) return rc;
@@ -2115,7 +2174,7 @@ int cc_record_iteration(uns_cc_handle* h, double cfl, CCRecHook hook, void* ctx)
                 CCView w = v;
                 w.grad_type = UNS_GRAD_GGFC;
                 LAUNCH(k_face_ggfc, w.nof, w);
-                LAUNCH_SPREAD(k_cell_grad, w.noc, w, (int)CG_GRAD, cfl);
+                LAUNCH_FP64_GRAD(w, CG_GRAD, cfl);
             }
             LAUNCH(k_face_visc, v.nof, v);
             if ((rc = hook(h, REC_AFTER_FACE_VISC, irk, ctx))) return rc;
@@ -3033,7 +3092,7 @@ int uns_cc_autotune(uns_cc_handle* h, int reps, int* blocks) {
     };
     int bf = 0, bv = 0, bg = 0;
     if (rc == UNS_OK && v.nof > 0)
-        bf = pick({64, 128, 256, 512}, [&](int bs) {
+        bf = pick({64, 128, 256, v.mixed ? 512 : 256}, [&](int bs) {
             const int nb = std::max(1, (v.nbf + bs - 1) / bs + (v.nfi + bs - 1) / bs);
             if (v.mixed) k_face_conv<float><<<nb, bs, 0, h->stream>>>(t);
             else k_face_conv<double><<<nb, bs, 0, h->stream>>>(t);

@@ -175,6 +175,23 @@ __device__ __forceinline__ bool dle(double a, double b) {
     const unsigned long long ax = (unsigned long long)x << 1, ay = (unsigned long long)y << 1;
     return (kx <= ky || (ax | ay) == 0) && ax <= 0xffe0000000000000ULL && ay <= 0xffe0000000000000ULL;
 }
+// Running extremes as order-preserving signed keys (11 integer operations for
+// both, where a maximum and a minimum instruction hold the FP64 unit 76 cycles
+// each): a NaN changes neither.
+__device__ __forceinline__ long long order_key(double a) {
+    const long long x = __double_as_longlong(a);
+    return x ^ (long long)((unsigned long long)(x >> 63) >> 1);
+}
+__device__ __forceinline__ double from_key(long long k) {
+    return __longlong_as_double(k ^ (long long)((unsigned long long)(k >> 63) >> 1));
+}
+__device__ __forceinline__ void extend(double a, long long& lo, long long& hi) {
+    const long long k = order_key(a);
+    if (((unsigned long long)__double_as_longlong(a) << 1) > 0xffe0000000000000ULL) return;
+    hi = k > hi ? k : hi;
+    lo = k < lo ? k : lo;
+}
+
 // 0 < a and a < 0 (false for NaN).
 __device__ __forceinline__ bool dpos(double a) {
     return (unsigned long long)__double_as_longlong(a) - 1ULL < 0x7ff0000000000000ULL;

@@ -480,12 +480,17 @@ __device__ __forceinline__ bool ratio_less(double n1, double d1, double n2, doub
     return __fma_rn(n1, d2, -p1) < __fma_rn(n2, d1, -p2);
 }
 
-// The same on F64 or F64I (their products and comparison are the same bits).
+// The same on F64 or F64I (their products and comparison are the same bits);
+// equal products, which are rare, in a call (see uns_fp64.cuh's rare paths).
+static __device__ __noinline__ bool ratio_less_tie(double n1, double d1, double n2, double d2, double p) {
+    return __fma_rn(n1, d2, -p) < __fma_rn(n2, d1, -p);
+}
+static __device__ __noinline__ double vk_limit_rare(double a, double b, double tol) { return vk_limit(a, b, tol); }
 template <class S>
 __device__ __forceinline__ bool ratio_less(S n1, S d1, S n2, S d2) {
     const S p1 = n1 * d2, p2 = n2 * d1;
     if (__double_as_longlong(p1.v) != __double_as_longlong(p2.v)) return p1 < p2;
-    return __fma_rn(n1.v, d2.v, -p1.v) < __fma_rn(n2.v, d1.v, -p2.v);
+    return ratio_less_tie(n1.v, d1.v, n2.v, d2.v, p1.v);
 }
 
 // Whether the ratio test above is exact for these operands: d positive,

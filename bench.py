@@ -92,7 +92,7 @@ WORKLOADS = {
 # face_conv, cell_res (stage 1), cell_rk23_wall + cell_rk23 (stages 2-3), res_final.
 # Mixed GG form: reset_minmax, begin, vertex_avg, cell_grad_side, face_conv,
 # cell_rk23_wall (wall cells, stages 1-3), cell_res_mixed, res_final.
-LAUNCHES = {("nc", "lusgs"): 9, ("nc", "rk3"): 11, ("cc", "rk3"): 10, ("cc", "lusgs"): 12, ("cc", "rk3_mixed_gg"): 8}
+LAUNCHES = {("nc", "lusgs"): 9, ("nc", "rk3"): 5, ("cc", "rk3"): 10, ("cc", "lusgs"): 12, ("cc", "rk3_mixed_gg"): 8}
 
 
 def cc_launches(p) -> int:
@@ -290,9 +290,9 @@ def launches_per_iter(kind: str, rk3: bool, laminar: bool, irs: bool = False, si
     (stage 1) and runs stages 2 and 3 as one pass over the cells (cell_rk23),
     recomputing only the wall faces' fluxes; the mixed Green-Gauss step
     (sides) has no face pass and runs its wall cells as the cell_rk23 phase."""
+    if kind == "nc":  # RK3: the stages share one residual
+        return {"grad_lim": 1, "edge": 1, "node_res": 1}
     n = 3 if rk3 else 1
-    if kind == "nc":
-        return {"grad_lim": n, "edge": n, "node_res": n}
     if rk3 and not laminar and not irs:
         return {"face_conv": 1, "cell_res": 1, "cell_rk23": 1, "viscous": 0, "cirs": 0,
                 "face_prim_spec": 0 if sides else 1}

@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(kBlock, std::is_same<S, F64I>::value ? 3 : 1) 
                 f4get(v.fq[f], q);
                 // + on the `in` side of an interior face, - on the other and on a boundary face
                 const bool minus = f >= v.nfi || (e & SIDE_BIT);
-                const S dx = S(minus ? -n.x : n.x) * area, dy = S(minus ? -n.y : n.y) * area;
+                const S dx = S(flip64(n.x, minus)) * area, dy = S(flip64(n.y, minus)) * area;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) { gx[j] = gx[j] + q[j] * dx; gy[j] = gy[j] + q[j] * dy; }
             }
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kBlock, std::is_same<S, F64I>::value ? 3 : 1) 
                 f4get(v.qp[nb.x], qa);
                 f4get(v.qp[nb.y], qb);
                 const bool out = f < v.nfi && (e & SIDE_BIT);
-                const S wx = out ? -w.z : w.x, wy = out ? -w.w : w.y;
+                const S wx = flip64(out ? w.z : w.x, out), wy = flip64(out ? w.w : w.y, out);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const S var = qb[j] - qa[j];
@@ -922,10 +922,10 @@ __device__ __forceinline__ void sub4(double r[4], const double4& a) { r[0] = r[0
 // The same on F64 or F64I, the sign by a flip of the operand's sign bit.
 template <class S>
 __device__ __forceinline__ void signed_add4(S r[4], const double4& a, bool minus) {
-    r[0] = r[0] + S(minus ? -a.x : a.x);
-    r[1] = r[1] + S(minus ? -a.y : a.y);
-    r[2] = r[2] + S(minus ? -a.z : a.z);
-    r[3] = r[3] + S(minus ? -a.w : a.w);
+    r[0] = r[0] + S(flip64(a.x, minus));
+    r[1] = r[1] + S(flip64(a.y, minus));
+    r[2] = r[2] + S(flip64(a.z, minus));
+    r[3] = r[3] + S(flip64(a.w, minus));
 }
 // The face fluxes of a cell in the reference's order, boundary faces first;
 // the sum's first term (0.0 + F) costs no FP64 instruction.
@@ -934,10 +934,10 @@ __device__ __forceinline__ void gather_res(const CCView& v, int k0, int k1, S r[
     bool first = true;
     auto take = [&](const double4& F, bool minus) {
         if (first) {
-            r[0] = zero_plus(minus ? -F.x : F.x);
-            r[1] = zero_plus(minus ? -F.y : F.y);
-            r[2] = zero_plus(minus ? -F.z : F.z);
-            r[3] = zero_plus(minus ? -F.w : F.w);
+            r[0] = zero_plus(flip64(F.x, minus));
+            r[1] = zero_plus(flip64(F.y, minus));
+            r[2] = zero_plus(flip64(F.z, minus));
+            r[3] = zero_plus(flip64(F.w, minus));
             first = false;
         } else {
             signed_add4(r, F, minus);

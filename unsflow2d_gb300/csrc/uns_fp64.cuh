@@ -72,9 +72,15 @@ __device__ __forceinline__ unsigned long long u64(unsigned hi, unsigned lo) {
     return ((unsigned long long)hi << 32) | lo;
 }
 
+// -a on the sign bit, and a with its sign flipped where minus (a negation that
+// no FMA operand absorbs is an addition on the FP64 unit).
+__device__ __forceinline__ double neg64(double a) { return dmake(dhi(a) ^ 0x80000000u, dlo(a)); }
+__device__ __forceinline__ double flip64(double a, bool minus) { return dmake(dhi(a) ^ (minus ? 0x80000000u : 0u), dlo(a)); }
+
 // The native operations where they are rarely needed, as calls: branched
 // around (predicated off, they would hold the FP64 unit all the same), and
 // once in a kernel's code.
+static __device__ __noinline__ double add_rare(double a, double b) { return a + b; }
 static __device__ __noinline__ double mul_rare(double a, double b) { return a * b; }
 static __device__ __noinline__ double div_rare(double a, double b) { return a / b; }
 static __device__ __noinline__ double sqrt_rare(double a) { return sqrt(a); }
@@ -196,7 +202,7 @@ __device__ __forceinline__ void extend(double a, long long& lo, long long& hi) {
 __device__ __forceinline__ bool dpos(double a) {
     return (unsigned long long)__double_as_longlong(a) - 1ULL < 0x7ff0000000000000ULL;
 }
-__device__ __forceinline__ bool dneg(double a) { return dpos(-a); }
+__device__ __forceinline__ bool dneg(double a) { return dpos(neg64(a)); }
 
 // 0.5 * a: the exponent field less one; zero stays, the ends of the range take the multiplication.
 __device__ __forceinline__ double dhalf(double a) {
@@ -238,7 +244,7 @@ struct F64 {
 };
 __device__ __forceinline__ F64 operator+(F64 a, F64 b) { return add64(a.v, b.v); }
 __device__ __forceinline__ F64 operator-(F64 a, F64 b) { return sub64(a.v, b.v); }
-__device__ __forceinline__ F64 operator-(F64 a) { return -a.v; }
+__device__ __forceinline__ F64 operator-(F64 a) { return neg64(a.v); }
 __device__ __forceinline__ F64 operator*(F64 a, F64 b) { return mul64(a.v, b.v); }
 __device__ __forceinline__ F64 operator/(F64 a, F64 b) { return div_digits(a.v, b.v); }
 __device__ __forceinline__ bool operator<(F64 a, F64 b) { return dlt(a.v, b.v); }
@@ -267,7 +273,7 @@ struct F64I {
 };
 __device__ __forceinline__ F64I operator+(F64I a, F64I b) { return add64(a.v, b.v); }
 __device__ __forceinline__ F64I operator-(F64I a, F64I b) { return sub64(a.v, b.v); }
-__device__ __forceinline__ F64I operator-(F64I a) { return -a.v; }
+__device__ __forceinline__ F64I operator-(F64I a) { return neg64(a.v); }
 #ifdef UNS_FP64_CONTRACT
 __device__ __forceinline__ F64I operator*(F64I a, F64I b) { return a.v * b.v; }
 #else

@@ -100,6 +100,8 @@ struct NCView {
 
 __device__ __forceinline__ bool stopped(const NCView& v) { return v.done != nullptr && *((volatile int*)v.done) != 0; }
 __device__ __forceinline__ void g4(const double4& q, double o[4]) { o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w; }
+template <class S> __device__ __forceinline__ void g4s(const double4& q, S o[4]) { o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w; }
+template <class S> __device__ __forceinline__ double4 m4s(const S o[4]) { return make_double4(o[0].v, o[1].v, o[2].v, o[3].v); }
 __device__ __forceinline__ double4 m4(const double o[4]) { return make_double4(o[0], o[1], o[2], o[3]); }
 
 // save_old (common.f90:88-104): con2prim + qold.
@@ -108,10 +110,18 @@ __global__ void __launch_bounds__(kBlock) k_nc_save_old(NCView v) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= v.nop) return;
     double4 q = v.qc[i];
-    Prim P = con2prim(v.g, q.x, q.y, q.z, q.w);
-    v.qp[i] = make_double4(P.rho, P.u, P.v, P.p);
-    v.qpf[i] = make_float4((float)P.rho, (float)P.u, (float)P.v, (float)P.p);
+    const PrimT<F64I> P = con2prim_t<F64I>(v.g, q.x, q.y, q.z, q.w);
+    v.qp[i] = make_double4(q.y, P.u.v, P.v.v, P.p.v);
+    v.qpf[i] = make_float4((float)q.y, (float)P.u, (float)P.v, (float)P.p);
     v.qold[i] = q;
+}
+
+// The VKN ratio of the reference's expressions where its terms leave the
+// range of ratio_ok.
+static __device__ __noinline__ double nc_vkn_rare(double alfa, double D_L, double TOL) {
+    const double n = alfa * alfa + 2.0 * D_L * alfa + TOL;
+    const double d = alfa * alfa + 2.0 * D_L * D_L + D_L * alfa + TOL;
+    return n / d;
 }
 
 // k_nc_grad_lim in the mixed form: the LSQ gradient and the limiter in FP32
@@ -192,46 +202,54 @@ __global__ void __launch_bounds__(kBlock) k_nc_grad_lim_mixed(NCView v) {
     pk[2] = make_float4((float)ph[0], (float)ph[1], (float)ph[2], (float)ph[3]);
 }
 
-__global__ void __launch_bounds__(kBlock) k_nc_grad_lim(NCView v) {
+// The FP64 form.  S = F64I (sums on the FP64 unit, products, divisions and
+// tests on the integer pipe) where the launch fills the SMs, S = F64 on small
+// meshes, where the products' latency is in the way.
+template <class S>
+__global__ void __launch_bounds__(kBlock, std::is_same<S, F64I>::value ? 3 : 1) k_nc_grad_lim(NCView v) {
     if (stopped(v)) return;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= v.nop) return;
-    double qi[4], gx[4] = {0, 0, 0, 0}, gy[4] = {0, 0, 0, 0};
-    g4(v.qp[i], qi);
+    S qi[4], gx[4], gy[4];
+    g4s(v.qp[i], qi);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { gx[k] = 0.0; gy[k] = 0.0; }
     for (int j = v.v2v_off[i]; j < v.v2v_off[i + 1]; ++j) {
         int c = v.v2v[j];
-        double2 w = v.wxy[j];
-        double qc[4];
-        g4(v.qp[c], qc);
+        const double2 w = v.wxy[j];
+        S qc[4];
+        g4s(v.qp[c], qc);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            gx[k] = gx[k] + (qc[k] - qi[k]) * w.x;
-            gy[k] = gy[k] + (qc[k] - qi[k]) * w.y;
+            const S d = qc[k] - qi[k];
+            gx[k] = gx[k] + d * w.x;
+            gy[k] = gy[k] + d * w.y;
         }
     }
-    v.gx[i] = m4(gx);
-    v.gy[i] = m4(gy);
-    // DUmax/DUmin over the node's edges (limiter.f90:24-39).
-    double dmx[4], dmn[4], ph[4];
+    v.gx[i] = m4s(gx);
+    v.gy[i] = m4s(gy);
+    // DUmax/DUmin over the node's edges (limiter.f90:24-39), as order keys
+    // (of two zeros they prefer the positive, rmax / rmin the first; a zero
+    // extreme has magnitude below eps or is the ratio's numerator, where its
+    // sign drops out).
+    long long dmx[4], dmn[4];
+    S ph[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) { dmn[k] = v.eps; dmx[k] = -v.eps; }
+    for (int k = 0; k < 4; ++k) { dmn[k] = order_key(v.eps); dmx[k] = order_key(-v.eps); }
     const int k0 = v.v2f_off[i], k1 = v.v2f_off[i + 1];
     for (int k = k0; k < k1; ++k) {
         int e = v.v2f[k], f = e & EDGE_MASK;
         int2 p = v.fpt[f];
-        double a[4], b[4];
-        g4(v.qp[p.x], a);
-        g4(v.qp[p.y], b);
+        S a[4], b[4];
+        g4s(v.qp[p.x], a);
+        g4s(v.qp[p.y], b);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            double du = b[j] - a[j];
-            if (e & P2_BIT) du = -du;
-            dmx[j] = rmax(dmx[j], du);
-            dmn[j] = rmin(dmn[j], du);
+            const double du = (b[j] - a[j]).v;
+            extend(flip64(du, (e & P2_BIT) != 0), dmn[j], dmx[j]);
         }
     }
-    g4(v.phi[i], ph);
-    double sq = sqrt(v.cv[i]);
+    g4s(v.phi[i], ph);
     // phi = min(phi, phj of every edge).  Each phj is min(1, n/d) (Barth:
     // clamped to [0, 1] in the corrected form) and the clamps are monotonic,
     // so only the smallest ratio needs a division: the edges' ratios are
@@ -240,42 +258,54 @@ __global__ void __launch_bounds__(kBlock) k_nc_grad_lim(NCView v) {
     // rounded minimum.  One IEEE division per variable instead of one per
     // edge and variable; the values are those of the per-edge form.
     const bool vkn = v.limiter == UNS_LIM_VKN, corrected = v.limiter == UNS_LIM_BARTH_CORRECTED;
-    double bn[4], bd[4];
+    S TOL = 0.0;
+    if (vkn) {
+        const S kk = S(v.kappa) * sqrt(S(v.cv[i]));
+        TOL = kk * kk * kk;
+    }
+    S bn[4], bd[4];
     bool have[4] = {false, false, false, false};
-    auto clamp = [&](double q) {
-        double phj = rmin(1.0, q);
-        return (!vkn && corrected) ? rmax(0.0, phj) : phj;
+    auto clamp = [&](S q) {
+        const S phj = rmin(S(1.0), q);
+        return (!vkn && corrected) ? rmax(S(0.0), phj) : phj;
     };
     for (int k = k0; k < k1; ++k) {
         int e = v.v2f[k], f = e & EDGE_MASK;
         int2 p = v.fpt[f];
-        double2 a = v.pxy[p.x], b = v.pxy[p.y];
-        double d0 = b.x - a.x, d1 = b.y - a.y;
+        const double2 a = v.pxy[p.x], b = v.pxy[p.y];
+        const S d0 = S(b.x) - a.x, d1 = S(b.y) - a.y;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            double s = gx[j] * d0 + gy[j] * d1;
-            double n, d;  // phj = clamp(n / d), or 1 where there is no ratio
-            bool ratio = true;
+            S D_L = half(gx[j] * d0 + gy[j] * d1);
+            S n, d;  // phj = clamp(n / d), or 1 where there is no ratio
+            bool ratio = true, exact = true;
             if (vkn) {
-                double D_L = (e & P2_BIT) ? -(0.5 * s) : 0.5 * s;
-                double kk = v.kappa * sq;
-                double TOL = kk * kk * kk;
-                double alfa = D_L > 0.0 ? dmx[j] : dmn[j];
-                if (fabs(alfa) < v.eps) alfa = 0.0;
-                n = alfa * alfa + 2.0 * D_L * alfa + TOL;
-                d = alfa * alfa + 2.0 * D_L * D_L + D_L * alfa + TOL;
+                D_L = flip64(D_L.v, (e & P2_BIT) != 0);
+                double alfa = from_key(dpos(D_L.v) ? dmx[j] : dmn[j]);
+                if (fabs(S(alfa)) < S(v.eps)) alfa = 0.0;
+                // 2 D alfa and 2 D D scaled after the product: the same bits
+                // unless it is subnormal, which terms that ratio_ok accepts
+                // do not show
+                const S aa = S(alfa) * alfa, da = D_L * alfa;
+                n = aa + twice(da) + TOL;
+                d = aa + twice(D_L * D_L) + da + TOL;
+                if (!ratio_ok(n.v, d.v)) {
+                    exact = false;
+                    ph[j] = rmin(ph[j], clamp(S(nc_vkn_rare(alfa, D_L.v, TOL.v))));
+                }
             } else {  // Barth-Jespersen: reference form projects fp2 with +1/2
-                double D_L = 0.5 * s;
-                if (corrected && (e & P2_BIT)) D_L = -D_L;
-                if (D_L > 0.0) { n = dmx[j]; d = D_L; }
-                else if (D_L < 0.0) { n = -dmn[j]; d = -D_L; }  // dmn / D_L with a positive denominator
+                D_L = flip64(D_L.v, corrected && (e & P2_BIT));
+                if (dpos(D_L.v)) { n = from_key(dmx[j]); d = D_L; }
+                else if (dneg(D_L.v)) { n = neg64(from_key(dmn[j])); d = -D_L; }  // dmn / D_L with a positive denominator
                 else ratio = false;
+                if (ratio && !ratio_ok(n.v, d.v)) {
+                    exact = false;
+                    ph[j] = rmin(ph[j], clamp(S(div_rare(n.v, d.v))));
+                }
             }
             if (!ratio) {
-                ph[j] = rmin(ph[j], clamp(1.0));
-            } else if (!ratio_ok(n, d)) {
-                ph[j] = rmin(ph[j], clamp(n / d));
-            } else if (!have[j] || ratio_less(n, d, bn[j], bd[j])) {
+                ph[j] = rmin(ph[j], clamp(S(1.0)));
+            } else if (exact && (!have[j] || ratio_less(n, d, bn[j], bd[j]))) {
                 bn[j] = n; bd[j] = d; have[j] = true;
             }
         }
@@ -283,11 +313,56 @@ __global__ void __launch_bounds__(kBlock) k_nc_grad_lim(NCView v) {
 #pragma unroll
     for (int j = 0; j < 4; ++j)
         if (have[j]) ph[j] = rmin(ph[j], clamp(bn[j] / bd[j]));
-    v.phi[i] = m4(ph);
+    v.phi[i] = m4s(ph);
+}
+
+// The boundary closure of edge f (wall or farfield) with nodes p.
+static __device__ __noinline__ void nc_boundary_edge(const NCView& v, int f, int2 p, double2 X1, double2 X2, int bc) {
+    double q1[4], q2[4];
+    g4(v.qp[p.x], q1);
+    g4(v.qp[p.y], q2);
+    const int s = v.fslot[f];
+    const Gas& g = v.g;
+    if (bc == 1001) {  // solid_flux (solid_flux.f90:26-41)
+        double pa = 0.75 * q1[3] + 0.25 * q2[3];
+        double pb = 0.25 * q1[3] + 0.75 * q2[3];
+        double nx = 0.5 * (X2.y - X1.y);
+        double ny = -0.5 * (X2.x - X1.x);
+        double ar = sqrt(nx * nx + ny * ny);
+        v.bla[s] = make_double2(sqrt(g.gamma * q1[3] / q1[0]) * ar, sqrt(g.gamma * q2[3] / q2[0]) * ar);
+        v.bres1[s] = make_double4(0.0, 0.0, pa * nx, pa * ny);
+        v.bres2[s] = make_double4(0.0, 0.0, pb * nx, pb * ny);
+    } else {  // farfield_flux1 (farfield_flux.f90:13-95)
+        double nx = -(0.5 * (X2.y - X1.y));
+        double ny = 0.5 * (X2.x - X1.x);
+        double dr = sqrt(nx * nx + ny * ny);
+        nx = nx / dr; ny = ny / dr;
+        double un_inf = g.u_inf * nx + g.v_inf * ny;
+        double rho = 0.5 * (q1[0] + q2[0]), uu = 0.5 * (q1[1] + q2[1]), vq = 0.5 * (q1[2] + q2[2]), pp = 0.5 * (q1[3] + q2[3]);
+        double a0 = sqrt(g.gamma * pp / rho);
+        double unn = uu * nx + vq * ny;
+        double Rp = unn + 2.0 * a0 / g.gamma1;
+        double Rm = un_inf - 2.0 * g.a_inf / g.gamma1;
+        double Unf = 0.5 * (Rp + Rm);
+        double af = 0.25 * (Rp - Rm) * g.gamma1;
+        double uf, vf, Sf;
+        if (Unf > 0.0) { uf = uu + nx * (Unf - unn); vf = vq + ny * (Unf - unn); Sf = pp / pow(rho, g.gamma); }
+        else { uf = g.u_inf + nx * (Unf - un_inf); vf = g.v_inf + ny * (Unf - un_inf); Sf = g.p_inf / pow(g.r_inf, g.gamma); }
+        double rhof = pow(af * af / g.gamma / Sf, 1.0 / g.gamma1);
+        double pf = rhof * af * af / g.gamma;
+        double ef = pf / g.gamma1 + 0.5 * rhof * (uf * uf + vf * vf);
+        double fl0 = (ef + pf) * Unf, fl1 = rhof * Unf;
+        double fl2 = fl1 * uf + pf * nx, fl3 = fl1 * vf + pf * ny;
+        double ar = sqrt(nx * nx + ny * ny);
+        v.bla[s] = make_double2((fabs(Unf) + sqrt(g.gamma * q1[3] / q1[0])) * ar, (fabs(Unf) + sqrt(g.gamma * q2[3] / q2[0])) * ar);
+        double4 r = make_double4(dr * fl0, dr * fl1, dr * fl2, dr * fl3);
+        v.bres1[s] = r;
+        v.bres2[s] = r;
+    }
 }
 
 template <class R>
-__global__ void __launch_bounds__(kBlock) k_nc_edge(NCView v) {
+__global__ void __launch_bounds__(kBlock, std::is_same<R, float>::value ? 1 : 3) k_nc_edge(NCView v) {
     if (stopped(v)) return;
     int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= v.nof) return;
@@ -332,77 +407,45 @@ __global__ void __launch_bounds__(kBlock) k_nc_edge(NCView v) {
             return;
         }
     }
+    // FP64 edges, and the boundary edges of the mixed form (flux alone in FP32)
+    typedef F64I S;
     int2 p = v.fpt[f];
     double2 X1 = v.pxy[p.x], X2 = v.pxy[p.y];
-    double d0 = X2.x - X1.x, d1 = X2.y - X1.y;
-    double q1[4], q2[4], a[4], b[4], c[4], d[4], f1[4], f2[4];
-    g4(v.qp[p.x], q1); g4(v.qp[p.y], q2);
-    g4(v.gx[p.x], a); g4(v.gy[p.x], b); g4(v.gx[p.y], c); g4(v.gy[p.y], d);
-    g4(v.phi[p.x], f1); g4(v.phi[p.y], f2);
-    V4<R> L, Rt, F;
+    const S d0 = S(X2.x) - X1.x, d1 = S(X2.y) - X1.y;
+    S q1[4], q2[4], a[4], b[4], c[4], d[4], f1[4], f2[4];
+    g4s(v.qp[p.x], q1); g4s(v.qp[p.y], q2);
+    g4s(v.gx[p.x], a); g4s(v.gy[p.x], b); g4s(v.gx[p.y], c); g4s(v.gy[p.y], d);
+    g4s(v.phi[p.x], f1); g4s(v.phi[p.y], f2);
+    typedef typename std::conditional<std::is_same<R, float>::value, float, F64I>::type FT;
+    V4<FT> L, Rt, F;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {  // fvresidual.f90:41-54
-        double g = a[k] * d0 + b[k] * d1;
-        L[k] = (R)(q1[k] + 0.5 * g * f1[k]);
+        S g = a[k] * d0 + b[k] * d1;
+        L[k] = Cvt<FT, S>::f(q1[k] + half(g) * f1[k]);
         g = c[k] * d0 + d[k] * d1;
-        Rt[k] = (R)(q2[k] - 0.5 * g * f2[k]);
+        Rt[k] = Cvt<FT, S>::f(q2[k] - half(g) * f2[k]);
     }
     double2 n = v.fn[f];
-    double area = v.farea[f];
-    const R G = (R)v.g.gamma, G1 = (R)v.g.gamma1;
-    R hl, hr;
-    if (v.g.flux == UNS_FLUX_AUSM) ausm_core<R>(G, G1, (R)n.x, (R)n.y, (R)v.g.mref, L, Rt, F, hl, hr);
-    else vanleer_core<R>(G, G1, (R)n.x, (R)n.y, L, Rt, F, hl, hr);
-    v.fF[f] = make_double4((double)F[0] * area, (double)F[1] * area, (double)F[2] * area, (double)F[3] * area);
+    const S area = v.farea[f];
+    const FT G = (FT)v.g.gamma, G1 = (FT)v.g.gamma1;
+    FT hlr, hrr;
+    if (v.g.flux == UNS_FLUX_AUSM) ausm_core<FT>(G, G1, (FT)n.x, (FT)n.y, (FT)v.g.mref, L, Rt, F, hlr, hrr);
+    else vanleer_core<FT>(G, G1, (FT)n.x, (FT)n.y, L, Rt, F, hlr, hrr);
+    const S F0 = Cvt<S, FT>::f(F[0]), F1 = Cvt<S, FT>::f(F[1]), F2 = Cvt<S, FT>::f(F[2]), F3 = Cvt<S, FT>::f(F[3]);
+    v.fF[f] = make_double4((F0 * area).v, (F1 * area).v, (F2 * area).v, (F3 * area).v);
     // Roe-averaged spectral radius (vanleer_flux.f90:102-115).
-    double rL = (double)L[0], rR = (double)Rt[0];
-    double RT = sqrt(rR / rL);
-    double u = ((double)L[1] + RT * (double)Rt[1]) / (1.0 + RT);
-    double vv = ((double)L[2] + RT * (double)Rt[2]) / (1.0 + RT);
-    double H = ((double)hl + RT * (double)hr) / (1.0 + RT);
-    double aa = sqrt((v.g.gamma1) * (H - 0.5 * (u * u + vv * vv)));
-    double un = fabs(u * n.x + vv * n.y);
-    v.fla[f] = (un + aa) * area;
+    const S L0 = Cvt<S, FT>::f(L[0]), L1 = Cvt<S, FT>::f(L[1]), L2 = Cvt<S, FT>::f(L[2]);
+    const S R0 = Cvt<S, FT>::f(Rt[0]), R1 = Cvt<S, FT>::f(Rt[1]), R2 = Cvt<S, FT>::f(Rt[2]);
+    const S RT1 = sqrt(R0 / L0), den = S(1.0) + RT1;
+    const S u = (L1 + RT1 * R1) / den;
+    const S vv = (L2 + RT1 * R2) / den;
+    const S H = (Cvt<S, FT>::f(hlr) + RT1 * Cvt<S, FT>::f(hrr)) / den;
+    const S aa = sqrt(S(v.g.gamma1) * (H - half(u * u + vv * vv)));
+    const S un = fabs(u * n.x + vv * n.y);
+    v.fla[f] = ((un + aa) * area).v;
     int bc = v.fbc[f];
     if (bc != 1001 && bc != 2001) return;
-    int s = v.fslot[f];
-    const Gas& g = v.g;
-    if (bc == 1001) {  // solid_flux (solid_flux.f90:26-41)
-        double pa = 0.75 * q1[3] + 0.25 * q2[3];
-        double pb = 0.25 * q1[3] + 0.75 * q2[3];
-        double nx = 0.5 * (X2.y - X1.y);
-        double ny = -0.5 * (X2.x - X1.x);
-        double ar = sqrt(nx * nx + ny * ny);
-        v.bla[s] = make_double2(sqrt(g.gamma * q1[3] / q1[0]) * ar, sqrt(g.gamma * q2[3] / q2[0]) * ar);
-        v.bres1[s] = make_double4(0.0, 0.0, pa * nx, pa * ny);
-        v.bres2[s] = make_double4(0.0, 0.0, pb * nx, pb * ny);
-    } else {  // farfield_flux1 (farfield_flux.f90:13-95)
-        double nx = -(0.5 * (X2.y - X1.y));
-        double ny = 0.5 * (X2.x - X1.x);
-        double dr = sqrt(nx * nx + ny * ny);
-        nx = nx / dr; ny = ny / dr;
-        double un_inf = g.u_inf * nx + g.v_inf * ny;
-        double rho = 0.5 * (q1[0] + q2[0]), uu = 0.5 * (q1[1] + q2[1]), vq = 0.5 * (q1[2] + q2[2]), pp = 0.5 * (q1[3] + q2[3]);
-        double a0 = sqrt(g.gamma * pp / rho);
-        double unn = uu * nx + vq * ny;
-        double Rp = unn + 2.0 * a0 / g.gamma1;
-        double Rm = un_inf - 2.0 * g.a_inf / g.gamma1;
-        double Unf = 0.5 * (Rp + Rm);
-        double af = 0.25 * (Rp - Rm) * g.gamma1;
-        double uf, vf, Sf;
-        if (Unf > 0.0) { uf = uu + nx * (Unf - unn); vf = vq + ny * (Unf - unn); Sf = pp / pow(rho, g.gamma); }
-        else { uf = g.u_inf + nx * (Unf - un_inf); vf = g.v_inf + ny * (Unf - un_inf); Sf = g.p_inf / pow(g.r_inf, g.gamma); }
-        double rhof = pow(af * af / g.gamma / Sf, 1.0 / g.gamma1);
-        double pf = rhof * af * af / g.gamma;
-        double ef = pf / g.gamma1 + 0.5 * rhof * (uf * uf + vf * vf);
-        double fl0 = (ef + pf) * Unf, fl1 = rhof * Unf;
-        double fl2 = fl1 * uf + pf * nx, fl3 = fl1 * vf + pf * ny;
-        double ar = sqrt(nx * nx + ny * ny);
-        v.bla[s] = make_double2((fabs(Unf) + sqrt(g.gamma * q1[3] / q1[0])) * ar, (fabs(Unf) + sqrt(g.gamma * q2[3] / q2[0])) * ar);
-        double4 r = make_double4(dr * fl0, dr * fl1, dr * fl2, dr * fl3);
-        v.bres1[s] = r;
-        v.bres2[s] = r;
-    }
+    nc_boundary_edge(v, f, p, X1, X2, bc);
 }
 
 // Node gather in edge-index order (the reference's accumulation order):
@@ -421,53 +464,60 @@ __global__ void __launch_bounds__(kBlock) k_nc_node_res(NCView v, double cfl_in,
     double fr = 0.0, frs = -1.0;
     int fri = 0x7fffffff;
     if (i < v.nop) {
-        double r[4] = {0, 0, 0, 0}, la = 0.0;
-        for (int k = v.v2f_off[i]; k < v.v2f_off[i + 1]; ++k) {
+        F64I r[4], la;
+        const int k0 = v.v2f_off[i], k1 = v.v2f_off[i + 1];
+        r[0] = r[1] = r[2] = r[3] = la = 0.0;
+        for (int k = k0; k < k1; ++k) {
             int e = v.v2f[k], f = e & EDGE_MASK;
-            double F[4];
-            g4(v.fF[f], F);
-            bool is2 = (e & P2_BIT) != 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) r[j] = is2 ? r[j] - F[j] : r[j] + F[j];
-            la = la + v.fla[f];
+            const double4 F = v.fF[f];
+            const double fl = v.fla[f];
+            const bool is2 = (e & P2_BIT) != 0;
+            if (k == k0) {  // 0.0 + F
+                r[0] = zero_plus(flip64(F.x, is2)); r[1] = zero_plus(flip64(F.y, is2));
+                r[2] = zero_plus(flip64(F.z, is2)); r[3] = zero_plus(flip64(F.w, is2));
+                la = zero_plus(fl);
+            } else {
+                r[0] = r[0] + F64I(flip64(F.x, is2)); r[1] = r[1] + F64I(flip64(F.y, is2));
+                r[2] = r[2] + F64I(flip64(F.z, is2)); r[3] = r[3] + F64I(flip64(F.w, is2));
+                la = la + fl;
+            }
             int s = v.fslot[f];
             if (s >= 0) {
                 double2 bl = v.bla[s];
-                la = la + (is2 ? bl.y : bl.x);
-                double B[4];
-                g4(is2 ? v.bres2[s] : v.bres1[s], B);
-                int bc = v.fbc[f];
-                if (bc == 1001) { r[2] = r[2] + B[2]; r[3] = r[3] + B[3]; }
-                else {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) r[j] = r[j] + B[j];
-                }
+                la = add_rare(la.v, is2 ? bl.y : bl.x);
+                const double4 B = is2 ? v.bres2[s] : v.bres1[s];
+                if (v.fbc[f] != 1001) { r[0] = add_rare(r[0].v, B.x); r[1] = add_rare(r[1].v, B.y); }
+                r[2] = add_rare(r[2].v, B.z);
+                r[3] = add_rare(r[3].v, B.w);
             }
         }
-        v.res[i] = m4(r);
-        v.la[i] = la;
-        double cfl = v.cfl_sched ? v.cfl_sched[*v.iter] : cfl_in;
-        double dt = cfl * v.cv[i] / la;
-        v.dt[i] = dt;
-        v.diag[i] = v.cv[i] / dt + 0.5 * 1.5 * la;
-        v.diaginv[i] = 1.0 / v.diag[i];
+        v.res[i] = m4s(r);
+        v.la[i] = la.v;
+        const F64I cv = v.cv[i], cfl = v.cfl_sched ? v.cfl_sched[*v.iter] : cfl_in;
+        const F64I dt = cfl * cv / la;
+        v.dt[i] = dt.v;
+        const F64I diag = cv / dt + F64I(0.5 * 1.5) * la;
+        v.diag[i] = diag.v;
+        v.diaginv[i] = (F64I(1.0) / diag).v;
         if (rk3) {
-            double dtbyarea = dt / v.cv[i];
-            double o[4], q[4];
-            g4(v.qold[i], o);
-            g4(v.qc[i], q);
-            for (int irk = 1; irk <= 3; ++irk) {
-                const double a = rk3_a(irk), b = rk3_b(irk);
+            const F64I dtbyarea = dt / cv;
+            F64I o[4], q[4];
+            g4s(v.qold[i], o);
+            g4s(v.qc[i], q);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) q[j] = a * o[j] + b * (q[j] - dtbyarea * r[j]);
+            for (int j = 0; j < 4; ++j) {  // weights 0, 1; 3/4, 1/4; 1/3, 2/3
+                const F64I D = dtbyarea * r[j];
+                q[j] = q[j] - D;
+                q[j] = F64I(rk3_a(2)) * o[j] + quarter(q[j] - D);
+                q[j] = F64I(rk3_a(3)) * o[j] + F64I(rk3_b(3)) * (q[j] - D);
             }
-            v.qc[i] = m4(q);
+            v.qc[i] = m4s(q);
         }
-        double t = 0.0;
+        F64I t = zero_plus((r[0] * r[0]).v);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) t = t + r[j] * r[j];
-        fr = t;
-        frs = sqrt(t);
+        for (int j = 1; j < 4; ++j) t = t + r[j] * r[j];
+        fr = t.v;
+        frs = sqrt(t).v;
         fri = i;
     }
     if (!partial) return;
@@ -592,20 +642,6 @@ __global__ void __launch_bounds__(kBlock) k_nc_res_final(NCView v, int nparts, d
     }
 }
 
-// normalflux(qold) of both end nodes on every edge (lusgs.f90:137-155); it
-// does not change during the sweeps, so it is evaluated once per edge.
-__device__ __forceinline__ void normalflux_nc(const Gas& g, const double4& q, double nx, double ny, double ds, double o[4]) {
-    Prim P = con2prim(g, q.x, q.y, q.z, q.w);
-    double et = P.e * P.rho;
-    double un = P.u * nx + P.v * ny;
-    o[0] = (et + P.p) * un;
-    o[1] = P.rho * un;
-    o[2] = o[1] * P.u + P.p * nx;
-    o[3] = o[1] * P.v + P.p * ny;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) o[k] = o[k] * ds;
-}
-
 constexpr int kSweepBlock = 128;
 // One sweep block per SM: one warp per SM sub-partition, so concurrently
 // active items never share an FP64 unit.
@@ -626,15 +662,14 @@ __global__ void __launch_bounds__(kBlock) k_nc_qold_prim(NCView v) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= v.nop) return;
     const double4 q = v.qold[i];
-    Prim P = con2prim(v.g, q.x, q.y, q.z, q.w);
-    v.qoldp[i] = make_double4(P.u, P.v, P.p, P.e * P.rho);
+    const PrimT<F64I> P = con2prim_t<F64I>(v.g, q.x, q.y, q.z, q.w);
+    v.qoldp[i] = make_double4(P.u.v, P.v.v, P.p.v, (P.e * P.rho).v);
 }
 
 // normalflux_nc from the node's precomputed primitives (rho = qold.rho).
-__device__ __forceinline__ void normalflux_nc_p(const double4& P, double rho, double nx, double ny, double ds,
-                                                double o[4]) {
-    const double u = P.x, vv = P.y, p = P.z, et = P.w;
-    double un = u * nx + vv * ny;
+__device__ __forceinline__ void normalflux_nc_p(const double4& P, F64I rho, F64I nx, F64I ny, F64I ds, F64I o[4]) {
+    const F64I u = P.x, vv = P.y, p = P.z, et = P.w;
+    const F64I un = u * nx + vv * ny;
     o[0] = (et + p) * un;
     o[1] = rho * un;
     o[2] = o[1] * u + p * nx;
@@ -651,11 +686,11 @@ __global__ void __launch_bounds__(kBlock) k_nc_sweep_prep(NCView v) {
     const double2 n = v.fn[c];
     const double ds = v.farea[c];
     const double4 q = v.qold[nb];
-    double o[4];
+    F64I o[4];
     normalflux_nc_p(v.qoldp[nb], q.y, n.x, n.y, ds, o);
-    v.rec[3 * (size_t)r] = m4(o);
-    v.rec[3 * (size_t)r + 1] = make_double4(n.x, n.y, ds, kOmega * v.fla[c]);
-    v.rec[3 * (size_t)r + 2] = make_double4(q.y, (double)v.rec_sign[r], __longlong_as_double((long long)nb), 0.0);
+    v.rec[3 * (size_t)r] = m4s(o);
+    v.rec[3 * (size_t)r + 1] = make_double4(n.x, n.y, ds, (F64I(kOmega) * v.fla[c]).v);
+    v.rec[3 * (size_t)r + 2] = make_double4(q.y, v.rec_sign[r] < 0 ? -1.0 : 1.0, __longlong_as_double((long long)nb), 0.0);
 }
 
 // Mixed-precision sweeps (delta form): per record, in FP32, the neighbour's
@@ -669,11 +704,11 @@ __global__ void __launch_bounds__(kBlock) k_nc_sweep_prep_mixed(NCView v) {
     const int c = v.rec_edge[r], nb = v.rec_nb[r];
     const double2 n = v.fn[c];
     const double4 q = v.qold[nb];
-    Prim P = con2prim(v.g, q.x, q.y, q.z, q.w);
+    const PrimT<F64I> P = con2prim_t<F64I>(v.g, q.x, q.y, q.z, q.w);
     float4* rf = reinterpret_cast<float4*>(v.rec) + 4 * (size_t)r;
     rf[0] = make_float4((float)q.y, (float)q.z, (float)q.w, (float)q.x);
     rf[1] = make_float4((float)P.u, (float)P.v, (float)P.p, (float)(P.u * n.x + P.v * n.y));
-    rf[2] = make_float4((float)n.x, (float)n.y, (float)v.farea[c], (float)(kOmega * v.fla[c]));
+    rf[2] = make_float4((float)n.x, (float)n.y, (float)v.farea[c], (float)(F64I(kOmega) * v.fla[c]));
     rf[3] = make_float4((float)v.rec_sign[r], __int_as_float(nb), 0.f, 0.f);
 }
 
@@ -1104,6 +1139,7 @@ struct uns_nc_handle {
     int nparts = 0;
     int* woff = nullptr;    // LU-SGS warp schedule: per-warp ranges of v.sched
     int coop_blocks = 0;
+    int nsm = 1;            // SMs of the device
     int lev_fwd = 0, lev_bwd = 0;  // dependency levels of the two sweeps (their critical path)
     double4 qinf;
     cudaGraphExec_t graph = nullptr;
@@ -1162,11 +1198,28 @@ int check_err_nc(uns_nc_handle* h) {
         UNS_CUDA(cudaGetLastError());                                                \
     } while (0)
 
+// Small meshes in narrower blocks, so that their warps spread over the SMs.
+inline int spread_bs_nc(const uns_nc_handle* h, int n) {
+    int bs = kBlock;
+    while (bs > 32 && nblocks(n, bs) < 2 * h->nsm) bs >>= 1;
+    return bs;
+}
+inline void launch_grad_lim(uns_nc_handle* h, NCView& v) {
+    const int bs = spread_bs_nc(h, v.nop);
+    if (bs < kBlock) k_nc_grad_lim<F64><<<nblocks(v.nop, bs), bs, 0, h->stream>>>(v);
+    else k_nc_grad_lim<F64I><<<nblocks(v.nop, bs), bs, 0, h->stream>>>(v);
+}
+inline void launch_edge(uns_nc_handle* h, NCView& v) {
+    int bs = kBlock;
+    while (bs > 32 && nblocks(v.nof, bs) < 4 * h->nsm) bs >>= 1;
+    k_nc_edge<double><<<nblocks(v.nof, bs), bs, 0, h->stream>>>(v);
+}
+
 int enqueue_fvres_nc(uns_nc_handle* h, NCView& v, double cfl, int rk3, int partial) {
     if (h->P.precision == UNS_PREC_MIXED) NLAUNCH(k_nc_grad_lim_mixed, v.nop, v);
-    else NLAUNCH(k_nc_grad_lim, v.nop, v);
+    else launch_grad_lim(h, v);
     if (h->P.precision == UNS_PREC_MIXED) NLAUNCH(k_nc_edge<float>, v.nof, v);
-    else NLAUNCH(k_nc_edge<double>, v.nof, v);
+    else launch_edge(h, v);
     NLAUNCH(k_nc_node_res, v.nop, v, cfl, rk3, partial);
     return UNS_OK;
 }
@@ -1353,6 +1406,7 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
             set_last_error("uns_nc_create: cannot size the cooperative LU-SGS launch");
             return fail(UNS_ERR_CUDA);
         }
+        h->nsm = nsm;
         h->coop_blocks = nsm * std::min(per, kSweepBlocksPerSM);
         // other end of each v2f edge, and the reference's orientation sign
         auto other = [&](int i, int e, int* sign) {
@@ -1638,12 +1692,12 @@ int uns_nc_profile(uns_nc_handle* h, double cfl, int reps, double* ms, const cha
         rc = timed(0, [&]() -> int { NLAUNCH(k_nc_save_old, v.nop, v); return UNS_OK; });
         if (!rc) rc = timed(1, [&]() -> int {
             if (h->P.precision == UNS_PREC_MIXED) NLAUNCH(k_nc_grad_lim_mixed, v.nop, v);
-            else NLAUNCH(k_nc_grad_lim, v.nop, v);
+            else launch_grad_lim(h, v);
             return UNS_OK;
         });
         if (!rc) rc = timed(2, [&]() -> int {
             if (h->P.precision == UNS_PREC_MIXED) NLAUNCH(k_nc_edge<float>, v.nof, v);
-            else NLAUNCH(k_nc_edge<double>, v.nof, v);
+            else launch_edge(h, v);
             return UNS_OK;
         });
         if (!rc) rc = timed(3, [&]() -> int { NLAUNCH(k_nc_node_res, v.nop, v, cfl, rk3 ? 1 : 0, 1); return UNS_OK; });

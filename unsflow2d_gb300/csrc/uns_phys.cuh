@@ -336,6 +336,10 @@ struct Cvt<T, T> {
     __device__ __forceinline__ static T f(T x) { return x; }
 };
 template <>
+struct Cvt<F64I, float> {
+    __device__ __forceinline__ static F64I f(float x) { return F64I((double)x); }
+};
+template <>
 struct Cvt<F64, float> {
     __device__ __forceinline__ static F64 f(float x) { return F64((double)x); }
 };

@@ -16,7 +16,8 @@ D = C.POINTER(C.c_double)
 OPS = {"add": np.add, "sub": np.subtract, "mul": np.multiply, "div": np.divide, "sqrt": lambda a, b: np.sqrt(a),
        "half": lambda a, b: 0.5 * a, "twice": lambda a, b: 2.0 * a, "lt": lambda a, b: (a < b).astype(float),
        "le": lambda a, b: (a <= b).astype(float), "sign": lambda a, b: (a > 0).astype(float) - (a < 0).astype(float),
-       "mul_digits": np.multiply}
+       "mul_digits": np.multiply, "narrow": lambda a, b: a.astype(np.float32).astype(float),
+       "widen": lambda a, b: a.astype(np.float32).astype(float)}
 
 
 def _operands(op):
@@ -46,6 +47,10 @@ def _operands(op):
         r = np.abs(rng.standard_normal(2 * k))
         a[8 * k:10 * k] = r * r
         a[9 * k:10 * k] = np.nextafter(a[9 * k:10 * k], rng.choice([0.0, np.inf], k))
+    if op in ("narrow", "widen"):  # FP32's exponent range, its ends and rounding ties
+        e[0] = rng.integers(860, 1170, n).astype(np.uint64)
+        m[0, : n // 2] &= ~np.uint64((1 << 28) - 1)
+        a = (s[0] | (e[0] << np.uint64(52)) | m[0]).view(np.float64)
     if op in ("lt", "le"):
         b[8 * k:9 * k] = a[8 * k:9 * k]
         b[9 * k:10 * k] = np.nextafter(a[9 * k:10 * k], np.inf)

@@ -35,6 +35,8 @@ __global__ void k_selftest_fp64(int op, const double* a, const double* b, double
         case 7: r = uns::dlt(x, y) ? 1.0 : 0.0; break;
         case 8: r = uns::dle(x, y) ? 1.0 : 0.0; break;
         case 10: r = uns::mul_digits(x, y); break;
+        case 11: r = (double)uns::narrow(x); break;
+        case 12: r = uns::widen((float)x); break;
         case 9: r = uns::dpos(x) ? 1.0 : (uns::dneg(x) ? -1.0 : 0.0); break;
     }
     out[i] = r;

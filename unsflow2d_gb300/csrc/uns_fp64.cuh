@@ -84,6 +84,26 @@ static __device__ __noinline__ double add_rare(double a, double b) { return a + 
 static __device__ __noinline__ double mul_rare(double a, double b) { return a * b; }
 static __device__ __noinline__ double div_rare(double a, double b) { return a / b; }
 static __device__ __noinline__ double sqrt_rare(double a) { return sqrt(a); }
+static __device__ __noinline__ double widen_rare(float a) { return (double)a; }
+static __device__ __noinline__ float narrow_rare(double a) { return (float)a; }
+
+// (double)a and (float)a on the integer pipe (the conversions hold the FP64
+// unit 76-99 cycles).
+__device__ __forceinline__ double widen(float a) {
+    const unsigned b = __float_as_uint(a);
+    const bool zero = (b << 1) == 0;
+    if ((b & 0x7f800000u) - 0x00800000u >= 0x7f000000u && !zero) return widen_rare(a);  // subnormal, infinite, NaN
+    const unsigned hi = ((b >> 3) & 0x0fffffffu) + 0x38000000u;
+    return dmake((b & 0x80000000u) | (zero ? 0u : hi), b << 29);
+}
+__device__ __forceinline__ float narrow(double a) {
+    const unsigned h = dhi(a), l = dlo(a), m = h & 0x7fffffffu;
+    const bool zero = (m | l) == 0;
+    if (m - 0x38100000u >= 0x0fd00000u && !zero) return narrow_rare(a);  // outside [2^-126, 2^127)
+    const unsigned r = __funnelshift_l(l, m - 0x38000000u, 3), rem = l << 3;  // 24-bit significand and what it drops
+    const unsigned up = (rem >= 0x80000000u && (rem > 0x80000000u || (r & 1u))) ? 1u : 0u;
+    return __uint_as_float((h & 0x80000000u) | (zero ? 0u : r + up));
+}
 
 // Division and square root by digit recurrence with accurate quotient digits
 // (D. Wong, M. Flynn, "Fast division using accurate quotient
@@ -100,17 +120,21 @@ __device__ __forceinline__ unsigned recip_digits(float y) {
     return __float_as_uint(__fmaf_rd(y, 1.0f - 0x1p-21f, 1.0f)) << 9;
 }
 
-__device__ __forceinline__ double div_digits(double a, double b) {
+// The reciprocal of b's significand for div_digits: from its leading 24 bits.
+__device__ __forceinline__ unsigned div_recip(double b) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(0x3f800000u | (__funnelshift_l(dlo(b), dhi(b), 3) & 0x7fffffu))));
+    return recip_digits(y);
+}
+
+// a / b with Y = div_recip(b), which a caller that has b early forms early.
+__device__ __forceinline__ double div_digits(double a, double b, unsigned Y) {
     const unsigned ha = dhi(a), la = dlo(a), hb = dhi(b), lb = dlo(b);
     const unsigned ea = ha & 0x7ff00000u, eb = hb & 0x7ff00000u, sign = (ha ^ hb) & 0x80000000u;
     const bool zero = ((ha << 1) | la) == 0;
     // exponent fields of both within [768, 1279]
     if ((((zero ? 0u : ea - 0x30000000u) | (eb - 0x30000000u)) & 0xe0000000u) != 0) return div_rare(a, b);
-    const unsigned mbh = (hb & 0xfffffu) | 0x100000u;
-    const unsigned long long ma = u64((ha & 0xfffffu) | 0x100000u, la), mb = u64(mbh, lb);
-    float y;  // 1 / significand of b from its leading 24 bits
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(0x3f800000u | (((mbh << 3) | (lb >> 29)) & 0x7fffffu))));
-    const unsigned Y = recip_digits(y);
+    const unsigned long long ma = u64((ha & 0xfffffu) | 0x100000u, la), mb = u64((hb & 0xfffffu) | 0x100000u, lb);
     const unsigned d1 = __umulhi((unsigned)(ma >> 21), Y) >> 2;                   // q to 2^-29
     const unsigned long long r1 = (ma << 29) - (unsigned long long)d1 * mb;      // < 2^63.2
     const unsigned d2 = __umulhi((unsigned)(r1 >> 32), Y);                        // to 2^-49
@@ -123,6 +147,7 @@ __device__ __forceinline__ double div_digits(double a, double b) {
     const unsigned hi = (unsigned)(f >> 32) + (ea - eb) + ((1021u + t) << 20);
     return dmake(zero ? sign : (hi | sign), zero ? 0u : (unsigned)f);
 }
+__device__ __forceinline__ double div_digits(double a, double b) { return div_digits(a, b, div_recip(b)); }
 
 __device__ __forceinline__ double sqrt_digits(double a) {
     const unsigned ha = dhi(a), la = dlo(a);

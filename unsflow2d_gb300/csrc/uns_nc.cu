@@ -24,6 +24,7 @@
 #include "uns_common.cuh"
 #include "uns_phys.cuh"
 #include "uns_sched.hpp"
+#include "uns_sweep.cuh"
 #include "unsflow_gpu.h"
 
 using namespace uns;
@@ -642,8 +643,7 @@ __global__ void __launch_bounds__(kBlock) k_nc_res_final(NCView v, int nparts, d
     }
 }
 
-constexpr int kSweepBlock = 128;
-// One sweep block per SM: one warp per SM sub-partition, so concurrently
+// One sweep block per SM: one sweep warp per SM sub-partition, so concurrently
 // active items never share an FP64 unit.
 constexpr int kSweepBlocksPerSM = 1;
 constexpr double kOmega = 1.5;  // lusgs.f90:26
@@ -716,227 +716,259 @@ __device__ __forceinline__ double pick4(int k, double a, double b, double c, dou
     return k == 0 ? a : (k == 1 ? b : (k == 2 ? c : d));
 }
 
-// The node's own diagonal, qold and res (variable `lane`) in lanes 0..3;
-// benign operands elsewhere, so the warp-wide divides meet no 0 or inf.
-// (The mixed form's sweep.)
-__device__ __forceinline__ void own_load(const NCView& v, const int4& S, int lane, double& D, double& o, double& r) {
-    if (lane < 4) {
-        D = v.diag[S.x];
-        o = reinterpret_cast<const double*>(&v.qold[S.x])[lane];
-        if (S.y == 0) r = reinterpret_cast<const double*>(&v.res[S.x])[lane];
-    } else {
-        D = 1.0;
-        o = 1.0;
-        r = 0.0;
-    }
-}
-
 // Lanes of a sweep item: lane = 4 * slot + k, slot = the taken edge (up to 8
-// per round), k = the variable.  An FP64 instruction costs its SM
-// sub-partition the same whatever the number of active lanes (about 70
-// cycles on GB300), so each item's arithmetic is spread over the lanes: the
-// four flux components of up to eight edges in one pass, the per-variable
-// sums and divides in lanes 0..3, and the three divisions of con2prim in
-// lanes 0, 2 and 3 at once.  Chosen by measurement on GB300 (sweeps at
-// 1024x512, bit-identical variants): the consumer reads rho from the record
-// rather than forming qold.rho + dqc.rho; the warp exchanges its per-lane
-// values through shared memory rather than shuffles; the division by the
-// diagonal stays an IEEE division (through a precomputed reciprocal with
-// Markstein's correction it was slower, as was halving on the integer pipe);
-// the next item's inputs are loaded after this item's polls.
-struct SweepIn {
-    double f1, nx, ny, ds, ol;  // the slot's record; f1 = component k
-    double sgn;                 // orientation sign +-1 (tested where used, so no load is waited on here)
-    int nb;
-    double D, o, r;             // lanes 0..3: the diagonal, qold and res (pass 0) / the early-read
-                                // forward dqc (pass 1), variable k
+// per round), k = the variable.  An FP64 instruction holds its SM
+// sub-partition's unit the same 64-76 cycles whatever the number of active
+// lanes, so each item's arithmetic is spread over the lanes: the four flux
+// components of up to eight edges in one pass, the per-variable sums and
+// divisions in lanes 0..3, and the three divisions of con2prim in lanes 0, 2
+// and 3 at once.  Chosen by measurement on GB300 (sweeps at 1024x512,
+// bit-identical variants): the consumer reads rho from the record rather than
+// forming qold.rho + dqc.rho; the warp exchanges its per-lane values through
+// shared memory rather than shuffles; the next item's inputs are loaded after
+// this item's polls.
+__device__ __forceinline__ double ld_relaxed(const double* p) {
+    double x;
+    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(x) : "l"(p) : "memory");
+    return x;
+}
+
+// What an edge term reads of a neighbour's record: (u, v, p, e*rho), rho and
+// component k of dqc.
+struct SweepNb {
+    double u, v, p, et, rho, dq;
 };
-
-__device__ __forceinline__ void sweep_load_edge(const NCView& v, int rec, int k, SweepIn& x) {
-    const double4* p = v.rec + 3 * (size_t)rec;
-    x.f1 = reinterpret_cast<const double*>(p)[k];
-    double4 b = p[1], c = p[2];
-    x.nx = b.x; x.ny = b.y; x.ds = b.z; x.ol = b.w;
-    x.sgn = c.y;
-    x.nb = (int)__double_as_longlong(c.z);
-}
-
-__device__ __forceinline__ void sweep_load(const NCView& v, const int4& S, int lane, SweepIn& x) {
-    if ((lane >> 2) < S.w) sweep_load_edge(v, S.z + (lane >> 2), lane & 3, x);
-    if (lane < 4) {
-        x.D = v.diag[S.x];
-        x.o = reinterpret_cast<const double*>(&v.qold[S.x])[lane];
-        if (S.y == 0) {
-            x.r = reinterpret_cast<const double*>(&v.res[S.x])[lane];
-        } else {  // the node's forward dqc: usually published long before; checked when used
-            asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];"
-                         : "=d"(x.r) : "l"(reinterpret_cast<const double*>(v.rec_b + S.x) + lane) : "memory");
-        }
-    } else {
-        x.D = 1.0;
-        x.o = 1.0;
-        x.r = 0.0;
-    }
-}
-
-// A neighbour's record: (u, v, p, e*rho) in w[0..4), dqc in w[4..8), rho.
-__device__ __forceinline__ void peek_neighbour(const NCView& v, size_t rs, double w[8], double& rho) {
+__device__ __forceinline__ SweepNb peek_neighbour(const NCView& v, size_t rs, int k) {
     const double2* pa = reinterpret_cast<const double2*>(v.rec_a + rs);
-    const double2* pb = reinterpret_cast<const double2*>(v.rec_b + rs);
-    double2 x0 = ld_relaxed2(pa), x1 = ld_relaxed2(pa + 1), x2 = ld_relaxed2(pb), x3 = ld_relaxed2(pb + 1);
-    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(rho) : "l"(v.rec_r + rs) : "memory");
-    w[0] = x0.x; w[1] = x0.y; w[2] = x1.x; w[3] = x1.y;
-    w[4] = x2.x; w[5] = x2.y; w[6] = x3.x; w[7] = x3.y;
+    const double2 x0 = ld_relaxed2(pa), x1 = ld_relaxed2(pa + 1);
+    SweepNb w;
+    w.u = x0.x; w.v = x0.y; w.p = x1.x; w.et = x1.y;
+    w.rho = ld_relaxed(v.rec_r + rs);
+    w.dq = ld_relaxed(reinterpret_cast<const double*>(v.rec_b + rs) + k);
+    return w;
 }
 
-__device__ __forceinline__ bool record_set(const double w[8], double rho) {
-    bool ready = !is_unset(rho);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) ready = ready && !is_unset(w[j]);
-    return ready;
+__device__ __forceinline__ bool record_set(const SweepNb& w) {
+    return !is_unset(w.u) && !is_unset(w.v) && !is_unset(w.p) && !is_unset(w.et) && !is_unset(w.rho) && !is_unset(w.dq);
 }
 
 // A neighbour's record, waiting (bounded) until every value is published.
-__device__ __forceinline__ bool poll_neighbour(const NCView& v, size_t rs, double w[8], double& rho) {
+__device__ __forceinline__ bool poll_neighbour(const NCView& v, size_t rs, int k, SweepNb& w) {
     long long t0 = 0;
     for (int spins = 0;; ++spins) {
-        peek_neighbour(v, rs, w, rho);
-        if (record_set(w, rho)) return true;
+        w = peek_neighbour(v, rs, k);
+        if (record_set(w)) return true;
         if (!poll_continue(spins, t0, v.err, v.wait_cycles)) return false;
     }
 }
 
-// lusgs sweeps (lusgs.f90:48-124) as one cooperative launch.  Each warp runs
-// its own list of items (node, pass) from the host-side list schedule, in
-// order, loading the next item's inputs while it works on the current one.
-// Per item, for each edge whose neighbour precedes the node in this pass
-// (reference v2f order): the neighbour's values come from registers when the
-// warp itself computed that neighbour last, else from its record (read
-// during the previous item, or polled); the edge term
-// 0.5*(sign*(F(qc) - F(qold)) - omega*la*dqc) is formed per component; lanes
-// 0..3 add the terms in edge order (the reference's summation order) and
-// divide by the diagonal; the new state is spread to all lanes, which keep
-// its primitives for the next item while lanes 0..2 publish the record.
-// Every rounded operation and its operand order is the reference's.
-__global__ void __launch_bounds__(kSweepBlock, 1) k_nc_lusgs(NCView v, const int* __restrict__ woff) {
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    __shared__ __align__(16) double wxs[kSweepBlock / 32][32];  // per-warp exchange of lane values
-    double* wx = wxs[wib];
-    const int gw = blockIdx.x * (kSweepBlock / 32) + wib;
+// Fields of a ring entry (per lane): the slot's record, f1 its component k;
+// the neighbour's record; the node's own diagonal, qold and res (pass 0) or
+// forward dqc (pass 1), variable k; and the neighbour's code (node << 1 |
+// pass, -1 in an idle slot) with the orientation sign in the upper word.
+enum { SF_F1, SF_NX, SF_NY, SF_DS, SF_OL, SF_U, SF_V, SF_P, SF_ET, SF_RHO, SF_DQ, SF_D2, SF_O, SF_R, SF_CODE, SF_N };
+typedef SweepRing<SF_N> RingNC;
+
+// The feeder: for each item of the warp's list, in order and as far ahead as
+// the ring allows, its inputs and its neighbours' records.  A neighbour that
+// is the list's previous item comes from the sweep warp's registers.
+__device__ void nc_feed(const NCView& v, RingNC& R, int kbeg, int kend, int lane) {
     const int slot = lane >> 2, k = lane & 3;
-    if (stopped(v)) return;
     const int n = v.nop;
-    const double gm1 = v.g.gamma - 1.0;
+    RingPos pos;
+    int last = -1;
+    int4 S = v.sched[kbeg];
+    for (int kk = kbeg; kk < kend; ++kk) {
+        const int4 Sn = kk + 1 < kend ? v.sched[kk + 1] : make_int4(0, 0, 0, 0);
+        const int it = S.x, pass = S.y, ntake = S.w;
+        int base = 0;
+        do {
+            const bool take = base + slot < ntake;
+            double4 b = make_double4(0.0, 0.0, 0.0, 0.0), c = b;
+            double f1 = 0.0, D = 1.0, o = 1.0, r = 0.0;
+            if (take) {
+                const double4* p = v.rec + 3 * (size_t)(S.z + base + slot);
+                f1 = reinterpret_cast<const double*>(p)[k];
+                b = p[1];
+                c = p[2];
+            }
+            if (base == 0 && lane < 4) {
+                D = v.diag[it];
+                o = reinterpret_cast<const double*>(&v.qold[it])[lane];
+                if (pass == 0) r = reinterpret_cast<const double*>(&v.res[it])[lane];
+            }
+            const int code = take ? ((int)__double_as_longlong(c.z) << 1) | pass : -1;
+            // the entry's stage is free once the sweep warp has read it
+            if (!mbar_wait(&R.empty[pos.stage], pos.phase ^ 1, &R.abort, ring_limit(v.wait_cycles))) {
+                if (!*(volatile int*)&R.abort) set_err(v.err, UNS_ERR_TIMEOUT, -1);
+                *(volatile int*)&R.abort = 1;
+                return;
+            }
+            double(*f)[32] = R.f[pos.stage];
+            f[SF_F1][lane] = f1;
+            f[SF_NX][lane] = b.x; f[SF_NY][lane] = b.y; f[SF_DS][lane] = b.z; f[SF_OL][lane] = b.w;
+            f[SF_CODE][lane] = __longlong_as_double(((long long)(c.y < 0.0 ? 0x80000000u : 0u) << 32) | (unsigned)code);
+            if (base == 0) {
+                f[SF_D2][lane] = D + D;
+                f[SF_O][lane] = o;
+                if (lane == 0) R.item[pos.stage] = S;
+            }
+            bool ok = true;
+            SweepNb w = {};
+            if (code != last && take) ok = poll_neighbour(v, (size_t)pass * n + (code >> 1), k, w);
+            if (base == 0 && pass == 1 && lane < 4 && (it << 1) != last)  // own forward dqc
+                ok = poll_value(reinterpret_cast<const double*>(v.rec_b + it) + lane, r, v.err, v.wait_cycles) && ok;
+            f[SF_U][lane] = w.u; f[SF_V][lane] = w.v; f[SF_P][lane] = w.p; f[SF_ET][lane] = w.et;
+            f[SF_RHO][lane] = w.rho; f[SF_DQ][lane] = w.dq;
+            if (base == 0) f[SF_R][lane] = pass == 0 ? r + r : r;
+            if (__any_sync(0xffffffffu, !ok)) {  // a wait gave up; the error is recorded
+                *(volatile int*)&R.abort = 1;
+                return;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&R.full[pos.stage]);
+            pos.next();
+            base += 8;
+        } while (base < ntake);
+        last = (it << 1) | pass;
+        if (last == v.skip_code) last = -1;  // test hook: that item hands nothing on
+        S = Sn;
+    }
+}
+
+// lusgs sweeps (lusgs.f90:48-124) as one cooperative launch.  Each sweep warp
+// runs its own list of items (node, pass) from the host-side list schedule, in
+// order, on what its feeder has put into the ring (uns_sweep.cuh).  Per item,
+// for each edge whose neighbour precedes the node in this pass (reference v2f
+// order): the neighbour's values come from registers when the warp itself
+// computed that neighbour last, else from the ring; the edge term
+// sign*(F(qc) - F(qold)) - omega*la*dqc is formed per component, lanes 0..3
+// add the terms in edge order (the reference's summation order) and divide by
+// the diagonal; the new state is spread to all lanes, which keep its
+// primitives for the next item while lanes 0..2 publish the record.
+// Every rounded operation and its operand order is the reference's, but for
+// its factor 0.5 on the terms, which doubles res and the diagonal instead
+// (a scaling by two commutes with every rounding short of the subnormal
+// range).
+//
+// The FP64 unit takes one instruction of the warp per 64 cycles whatever its
+// lanes, so sums and products are register FMAs, and the two divisions (590
+// cycles each there) run on the integer pipe (240).  %PERF%
+__global__ void __launch_bounds__(kSweepBlock, 1) k_nc_lusgs(NCView v, const int* __restrict__ woff) {
+    extern __shared__ __align__(16) unsigned char sweep_smem[];
+    RingNC* rings = reinterpret_cast<RingNC*>(sweep_smem);
+    __shared__ __align__(16) double wxs[kSweepPairs][32];  // per-warp exchange of lane values
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wib = (threadIdx.x >> 5) & (kSweepPairs - 1);
+    const bool feeder = threadIdx.x >= 32 * kSweepPairs;
+    if (stopped(v)) return;
+    if (threadIdx.x < kSweepPairs) ring_init(rings[threadIdx.x]);
+    __syncthreads();
+    const int gw = blockIdx.x * kSweepPairs + wib;
     const int kbeg = woff[gw], kend = woff[gw + 1];
     if (kbeg >= kend) return;
-    const int4 none = make_int4(0, 0, 0, 0);
-    int4 S = v.sched[kbeg];
-    int4 Sn = kbeg + 1 < kend ? v.sched[kbeg + 1] : none;
-    SweepIn X = {}, Xn = {};
-    sweep_load(v, S, lane, X);
-    int last = -1;  // code of the warp's previous item; its values below, in every lane
-    double Lrho = 0.0, Lu = 0.0, Lv = 0.0, Lp = 0.0, Le = 0.0, L0 = 0.0, L1 = 0.0, L2 = 0.0, L3 = 0.0;
-    // early read of the current item's first-round neighbour record, issued
-    // during the previous item (usually already published)
-    double Sw[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, Srho = 0.0;
-    bool spec = false;
+    RingNC& R = rings[wib];
+    if (feeder) {
+        nc_feed(v, R, kbeg, kend, lane);
+        return;
+    }
+    double* wx = wxs[wib];
+    const int k = lane & 3;
+    const int n = v.nop;
+    const double gm1 = in_register(v.g.gamma - 1.0);
+    RingPos pos;
+    int last = -1;  // code of the warp's previous item; its values in L, in every lane
+    SweepNb L = {};
     for (int kk = kbeg; kk < kend; ++kk) {
-        const int4 Snn = kk + 2 < kend ? v.sched[kk + 2] : none;
-        const int it = S.x, pass = S.y, ntake = S.w;
         double cres = 0.0;  // lanes 0..3: sum over edges of component k
-        for (int base = 0; base < ntake; base += 8) {
-            SweepIn E = X;
-            if (base > 0 && base + slot < ntake) sweep_load_edge(v, S.z + base + slot, k, E);
-            bool ok = true;
-            double t = 0.0;
-            if (base + slot < ntake) {
-                double w[8], rho;
-                if (((E.nb << 1) | pass) == last) {
-                    w[0] = Lu; w[1] = Lv; w[2] = Lp; w[3] = Le; w[4] = L0; w[5] = L1; w[6] = L2; w[7] = L3;
-                    rho = Lrho;
-                } else if (base == 0 && spec && record_set(Sw, Srho)) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) w[j] = Sw[j];
-                    rho = Srho;
-                } else {
-                    ok = poll_neighbour(v, (size_t)pass * n + E.nb, w, rho);
-                }
-                // normalflux (lusgs.f90:144-150) component k, then the edge term
-                const double u = w[0], vv = w[1], p = w[2], et = w[3];
-                const double un = u * E.nx + vv * E.ny;
-                const double o1 = rho * un;
-                const double prod = (k == 0 ? et + p : o1) * (k == 0 ? un : (k == 2 ? u : vv));
-                const double pn = p * (k == 2 ? E.nx : E.ny);
-                double o = k == 1 ? o1 : (k == 0 ? prod : prod + pn);
-                o = o * E.ds;
-                const double diff = o - E.f1;
-                const double dqk = pick4(k, w[4], w[5], w[6], w[7]);
-                t = 0.5 * ((__double_as_longlong(E.sgn) < 0 ? -diff : diff) - E.ol * dqk);
+        double D2 = 2.0, xo = 1.0, xr = 0.0;
+        unsigned Y = 0;  // the diagonal's reciprocal digits, off the chain
+        int it = 0, pass = 0, ntake = 0, base = 0;
+        do {
+            if (!mbar_wait(&R.full[pos.stage], pos.phase, &R.abort, ring_limit(v.wait_cycles))) {
+                if (!*(volatile int*)&R.abort) set_err(v.err, UNS_ERR_TIMEOUT, -1);
+                *(volatile int*)&R.abort = 1;
+                return;
             }
-            if (__ballot_sync(full, !ok)) return;  // a wait gave up; the error is recorded
+            const double(*f)[32] = R.f[pos.stage];
+            if (base == 0) {
+                const int4 S = R.item[pos.stage];
+                it = S.x; pass = S.y; ntake = S.w;
+                D2 = f[SF_D2][lane]; xo = f[SF_O][lane]; xr = f[SF_R][lane];
+                Y = div_recip(D2);
+            }
+            const long long cs = __double_as_longlong(f[SF_CODE][lane]);
+            const double f1 = f[SF_F1][lane], nx = f[SF_NX][lane], ny = f[SF_NY][lane], ds = f[SF_DS][lane], ol = f[SF_OL][lane];
+            SweepNb w;
+            w.u = f[SF_U][lane]; w.v = f[SF_V][lane]; w.p = f[SF_P][lane]; w.et = f[SF_ET][lane];
+            w.rho = f[SF_RHO][lane]; w.dq = f[SF_DQ][lane];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&R.empty[pos.stage]);
+            pos.next();
+            if (ntake == 0) break;
+            const int code = (int)cs;
+            if (code == last && code >= 0) w = L;
+            // normalflux (lusgs.f90:144-150) component k, then the edge term;
+            // idle slots compute on zeros
+            const double un = add64(mul64(w.u, nx), mul64(w.v, ny));
+            const double o1 = mul64(w.rho, un);
+            const double h = add64(w.et, w.p);
+            const double prod = mul64(k == 0 ? h : o1, k == 0 ? un : (k == 2 ? w.u : w.v));
+            const double sum = add64(prod, mul64(w.p, k == 2 ? nx : ny));
+            const double o = mul64(k == 1 ? o1 : (k == 0 ? prod : sum), ds);
+            const double diff = sub64(o, f1);
+            const double t = sub64(flip64(diff, cs < 0), mul64(ol, w.dq));
             // the terms in edge order, from 0.0 (the first addition is exact)
             const int nr = min(8, ntake - base);
             wx[lane] = t;
             __syncwarp();
             int e = 0;
             if (base == 0) { cres = zero_plus(wx[k]); e = 1; }
-            for (; e < nr; ++e) cres = cres + wx[4 * e + k];
+            for (; e < nr; ++e) cres = add64(cres, wx[4 * e + k]);
             __syncwarp();
-        }
-        // next item's inputs (independent of the sweep), issued once this
-        // item's polls are done so they do not queue ahead of them
-        if (kk + 1 < kend) sweep_load(v, Sn, lane, Xn);
-        double r = X.r;
-        bool ok = true;
-        if (pass == 1 && lane < 4) {  // own forward dqc
-            if ((it << 1) == last) r = pick4(lane, L0, L1, L2, L3);
-            else if (is_unset(r)) ok = poll_value(reinterpret_cast<const double*>(v.rec_b + it) + lane, r, v.err, v.wait_cycles);
-        }
-        if (__ballot_sync(full, !ok)) return;
+            base += 8;
+        } while (base < ntake);
         // dqc and qc = qold + dqc (lusgs.f90:78-81 / 117-120), component k in lane k
-        const double d = pass == 0 ? (-r - cres) / X.D : r - cres / X.D;
-        const double q = X.o + d;
-        // the next item's first-round neighbour records, while this item finishes
-        spec = false;
-        if (kk + 1 < kend && slot < Sn.w && ((Xn.nb << 1) | Sn.y) != ((it << 1) | pass)) {
-            peek_neighbour(v, (size_t)Sn.y * n + Xn.nb, Sw, Srho);
-            spec = true;
+        double d;
+        if (pass == 0) {
+            d = div_digits(sub64(neg64(xr), cres), D2, Y);
+        } else {  // from the node's own forward dqc
+            const double r = (it << 1) == last ? L.dq : xr;
+            d = sub64(r, div_digits(cres, D2, Y));
         }
+        const double q = add64(xo, d);
         // con2prim (All_modules.f90:146-169): rho = q1, then E/rho, rhou/rho,
         // rhov/rho in lanes 0, 2, 3
         if (lane < 4) { wx[lane] = q; wx[4 + lane] = d; }
         __syncwarp();
         const double2 qa = reinterpret_cast<const double2*>(wx)[0], qb = reinterpret_cast<const double2*>(wx)[1];
-        const double E0 = qa.x, rho = qa.y, Q2 = qb.x, Q3 = qb.y;
-        const double quo = q / rho;
+        const double E1 = qa.x, rho = qa.y, Q2 = qb.x, Q3 = qb.y;
+        const double quo = div_digits(q, rho);
         // the four products of the pressure and the record as one
         // multiplication: lane 0 e*rho, lane 1 0.5*rho, lane 2 u*u, lane 3 v*v
-        // (an FP64 instruction costs the warp the same for one lane or four)
         const double ma = lane == 1 ? 0.5 : quo, mb = lane < 2 ? rho : quo;
-        const double pr = ma * mb;
+        const double pr = mul64(ma, mb);
         if (lane < 4) { wx[8 + lane] = quo; wx[12 + lane] = pr; }
         __syncwarp();
-        const double2 da = reinterpret_cast<const double2*>(wx)[2], db = reinterpret_cast<const double2*>(wx)[3];
         const double2 pa = reinterpret_cast<const double2*>(wx)[6], pb = reinterpret_cast<const double2*>(wx)[7];
-        const double u = wx[10], vv = wx[11];
-        L0 = da.x; L1 = da.y; L2 = db.x; L3 = db.y;
+        const double uu = wx[10], vv = wx[11], dk = wx[4 + k];
+        const double2 da = reinterpret_cast<const double2*>(wx)[2], db = reinterpret_cast<const double2*>(wx)[3];
         __syncwarp();
-        const double qq = pb.x + pb.y;                // u*u + v*v
-        const double p = gm1 * (E0 - pa.y * qq);      // gm1*(E - 0.5*rho*qq)
-        Lrho = rho; Lu = u; Lv = vv; Lp = p; Le = pa.x;
+        const double qq = add64(pb.x, pb.y);                       // u*u + v*v
+        const double p = mul64(gm1, sub64(E1, mul64(pa.y, qq)));   // gm1*(E - 0.5*rho*qq)
+        L.u = uu; L.v = vv; L.p = p; L.et = pa.x; L.rho = rho; L.dq = dk;
         last = (it << 1) | pass;
         const size_t slotr = (size_t)pass * n + it;
-        if (last == v.skip_code) {  // test hook: this item publishes nothing and hands nothing on
-            last = -1;
+        if (last == v.skip_code) {
+            last = -1;  // test hook: this item publishes nothing and hands nothing on
         } else {
             // Lane 0 stores (u, v, p, e*rho), lane 1 dqc, lane 2 rho, as
             // predicated stores of one instruction sequence: lane-divergent
             // branches here cost the critical path more than the stores
             // (sweeps 11.07 -> 10.39 ms at 1024x512, measured).
             double2* dst = reinterpret_cast<double2*>(lane == 0 ? v.rec_a + slotr : v.rec_b + slotr);
-            const double x0 = lane == 0 ? Lu : L0, x1 = lane == 0 ? Lv : L1;
-            const double x2 = lane == 0 ? Lp : L2, x3 = lane == 0 ? Le : L3;
+            const double x0 = lane == 0 ? uu : da.x, x1 = lane == 0 ? vv : da.y;
+            const double x2 = lane == 0 ? p : db.x, x3 = lane == 0 ? pa.x : db.y;
             const int st_ab = lane < 2, st_r = lane == 2;
             asm volatile(
                 "{\n\t.reg .pred pa, pr;\n\t"
@@ -949,11 +981,8 @@ __global__ void __launch_bounds__(kSweepBlock, 1) k_nc_lusgs(NCView v, const int
                 : "r"(st_ab), "r"(st_r), "l"(dst), "d"(x0), "d"(x1), "l"(dst + 1), "d"(x2), "d"(x3), "l"(v.rec_r + slotr),
                   "d"(rho)
                 : "memory");
-            if (pass == 1 && lane == 2) v.qc[it] = make_double4(E0, rho, Q2, Q3);
+            if (pass == 1 && lane == 2) v.qc[it] = make_double4(E1, rho, Q2, Q3);
         }
-        S = Sn;
-        Sn = Snn;
-        X = Xn;
     }
 }
 
@@ -964,104 +993,160 @@ __global__ void __launch_bounds__(kSweepBlock, 1) k_nc_lusgs(NCView v, const int
 // FP32 error is relative to the change itself; items publish dqc only (FP32
 // for the edge terms, FP64 for the node's own backward step) and form no
 // primitives.
-struct SweepInM {
-    float rho, ru, rv, E, u, v, p, un, nx, ny, ds, ol, sign;  // the slot's record
-    int nb;
-    double D, o, r;  // lanes 0..3: the reciprocal of the node's diagonal, qold and res, variable k
+struct SweepRecM {
+    float rho, ru, rv, E, u, v, p, un, nx, ny;  // the slot's record, as dflux_k reads it
 };
 
-__device__ __forceinline__ void sweep_load_edge_m(const NCView& v, int rec, SweepInM& x) {
-    const float4* p = reinterpret_cast<const float4*>(v.rec) + 4 * (size_t)rec;
-    float4 a = p[0], b = p[1], c = p[2], d = p[3];
-    x.rho = a.x; x.ru = a.y; x.rv = a.z; x.E = a.w;
-    x.u = b.x; x.v = b.y; x.p = b.z; x.un = b.w;
-    x.nx = c.x; x.ny = c.y; x.ds = c.z; x.ol = c.w;
-    x.sign = d.x; x.nb = __float_as_int(d.y);
-}
+// Fields of a ring entry of the mixed form: two floats to a field.
+enum { MF_R01, MF_R23, MF_UV, MF_PUN, MF_N, MF_DSOL, MF_DQ01, MF_DQ23, MF_D, MF_O, MF_R, MF_CODE, MF_COUNT };
+typedef SweepRing<MF_COUNT> RingNCM;
 
-__device__ __forceinline__ void sweep_load_m(const NCView& v, const int4& S, int lane, SweepInM& x) {
-    if ((lane >> 2) < S.w) sweep_load_edge_m(v, S.z + (lane >> 2), x);
-    own_load(v, S, lane, x.D, x.o, x.r);
-    if (lane < 4) x.D = v.diaginv[S.x];  // the FP32 sweep multiplies by the FP64 reciprocal
+__device__ __forceinline__ double pack2(float a, float b) {
+    return dmake(__float_as_uint(b), __float_as_uint(a));
 }
+__device__ __forceinline__ float low_f(double x) { return __uint_as_float(dlo(x)); }
+__device__ __forceinline__ float high_f(double x) { return __uint_as_float(dhi(x)); }
 
-// lusgs sweeps in the mixed form: the schedule, lanes, hand-offs and FP64
-// sums / diagonal division of k_nc_lusgs; FP32 delta-form edge terms.
-__global__ void __launch_bounds__(kSweepBlock, 1) k_nc_lusgs_mixed(NCView v, const int* __restrict__ woff) {
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int gw = blockIdx.x * (kSweepBlock / 32) + wib;
-    const int slot = lane >> 2, k = lane & 3;
-    if (stopped(v)) return;
+__device__ void nc_feed_mixed(const NCView& v, RingNCM& R, int kbeg, int kend, int lane) {
+    const int slot = lane >> 2;
     const int n = v.nop;
-    const float gm1 = (float)(v.g.gamma - 1.0);
     const float4* recf = reinterpret_cast<const float4*>(v.rec_a);
+    RingPos pos;
+    int last = -1;
+    int4 S = v.sched[kbeg];
+    for (int kk = kbeg; kk < kend; ++kk) {
+        const int4 Sn = kk + 1 < kend ? v.sched[kk + 1] : make_int4(0, 0, 0, 0);
+        const int it = S.x, pass = S.y, ntake = S.w;
+        int base = 0;
+        do {
+            const bool take = base + slot < ntake;
+            float4 a = make_float4(1.f, 0.f, 0.f, 0.f), b = make_float4(0.f, 0.f, 0.f, 0.f), c = b, d = b;
+            double D = 1.0, o = 1.0, r = 0.0;
+            if (take) {
+                const float4* p = reinterpret_cast<const float4*>(v.rec) + 4 * (size_t)(S.z + base + slot);
+                a = p[0]; b = p[1]; c = p[2]; d = p[3];
+            }
+            if (base == 0 && lane < 4) {
+                D = v.diaginv[it];  // the FP32 sweep multiplies by the FP64 reciprocal
+                o = reinterpret_cast<const double*>(&v.qold[it])[lane];
+                if (pass == 0) r = reinterpret_cast<const double*>(&v.res[it])[lane];
+            }
+            const int code = take ? (__float_as_int(d.y) << 1) | pass : -1;
+            if (!mbar_wait(&R.empty[pos.stage], pos.phase ^ 1, &R.abort, ring_limit(v.wait_cycles))) {
+                if (!*(volatile int*)&R.abort) set_err(v.err, UNS_ERR_TIMEOUT, -1);
+                *(volatile int*)&R.abort = 1;
+                return;
+            }
+            double(*f)[32] = R.f[pos.stage];
+            f[MF_R01][lane] = pack2(a.x, a.y); f[MF_R23][lane] = pack2(a.z, a.w);
+            f[MF_UV][lane] = pack2(b.x, b.y); f[MF_PUN][lane] = pack2(b.z, b.w);
+            f[MF_N][lane] = pack2(c.x, c.y); f[MF_DSOL][lane] = pack2(c.z, c.w);
+            f[MF_CODE][lane] = dmake(d.x < 0.f ? 0x80000000u : 0u, (unsigned)code);
+            if (base == 0) {
+                f[MF_D][lane] = D;
+                f[MF_O][lane] = o;
+                if (lane == 0) R.item[pos.stage] = S;
+            }
+            bool ok = true;
+            float dq[4] = {0.f, 0.f, 0.f, 0.f};
+            if (code != last && take) ok = poll_f4(recf + (size_t)pass * n + (code >> 1), dq, v.err, v.wait_cycles);
+            if (base == 0 && pass == 1 && lane < 4 && (it << 1) != last)  // own forward dqc
+                ok = poll_value(reinterpret_cast<const double*>(v.rec_b + it) + lane, r, v.err, v.wait_cycles) && ok;
+            f[MF_DQ01][lane] = pack2(dq[0], dq[1]);
+            f[MF_DQ23][lane] = pack2(dq[2], dq[3]);
+            if (base == 0) f[MF_R][lane] = r;
+            if (__any_sync(0xffffffffu, !ok)) {
+                *(volatile int*)&R.abort = 1;
+                return;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&R.full[pos.stage]);
+            pos.next();
+            base += 8;
+        } while (base < ntake);
+        last = (it << 1) | pass;
+        if (last == v.skip_code) last = -1;
+        S = Sn;
+    }
+}
+
+// lusgs sweeps in the mixed form: the schedule, lanes, ring and FP64 sums of
+// k_nc_lusgs; FP32 delta-form edge terms.  %PERFM%
+__global__ void __launch_bounds__(kSweepBlock, 1) k_nc_lusgs_mixed(NCView v, const int* __restrict__ woff) {
+    extern __shared__ __align__(16) unsigned char sweep_smem[];
+    RingNCM* rings = reinterpret_cast<RingNCM*>(sweep_smem);
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wib = (threadIdx.x >> 5) & (kSweepPairs - 1);
+    const bool feeder = threadIdx.x >= 32 * kSweepPairs;
+    if (stopped(v)) return;
+    if (threadIdx.x < kSweepPairs) ring_init(rings[threadIdx.x]);
+    __syncthreads();
+    const int gw = blockIdx.x * kSweepPairs + wib;
     const int kbeg = woff[gw], kend = woff[gw + 1];
     if (kbeg >= kend) return;
-    const int4 none = make_int4(0, 0, 0, 0);
-    int4 S = v.sched[kbeg];
-    int4 Sn = kbeg + 1 < kend ? v.sched[kbeg + 1] : none;
-    SweepInM X = {}, Xn = {};
-    sweep_load_m(v, S, lane, X);
+    RingNCM& R = rings[wib];
+    if (feeder) {
+        nc_feed_mixed(v, R, kbeg, kend, lane);
+        return;
+    }
+    const int k = lane & 3;
+    const int n = v.nop;
+    const float gm1 = (float)(v.g.gamma - 1.0);
+    RingPos pos;
     int last = -1;
     float LF[4] = {0.f, 0.f, 0.f, 0.f};             // previous item's dqc (FP32)
-    double L0 = 0.0, L1 = 0.0, L2 = 0.0, L3 = 0.0;  // and in FP64
-    float Sf[4] = {0.f, 0.f, 0.f, 0.f};
-    bool spec = false;
+    double Lk = 0.0;                                // and in FP64, component k
     for (int kk = kbeg; kk < kend; ++kk) {
-        const int4 Snn = kk + 2 < kend ? v.sched[kk + 2] : none;
-        const int it = S.x, pass = S.y, ntake = S.w;
-        double cres = 0.0;
-        for (int base = 0; base < ntake; base += 8) {
-            SweepInM E = X;
-            if (base > 0 && base + slot < ntake) sweep_load_edge_m(v, S.z + base + slot, E);
-            bool ok = true;
-            double t = 0.0;
-            if (base + slot < ntake) {
-                float dq[4];
-                if (((E.nb << 1) | pass) == last) {
-                    dq[0] = LF[0]; dq[1] = LF[1]; dq[2] = LF[2]; dq[3] = LF[3];
-                } else if (base == 0 && spec && set_f4(Sf)) {
-                    dq[0] = Sf[0]; dq[1] = Sf[1]; dq[2] = Sf[2]; dq[3] = Sf[3];
-                } else {
-                    ok = poll_f4(recf + (size_t)pass * n + E.nb, dq, v.err, v.wait_cycles);
-                }
-                const float df = dflux_k(E, gm1, dq, k);
-                const float dqk = k == 0 ? dq[0] : (k == 1 ? dq[1] : (k == 2 ? dq[2] : dq[3]));
-                t = (double)(0.5f * ((E.sign < 0.f ? -df : df) * E.ds - E.ol * dqk));
+        double cres = 0.0, xd = 1.0, xo = 1.0, xr = 0.0;
+        int it = 0, pass = 0, ntake = 0, base = 0;
+        do {
+            if (!mbar_wait(&R.full[pos.stage], pos.phase, &R.abort, ring_limit(v.wait_cycles))) {
+                if (!*(volatile int*)&R.abort) set_err(v.err, UNS_ERR_TIMEOUT, -1);
+                *(volatile int*)&R.abort = 1;
+                return;
             }
-            if (__ballot_sync(full, !ok)) return;
+            const double(*f)[32] = R.f[pos.stage];
+            if (base == 0) {
+                const int4 S = R.item[pos.stage];
+                it = S.x; pass = S.y; ntake = S.w;
+                xd = f[MF_D][lane]; xo = f[MF_O][lane]; xr = f[MF_R][lane];
+            }
+            const double r01 = f[MF_R01][lane], r23 = f[MF_R23][lane], uv = f[MF_UV][lane], pun = f[MF_PUN][lane];
+            const double nn = f[MF_N][lane], dsol = f[MF_DSOL][lane], q01 = f[MF_DQ01][lane], q23 = f[MF_DQ23][lane];
+            const long long cs = __double_as_longlong(f[MF_CODE][lane]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&R.empty[pos.stage]);
+            pos.next();
+            if (ntake == 0) break;
+            const bool mine = (int)cs == last && (int)cs >= 0;
+            const float dq[4] = {mine ? LF[0] : low_f(q01), mine ? LF[1] : high_f(q01), mine ? LF[2] : low_f(q23),
+                                 mine ? LF[3] : high_f(q23)};
+            const SweepRecM E = {low_f(r01), high_f(r01), low_f(r23), high_f(r23), low_f(uv), high_f(uv),
+                                 low_f(pun), high_f(pun), low_f(nn), high_f(nn)};
+            const float df = dflux_k(E, gm1, dq, k);
+            const float dqk = k == 0 ? dq[0] : (k == 1 ? dq[1] : (k == 2 ? dq[2] : dq[3]));
+            const double t = widen(0.5f * ((cs < 0 ? -df : df) * low_f(dsol) - high_f(dsol) * dqk));
             const int nr = min(8, ntake - base);
             int e = 0;
             if (base == 0) { cres = zero_plus(__shfl_sync(full, t, k)); e = 1; }  // 0.0 + t0, exact
-            for (; e < nr; ++e) cres = cres + __shfl_sync(full, t, 4 * e + k);
+            for (; e < nr; ++e) cres = add64(cres, __shfl_sync(full, t, 4 * e + k));
+            base += 8;
+        } while (base < ntake);
+        double d;
+        if (pass == 0) {
+            d = mul64(sub64(neg64(xr), cres), xd);
+        } else {  // from the node's own forward dqc
+            const double r = (it << 1) == last ? Lk : xr;
+            d = sub64(r, mul64(cres, xd));
         }
-        if (kk + 1 < kend) sweep_load_m(v, Sn, lane, Xn);
-        double r = X.r;
-        bool ok = true;
-        if (pass == 1 && lane < 4) {  // own forward dqc
-            if ((it << 1) == last) r = pick4(lane, L0, L1, L2, L3);
-            else ok = poll_value(reinterpret_cast<const double*>(v.rec_b + it) + lane, r, v.err, v.wait_cycles);
-        }
-        if (__ballot_sync(full, !ok)) return;
-        const double d = pass == 0 ? (-r - cres) * X.D : r - cres * X.D;
-        const double q = X.o + d;
-        spec = false;
-        if (kk + 1 < kend && slot < Sn.w && ((Xn.nb << 1) | Sn.y) != ((it << 1) | pass)) {
-            peek_f4(recf + (size_t)Sn.y * n + Xn.nb, Sf);
-            spec = true;
-        }
-        const float df = (float)d;
+        const float df = narrow(d);
         LF[0] = __shfl_sync(full, df, 0);
         LF[1] = __shfl_sync(full, df, 1);
         LF[2] = __shfl_sync(full, df, 2);
         LF[3] = __shfl_sync(full, df, 3);
-        L0 = __shfl_sync(full, d, 0);
-        L1 = __shfl_sync(full, d, 1);
-        L2 = __shfl_sync(full, d, 2);
-        L3 = __shfl_sync(full, d, 3);
-        const double Q0 = __shfl_sync(full, q, 0), Q1 = __shfl_sync(full, q, 1), Q2 = __shfl_sync(full, q, 2),
-                     Q3 = __shfl_sync(full, q, 3);
+        const double L0 = __shfl_sync(full, d, 0), L1 = __shfl_sync(full, d, 1), L2 = __shfl_sync(full, d, 2),
+                     L3 = __shfl_sync(full, d, 3);
+        Lk = pick4(k, L0, L1, L2, L3);
         last = (it << 1) | pass;
         const size_t slotr = (size_t)pass * n + it;
         if (last == v.skip_code) {  // test hook: this item publishes nothing and hands nothing on
@@ -1069,11 +1154,8 @@ __global__ void __launch_bounds__(kSweepBlock, 1) k_nc_lusgs_mixed(NCView v, con
         } else {
             publish_mixed(lane, reinterpret_cast<float4*>(v.rec_a) + slotr, reinterpret_cast<double2*>(v.rec_b + slotr), LF,
                           L0, L1, L2, L3);
-            if (pass == 1 && lane == 2) v.qc[it] = make_double4(Q0, Q1, Q2, Q3);
+            if (pass == 1 && lane < 4) reinterpret_cast<double*>(&v.qc[it])[lane] = add64(xo, d);
         }
-        S = Sn;
-        Sn = Snn;
-        X = Xn;
     }
 }
 
@@ -1240,6 +1322,7 @@ int launch_sweeps_nc(uns_nc_handle* h, NCView& v) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(h->coop_blocks);
     cfg.blockDim = dim3(kSweepBlock);
+    cfg.dynamicSmemBytes = kSweepPairs * (mixed ? sizeof(RingNCM) : sizeof(RingNC));
     cfg.stream = h->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -1402,7 +1485,7 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
         if (nop >= (1 << 30)) { set_last_error("uns_nc_create: too many nodes"); return fail(UNS_ERR_MESH); }
         int dev = 0, nsm = 0, per = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_nc_lusgs, kSweepBlock, 0) != cudaSuccess || per < 1) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_nc_lusgs, kSweepBlock, kSweepPairs * sizeof(RingNC)) != cudaSuccess || per < 1) {
             set_last_error("uns_nc_create: cannot size the cooperative LU-SGS launch");
             return fail(UNS_ERR_CUDA);
         }
@@ -1420,7 +1503,7 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
                 int sg;
                 nbr[k] = other(i, m->v2f[k], &sg);
             }
-        WarpSchedule ws = list_schedule(nop, m->v2f_off, nbr.data(), h->coop_blocks * (kSweepBlock / 32));
+        WarpSchedule ws = list_schedule(nop, m->v2f_off, nbr.data(), h->coop_blocks * kSweepPairs);
         h->lev_fwd = ws.nlev_fwd;
         h->lev_bwd = ws.nlev_bwd;
         std::vector<int4> sched(ws.items.size());

@@ -35,6 +35,7 @@
 #include "uns_common.cuh"
 #include "uns_phys.cuh"
 #include "uns_sched.hpp"
+#include "uns_sweep.cuh"
 #include "unsflow_gpu.h"
 
 using namespace uns;
@@ -1444,40 +1445,15 @@ __global__ void k_unpack_f32(CCView v) {
     v.phi[i] = make_double4(c.x, c.y, c.z, c.w);
 }
 
-// lusgs2 sweep pieces (lusgs.F90:245-318).  The per-cell neighbour sum keeps
-// the reference c2f order, so the result equals the sequential sweep.
-__device__ __forceinline__ void normal_flux_d(const Gas& g, const double4& qo, const double4& dq, double nx, double ny,
-                                              double area, double out[4]) {
-    Prim P = con2prim(g, qo.x, qo.y, qo.z, qo.w);
-    double et = P.e * P.rho;
-    double un = P.u * nx + P.v * ny;
-    double f1[4] = {(et + P.p) * un, P.rho * un, 0.0, 0.0};
-    f1[2] = f1[1] * P.u + P.p * nx;
-    f1[3] = f1[1] * P.v + P.p * ny;
-    Prim Q = con2prim(g, qo.x + dq.x, qo.y + dq.y, qo.z + dq.z, qo.w + dq.w);
-    et = Q.e * Q.rho;
-    un = Q.u * nx + Q.v * ny;
-    double f2[4] = {(et + Q.p) * un, Q.rho * un, 0.0, 0.0};
-    f2[2] = f2[1] * Q.u + Q.p * nx;
-    f2[3] = f2[1] * Q.v + Q.p * ny;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) out[k] = area * (f2[k] - f1[k]);
-}
-
 // normal_flux pieces (lusgs.F90:328-359): the flux of a state along (nx, ny).
-__device__ __forceinline__ void nflux_prims(const double4& w, double et, double nx, double ny, double o[4]) {
-    double un = w.y * nx + w.z * ny;
-    o[0] = (et + w.w) * un;
-    o[1] = w.x * un;
-    o[2] = o[1] * w.y + w.w * nx;
-    o[3] = o[1] * w.z + w.w * ny;
+__device__ __forceinline__ void nflux_prims(const PrimT<F64I>& w, F64I nx, F64I ny, F64I o[4]) {
+    const F64I et = w.e * w.rho;
+    const F64I un = w.u * nx + w.v * ny;
+    o[0] = (et + w.p) * un;
+    o[1] = w.rho * un;
+    o[2] = o[1] * w.u + w.p * nx;
+    o[3] = o[1] * w.v + w.p * ny;
 }
-
-constexpr int kSweepBlock = 128;
-// One sweep block per SM: one warp per SM sub-partition, so concurrently
-// active items never share an FP64 unit.
-constexpr int kSweepBlocksPerSM = 1;
-constexpr double kOmega = 1.5;  // lusgs.F90:229
 
 // Per LU-SGS call: everything a sweep item needs from a face that does not
 // change during the sweeps, contiguous in schedule order:
@@ -1491,13 +1467,14 @@ __global__ void __launch_bounds__(kBlock) k_cc_sweep_prep(CCView v) {
     if (r >= v.nrec) return;
     const int c = v.rec_face[r], nb = v.rec_nb[r];
     const double2 n = v.fn[c];
-    const double nx = v.rec_flip[r] ? -n.x : n.x, ny = v.rec_flip[r] ? -n.y : n.y;
+    const bool flip = v.rec_flip[r] != 0;
+    const double nx = flip64(n.x, flip), ny = flip64(n.y, flip);
     const double4 q = v.qold[nb];
-    Prim P = con2prim(v.g, q.x, q.y, q.z, q.w);
-    double o[4];
-    nflux_prims(make_double4(P.rho, P.u, P.v, P.p), P.e * P.rho, nx, ny, o);
-    v.rec[3 * (size_t)r] = d4(o);
-    v.rec[3 * (size_t)r + 1] = make_double4(nx, ny, v.farea[c], kOmega * v.fla[c]);
+    const PrimT<F64I> P = con2prim_t<F64I>(v.g, q.x, q.y, q.z, q.w);
+    F64I o[4];
+    nflux_prims(P, nx, ny, o);
+    v.rec[3 * (size_t)r] = f4(o);
+    v.rec[3 * (size_t)r + 1] = make_double4(nx, ny, v.farea[c], (F64I(kOmega) * v.fla[c]).v);
     v.rec[3 * (size_t)r + 2] = make_double4(q.y, 0.0, __longlong_as_double((long long)nb), 0.0);
 }
 
@@ -1510,329 +1487,37 @@ __global__ void __launch_bounds__(kBlock) k_cc_sweep_prep_mixed(CCView v) {
     if (r >= v.nrec) return;
     const int c = v.rec_face[r], nb = v.rec_nb[r];
     const double2 n = v.fn[c];
-    const double nx = v.rec_flip[r] ? -n.x : n.x, ny = v.rec_flip[r] ? -n.y : n.y;
+    const bool flip = v.rec_flip[r] != 0;
+    const double nx = flip64(n.x, flip), ny = flip64(n.y, flip);
     const double4 q = v.qold[nb];
-    Prim P = con2prim(v.g, q.x, q.y, q.z, q.w);
+    const PrimT<F64I> P = con2prim_t<F64I>(v.g, q.x, q.y, q.z, q.w);
     float4* rf = reinterpret_cast<float4*>(v.rec) + 4 * (size_t)r;
     rf[0] = make_float4((float)q.y, (float)q.z, (float)q.w, (float)q.x);
     rf[1] = make_float4((float)P.u, (float)P.v, (float)P.p, (float)(P.u * nx + P.v * ny));
-    rf[2] = make_float4((float)nx, (float)ny, (float)v.farea[c], (float)(kOmega * v.fla[c]));
+    rf[2] = make_float4((float)nx, (float)ny, (float)v.farea[c], (float)(F64I(kOmega) * v.fla[c]));
     rf[3] = make_float4(1.f, __int_as_float(nb), 0.f, 0.f);
 }
 
-__device__ __forceinline__ double pick4(int k, double a, double b, double c, double d) {
-    return k == 0 ? a : (k == 1 ? b : (k == 2 ? c : d));
+SweepArgs sweep_args(const CCView& v, bool mixed) {
+    SweepArgs a;
+    a.n = v.noc; a.sched = v.sched; a.rec = v.rec;
+    a.diag = mixed ? v.diaginv : v.diag;
+    a.qold = v.qold; a.res = v.res; a.qc = v.qc;
+    a.out = v.srec; a.outf = reinterpret_cast<float4*>(v.srec);
+    a.outd = reinterpret_cast<double4*>(v.srec + 2 * (size_t)v.noc);
+    a.err = v.err; a.wait_cycles = v.wait_cycles; a.skip_code = v.skip_code;
+    a.gm1 = v.g.gamma - 1.0;
+    return a;
 }
 
-// Lanes of a sweep item: lane = 4 * slot + k, slot = the taken face (up to 8
-// per round), k = the variable.  An FP64 instruction costs its SM
-// sub-partition the same whatever the number of active lanes, so each item's
-// arithmetic is spread over the lanes: the four flux components of up to
-// eight faces in one pass, the per-variable sums and divides in lanes 0..3,
-// and the three divisions of con2prim in lanes 0, 2 and 3 at once.
-struct SweepIn {
-    double f1, nx, ny, area, ol, rho_old;  // the slot's record; f1 = component k
-    int nb;
-    double D, o, r;  // lanes 0..3: the cell's diagonal, qold and res, variable k
-};
-
-__device__ __forceinline__ void sweep_load_face(const CCView& v, int rec, int k, SweepIn& x) {
-    const double4* p = v.rec + 3 * (size_t)rec;
-    x.f1 = reinterpret_cast<const double*>(p)[k];
-    double4 b = p[1], c = p[2];
-    x.nx = b.x; x.ny = b.y; x.area = b.z; x.ol = b.w;
-    x.rho_old = c.x; x.nb = (int)__double_as_longlong(c.z);
+// The sweeps (uns_sweep.cuh) over the interior cells.
+__global__ void __launch_bounds__(kSweepBlock, 1) k_lusgs(SweepArgs a, const int* done, const int* __restrict__ woff) {
+    if (done && *((volatile const int*)done) != 0) return;
+    sweep_block<true, false>(a, woff);
 }
-
-// The cell's own diagonal, qold and res (variable `lane`) in lanes 0..3;
-// benign operands elsewhere, so the warp-wide divides meet no 0 or inf.
-__device__ __forceinline__ void own_load(const CCView& v, const int4& S, int lane, double& D, double& o, double& r) {
-    if (lane < 4) {
-        D = v.diag[S.x];
-        o = reinterpret_cast<const double*>(&v.qold[S.x])[lane];
-        if (S.y == 0) r = reinterpret_cast<const double*>(&v.res[S.x])[lane];
-    } else {
-        D = 1.0;
-        o = 1.0;
-        r = 0.0;
-    }
-}
-
-__device__ __forceinline__ void sweep_load(const CCView& v, const int4& S, int lane, SweepIn& x) {
-    if ((lane >> 2) < S.w) sweep_load_face(v, S.z + (lane >> 2), lane & 3, x);
-    own_load(v, S, lane, x.D, x.o, x.r);
-}
-
-// One unconditional read of a neighbour record, issued early; the values are
-// checked (record_set) only when the item that needs them starts.
-__device__ __forceinline__ void peek_neighbour(const CCView& v, size_t rs, double w[4], double dq[4]) {
-    const double2* pa = reinterpret_cast<const double2*>(v.rec_a + rs);
-    const double2* pb = reinterpret_cast<const double2*>(v.rec_b + rs);
-    double2 x0 = ld_relaxed2(pa), x1 = ld_relaxed2(pa + 1), x2 = ld_relaxed2(pb), x3 = ld_relaxed2(pb + 1);
-    w[0] = x0.x; w[1] = x0.y; w[2] = x1.x; w[3] = x1.y;
-    dq[0] = x2.x; dq[1] = x2.y; dq[2] = x3.x; dq[3] = x3.y;
-}
-
-__device__ __forceinline__ bool record_set(const double w[4], const double dq[4]) {
-    bool ready = true;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) ready = ready && !is_unset(w[j]) && !is_unset(dq[j]);
-    return ready;
-}
-
-// lusgs2 sweeps (lusgs.F90:245-318) as one cooperative launch.  Each warp runs
-// its own list of items (cell, pass) from the host-side list schedule, in
-// order, loading the next item's inputs while it works on the current one.
-// Per item, for each face whose neighbour precedes the cell in this pass
-// (reference c2f order): the neighbour's values come from registers when the
-// warp itself computed that neighbour last, else from its record (read early
-// or polled); the face term area*(F(qold+dq) - F(qold)) - omega*lam*dq is
-// formed per component; lanes 0..3 add the terms in c2f order and apply the
-// diagonal; the new values are spread to all lanes, which keep the
-// primitives of qold + dq for the next item while lanes 0 and 1 publish the
-// record.  Every operation and operand order is the reference's.
-__global__ void __launch_bounds__(kSweepBlock, 1) k_lusgs(CCView v, const int* __restrict__ woff) {
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int gw = blockIdx.x * (kSweepBlock / 32) + wib;
-    const int slot = lane >> 2, k = lane & 3;
-    if (stopped(v)) return;
-    const int n = v.noc;
-    const double gm1 = v.g.gamma - 1.0;
-    const int kbeg = woff[gw], kend = woff[gw + 1];
-    if (kbeg >= kend) return;
-    const int4 none = make_int4(0, 0, 0, 0);
-    int4 S = v.sched[kbeg];
-    int4 Sn = kbeg + 1 < kend ? v.sched[kbeg + 1] : none;
-    SweepIn X = {}, Xn = {};
-    sweep_load(v, S, lane, X);
-    int last = -1;  // code of the warp's previous item; its values below, in every lane
-    double Lrho = 0.0, Lu = 0.0, Lv = 0.0, Lp = 0.0, Le = 0.0, L0 = 0.0, L1 = 0.0, L2 = 0.0, L3 = 0.0;
-    // early read of the current item's first-round neighbour record, issued
-    // during the previous item (usually already published)
-    double Sw[4] = {0.0, 0.0, 0.0, 0.0}, Sdq[4] = {0.0, 0.0, 0.0, 0.0};
-    bool spec = false;
-    for (int kk = kbeg; kk < kend; ++kk) {
-        const int4 Snn = kk + 2 < kend ? v.sched[kk + 2] : none;
-        const int it = S.x, pass = S.y, ntake = S.w;
-        double cres = 0.0;  // lanes 0..3: sum over faces of component k
-        for (int base = 0; base < ntake; base += 8) {
-            SweepIn E = X;
-            if (base > 0 && base + slot < ntake) sweep_load_face(v, S.z + base + slot, k, E);
-            bool ok = true;
-            double t = 0.0;
-            if (base + slot < ntake) {
-                double w[8], rho;
-                if (((E.nb << 1) | pass) == last) {
-                    w[0] = Lu; w[1] = Lv; w[2] = Lp; w[3] = Le; w[4] = L0; w[5] = L1; w[6] = L2; w[7] = L3;
-                    rho = Lrho;
-                } else if (base == 0 && spec && record_set(Sw, Sdq)) {
-                    w[0] = Sw[0]; w[1] = Sw[1]; w[2] = Sw[2]; w[3] = Sw[3];
-                    w[4] = Sdq[0]; w[5] = Sdq[1]; w[6] = Sdq[2]; w[7] = Sdq[3];
-                    rho = E.rho_old + w[5];
-                } else {
-                    const size_t rs = (size_t)pass * n + E.nb;
-                    ok = poll_record2(v.rec_a + rs, v.rec_b + rs, w, v.err, v.wait_cycles);
-                    rho = E.rho_old + w[5];
-                }
-                // normal_flux (lusgs.F90:348-357) component k, then the face term
-                const double u = w[0], vv = w[1], p = w[2], et = w[3];
-                const double un = u * E.nx + vv * E.ny;
-                const double o1 = rho * un;
-                const double prod = (k == 0 ? et + p : o1) * (k == 0 ? un : (k == 2 ? u : vv));
-                const double pn = p * (k == 2 ? E.nx : E.ny);
-                const double o = k == 1 ? o1 : (k == 0 ? prod : prod + pn);
-                t = E.area * (o - E.f1) - E.ol * pick4(k, w[4], w[5], w[6], w[7]);
-            }
-            if (__ballot_sync(full, !ok)) return;  // a wait gave up; the error is recorded
-            const int nr = min(8, ntake - base);
-            int e = 0;
-            if (base == 0) { cres = zero_plus(__shfl_sync(full, t, k)); e = 1; }  // 0.0 + t0, exact
-            for (; e < nr; ++e) cres = cres + __shfl_sync(full, t, 4 * e + k);
-        }
-        // next item's inputs (independent of the sweep), issued once this
-        // item's polls are done so they do not queue ahead of them
-        if (kk + 1 < kend) sweep_load(v, Sn, lane, Xn);
-        double r = X.r;
-        bool ok = true;
-        if (pass == 1 && lane < 4) {  // own lower
-            if ((it << 1) == last) r = pick4(lane, L0, L1, L2, L3);
-            else ok = poll_value(reinterpret_cast<const double*>(v.rec_b + it) + lane, r, v.err, v.wait_cycles);
-        }
-        if (__ballot_sync(full, !ok)) return;
-        // lower / upper (lusgs.F90:276-279 / 314-317), component k in lane k
-        const double d = pass == 0 ? (-r - 0.5 * cres) / X.D : r - 0.5 * cres / X.D;
-        const double q = X.o + d;  // qold + dq (and, after the backward sweep, the new qc)
-        spec = false;
-        if (kk + 1 < kend && slot < Sn.w && ((Xn.nb << 1) | Sn.y) != ((it << 1) | pass)) {
-            peek_neighbour(v, (size_t)Sn.y * n + Xn.nb, Sw, Sdq);
-            spec = true;
-        }
-        // con2prim (pri.F90:13-37): rho = q1, then E/rho, rhou/rho, rhov/rho in lanes 0, 2, 3
-        const double rho = __shfl_sync(full, q, 1);
-        const double quo = q / rho;
-        const double E0 = __shfl_sync(full, q, 0), Q2 = __shfl_sync(full, q, 2), Q3 = __shfl_sync(full, q, 3);
-        // the four products of the pressure and the record as one
-        // multiplication: lane 0 e*rho, lane 1 0.5*rho, lane 2 u*u, lane 3 v*v
-        // (an FP64 instruction costs the warp the same for one lane or four)
-        const double ma = lane == 1 ? 0.5 : quo, mb = lane < 2 ? rho : quo;
-        const double pr = ma * mb;
-        const double u = __shfl_sync(full, quo, 2), vv = __shfl_sync(full, quo, 3);
-        const double erho = __shfl_sync(full, pr, 0), hrho = __shfl_sync(full, pr, 1);
-        const double qq = __shfl_sync(full, pr, 2) + __shfl_sync(full, pr, 3);  // u*u + v*v
-        const double p = gm1 * (E0 - hrho * qq);                                  // gm1*(E - 0.5*rho*qq)
-        L0 = __shfl_sync(full, d, 0);
-        L1 = __shfl_sync(full, d, 1);
-        L2 = __shfl_sync(full, d, 2);
-        L3 = __shfl_sync(full, d, 3);
-        Lrho = rho; Lu = u; Lv = vv; Lp = p; Le = erho;
-        last = (it << 1) | pass;
-        const size_t slotr = (size_t)pass * n + it;
-        if (last == v.skip_code) {  // test hook: this item publishes nothing and hands nothing on
-            last = -1;
-        } else {
-            // Lane 0 stores (u, v, p, e*rho), lane 1 dq, as predicated stores
-            // of one instruction sequence (lane-divergent branches around the
-            // stores cost the sweep's critical path more than the stores).
-            double2* dst = reinterpret_cast<double2*>(lane == 0 ? v.rec_a + slotr : v.rec_b + slotr);
-            const double x0 = lane == 0 ? Lu : L0, x1 = lane == 0 ? Lv : L1;
-            const double x2 = lane == 0 ? Lp : L2, x3 = lane == 0 ? Le : L3;
-            const int st_ab = lane < 2;
-            asm volatile(
-                "{\n\t.reg .pred pa;\n\t"
-                "setp.ne.s32 pa, %0, 0;\n\t"
-                "@pa st.relaxed.gpu.global.v2.f64 [%1], {%2, %3};\n\t"
-                "@pa st.relaxed.gpu.global.v2.f64 [%4], {%5, %6};\n\t}"
-                :
-                : "r"(st_ab), "l"(dst), "d"(x0), "d"(x1), "l"(dst + 1), "d"(x2), "d"(x3)
-                : "memory");
-            if (pass == 1 && lane == 2) v.qc[it] = make_double4(E0, rho, Q2, Q3);
-        }
-        S = Sn;
-        Sn = Snn;
-        X = Xn;
-    }
-}
-
-// ------------------------------------------------------------ mixed (delta form)
-// The FP32 sweep cannot form F(qold + dq) - F(qold) as a difference of two
-// O(1) fluxes: near convergence that difference drowns in FP32 rounding and
-// the solve stalls.  It forms the change directly from dq (dflux_k), so its
-// FP32 error is relative to the change itself; items publish dq only (FP32
-// for the face terms, FP64 for the cell's own backward step) and form no
-// primitives.
-struct SweepInM {
-    float rho, ru, rv, E, u, v, p, un, nx, ny, area, ol;  // the slot's record
-    int nb;
-    double D, o, r;  // lanes 0..3: the reciprocal of the cell's diagonal, qold and res, variable k
-};
-
-__device__ __forceinline__ void sweep_load_face_m(const CCView& v, int rec, SweepInM& x) {
-    const float4* p = reinterpret_cast<const float4*>(v.rec) + 4 * (size_t)rec;
-    float4 a = p[0], b = p[1], c = p[2], d = p[3];
-    x.rho = a.x; x.ru = a.y; x.rv = a.z; x.E = a.w;
-    x.u = b.x; x.v = b.y; x.p = b.z; x.un = b.w;
-    x.nx = c.x; x.ny = c.y; x.area = c.z; x.ol = c.w;
-    x.nb = __float_as_int(d.y);
-}
-
-__device__ __forceinline__ void sweep_load_m(const CCView& v, const int4& S, int lane, SweepInM& x) {
-    if ((lane >> 2) < S.w) sweep_load_face_m(v, S.z + (lane >> 2), x);
-    own_load(v, S, lane, x.D, x.o, x.r);
-    if (lane < 4) x.D = v.diaginv[S.x];  // the FP32 sweep multiplies by the FP64 reciprocal
-}
-
-// lusgs2 sweeps in the mixed form: the schedule, lanes, hand-offs and FP64
-// sums of k_lusgs, the diagonal as its FP64 reciprocal (formed with the
-// diagonal, off the sweep's critical path); FP32 delta-form face terms.
-__global__ void __launch_bounds__(kSweepBlock, 1) k_lusgs_mixed(CCView v, const int* __restrict__ woff) {
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int gw = blockIdx.x * (kSweepBlock / 32) + wib;
-    const int slot = lane >> 2, k = lane & 3;
-    if (stopped(v)) return;
-    const int n = v.noc;
-    const float gm1 = (float)(v.g.gamma - 1.0);
-    const float4* recf = reinterpret_cast<const float4*>(v.rec_a);
-    const int kbeg = woff[gw], kend = woff[gw + 1];
-    if (kbeg >= kend) return;
-    const int4 none = make_int4(0, 0, 0, 0);
-    int4 S = v.sched[kbeg];
-    int4 Sn = kbeg + 1 < kend ? v.sched[kbeg + 1] : none;
-    SweepInM X = {}, Xn = {};
-    sweep_load_m(v, S, lane, X);
-    int last = -1;
-    float LF[4] = {0.f, 0.f, 0.f, 0.f};             // previous item's dq (FP32)
-    double L0 = 0.0, L1 = 0.0, L2 = 0.0, L3 = 0.0;  // and in FP64
-    float Sf[4] = {0.f, 0.f, 0.f, 0.f};
-    bool spec = false;
-    for (int kk = kbeg; kk < kend; ++kk) {
-        const int4 Snn = kk + 2 < kend ? v.sched[kk + 2] : none;
-        const int it = S.x, pass = S.y, ntake = S.w;
-        double cres = 0.0;
-        for (int base = 0; base < ntake; base += 8) {
-            SweepInM E = X;
-            if (base > 0 && base + slot < ntake) sweep_load_face_m(v, S.z + base + slot, E);
-            bool ok = true;
-            double t = 0.0;
-            if (base + slot < ntake) {
-                float dq[4];
-                if (((E.nb << 1) | pass) == last) {
-                    dq[0] = LF[0]; dq[1] = LF[1]; dq[2] = LF[2]; dq[3] = LF[3];
-                } else if (base == 0 && spec && set_f4(Sf)) {
-                    dq[0] = Sf[0]; dq[1] = Sf[1]; dq[2] = Sf[2]; dq[3] = Sf[3];
-                } else {
-                    ok = poll_f4(recf + (size_t)pass * n + E.nb, dq, v.err, v.wait_cycles);
-                }
-                const float df = dflux_k(E, gm1, dq, k);
-                const float dqk = k == 0 ? dq[0] : (k == 1 ? dq[1] : (k == 2 ? dq[2] : dq[3]));
-                t = (double)(E.area * df - E.ol * dqk);
-            }
-            if (__ballot_sync(full, !ok)) return;
-            const int nr = min(8, ntake - base);
-            int e = 0;
-            if (base == 0) { cres = zero_plus(__shfl_sync(full, t, k)); e = 1; }  // 0.0 + t0, exact
-            for (; e < nr; ++e) cres = cres + __shfl_sync(full, t, 4 * e + k);
-        }
-        if (kk + 1 < kend) sweep_load_m(v, Sn, lane, Xn);
-        double r = X.r;
-        bool ok = true;
-        if (pass == 1 && lane < 4) {  // own lower
-            if ((it << 1) == last) r = pick4(lane, L0, L1, L2, L3);
-            else ok = poll_value(reinterpret_cast<const double*>(v.rec_b + it) + lane, r, v.err, v.wait_cycles);
-        }
-        if (__ballot_sync(full, !ok)) return;
-        const double d = pass == 0 ? (-r - 0.5 * cres) * X.D : r - 0.5 * cres * X.D;
-        const double q = X.o + d;
-        spec = false;
-        if (kk + 1 < kend && slot < Sn.w && ((Xn.nb << 1) | Sn.y) != ((it << 1) | pass)) {
-            peek_f4(recf + (size_t)Sn.y * n + Xn.nb, Sf);
-            spec = true;
-        }
-        const float df = (float)d;
-        LF[0] = __shfl_sync(full, df, 0);
-        LF[1] = __shfl_sync(full, df, 1);
-        LF[2] = __shfl_sync(full, df, 2);
-        LF[3] = __shfl_sync(full, df, 3);
-        L0 = __shfl_sync(full, d, 0);
-        L1 = __shfl_sync(full, d, 1);
-        L2 = __shfl_sync(full, d, 2);
-        L3 = __shfl_sync(full, d, 3);
-        const double Q0 = __shfl_sync(full, q, 0), Q1 = __shfl_sync(full, q, 1), Q2 = __shfl_sync(full, q, 2),
-                     Q3 = __shfl_sync(full, q, 3);
-        last = (it << 1) | pass;
-        const size_t slotr = (size_t)pass * n + it;
-        if (last == v.skip_code) {  // test hook: this item publishes nothing and hands nothing on
-            last = -1;
-        } else {
-            publish_mixed(lane, reinterpret_cast<float4*>(v.rec_a) + slotr, reinterpret_cast<double2*>(v.rec_b + slotr), LF,
-                          L0, L1, L2, L3);
-            if (pass == 1 && lane == 2) v.qc[it] = make_double4(Q0, Q1, Q2, Q3);
-        }
-        S = Sn;
-        Sn = Snn;
-        X = Xn;
-    }
+__global__ void __launch_bounds__(kSweepBlock, 1) k_lusgs_mixed(SweepArgs a, const int* done, const int* __restrict__ woff) {
+    if (done && *((volatile const int*)done) != 0) return;
+    sweep_block<true, true>(a, woff);
 }
 
 }  // namespace
@@ -2065,25 +1750,28 @@ int enqueue_lusgs(uns_cc_handle* h, CCView& v) {
         if (mixed) LAUNCH(k_cc_sweep_prep_mixed, v.nrec, v);
         else LAUNCH(k_cc_sweep_prep, v.nrec, v);
     }
-    const long long n2 = 2LL * v.noc * 2;  // double2 per record array
-    if (mixed)
-        k_fill_unset_f<<<std::min<long long>(nblocks(2LL * v.noc), 4096), kBlock, 0, h->stream>>>((float4*)v.rec_a,
-                                                                                                   2LL * v.noc);
-    else
-        k_fill_unset<<<std::min<long long>(nblocks(n2), 4096), kBlock, 0, h->stream>>>((double2*)v.rec_a, n2);
-    k_fill_unset<<<std::min<long long>(nblocks(n2), 4096), kBlock, 0, h->stream>>>((double2*)v.rec_b, n2);
+    // re-arm the records
+    const long long n2 = 2LL * v.noc;
+    if (mixed) {
+        k_fill_unset_f<<<std::min<long long>(nblocks(n2), 4096), kBlock, 0, h->stream>>>((float4*)v.srec, n2);
+        k_fill_unset<<<std::min<long long>(nblocks(2 * n2), 4096), kBlock, 0, h->stream>>>(v.srec + n2, 2 * n2);
+    } else {
+        k_fill_unset<<<std::min<long long>(nblocks(5 * n2), 4096), kBlock, 0, h->stream>>>(v.srec, 5 * n2);
+    }
     UNS_CUDA(cudaGetLastError());
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(h->coop_blocks);
     cfg.blockDim = dim3(kSweepBlock);
+    cfg.dynamicSmemBytes = mixed ? sweep_smem_bytes<true>() : sweep_smem_bytes<false>();
     cfg.stream = h->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (mixed) UNS_CUDA(cudaLaunchKernelEx(&cfg, k_lusgs_mixed, v, (const int*)h->woff));
-    else UNS_CUDA(cudaLaunchKernelEx(&cfg, k_lusgs, v, (const int*)h->woff));
+    const SweepArgs a = sweep_args(v, mixed);
+    if (mixed) UNS_CUDA(cudaLaunchKernelEx(&cfg, k_lusgs_mixed, a, (const int*)v.done, (const int*)h->woff));
+    else UNS_CUDA(cudaLaunchKernelEx(&cfg, k_lusgs, a, (const int*)v.done, (const int*)h->woff));
     return UNS_OK;
 }
 
@@ -2398,7 +2086,7 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
     AL(pp, nop); AL(ppT, nop); AL(fq, nof); AL(fqT, nof); AL(fla, nof); AL(fmu, nof);
     AL(fF, nof); AL(fV, nof); AL(fgx, nof); AL(fgy, nof); AL(fgT, nof); AL(fasum, nof);
     AL(fwall, nbf); AL(fwallv, nbf);
-    AL(diag, noc); AL(diaginv, noc); AL(rec_a, 2 * (size_t)noc); AL(rec_b, 2 * (size_t)noc);
+    AL(diag, noc); AL(diaginv, noc);
     UP(fgeof, fgeof); UP(fnaf, fnaf); UP(lswf, lswf);
     AL(qpf, ntot); AL(fqf, nof); AL(flaf, nof); AL(packf, 4 * (size_t)noc); AL(ppf, nop); AL(dcv, noc);
     { std::vector<float> t(m->v2c_wt, m->v2c_wt + m->v2c_off[nop]); UP(v2c_wtf, t); }
@@ -2419,7 +2107,7 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
         if (noc >= (1 << 30)) { set_last_error("uns_cc_create: too many cells"); return fail(UNS_ERR_MESH); }
         int dev = 0, nsm = 0, per = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_lusgs, kSweepBlock, 0) != cudaSuccess || per < 1) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_lusgs, kSweepBlock, sweep_smem_bytes<false>()) != cudaSuccess || per < 1) {
             set_last_error("uns_cc_create: cannot size the cooperative LU-SGS launch");
             return fail(UNS_ERR_CUDA);
         }
@@ -2437,7 +2125,7 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
                 int fl;
                 nbr[k] = other(i, m->c2f[k], &fl);
             }
-        WarpSchedule ws = list_schedule(noc, m->c2f_off, nbr.data(), h->coop_blocks * (kSweepBlock / 32));
+        WarpSchedule ws = list_schedule(noc, m->c2f_off, nbr.data(), h->coop_blocks * kSweepPairs);
         std::vector<int4> sched(ws.items.size());
         std::vector<int> rf, rn, rl;
         for (size_t pos = 0; pos < ws.items.size(); ++pos) {
@@ -2454,6 +2142,7 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
         if ((rc = h->upload(h->woff, ws.off.data(), ws.off.size()))) return fail(rc);
         UP(sched, sched); UP(rec_face, rf); UP(rec_nb, rn); UP(rec_flip, rl);
         AL(rec, 3 * rf.size());
+        AL(srec, 10 * (size_t)noc);
     }
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) { set_last_error("uns_cc_create: upload failed"); return fail(UNS_ERR_CUDA); }
     rc = uns_cc_initialize(h);

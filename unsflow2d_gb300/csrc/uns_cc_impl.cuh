@@ -84,8 +84,7 @@ struct CCView {
     const int* rec_flip;
     int nrec;
     double4* rec;     // per record, per LU-SGS call: 3 x double4 (k_cc_sweep_prep) or 4 x float4 (k_cc_sweep_prep_mixed)
-    double4* rec_a;   // sweep records [pass * noc + cell]: (u, v, p, e*rho) of qold + dq
-    double4* rec_b;   //   and dq (lower / upper); rho is rebuilt as qold.rho + dq.rho
+    double2* srec;    // sweep records (sweep_args): 10 per cell
     unsigned long long* minmax;  // encoded qmax[4], qmin[4]
     unsigned long long* dtmin;   // encoded dtglobal
     double* partial;

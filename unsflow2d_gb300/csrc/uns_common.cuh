@@ -76,9 +76,6 @@ __device__ __forceinline__ double2 ld_relaxed2(const double2* p) {
     asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_relaxed2(double2* p, double a, double b) {
-    asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" : : "l"(p), "d"(a), "d"(b) : "memory");
-}
 
 // Bounded wait shared by the record polls: false (and UNS_ERR_TIMEOUT
 // recorded) once `limit` cycles have passed or another thread has timed out.
@@ -96,35 +93,6 @@ __device__ __forceinline__ bool poll_continue(int spins, long long& t0, DevErr* 
     return true;
 }
 
-// Reads the 2 x 32-byte record (a, b) of a sweep item into out[0..8), all
-// four loads in flight together, waiting (bounded) until none is kUnset.
-__device__ __forceinline__ bool poll_record2(const double4* a, const double4* b, double out[8], DevErr* err,
-                                             long long limit = kWaitCycles) {
-    const double2* pa = reinterpret_cast<const double2*>(a);
-    const double2* pb = reinterpret_cast<const double2*>(b);
-    long long t0 = 0;
-    for (int spins = 0;; ++spins) {
-        double2 x0 = ld_relaxed2(pa), x1 = ld_relaxed2(pa + 1), x2 = ld_relaxed2(pb), x3 = ld_relaxed2(pb + 1);
-        out[0] = x0.x; out[1] = x0.y; out[2] = x1.x; out[3] = x1.y;
-        out[4] = x2.x; out[5] = x2.y; out[6] = x3.x; out[7] = x3.y;
-        bool ready = true;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) ready = ready && !is_unset(out[j]);
-        if (ready) return true;
-        if (!poll_continue(spins, t0, err, limit)) return false;
-    }
-}
-
-// One published value, waiting (bounded) until it is not kUnset.
-__device__ __forceinline__ bool poll_value(const double* p, double& out, DevErr* err, long long limit = kWaitCycles) {
-    long long t0 = 0;
-    for (int spins = 0;; ++spins) {
-        asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(out) : "l"(p) : "memory");
-        if (!is_unset(out)) return true;
-        if (!poll_continue(spins, t0, err, limit)) return false;
-    }
-}
-
 // FP32 records (mixed precision) use a signalling-NaN float pattern the same way.
 constexpr unsigned kUnsetF = 0x7FA0DEADu;
 __device__ __forceinline__ bool is_unset(float x) { return (unsigned)__float_as_int(x) == kUnsetF; }
@@ -137,16 +105,6 @@ __device__ __forceinline__ void peek_f4(const float4* a, float w[4]) {
 
 __device__ __forceinline__ bool set_f4(const float w[4]) {
     return !is_unset(w[0]) && !is_unset(w[1]) && !is_unset(w[2]) && !is_unset(w[3]);
-}
-
-// A float4 record, waiting (bounded) until none of its values is kUnsetF.
-__device__ __forceinline__ bool poll_f4(const float4* a, float w[4], DevErr* err, long long limit = kWaitCycles) {
-    long long t0 = 0;
-    for (int spins = 0;; ++spins) {
-        peek_f4(a, w);
-        if (set_f4(w)) return true;
-        if (!poll_continue(spins, t0, err, limit)) return false;
-    }
 }
 
 // LU-SGS normal flux change F(q + dq) - F(q) along (nx, ny), component k, in

@@ -80,9 +80,7 @@ struct NCView {
     double4* rec;    // per record, per LU-SGS call: 3 x double4 (k_nc_sweep_prep) or 4 x float4 (k_nc_sweep_prep_mixed)
     double* diag;    // LU-SGS diagonal cv/dt + 0.5*omega*la (lusgs.f90:36)
     double* diaginv; // its FP64 reciprocal, read by the FP32 sweeps (a multiply on their critical path)
-    double4* rec_a;  // sweep records [pass * nop + node]: (u, v, p, e*rho) of qc
-    double4* rec_b;  //   and dqc
-    double* rec_r;   //   and rho (FP64 sweep)
+    double2* srec;   // sweep records (sweep_args): 10 per node
     double* partial;   // [2*nblk]: sum, max
     int* partial_i;    // argmax
     DevErr* err;
@@ -643,11 +641,6 @@ __global__ void __launch_bounds__(kBlock) k_nc_res_final(NCView v, int nparts, d
     }
 }
 
-// One sweep block per SM: one sweep warp per SM sub-partition, so concurrently
-// active items never share an FP64 unit.
-constexpr int kSweepBlocksPerSM = 1;
-constexpr double kOmega = 1.5;  // lusgs.f90:26
-
 // Per LU-SGS call: everything a sweep item needs from an edge that does not
 // change during the sweeps, laid out contiguously in schedule order so a
 // lane fetches it with three 32-byte loads and no index chasing:
@@ -712,451 +705,25 @@ __global__ void __launch_bounds__(kBlock) k_nc_sweep_prep_mixed(NCView v) {
     rf[3] = make_float4((float)v.rec_sign[r], __int_as_float(nb), 0.f, 0.f);
 }
 
-__device__ __forceinline__ double pick4(int k, double a, double b, double c, double d) {
-    return k == 0 ? a : (k == 1 ? b : (k == 2 ? c : d));
+SweepArgs sweep_args(const NCView& v, bool mixed) {
+    SweepArgs a;
+    a.n = v.nop; a.sched = v.sched; a.rec = v.rec;
+    a.diag = mixed ? v.diaginv : v.diag;
+    a.qold = v.qold; a.res = v.res; a.qc = v.qc;
+    a.out = v.srec; a.outf = reinterpret_cast<float4*>(v.srec); a.outd = reinterpret_cast<double4*>(v.srec + 2 * (size_t)v.nop);
+    a.err = v.err; a.wait_cycles = v.wait_cycles; a.skip_code = v.skip_code;
+    a.gm1 = v.g.gamma - 1.0;
+    return a;
 }
 
-// Lanes of a sweep item: lane = 4 * slot + k, slot = the taken edge (up to 8
-// per round), k = the variable.  An FP64 instruction holds its SM
-// sub-partition's unit the same 64-76 cycles whatever the number of active
-// lanes, so each item's arithmetic is spread over the lanes: the four flux
-// components of up to eight edges in one pass, the per-variable sums and
-// divisions in lanes 0..3, and the three divisions of con2prim in lanes 0, 2
-// and 3 at once.  Chosen by measurement on GB300 (sweeps at 1024x512,
-// bit-identical variants): the consumer reads rho from the record rather than
-// forming qold.rho + dqc.rho; the warp exchanges its per-lane values through
-// shared memory rather than shuffles; the next item's inputs are loaded after
-// this item's polls.
-__device__ __forceinline__ double ld_relaxed(const double* p) {
-    double x;
-    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(x) : "l"(p) : "memory");
-    return x;
+// The sweeps (uns_sweep.cuh) over the nodes.
+__global__ void __launch_bounds__(kSweepBlock, 1) k_nc_lusgs(SweepArgs a, const int* done, const int* __restrict__ woff) {
+    if (done && *((volatile const int*)done) != 0) return;
+    sweep_block<false, false>(a, woff);
 }
-
-// What an edge term reads of a neighbour's record: (u, v, p, e*rho), rho and
-// component k of dqc.
-struct SweepNb {
-    double u, v, p, et, rho, dq;
-};
-__device__ __forceinline__ SweepNb peek_neighbour(const NCView& v, size_t rs, int k) {
-    const double2* pa = reinterpret_cast<const double2*>(v.rec_a + rs);
-    const double2 x0 = ld_relaxed2(pa), x1 = ld_relaxed2(pa + 1);
-    SweepNb w;
-    w.u = x0.x; w.v = x0.y; w.p = x1.x; w.et = x1.y;
-    w.rho = ld_relaxed(v.rec_r + rs);
-    w.dq = ld_relaxed(reinterpret_cast<const double*>(v.rec_b + rs) + k);
-    return w;
-}
-
-__device__ __forceinline__ bool record_set(const SweepNb& w) {
-    return !is_unset(w.u) && !is_unset(w.v) && !is_unset(w.p) && !is_unset(w.et) && !is_unset(w.rho) && !is_unset(w.dq);
-}
-
-// A neighbour's record, waiting (bounded) until every value is published.
-__device__ __forceinline__ bool poll_neighbour(const NCView& v, size_t rs, int k, SweepNb& w) {
-    long long t0 = 0;
-    for (int spins = 0;; ++spins) {
-        w = peek_neighbour(v, rs, k);
-        if (record_set(w)) return true;
-        if (!poll_continue(spins, t0, v.err, v.wait_cycles)) return false;
-    }
-}
-
-// Fields of a ring entry (per lane): the slot's record, f1 its component k;
-// the neighbour's record; the node's own diagonal, qold and res (pass 0) or
-// forward dqc (pass 1), variable k; and the neighbour's code (node << 1 |
-// pass, -1 in an idle slot) with the orientation sign in the upper word.
-enum { SF_F1, SF_NX, SF_NY, SF_DS, SF_OL, SF_U, SF_V, SF_P, SF_ET, SF_RHO, SF_DQ, SF_D2, SF_O, SF_R, SF_CODE, SF_N };
-typedef SweepRing<SF_N> RingNC;
-
-// The feeder: for each item of the warp's list, in order and as far ahead as
-// the ring allows, its inputs and its neighbours' records.  A neighbour that
-// is the list's previous item comes from the sweep warp's registers.
-__device__ void nc_feed(const NCView& v, RingNC& R, int kbeg, int kend, int lane) {
-    const int slot = lane >> 2, k = lane & 3;
-    const int n = v.nop;
-    RingPos pos;
-    int last = -1;
-    int4 S = v.sched[kbeg];
-    for (int kk = kbeg; kk < kend; ++kk) {
-        const int4 Sn = kk + 1 < kend ? v.sched[kk + 1] : make_int4(0, 0, 0, 0);
-        const int it = S.x, pass = S.y, ntake = S.w;
-        int base = 0;
-        do {
-            const bool take = base + slot < ntake;
-            double4 b = make_double4(0.0, 0.0, 0.0, 0.0), c = b;
-            double f1 = 0.0, D = 1.0, o = 1.0, r = 0.0;
-            if (take) {
-                const double4* p = v.rec + 3 * (size_t)(S.z + base + slot);
-                f1 = reinterpret_cast<const double*>(p)[k];
-                b = p[1];
-                c = p[2];
-            }
-            if (base == 0 && lane < 4) {
-                D = v.diag[it];
-                o = reinterpret_cast<const double*>(&v.qold[it])[lane];
-                if (pass == 0) r = reinterpret_cast<const double*>(&v.res[it])[lane];
-            }
-            const int code = take ? ((int)__double_as_longlong(c.z) << 1) | pass : -1;
-            // the entry's stage is free once the sweep warp has read it
-            if (!mbar_wait(&R.empty[pos.stage], pos.phase ^ 1, &R.abort, ring_limit(v.wait_cycles))) {
-                if (!*(volatile int*)&R.abort) set_err(v.err, UNS_ERR_TIMEOUT, -1);
-                *(volatile int*)&R.abort = 1;
-                return;
-            }
-            double(*f)[32] = R.f[pos.stage];
-            f[SF_F1][lane] = f1;
-            f[SF_NX][lane] = b.x; f[SF_NY][lane] = b.y; f[SF_DS][lane] = b.z; f[SF_OL][lane] = b.w;
-            f[SF_CODE][lane] = __longlong_as_double(((long long)(c.y < 0.0 ? 0x80000000u : 0u) << 32) | (unsigned)code);
-            if (base == 0) {
-                f[SF_D2][lane] = D + D;
-                f[SF_O][lane] = o;
-                if (lane == 0) R.item[pos.stage] = S;
-            }
-            bool ok = true;
-            SweepNb w = {};
-            if (code != last && take) ok = poll_neighbour(v, (size_t)pass * n + (code >> 1), k, w);
-            if (base == 0 && pass == 1 && lane < 4 && (it << 1) != last)  // own forward dqc
-                ok = poll_value(reinterpret_cast<const double*>(v.rec_b + it) + lane, r, v.err, v.wait_cycles) && ok;
-            f[SF_U][lane] = w.u; f[SF_V][lane] = w.v; f[SF_P][lane] = w.p; f[SF_ET][lane] = w.et;
-            f[SF_RHO][lane] = w.rho; f[SF_DQ][lane] = w.dq;
-            if (base == 0) f[SF_R][lane] = pass == 0 ? r + r : r;
-            if (__any_sync(0xffffffffu, !ok)) {  // a wait gave up; the error is recorded
-                *(volatile int*)&R.abort = 1;
-                return;
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&R.full[pos.stage]);
-            pos.next();
-            base += 8;
-        } while (base < ntake);
-        last = (it << 1) | pass;
-        if (last == v.skip_code) last = -1;  // test hook: that item hands nothing on
-        S = Sn;
-    }
-}
-
-// lusgs sweeps (lusgs.f90:48-124) as one cooperative launch.  Each sweep warp
-// runs its own list of items (node, pass) from the host-side list schedule, in
-// order, on what its feeder has put into the ring (uns_sweep.cuh).  Per item,
-// for each edge whose neighbour precedes the node in this pass (reference v2f
-// order): the neighbour's values come from registers when the warp itself
-// computed that neighbour last, else from the ring; the edge term
-// sign*(F(qc) - F(qold)) - omega*la*dqc is formed per component, lanes 0..3
-// add the terms in edge order (the reference's summation order) and divide by
-// the diagonal; the new state is spread to all lanes, which keep its
-// primitives for the next item while lanes 0..2 publish the record.
-// Every rounded operation and its operand order is the reference's, but for
-// its factor 0.5 on the terms, which doubles res and the diagonal instead
-// (a scaling by two commutes with every rounding short of the subnormal
-// range).
-//
-// The FP64 unit takes one instruction of the warp per 64 cycles whatever its
-// lanes, so sums and products are register FMAs, and the two divisions (590
-// cycles each there) run on the integer pipe (240).  %PERF%
-__global__ void __launch_bounds__(kSweepBlock, 1) k_nc_lusgs(NCView v, const int* __restrict__ woff) {
-    extern __shared__ __align__(16) unsigned char sweep_smem[];
-    RingNC* rings = reinterpret_cast<RingNC*>(sweep_smem);
-    __shared__ __align__(16) double wxs[kSweepPairs][32];  // per-warp exchange of lane values
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, wib = (threadIdx.x >> 5) & (kSweepPairs - 1);
-    const bool feeder = threadIdx.x >= 32 * kSweepPairs;
-    if (stopped(v)) return;
-    if (threadIdx.x < kSweepPairs) ring_init(rings[threadIdx.x]);
-    __syncthreads();
-    const int gw = blockIdx.x * kSweepPairs + wib;
-    const int kbeg = woff[gw], kend = woff[gw + 1];
-    if (kbeg >= kend) return;
-    RingNC& R = rings[wib];
-    if (feeder) {
-        nc_feed(v, R, kbeg, kend, lane);
-        return;
-    }
-    double* wx = wxs[wib];
-    const int k = lane & 3;
-    const int n = v.nop;
-    const double gm1 = in_register(v.g.gamma - 1.0);
-    RingPos pos;
-    int last = -1;  // code of the warp's previous item; its values in L, in every lane
-    SweepNb L = {};
-    for (int kk = kbeg; kk < kend; ++kk) {
-        double cres = 0.0;  // lanes 0..3: sum over edges of component k
-        double D2 = 2.0, xo = 1.0, xr = 0.0;
-        unsigned Y = 0;  // the diagonal's reciprocal digits, off the chain
-        int it = 0, pass = 0, ntake = 0, base = 0;
-        do {
-            if (!mbar_wait(&R.full[pos.stage], pos.phase, &R.abort, ring_limit(v.wait_cycles))) {
-                if (!*(volatile int*)&R.abort) set_err(v.err, UNS_ERR_TIMEOUT, -1);
-                *(volatile int*)&R.abort = 1;
-                return;
-            }
-            const double(*f)[32] = R.f[pos.stage];
-            if (base == 0) {
-                const int4 S = R.item[pos.stage];
-                it = S.x; pass = S.y; ntake = S.w;
-                D2 = f[SF_D2][lane]; xo = f[SF_O][lane]; xr = f[SF_R][lane];
-                Y = div_recip(D2);
-            }
-            const long long cs = __double_as_longlong(f[SF_CODE][lane]);
-            const double f1 = f[SF_F1][lane], nx = f[SF_NX][lane], ny = f[SF_NY][lane], ds = f[SF_DS][lane], ol = f[SF_OL][lane];
-            SweepNb w;
-            w.u = f[SF_U][lane]; w.v = f[SF_V][lane]; w.p = f[SF_P][lane]; w.et = f[SF_ET][lane];
-            w.rho = f[SF_RHO][lane]; w.dq = f[SF_DQ][lane];
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&R.empty[pos.stage]);
-            pos.next();
-            if (ntake == 0) break;
-            const int code = (int)cs;
-            if (code == last && code >= 0) w = L;
-            // normalflux (lusgs.f90:144-150) component k, then the edge term;
-            // idle slots compute on zeros
-            const double un = add64(mul64(w.u, nx), mul64(w.v, ny));
-            const double o1 = mul64(w.rho, un);
-            const double h = add64(w.et, w.p);
-            const double prod = mul64(k == 0 ? h : o1, k == 0 ? un : (k == 2 ? w.u : w.v));
-            const double sum = add64(prod, mul64(w.p, k == 2 ? nx : ny));
-            const double o = mul64(k == 1 ? o1 : (k == 0 ? prod : sum), ds);
-            const double diff = sub64(o, f1);
-            const double t = sub64(flip64(diff, cs < 0), mul64(ol, w.dq));
-            // the terms in edge order, from 0.0 (the first addition is exact)
-            const int nr = min(8, ntake - base);
-            wx[lane] = t;
-            __syncwarp();
-            int e = 0;
-            if (base == 0) { cres = zero_plus(wx[k]); e = 1; }
-            for (; e < nr; ++e) cres = add64(cres, wx[4 * e + k]);
-            __syncwarp();
-            base += 8;
-        } while (base < ntake);
-        // dqc and qc = qold + dqc (lusgs.f90:78-81 / 117-120), component k in lane k
-        double d;
-        if (pass == 0) {
-            d = div_digits(sub64(neg64(xr), cres), D2, Y);
-        } else {  // from the node's own forward dqc
-            const double r = (it << 1) == last ? L.dq : xr;
-            d = sub64(r, div_digits(cres, D2, Y));
-        }
-        const double q = add64(xo, d);
-        // con2prim (All_modules.f90:146-169): rho = q1, then E/rho, rhou/rho,
-        // rhov/rho in lanes 0, 2, 3
-        if (lane < 4) { wx[lane] = q; wx[4 + lane] = d; }
-        __syncwarp();
-        const double2 qa = reinterpret_cast<const double2*>(wx)[0], qb = reinterpret_cast<const double2*>(wx)[1];
-        const double E1 = qa.x, rho = qa.y, Q2 = qb.x, Q3 = qb.y;
-        const double quo = div_digits(q, rho);
-        // the four products of the pressure and the record as one
-        // multiplication: lane 0 e*rho, lane 1 0.5*rho, lane 2 u*u, lane 3 v*v
-        const double ma = lane == 1 ? 0.5 : quo, mb = lane < 2 ? rho : quo;
-        const double pr = mul64(ma, mb);
-        if (lane < 4) { wx[8 + lane] = quo; wx[12 + lane] = pr; }
-        __syncwarp();
-        const double2 pa = reinterpret_cast<const double2*>(wx)[6], pb = reinterpret_cast<const double2*>(wx)[7];
-        const double uu = wx[10], vv = wx[11], dk = wx[4 + k];
-        const double2 da = reinterpret_cast<const double2*>(wx)[2], db = reinterpret_cast<const double2*>(wx)[3];
-        __syncwarp();
-        const double qq = add64(pb.x, pb.y);                       // u*u + v*v
-        const double p = mul64(gm1, sub64(E1, mul64(pa.y, qq)));   // gm1*(E - 0.5*rho*qq)
-        L.u = uu; L.v = vv; L.p = p; L.et = pa.x; L.rho = rho; L.dq = dk;
-        last = (it << 1) | pass;
-        const size_t slotr = (size_t)pass * n + it;
-        if (last == v.skip_code) {
-            last = -1;  // test hook: this item publishes nothing and hands nothing on
-        } else {
-            // Lane 0 stores (u, v, p, e*rho), lane 1 dqc, lane 2 rho, as
-            // predicated stores of one instruction sequence: lane-divergent
-            // branches here cost the critical path more than the stores
-            // (sweeps 11.07 -> 10.39 ms at 1024x512, measured).
-            double2* dst = reinterpret_cast<double2*>(lane == 0 ? v.rec_a + slotr : v.rec_b + slotr);
-            const double x0 = lane == 0 ? uu : da.x, x1 = lane == 0 ? vv : da.y;
-            const double x2 = lane == 0 ? p : db.x, x3 = lane == 0 ? pa.x : db.y;
-            const int st_ab = lane < 2, st_r = lane == 2;
-            asm volatile(
-                "{\n\t.reg .pred pa, pr;\n\t"
-                "setp.ne.s32 pa, %0, 0;\n\t"
-                "setp.ne.s32 pr, %1, 0;\n\t"
-                "@pa st.relaxed.gpu.global.v2.f64 [%2], {%3, %4};\n\t"
-                "@pa st.relaxed.gpu.global.v2.f64 [%5], {%6, %7};\n\t"
-                "@pr st.relaxed.gpu.global.f64 [%8], %9;\n\t}"
-                :
-                : "r"(st_ab), "r"(st_r), "l"(dst), "d"(x0), "d"(x1), "l"(dst + 1), "d"(x2), "d"(x3), "l"(v.rec_r + slotr),
-                  "d"(rho)
-                : "memory");
-            if (pass == 1 && lane == 2) v.qc[it] = make_double4(E1, rho, Q2, Q3);
-        }
-    }
-}
-
-// ------------------------------------------------------------ mixed (delta form)
-// The FP32 sweep cannot form F(qold + dqc) - F(qold) as a difference of two
-// O(1) fluxes: near convergence that difference drowns in FP32 rounding and
-// the solve stalls.  It forms the change directly from dqc (dflux_k), so its
-// FP32 error is relative to the change itself; items publish dqc only (FP32
-// for the edge terms, FP64 for the node's own backward step) and form no
-// primitives.
-struct SweepRecM {
-    float rho, ru, rv, E, u, v, p, un, nx, ny;  // the slot's record, as dflux_k reads it
-};
-
-// Fields of a ring entry of the mixed form: two floats to a field.
-enum { MF_R01, MF_R23, MF_UV, MF_PUN, MF_N, MF_DSOL, MF_DQ01, MF_DQ23, MF_D, MF_O, MF_R, MF_CODE, MF_COUNT };
-typedef SweepRing<MF_COUNT> RingNCM;
-
-__device__ __forceinline__ double pack2(float a, float b) {
-    return dmake(__float_as_uint(b), __float_as_uint(a));
-}
-__device__ __forceinline__ float low_f(double x) { return __uint_as_float(dlo(x)); }
-__device__ __forceinline__ float high_f(double x) { return __uint_as_float(dhi(x)); }
-
-__device__ void nc_feed_mixed(const NCView& v, RingNCM& R, int kbeg, int kend, int lane) {
-    const int slot = lane >> 2;
-    const int n = v.nop;
-    const float4* recf = reinterpret_cast<const float4*>(v.rec_a);
-    RingPos pos;
-    int last = -1;
-    int4 S = v.sched[kbeg];
-    for (int kk = kbeg; kk < kend; ++kk) {
-        const int4 Sn = kk + 1 < kend ? v.sched[kk + 1] : make_int4(0, 0, 0, 0);
-        const int it = S.x, pass = S.y, ntake = S.w;
-        int base = 0;
-        do {
-            const bool take = base + slot < ntake;
-            float4 a = make_float4(1.f, 0.f, 0.f, 0.f), b = make_float4(0.f, 0.f, 0.f, 0.f), c = b, d = b;
-            double D = 1.0, o = 1.0, r = 0.0;
-            if (take) {
-                const float4* p = reinterpret_cast<const float4*>(v.rec) + 4 * (size_t)(S.z + base + slot);
-                a = p[0]; b = p[1]; c = p[2]; d = p[3];
-            }
-            if (base == 0 && lane < 4) {
-                D = v.diaginv[it];  // the FP32 sweep multiplies by the FP64 reciprocal
-                o = reinterpret_cast<const double*>(&v.qold[it])[lane];
-                if (pass == 0) r = reinterpret_cast<const double*>(&v.res[it])[lane];
-            }
-            const int code = take ? (__float_as_int(d.y) << 1) | pass : -1;
-            if (!mbar_wait(&R.empty[pos.stage], pos.phase ^ 1, &R.abort, ring_limit(v.wait_cycles))) {
-                if (!*(volatile int*)&R.abort) set_err(v.err, UNS_ERR_TIMEOUT, -1);
-                *(volatile int*)&R.abort = 1;
-                return;
-            }
-            double(*f)[32] = R.f[pos.stage];
-            f[MF_R01][lane] = pack2(a.x, a.y); f[MF_R23][lane] = pack2(a.z, a.w);
-            f[MF_UV][lane] = pack2(b.x, b.y); f[MF_PUN][lane] = pack2(b.z, b.w);
-            f[MF_N][lane] = pack2(c.x, c.y); f[MF_DSOL][lane] = pack2(c.z, c.w);
-            f[MF_CODE][lane] = dmake(d.x < 0.f ? 0x80000000u : 0u, (unsigned)code);
-            if (base == 0) {
-                f[MF_D][lane] = D;
-                f[MF_O][lane] = o;
-                if (lane == 0) R.item[pos.stage] = S;
-            }
-            bool ok = true;
-            float dq[4] = {0.f, 0.f, 0.f, 0.f};
-            if (code != last && take) ok = poll_f4(recf + (size_t)pass * n + (code >> 1), dq, v.err, v.wait_cycles);
-            if (base == 0 && pass == 1 && lane < 4 && (it << 1) != last)  // own forward dqc
-                ok = poll_value(reinterpret_cast<const double*>(v.rec_b + it) + lane, r, v.err, v.wait_cycles) && ok;
-            f[MF_DQ01][lane] = pack2(dq[0], dq[1]);
-            f[MF_DQ23][lane] = pack2(dq[2], dq[3]);
-            if (base == 0) f[MF_R][lane] = r;
-            if (__any_sync(0xffffffffu, !ok)) {
-                *(volatile int*)&R.abort = 1;
-                return;
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&R.full[pos.stage]);
-            pos.next();
-            base += 8;
-        } while (base < ntake);
-        last = (it << 1) | pass;
-        if (last == v.skip_code) last = -1;
-        S = Sn;
-    }
-}
-
-// lusgs sweeps in the mixed form: the schedule, lanes, ring and FP64 sums of
-// k_nc_lusgs; FP32 delta-form edge terms.  %PERFM%
-__global__ void __launch_bounds__(kSweepBlock, 1) k_nc_lusgs_mixed(NCView v, const int* __restrict__ woff) {
-    extern __shared__ __align__(16) unsigned char sweep_smem[];
-    RingNCM* rings = reinterpret_cast<RingNCM*>(sweep_smem);
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, wib = (threadIdx.x >> 5) & (kSweepPairs - 1);
-    const bool feeder = threadIdx.x >= 32 * kSweepPairs;
-    if (stopped(v)) return;
-    if (threadIdx.x < kSweepPairs) ring_init(rings[threadIdx.x]);
-    __syncthreads();
-    const int gw = blockIdx.x * kSweepPairs + wib;
-    const int kbeg = woff[gw], kend = woff[gw + 1];
-    if (kbeg >= kend) return;
-    RingNCM& R = rings[wib];
-    if (feeder) {
-        nc_feed_mixed(v, R, kbeg, kend, lane);
-        return;
-    }
-    const int k = lane & 3;
-    const int n = v.nop;
-    const float gm1 = (float)(v.g.gamma - 1.0);
-    RingPos pos;
-    int last = -1;
-    float LF[4] = {0.f, 0.f, 0.f, 0.f};             // previous item's dqc (FP32)
-    double Lk = 0.0;                                // and in FP64, component k
-    for (int kk = kbeg; kk < kend; ++kk) {
-        double cres = 0.0, xd = 1.0, xo = 1.0, xr = 0.0;
-        int it = 0, pass = 0, ntake = 0, base = 0;
-        do {
-            if (!mbar_wait(&R.full[pos.stage], pos.phase, &R.abort, ring_limit(v.wait_cycles))) {
-                if (!*(volatile int*)&R.abort) set_err(v.err, UNS_ERR_TIMEOUT, -1);
-                *(volatile int*)&R.abort = 1;
-                return;
-            }
-            const double(*f)[32] = R.f[pos.stage];
-            if (base == 0) {
-                const int4 S = R.item[pos.stage];
-                it = S.x; pass = S.y; ntake = S.w;
-                xd = f[MF_D][lane]; xo = f[MF_O][lane]; xr = f[MF_R][lane];
-            }
-            const double r01 = f[MF_R01][lane], r23 = f[MF_R23][lane], uv = f[MF_UV][lane], pun = f[MF_PUN][lane];
-            const double nn = f[MF_N][lane], dsol = f[MF_DSOL][lane], q01 = f[MF_DQ01][lane], q23 = f[MF_DQ23][lane];
-            const long long cs = __double_as_longlong(f[MF_CODE][lane]);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&R.empty[pos.stage]);
-            pos.next();
-            if (ntake == 0) break;
-            const bool mine = (int)cs == last && (int)cs >= 0;
-            const float dq[4] = {mine ? LF[0] : low_f(q01), mine ? LF[1] : high_f(q01), mine ? LF[2] : low_f(q23),
-                                 mine ? LF[3] : high_f(q23)};
-            const SweepRecM E = {low_f(r01), high_f(r01), low_f(r23), high_f(r23), low_f(uv), high_f(uv),
-                                 low_f(pun), high_f(pun), low_f(nn), high_f(nn)};
-            const float df = dflux_k(E, gm1, dq, k);
-            const float dqk = k == 0 ? dq[0] : (k == 1 ? dq[1] : (k == 2 ? dq[2] : dq[3]));
-            const double t = widen(0.5f * ((cs < 0 ? -df : df) * low_f(dsol) - high_f(dsol) * dqk));
-            const int nr = min(8, ntake - base);
-            int e = 0;
-            if (base == 0) { cres = zero_plus(__shfl_sync(full, t, k)); e = 1; }  // 0.0 + t0, exact
-            for (; e < nr; ++e) cres = add64(cres, __shfl_sync(full, t, 4 * e + k));
-            base += 8;
-        } while (base < ntake);
-        double d;
-        if (pass == 0) {
-            d = mul64(sub64(neg64(xr), cres), xd);
-        } else {  // from the node's own forward dqc
-            const double r = (it << 1) == last ? Lk : xr;
-            d = sub64(r, mul64(cres, xd));
-        }
-        const float df = narrow(d);
-        LF[0] = __shfl_sync(full, df, 0);
-        LF[1] = __shfl_sync(full, df, 1);
-        LF[2] = __shfl_sync(full, df, 2);
-        LF[3] = __shfl_sync(full, df, 3);
-        const double L0 = __shfl_sync(full, d, 0), L1 = __shfl_sync(full, d, 1), L2 = __shfl_sync(full, d, 2),
-                     L3 = __shfl_sync(full, d, 3);
-        Lk = pick4(k, L0, L1, L2, L3);
-        last = (it << 1) | pass;
-        const size_t slotr = (size_t)pass * n + it;
-        if (last == v.skip_code) {  // test hook: this item publishes nothing and hands nothing on
-            last = -1;
-        } else {
-            publish_mixed(lane, reinterpret_cast<float4*>(v.rec_a) + slotr, reinterpret_cast<double2*>(v.rec_b + slotr), LF,
-                          L0, L1, L2, L3);
-            if (pass == 1 && lane < 4) reinterpret_cast<double*>(&v.qc[it])[lane] = add64(xo, d);
-        }
-    }
+__global__ void __launch_bounds__(kSweepBlock, 1) k_nc_lusgs_mixed(SweepArgs a, const int* done, const int* __restrict__ woff) {
+    if (done && *((volatile const int*)done) != 0) return;
+    sweep_block<false, true>(a, woff);
 }
 
 // tecplt's vertex table (NCFVM/main.f90:190-233): per node x, y and the
@@ -1308,29 +875,28 @@ int enqueue_fvres_nc(uns_nc_handle* h, NCView& v, double cfl, int rk3, int parti
 
 int launch_sweeps_nc(uns_nc_handle* h, NCView& v) {
     const bool mixed = h->P.precision != UNS_PREC_FP64;  // FP32 sweep arithmetic
-    const long long n2 = 2LL * v.nop * 2;  // double2 per record array
-    if (mixed)
-        k_fill_unset_f<<<std::min<long long>(nblocks(2LL * v.nop), 4096), kBlock, 0, h->stream>>>((float4*)v.rec_a,
-                                                                                                   2LL * v.nop);
-    else {
-        k_fill_unset<<<std::min<long long>(nblocks(n2), 4096), kBlock, 0, h->stream>>>((double2*)v.rec_a, n2);
-        k_fill_unset<<<std::min<long long>(nblocks(v.nop), 4096), kBlock, 0, h->stream>>>((double2*)v.rec_r,
-                                                                                           (long long)v.nop);
+    // re-arm the records
+    const long long n2 = 2LL * v.nop;
+    if (mixed) {
+        k_fill_unset_f<<<std::min<long long>(nblocks(n2), 4096), kBlock, 0, h->stream>>>((float4*)v.srec, n2);
+        k_fill_unset<<<std::min<long long>(nblocks(2 * n2), 4096), kBlock, 0, h->stream>>>(v.srec + n2, 2 * n2);
+    } else {
+        k_fill_unset<<<std::min<long long>(nblocks(5 * n2), 4096), kBlock, 0, h->stream>>>(v.srec, 5 * n2);
     }
-    k_fill_unset<<<std::min<long long>(nblocks(n2), 4096), kBlock, 0, h->stream>>>((double2*)v.rec_b, n2);
     UNS_CUDA(cudaGetLastError());
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(h->coop_blocks);
     cfg.blockDim = dim3(kSweepBlock);
-    cfg.dynamicSmemBytes = kSweepPairs * (mixed ? sizeof(RingNCM) : sizeof(RingNC));
+    cfg.dynamicSmemBytes = mixed ? sweep_smem_bytes<true>() : sweep_smem_bytes<false>();
     cfg.stream = h->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (mixed) UNS_CUDA(cudaLaunchKernelEx(&cfg, k_nc_lusgs_mixed, v, (const int*)h->woff));
-    else UNS_CUDA(cudaLaunchKernelEx(&cfg, k_nc_lusgs, v, (const int*)h->woff));
+    const SweepArgs a = sweep_args(v, mixed);
+    if (mixed) UNS_CUDA(cudaLaunchKernelEx(&cfg, k_nc_lusgs_mixed, a, (const int*)v.done, (const int*)h->woff));
+    else UNS_CUDA(cudaLaunchKernelEx(&cfg, k_nc_lusgs, a, (const int*)v.done, (const int*)h->woff));
     return UNS_OK;
 }
 
@@ -1466,7 +1032,7 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
     { std::vector<int> t(m->v2f, m->v2f + m->v2f_off[nop]); UPN(rv2f, t); }
     ALN(qc, nop); ALN(qp, nop); ALN(qpf, nop); ALN(packn, 3 * (size_t)nop); ALN(qold, nop); ALN(qoldp, nop); ALN(res, nop); ALN(gx, nop); ALN(gy, nop); ALN(phi, nop);
     ALN(dt, nop); ALN(la, nop); ALN(fla, nof); ALN(fF, nof); ALN(bres1, nbnd); ALN(bres2, nbnd); ALN(bla, nbnd);
-    ALN(diag, nop); ALN(diaginv, nop); ALN(rec_a, 2 * (size_t)nop); ALN(rec_b, 2 * (size_t)nop); ALN(rec_r, 2 * (size_t)nop);
+    ALN(diag, nop); ALN(diaginv, nop); ALN(srec, 10 * (size_t)nop);
     ALN(err, 1);
     h->v.wait_cycles = kWaitCycles;
     h->v.skip_code = -1;
@@ -1485,7 +1051,7 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
         if (nop >= (1 << 30)) { set_last_error("uns_nc_create: too many nodes"); return fail(UNS_ERR_MESH); }
         int dev = 0, nsm = 0, per = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_nc_lusgs, kSweepBlock, kSweepPairs * sizeof(RingNC)) != cudaSuccess || per < 1) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_nc_lusgs, kSweepBlock, sweep_smem_bytes<false>()) != cudaSuccess || per < 1) {
             set_last_error("uns_nc_create: cannot size the cooperative LU-SGS launch");
             return fail(UNS_ERR_CUDA);
         }

@@ -1500,7 +1500,7 @@ __global__ void __launch_bounds__(kBlock) k_cc_sweep_prep_mixed(CCView v) {
 
 SweepArgs sweep_args(const CCView& v, bool mixed) {
     SweepArgs a;
-    a.n = v.noc; a.sched = v.sched; a.rec = v.rec;
+    a.n = v.noc; a.sched = v.sched; a.rec = v.rec; a.rec_src = v.rec_src;
     a.diag = mixed ? v.diaginv : v.diag;
     a.qold = v.qold; a.res = v.res; a.qc = v.qc;
     a.out = v.srec; a.outf = reinterpret_cast<float4*>(v.srec);
@@ -2106,7 +2106,8 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
         if (maxdeg > 32) { set_last_error("uns_cc_create: a cell has more than 32 faces"); return fail(UNS_ERR_MESH); }
         if (noc >= (1 << 30)) { set_last_error("uns_cc_create: too many cells"); return fail(UNS_ERR_MESH); }
         int dev = 0, nsm = 0, per = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        if (sweep_allow_smem<false>(k_lusgs) != cudaSuccess || sweep_allow_smem<true>(k_lusgs_mixed) != cudaSuccess ||
+            cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_lusgs, kSweepBlock, sweep_smem_bytes<false>()) != cudaSuccess || per < 1) {
             set_last_error("uns_cc_create: cannot size the cooperative LU-SGS launch");
             return fail(UNS_ERR_CUDA);
@@ -2126,6 +2127,8 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
                 nbr[k] = other(i, m->c2f[k], &fl);
             }
         WarpSchedule ws = list_schedule(noc, m->c2f_off, nbr.data(), h->coop_blocks * kSweepPairs);
+        const std::vector<int> at = record_places(ws);
+        std::vector<int> src;
         std::vector<int4> sched(ws.items.size());
         std::vector<int> rf, rn, rl;
         for (size_t pos = 0; pos < ws.items.size(); ++pos) {
@@ -2134,13 +2137,15 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
             for (int k = m->c2f_off[it]; k < m->c2f_off[it + 1]; ++k) {
                 int fl, nb = other(it, m->c2f[k], &fl);
                 bool take = nb >= 0 && nb < noc && (pass == 0 ? nb < it : nb > it);
-                if (take) { rf.push_back(m->c2f[k]); rn.push_back(nb); rl.push_back(fl); }
+                if (take) { rf.push_back(m->c2f[k]); rn.push_back(nb); rl.push_back(fl);
+                    const int from = (nb << 1) | pass;
+                    src.push_back(ws.warp[from] / kSchedGroup == ws.warp[ws.items[pos]] / kSchedGroup ? at[from] : -1); }
             }
             sched[pos] = make_int4(it, pass, first, (int)rf.size() - first);
         }
         v.nrec = (int)rf.size();
         if ((rc = h->upload(h->woff, ws.off.data(), ws.off.size()))) return fail(rc);
-        UP(sched, sched); UP(rec_face, rf); UP(rec_nb, rn); UP(rec_flip, rl);
+        UP(sched, sched); UP(rec_face, rf); UP(rec_nb, rn); UP(rec_flip, rl); UP(rec_src, src);
         AL(rec, 3 * rf.size());
         AL(srec, 10 * (size_t)noc);
     }

@@ -123,10 +123,13 @@ __device__ __forceinline__ float dflux_k(const Rec& e, float gm1, const float dq
     const float un2 = e.un + dun;
     const float df1 = dr * un2 + e.rho * dun;  // change of rho u.n
     const float run = e.rho * e.un;
-    if (k == 0) return (dE + dp) * un2 + (e.E + e.p) * dun;
-    if (k == 1) return df1;
-    if (k == 2) return df1 * u2 + run * du + dp * e.nx;
-    return df1 * v2 + run * dv + dp * e.ny;
+    // the four components as one pass of selected operands (a warp's lanes
+    // hold all four): k = 0 (dE + dp) un2 + (E + p) dun, k = 1 df1, k = 2 and
+    // 3 df1 (u2 or v2) + run (du or dv) + dp (nx or ny)
+    const float x = k == 0 ? dE + dp : df1, y = k == 0 ? un2 : (k == 2 ? u2 : v2);
+    const float z = k == 0 ? e.E + e.p : run, w = k == 0 ? dun : (k == 2 ? du : dv);
+    const float s = x * y + z * w;
+    return k == 1 ? df1 : (k == 0 ? s : s + dp * (k == 2 ? e.nx : e.ny));
 }
 
 // Publishes a mixed-form sweep record: lane 0 the FP32 dq (one float4

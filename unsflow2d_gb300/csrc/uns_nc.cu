@@ -76,6 +76,7 @@ struct NCView {
     const int* rec_edge;
     const int* rec_nb;
     const int* rec_sign;
+    const int* rec_src;  // producer in the same block (record_places), or -1
     int nrec;
     double4* rec;    // per record, per LU-SGS call: 3 x double4 (k_nc_sweep_prep) or 4 x float4 (k_nc_sweep_prep_mixed)
     double* diag;    // LU-SGS diagonal cv/dt + 0.5*omega*la (lusgs.f90:36)
@@ -707,7 +708,7 @@ __global__ void __launch_bounds__(kBlock) k_nc_sweep_prep_mixed(NCView v) {
 
 SweepArgs sweep_args(const NCView& v, bool mixed) {
     SweepArgs a;
-    a.n = v.nop; a.sched = v.sched; a.rec = v.rec;
+    a.n = v.nop; a.sched = v.sched; a.rec = v.rec; a.rec_src = v.rec_src;
     a.diag = mixed ? v.diaginv : v.diag;
     a.qold = v.qold; a.res = v.res; a.qc = v.qc;
     a.out = v.srec; a.outf = reinterpret_cast<float4*>(v.srec); a.outd = reinterpret_cast<double4*>(v.srec + 2 * (size_t)v.nop);
@@ -1050,7 +1051,8 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
         if (maxdeg > 32) { set_last_error("uns_nc_create: a node has more than 32 edges"); return fail(UNS_ERR_MESH); }
         if (nop >= (1 << 30)) { set_last_error("uns_nc_create: too many nodes"); return fail(UNS_ERR_MESH); }
         int dev = 0, nsm = 0, per = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        if (sweep_allow_smem<false>(k_nc_lusgs) != cudaSuccess || sweep_allow_smem<true>(k_nc_lusgs_mixed) != cudaSuccess ||
+            cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_nc_lusgs, kSweepBlock, sweep_smem_bytes<false>()) != cudaSuccess || per < 1) {
             set_last_error("uns_nc_create: cannot size the cooperative LU-SGS launch");
             return fail(UNS_ERR_CUDA);
@@ -1072,6 +1074,8 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
         WarpSchedule ws = list_schedule(nop, m->v2f_off, nbr.data(), h->coop_blocks * kSweepPairs);
         h->lev_fwd = ws.nlev_fwd;
         h->lev_bwd = ws.nlev_bwd;
+        const std::vector<int> at = record_places(ws);
+        std::vector<int> src;
         std::vector<int4> sched(ws.items.size());
         std::vector<int> re, rn, rs;
         for (size_t pos = 0; pos < ws.items.size(); ++pos) {
@@ -1080,13 +1084,15 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
             for (int k = m->v2f_off[it]; k < m->v2f_off[it + 1]; ++k) {
                 int sg, nb = other(it, m->v2f[k], &sg);
                 bool take = nb >= 0 && nb < nop && (pass == 0 ? nb < it : nb > it);
-                if (take) { re.push_back(m->v2f[k]); rn.push_back(nb); rs.push_back(sg); }
+                if (take) { re.push_back(m->v2f[k]); rn.push_back(nb); rs.push_back(sg);
+                    const int from = (nb << 1) | pass;
+                    src.push_back(ws.warp[from] / kSchedGroup == ws.warp[ws.items[pos]] / kSchedGroup ? at[from] : -1); }
             }
             sched[pos] = make_int4(it, pass, first, (int)re.size() - first);
         }
         h->v.nrec = (int)re.size();
         if ((rc = h->upload(h->woff, ws.off.data(), ws.off.size()))) return fail(rc);
-        UPN(sched, sched); UPN(rec_edge, re); UPN(rec_nb, rn); UPN(rec_sign, rs);
+        UPN(sched, sched); UPN(rec_edge, re); UPN(rec_nb, rn); UPN(rec_sign, rs); UPN(rec_src, src);
         ALN(rec, 3 * re.size());
     }
 #undef UPN

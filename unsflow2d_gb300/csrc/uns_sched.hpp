@@ -8,12 +8,20 @@
 // latency-bound: what matters is how fast one item can follow another.
 //
 // An item that follows a predecessor computed by the same warp takes its
-// values from registers; one that follows another warp's item must see that
-// item's published record in L2.  list_schedule assigns the items to warps by
-// greedy list scheduling on that cost model (an item costs kCompute; a
-// cross-warp edge adds kSync): each item, in topological order, goes to the
-// warp of its last-finishing predecessor when that warp has nothing newer
-// queued, else to the warp that frees up first, whichever starts it earlier.
+// values from registers; one that follows an item of another warp of its block
+// reads them in shared memory; one that follows another block's must see the
+// published record in L2.  list_schedule assigns the items to warps by greedy
+// list scheduling on that cost model (an item costs kCompute, an edge between
+// warps of a block kNear, between blocks kSync): each item, in topological
+// order, goes to the warp that starts it earliest among those of its
+// predecessors whose newest item that is, the warps of its predecessors'
+// blocks, and the warp that frees up first.
+//
+// Costs by measurement and replay (NCFVM 1024x512, hand-offs of 0.1 of an item
+// inside a block and 0.55 between blocks, in levels of the graph): 1.27 with
+// one cost for every edge and no preference for a block, 1.13 with 0.05 and
+// 0.30 as below, 1.17 with the hand-offs' own 0.1 and 0.55, which spread the
+// chains less.
 //
 // Each warp's list is in increasing simulated start time and every
 // dependency of an item has a strictly earlier simulated start, so with all
@@ -32,14 +40,19 @@ namespace uns {
 struct WarpSchedule {
     std::vector<int> off;    // nwarps + 1 offsets into items
     std::vector<int> items;  // (entity << 1) | pass, pass 0 = forward, 1 = backward
+    std::vector<int> warp;   // item code -> its warp
     double makespan = 0.0;   // simulated length in units of one item's compute
     int nlev_fwd = 0, nlev_bwd = 0;
 };
 
+constexpr int kSchedGroup = 4;  // consecutive warps of a block
+
 // nbr_off / nbr: CSR neighbour lists of the n entities (any order, entries
-// outside [0, n) ignored).  nwarps: warps of the cooperative launch.  kSync:
-// the extra delay of a cross-warp dependency, in units of one item's compute.
-inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int nwarps, double kSync = 0.25) {
+// outside [0, n) ignored).  nwarps: warps of the cooperative launch.  kNear,
+// kSync: the extra delay of a dependency on another warp of the block and of
+// another block, in units of one item's compute.
+inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int nwarps, double kNear = 0.05,
+                                  double kSync = 0.30) {
     constexpr double kCompute = 1.0;
     // Topological orders: forward by dependency level (then index), backward
     // by backward level (then descending index).
@@ -89,28 +102,26 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
         // ready time of the item on warp w
         auto start_on = [&](int w) {
             double s = wfree[w];
-            for (int p : preds) s = std::max(s, fin[p] + (wof[p] == w ? 0.0 : kSync));
+            for (int p : preds) {
+                const int v = wof[p];
+                s = std::max(s, fin[p] + (v == w ? 0.0 : (v / kSchedGroup == w / kSchedGroup ? kNear : kSync)));
+            }
             return s;
         };
-        // candidate warps: those whose newest item is a predecessor (the
-        // chain continues there); ties go to the predecessor nearest in
-        // index, so chains follow the mesh numbering where they can
-        const int self = code >> 1;
-        int wa = -1, da = 0;
-        double sa = 0.0;
+        int w = -1;
+        double s = 0.0;
+        auto consider = [&](int c) {
+            const double t = start_on(c);
+            if (w < 0 || t < s - 1e-12) { w = c; s = t; }
+        };
+        for (int p : preds)
+            if (wlast[wof[p]] == p) consider(wof[p]);
         for (int p : preds) {
-            int w = wof[p];
-            if (wlast[w] != p) continue;
-            double s = start_on(w);
-            int dist = std::abs((p >> 1) - self);
-            if (wa < 0 || s < sa || (s == sa && dist < da)) { wa = w; sa = s; da = dist; }
+            const int g = wof[p] / kSchedGroup * kSchedGroup;
+            for (int c = g; c < g + kSchedGroup && c < nwarps; ++c) consider(c);
         }
         while (heap.top().first != wfree[heap.top().second]) heap.pop();  // drop stale entries
-        int wb = heap.top().second;
-        double sb = start_on(wb);
-        int w = wb;
-        double s = sb;
-        if (wa >= 0 && sa <= sb) { w = wa; s = sa; }
+        consider(heap.top().second);
         fin[code] = s + kCompute;
         wof[code] = w;
         wfree[w] = fin[code];
@@ -141,9 +152,20 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
     out.nlev_bwd = nlevb;
     out.off.assign(nwarps + 1, 0);
     for (int w = 0; w < nwarps; ++w) out.off[w + 1] = out.off[w] + (int)lists[w].size();
+    out.warp = wof;
     out.items.reserve(2 * (size_t)n);
     for (int w = 0; w < nwarps; ++w) out.items.insert(out.items.end(), lists[w].begin(), lists[w].end());
     return out;
+}
+
+// Per item code: where the sweep warps of its block find its record, (warp of
+// the block << 28) | list index.
+inline std::vector<int> record_places(const WarpSchedule& ws) {
+    std::vector<int> at(ws.items.size());
+    for (size_t w = 0; w + 1 < ws.off.size(); ++w)
+        for (int k = ws.off[w]; k < ws.off[w + 1]; ++k)
+            at[ws.items[k]] = (int)(w % kSchedGroup) << 28 | (k - ws.off[w]);
+    return at;
 }
 
 }  // namespace uns

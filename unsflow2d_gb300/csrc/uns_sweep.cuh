@@ -32,6 +32,8 @@
 #include "uns_common.cuh"
 #include "uns_fp64.cuh"
 
+#include <type_traits>
+
 namespace uns {
 
 constexpr int kSweepPairs = 4;                   // sweep warps per block: one per SM sub-partition
@@ -45,6 +47,7 @@ constexpr double kOmega = 1.5;                   // CCFVM/lusgs.F90:229, NCFVM/l
 struct SweepArgs {
     int n;                 // entities
     const int4* sched;     // (entity, pass, first record, records) per list position
+    const int* rec_src;    // per record: its producer in this block (warp << 28 | list index), or -1
     const double4* rec;    // inputs per record (k_*_sweep_prep): 3 x double4, or 4 x float4 in the mixed form
     const double* diag;    // the diagonal, or its reciprocal in the mixed form
     const double4* qold;
@@ -117,6 +120,43 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity
     }
 }
 
+// The last kBox records of a sweep warp, for the warps of its block: a record
+// that a neighbouring warp needs is read here a few hundred cycles after its
+// item ends, against 1 500-2 900 through L2 (store, poll, the two dies).
+// seq[slot] is the list index of the record in the slot, ~index from the start
+// of the item that will write it; a reader checks it before and after, and
+// where the slot has moved on, or is about to (the item that takes it over may
+// wait for the reader's), it takes the global record, published long before.
+constexpr int kBox = 16;
+template <int NP>
+struct __align__(16) SweepBox {
+    double2 rec[kBox][NP];
+    int seq[kBox];
+};
+template <int NP>
+__device__ __forceinline__ void box_init(SweepBox<NP>& b) {
+    for (int i = 0; i < kBox; ++i) b.seq[i] = ~0;
+}
+__device__ __forceinline__ int ld_acquire(const int* p) {
+    int x;
+    asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(x) : "r"(smem_addr(p)) : "memory");
+    return x;
+}
+__device__ __forceinline__ void st_release(int* p, int x) {
+    asm volatile("st.release.cta.shared.s32 [%0], %1;" : : "r"(smem_addr(p)), "r"(x) : "memory");
+}
+// Marks the slot of list index idx as being written (lane 0, early in the item).
+template <int NP>
+__device__ __forceinline__ void box_open(SweepBox<NP>& b, int idx) {
+    *(volatile int*)&b.seq[idx % kBox] = ~idx;
+    __threadfence_block();
+}
+
+// Where a record comes from, in the upper word of an entry's code field: bits
+// 0..30 one more than (warp of the block << 28 | list index), 0 for another
+// block's; bit 31 the orientation's sign.
+__device__ __forceinline__ int src_of(long long code) { return (int)((unsigned long long)code >> 32 & 0x7fffffffu) - 1; }
+
 // Position in the ring: stage and the parity of its next phase.
 struct RingPos {
     int stage = 0;
@@ -152,6 +192,7 @@ __device__ __forceinline__ bool poller_go_on(int spins, long long& t0, const Swe
 // sign of the record's orientation in the upper word.
 enum { SF_F1, SF_NX, SF_NY, SF_DS, SF_OL, SF_U, SF_V, SF_P, SF_ET, SF_RHO, SF_DQ, SF_D2, SF_O, SF_R, SF_CODE, SF_N };
 typedef SweepRing<SF_N> RingD;
+typedef SweepBox<5> BoxD;  // the record's five 16-byte pieces
 
 __device__ __forceinline__ void sweep_feed(const SweepArgs& a, RingD& R, int kbeg, int kend, int lane) {
     const int slot = lane >> 2, k = lane & 3;
@@ -166,7 +207,9 @@ __device__ __forceinline__ void sweep_feed(const SweepArgs& a, RingD& R, int kbe
             const bool take = base + slot < ntake;
             double4 b = make_double4(0.0, 0.0, 0.0, 0.0), c = b;
             double f1 = 0.0, D = 1.0, o = 1.0, r = 0.0;
+            int src = -1;
             if (take) {
+                src = a.rec_src[S.z + base + slot];
                 const double4* p = a.rec + 3 * (size_t)(S.z + base + slot);
                 f1 = reinterpret_cast<const double*>(p)[k];
                 b = p[1];
@@ -183,7 +226,7 @@ __device__ __forceinline__ void sweep_feed(const SweepArgs& a, RingD& R, int kbe
             double(*f)[32] = R.f[pos.stage];
             f[SF_F1][lane] = f1;
             f[SF_NX][lane] = b.x; f[SF_NY][lane] = b.y; f[SF_DS][lane] = b.z; f[SF_OL][lane] = b.w;
-            f[SF_CODE][lane] = dmake(dhi(c.y) & 0x80000000u, (unsigned)code);
+            f[SF_CODE][lane] = dmake((dhi(c.y) & 0x80000000u) | (unsigned)(src + 1), (unsigned)code);
             const double none = nb ? unset() : 0.0;
             f[SF_U][lane] = none; f[SF_V][lane] = none; f[SF_P][lane] = none;
             f[SF_ET][lane] = none; f[SF_RHO][lane] = none; f[SF_DQ][lane] = none;
@@ -204,7 +247,7 @@ __device__ __forceinline__ void sweep_feed(const SweepArgs& a, RingD& R, int kbe
     }
 }
 
-__device__ __forceinline__ void sweep_poll(const SweepArgs& a, RingD& R, int kbeg, int kend, int lane) {
+__device__ __forceinline__ void sweep_poll(const SweepArgs& a, RingD& R, const BoxD* boxes, int kbeg, int kend, int lane) {
     const int k = lane & 3;
     RingPos pos;
     for (int kk = kbeg; kk < kend; ++kk) {
@@ -214,7 +257,9 @@ __device__ __forceinline__ void sweep_poll(const SweepArgs& a, RingD& R, int kbe
             double(*f)[32] = R.f[pos.stage];
             const int4 S = R.item[pos.stage];  // (base > 0: the stage's older item, unused)
             if (base == 0) ntake = S.w;
-            const int code = (int)__double_as_longlong(ld_field(&f[SF_CODE][lane]));
+            const long long cs = __double_as_longlong(ld_field(&f[SF_CODE][lane]));
+            const int code = (int)cs;
+            int src = src_of(cs);
             bool nb = is_unset(ld_field(&f[SF_DQ][lane]));
             bool own = base == 0 && lane < 4 && is_unset(ld_field(&f[SF_R][lane]));
             const double2* p = a.out + 5 * ((size_t)(code & 1) * a.n + (nb ? code >> 1 : 0));
@@ -222,9 +267,23 @@ __device__ __forceinline__ void sweep_poll(const SweepArgs& a, RingD& R, int kbe
             long long t0 = 0;
             for (int spins = 0; nb || own; ++spins) {
                 if (nb) {
-                    const double2 x0 = ld_relaxed2(p), x1 = ld_relaxed2(p + 1);
-                    const double rho = ld_relaxed(reinterpret_cast<const double*>(p) + 4);
-                    const double dq = ld_relaxed(reinterpret_cast<const double*>(p) + 5 + k);
+                    double2 x0, x1;
+                    double rho, dq;
+                    if (src >= 0) {
+                        const BoxD& b = boxes[src >> 28];
+                        const int idx = src & 0xfffffff, seq = ld_acquire(&b.seq[idx % kBox]);
+                        const volatile double* q = reinterpret_cast<const volatile double*>(b.rec[idx % kBox]);
+                        x0.x = q[0]; x0.y = q[1]; x1.x = q[2]; x1.y = q[3];
+                        rho = q[4]; dq = q[5 + k];
+                        __threadfence_block();
+                        const bool same = seq == idx && *(const volatile int*)&b.seq[idx % kBox] == idx;
+                        if (!same) x0.x = unset();
+                        if ((seq < 0 ? ~seq : seq) > idx) src = -1;  // the slot has moved on
+                    } else {
+                        x0 = ld_relaxed2(p); x1 = ld_relaxed2(p + 1);
+                        rho = ld_relaxed(reinterpret_cast<const double*>(p) + 4);
+                        dq = ld_relaxed(reinterpret_cast<const double*>(p) + 5 + k);
+                    }
                     if (!(is_unset(x0.x) || is_unset(x0.y) || is_unset(x1.x) || is_unset(x1.y) || is_unset(rho) || is_unset(dq))) {
                         st_field(&f[SF_U][lane], x0.x); st_field(&f[SF_V][lane], x0.y); st_field(&f[SF_P][lane], x1.x);
                         st_field(&f[SF_ET][lane], x1.y); st_field(&f[SF_RHO][lane], rho); st_field(&f[SF_DQ][lane], dq);
@@ -263,55 +322,81 @@ __device__ __forceinline__ void sweep_poll(const SweepArgs& a, RingD& R, int kbe
 //
 // Sums and products are register FMAs (64 cycles each); the two divisions (590
 // cycles each on the FP64 unit) run on the integer pipe (240).  %PERF%
+// An entry of the ring in registers.
+struct SweepEntry {
+    double f1, nx, ny, ds, ol, u, v, p, et, rho, dq, D2, o, r;
+    long long code;
+    int4 item;
+    __device__ __forceinline__ void neighbour(const double (*f)[32], int lane) {
+        u = ld_field(&f[SF_U][lane]); v = ld_field(&f[SF_V][lane]); p = ld_field(&f[SF_P][lane]);
+        et = ld_field(&f[SF_ET][lane]); rho = ld_field(&f[SF_RHO][lane]); dq = ld_field(&f[SF_DQ][lane]);
+    }
+    __device__ __forceinline__ void load(const RingD& R, int stage, int lane, bool first) {
+        const double(*f)[32] = R.f[stage];
+        f1 = f[SF_F1][lane]; nx = f[SF_NX][lane]; ny = f[SF_NY][lane]; ds = f[SF_DS][lane]; ol = f[SF_OL][lane];
+        code = __double_as_longlong(f[SF_CODE][lane]);
+        neighbour(f, lane);
+        if (first) {
+            item = R.item[stage];
+            D2 = f[SF_D2][lane]; o = f[SF_O][lane];
+            r = ld_field(&f[SF_R][lane]);
+        }
+    }
+    __device__ __forceinline__ bool waits() const {
+        return is_unset(u) || is_unset(v) || is_unset(p) || is_unset(et) || is_unset(rho) || is_unset(dq) || is_unset(r);
+    }
+};
+
 template <bool kCC>
-__device__ __forceinline__ void sweep_items(const SweepArgs& a, RingD& R, double* wx, int kbeg, int kend, int lane) {
+__device__ __forceinline__ void sweep_items(const SweepArgs& a, RingD& R, BoxD& box, double* wx, int kbeg, int kend, int lane) {
+    const unsigned all = 0xffffffffu;
     const int k = lane & 3;
-    const double gm1 = in_register(a.gm1);
+    const double gm1 = in_register(a.gm1), one = opaque_one(), mzero = opaque_mzero();
     RingPos pos;
     int last = -1;  // code of the warp's previous item; its values below, in every lane
     double Lu = 0.0, Lv = 0.0, Lp = 0.0, Let = 0.0, Lrho = 0.0, Ldq = 0.0;
+    SweepEntry X;
+    X.r = 0.0;
     for (int kk = kbeg; kk < kend; ++kk) {
         double cres = 0.0;  // lanes 0..3: sum over the terms of component k
-        double D2 = 2.0, xo = 1.0, r = 0.0;
-        unsigned Y = 0;  // the diagonal's reciprocal digits, off the chain
+        unsigned Y = 0;     // the diagonal's reciprocal digits, off the chain
+        const int idx = kk - kbeg, bslot = idx % kBox;
+        if (lane == 0) box_open(box, idx);
         int it = 0, pass = 0, ntake = 0, base = 0;
         do {
             if (!mbar_wait(&R.full[pos.stage], pos.phase, RingWait(&R.abort, a))) return;
-            const double(*f)[32] = R.f[pos.stage];
-            if (base == 0) {
-                const int4 S = R.item[pos.stage];
-                it = S.x; pass = S.y; ntake = S.w;
-                D2 = f[SF_D2][lane]; xo = f[SF_O][lane];
-                Y = div_recip(D2);
-            }
-            const long long cs = __double_as_longlong(f[SF_CODE][lane]);
-            const double f1 = f[SF_F1][lane], nx = f[SF_NX][lane], ny = f[SF_NY][lane], ds = f[SF_DS][lane], ol = f[SF_OL][lane];
-            double u, v, p, et, rho, dq;
-            RingWait w(&R.abort, a);
-            for (int spins = 0;; ++spins) {
-                u = ld_field(&f[SF_U][lane]); v = ld_field(&f[SF_V][lane]); p = ld_field(&f[SF_P][lane]);
-                et = ld_field(&f[SF_ET][lane]); rho = ld_field(&f[SF_RHO][lane]); dq = ld_field(&f[SF_DQ][lane]);
-                if (base == 0) r = ld_field(&f[SF_R][lane]);
-                const bool wait = is_unset(u) || is_unset(v) || is_unset(p) || is_unset(et) || is_unset(rho) || is_unset(dq) || is_unset(r);
-                if (!__any_sync(0xffffffffu, wait)) break;
-                if (__any_sync(0xffffffffu, !w.go_on(spins))) return;
+            X.load(R, pos.stage, lane, base == 0);
+            if (__any_sync(all, X.waits())) {
+                RingWait w(&R.abort, a);
+                for (int spins = 0;; ++spins) {
+                    X.neighbour(R.f[pos.stage], lane);
+                    if (base == 0) X.r = ld_field(&R.f[pos.stage][SF_R][lane]);
+                    if (!__any_sync(all, X.waits())) break;
+                    if (__any_sync(all, !w.go_on(spins))) return;
+                }
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&R.empty[pos.stage]);
             pos.next();
-            if (ntake == 0) break;
-            const int code = (int)cs;
-            if (code == last && code >= 0) { u = Lu; v = Lv; p = Lp; et = Let; rho = Lrho; dq = Ldq; }
+            if (base == 0) {
+                it = X.item.x; pass = X.item.y; ntake = X.item.w;
+                Y = div_recip(X.D2);
+                if (ntake == 0) break;
+            }
+            const int code = (int)X.code;
+            if (code == last && code >= 0) { X.u = Lu; X.v = Lv; X.p = Lp; X.et = Let; X.rho = Lrho; X.dq = Ldq; }
             // normal flux (CCFVM/lusgs.F90:348-357, NCFVM/lusgs.f90:144-150)
-            // component k, then the term; idle slots compute on zeros
-            const double un = add64(mul64(u, nx), mul64(v, ny));
-            const double o1 = mul64(rho, un);
-            const double h = add64(et, p);
-            const double prod = mul64(k == 0 ? h : o1, k == 0 ? un : (k == 2 ? u : v));
-            const double sum = add64(prod, mul64(p, k == 2 ? nx : ny));
-            const double o = k == 1 ? o1 : (k == 0 ? prod : sum);
-            const double df = kCC ? mul64(ds, sub64(o, f1)) : flip64(sub64(mul64(o, ds), f1), cs < 0);
-            const double t = sub64(df, mul64(ol, dq));
+            // component k, then the term; idle slots compute on zeros.  Lane k
+            // = 0 forms (et + p)*un, k = 1 rho*un, k = 2 and 3 rho*un*(u or v)
+            // + p*(nx or ny): one FMA with per-lane operands does an addition
+            // in some lanes and a product in others (x*1 + y, x*y + -0).
+            const double un = add64(mul64(X.u, X.nx), mul64(X.v, X.ny));
+            const double hp = __fma_rn(k == 0 ? X.et : X.p, k == 0 ? one : (k == 2 ? X.nx : X.ny), k == 0 ? X.p : mzero);
+            const double A = mul64(k == 0 ? hp : X.rho, un);
+            const double B = __fma_rn(A, k < 2 ? one : (k == 2 ? X.u : X.v), mzero);
+            const double o = k < 2 ? B : add64(B, hp);
+            const double df = kCC ? mul64(X.ds, sub64(o, X.f1)) : flip64(sub64(mul64(o, X.ds), X.f1), X.code < 0);
+            const double t = sub64(df, mul64(X.ol, X.dq));
             // the terms in order, from 0.0 (the first addition is exact)
             const int nr = min(8, ntake - base);
             wx[lane] = t;
@@ -326,12 +411,11 @@ __device__ __forceinline__ void sweep_items(const SweepArgs& a, RingD& R, double
         // 78-81, 117-120), component k in lane k
         double d;
         if (pass == 0) {
-            d = div_digits(sub64(neg64(r), cres), D2, Y);
+            d = div_digits(sub64(neg64(X.r), cres), X.D2, Y);
         } else {  // from the entity's own forward dq
-            if ((it << 1) == last) r = Ldq;
-            d = sub64(r, div_digits(cres, D2, Y));
+            d = sub64((it << 1) == last ? Ldq : X.r, div_digits(cres, X.D2, Y));
         }
-        const double q = add64(xo, d);
+        const double q = add64(X.o, d);
         // con2prim (CCFVM/types/pri.F90:13-37, NCFVM/All_modules.f90:146-169):
         // rho = q1, then E/rho, rhou/rho, rhov/rho in lanes 0, 2, 3
         if (lane < 4) { wx[lane] = q; wx[5 + lane] = d; }
@@ -360,6 +444,9 @@ __device__ __forceinline__ void sweep_items(const SweepArgs& a, RingD& R, double
             // predicated instruction
             double2* dst = a.out + 5 * ((size_t)pass * a.n + it) + (lane < 5 ? lane : 0);
             const double x = lane == 1 ? Lp : piece.x, y = lane == 1 ? Let : piece.y;
+            if (lane < 5) box.rec[bslot][lane] = make_double2(x, y);
+            __syncwarp();
+            if (lane == 0) st_release(&box.seq[bslot], idx);
             asm volatile(
                 "{\n\t.reg .pred pa;\n\t"
                 "setp.ne.s32 pa, %0, 0;\n\t"
@@ -383,6 +470,7 @@ struct SweepRecM {
 // Fields of an entry: two floats to a field.
 enum { MF_R01, MF_R23, MF_UV, MF_PUN, MF_N, MF_DSOL, MF_DQ01, MF_DQ23, MF_D, MF_O, MF_R, MF_CODE, MF_COUNT };
 typedef SweepRing<MF_COUNT> RingM;
+typedef SweepBox<1> BoxM;  // dq in FP32
 
 // kCC: the reference halves the sum of the terms; here res is doubled and the
 // diagonal's reciprocal halved instead.  (NCFVM halves each term in FP32.)
@@ -400,7 +488,9 @@ __device__ __forceinline__ void sweep_feed_mixed(const SweepArgs& a, RingM& R, i
             const bool take = base + slot < ntake;
             float4 x = make_float4(1.f, 0.f, 0.f, 0.f), b = make_float4(0.f, 0.f, 0.f, 0.f), c = b, d = b;
             double D = 1.0, o = 1.0, r = 0.0;
+            int src = -1;
             if (take) {
+                src = a.rec_src[S.z + base + slot];
                 const float4* p = reinterpret_cast<const float4*>(a.rec) + 4 * (size_t)(S.z + base + slot);
                 x = p[0]; b = p[1]; c = p[2]; d = p[3];
             }
@@ -416,7 +506,7 @@ __device__ __forceinline__ void sweep_feed_mixed(const SweepArgs& a, RingM& R, i
             f[MF_R01][lane] = pack2(x.x, x.y); f[MF_R23][lane] = pack2(x.z, x.w);
             f[MF_UV][lane] = pack2(b.x, b.y); f[MF_PUN][lane] = pack2(b.z, b.w);
             f[MF_N][lane] = pack2(c.x, c.y); f[MF_DSOL][lane] = pack2(c.z, c.w);
-            f[MF_CODE][lane] = dmake(d.x < 0.f ? 0x80000000u : 0u, (unsigned)code);
+            f[MF_CODE][lane] = dmake((d.x < 0.f ? 0x80000000u : 0u) | (unsigned)(src + 1), (unsigned)code);
             const double none = nb ? unset() : 0.0;
             f[MF_DQ01][lane] = none; f[MF_DQ23][lane] = none;
             if (base == 0) {
@@ -436,7 +526,7 @@ __device__ __forceinline__ void sweep_feed_mixed(const SweepArgs& a, RingM& R, i
     }
 }
 
-__device__ __forceinline__ void sweep_poll_mixed(const SweepArgs& a, RingM& R, int kbeg, int kend, int lane) {
+__device__ __forceinline__ void sweep_poll_mixed(const SweepArgs& a, RingM& R, const BoxM* boxes, int kbeg, int kend, int lane) {
     RingPos pos;
     for (int kk = kbeg; kk < kend; ++kk) {
         int ntake = 0, base = 0;
@@ -445,7 +535,9 @@ __device__ __forceinline__ void sweep_poll_mixed(const SweepArgs& a, RingM& R, i
             double(*f)[32] = R.f[pos.stage];
             const int4 S = R.item[pos.stage];
             if (base == 0) ntake = S.w;
-            const int code = (int)__double_as_longlong(ld_field(&f[MF_CODE][lane]));
+            const long long cs = __double_as_longlong(ld_field(&f[MF_CODE][lane]));
+            const int code = (int)cs;
+            int src = src_of(cs);
             bool nb = is_unset(ld_field(&f[MF_DQ23][lane]));
             bool own = base == 0 && lane < 4 && is_unset(ld_field(&f[MF_R][lane]));
             const float4* p = a.outf + (size_t)(code & 1) * a.n + (nb ? code >> 1 : 0);
@@ -454,7 +546,18 @@ __device__ __forceinline__ void sweep_poll_mixed(const SweepArgs& a, RingM& R, i
             for (int spins = 0; nb || own; ++spins) {
                 if (nb) {
                     float w[4];
-                    peek_f4(p, w);
+                    if (src >= 0) {
+                        const BoxM& b = boxes[src >> 28];
+                        const int idx = src & 0xfffffff, seq = ld_acquire(&b.seq[idx % kBox]);
+                        const volatile float* q = reinterpret_cast<const volatile float*>(b.rec[idx % kBox]);
+                        w[0] = q[0]; w[1] = q[1]; w[2] = q[2]; w[3] = q[3];
+                        __threadfence_block();
+                        const bool same = seq == idx && *(const volatile int*)&b.seq[idx % kBox] == idx;
+                        if (!same) w[0] = __uint_as_float(kUnsetF);
+                        if ((seq < 0 ? ~seq : seq) > idx) src = -1;  // the slot has moved on
+                    } else {
+                        peek_f4(p, w);
+                    }
                     if (set_f4(w)) {
                         st_field(&f[MF_DQ01][lane], pack2(w[0], w[1]));
                         st_field(&f[MF_DQ23][lane], pack2(w[2], w[3]));
@@ -479,8 +582,30 @@ __device__ __forceinline__ void sweep_poll_mixed(const SweepArgs& a, RingM& R, i
     }
 }
 
+struct SweepEntryM {
+    double r01, r23, uv, pun, nn, dsol, q01, q23, D, o, r;
+    long long code;
+    int4 item;
+    __device__ __forceinline__ void neighbour(const double (*f)[32], int lane) {
+        q01 = ld_field(&f[MF_DQ01][lane]); q23 = ld_field(&f[MF_DQ23][lane]);
+    }
+    __device__ __forceinline__ void load(const RingM& R, int stage, int lane, bool first) {
+        const double(*f)[32] = R.f[stage];
+        r01 = f[MF_R01][lane]; r23 = f[MF_R23][lane]; uv = f[MF_UV][lane]; pun = f[MF_PUN][lane];
+        nn = f[MF_N][lane]; dsol = f[MF_DSOL][lane];
+        code = __double_as_longlong(f[MF_CODE][lane]);
+        neighbour(f, lane);
+        if (first) {
+            item = R.item[stage];
+            D = f[MF_D][lane]; o = f[MF_O][lane];
+            r = ld_field(&f[MF_R][lane]);
+        }
+    }
+    __device__ __forceinline__ bool waits() const { return is_unset(q01) || is_unset(q23) || is_unset(r); }
+};
+
 template <bool kCC>
-__device__ __forceinline__ void sweep_items_mixed(const SweepArgs& a, RingM& R, int kbeg, int kend, int lane) {
+__device__ __forceinline__ void sweep_items_mixed(const SweepArgs& a, RingM& R, BoxM& box, int kbeg, int kend, int lane) {
     const unsigned all = 0xffffffffu;
     const int k = lane & 3;
     const float gm1 = (float)a.gm1;
@@ -488,41 +613,41 @@ __device__ __forceinline__ void sweep_items_mixed(const SweepArgs& a, RingM& R, 
     int last = -1;
     float LF[4] = {0.f, 0.f, 0.f, 0.f};  // previous item's dq (FP32)
     double Lk = 0.0;                     // and in FP64, component k
+    SweepEntryM X;
+    X.r = 0.0;
     for (int kk = kbeg; kk < kend; ++kk) {
-        double cres = 0.0, xd = 1.0, xo = 1.0, r = 0.0;
+        double cres = 0.0;
+        const int idx = kk - kbeg, bslot = idx % kBox;
+        if (lane == 0) box_open(box, idx);
         int it = 0, pass = 0, ntake = 0, base = 0;
         do {
             if (!mbar_wait(&R.full[pos.stage], pos.phase, RingWait(&R.abort, a))) return;
-            const double(*f)[32] = R.f[pos.stage];
-            if (base == 0) {
-                const int4 S = R.item[pos.stage];
-                it = S.x; pass = S.y; ntake = S.w;
-                xd = f[MF_D][lane]; xo = f[MF_O][lane];
-            }
-            const double r01 = f[MF_R01][lane], r23 = f[MF_R23][lane], uv = f[MF_UV][lane], pun = f[MF_PUN][lane];
-            const double nn = f[MF_N][lane], dsol = f[MF_DSOL][lane];
-            const long long cs = __double_as_longlong(f[MF_CODE][lane]);
-            double q01, q23;
-            RingWait w(&R.abort, a);
-            for (int spins = 0;; ++spins) {
-                q01 = ld_field(&f[MF_DQ01][lane]); q23 = ld_field(&f[MF_DQ23][lane]);
-                if (base == 0) r = ld_field(&f[MF_R][lane]);
-                if (!__any_sync(all, is_unset(q01) || is_unset(q23) || is_unset(r))) break;
-                if (__any_sync(all, !w.go_on(spins))) return;
+            X.load(R, pos.stage, lane, base == 0);
+            if (__any_sync(all, X.waits())) {
+                RingWait w(&R.abort, a);
+                for (int spins = 0;; ++spins) {
+                    X.neighbour(R.f[pos.stage], lane);
+                    if (base == 0) X.r = ld_field(&R.f[pos.stage][MF_R][lane]);
+                    if (!__any_sync(all, X.waits())) break;
+                    if (__any_sync(all, !w.go_on(spins))) return;
+                }
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&R.empty[pos.stage]);
             pos.next();
-            if (ntake == 0) break;
-            const bool mine = (int)cs == last && (int)cs >= 0;
-            const float dq[4] = {mine ? LF[0] : low_f(q01), mine ? LF[1] : high_f(q01), mine ? LF[2] : low_f(q23),
-                                 mine ? LF[3] : high_f(q23)};
-            const SweepRecM E = {low_f(r01), high_f(r01), low_f(r23), high_f(r23), low_f(uv), high_f(uv),
-                                 low_f(pun), high_f(pun), low_f(nn), high_f(nn)};
+            if (base == 0) {
+                it = X.item.x; pass = X.item.y; ntake = X.item.w;
+                if (ntake == 0) break;
+            }
+            const bool mine = (int)X.code == last && (int)X.code >= 0;
+            const float dq[4] = {mine ? LF[0] : low_f(X.q01), mine ? LF[1] : high_f(X.q01), mine ? LF[2] : low_f(X.q23),
+                                 mine ? LF[3] : high_f(X.q23)};
+            const SweepRecM E = {low_f(X.r01), high_f(X.r01), low_f(X.r23), high_f(X.r23), low_f(X.uv), high_f(X.uv),
+                                 low_f(X.pun), high_f(X.pun), low_f(X.nn), high_f(X.nn)};
             const float df = dflux_k(E, gm1, dq, k);
             const float dqk = k == 0 ? dq[0] : (k == 1 ? dq[1] : (k == 2 ? dq[2] : dq[3]));
-            const double t = widen(kCC ? low_f(dsol) * df - high_f(dsol) * dqk
-                                       : 0.5f * ((cs < 0 ? -df : df) * low_f(dsol) - high_f(dsol) * dqk));
+            const double t = widen(kCC ? low_f(X.dsol) * df - high_f(X.dsol) * dqk
+                                       : 0.5f * ((X.code < 0 ? -df : df) * low_f(X.dsol) - high_f(X.dsol) * dqk));
             const int nr = min(8, ntake - base);
             int e = 0;
             if (base == 0) { cres = zero_plus(__shfl_sync(all, t, k)); e = 1; }  // 0.0 + t0, exact
@@ -531,10 +656,9 @@ __device__ __forceinline__ void sweep_items_mixed(const SweepArgs& a, RingM& R, 
         } while (base < ntake);
         double d;
         if (pass == 0) {
-            d = mul64(sub64(neg64(r), cres), xd);
+            d = mul64(sub64(neg64(X.r), cres), X.D);
         } else {  // from the entity's own forward dq
-            if ((it << 1) == last) r = Lk;
-            d = sub64(r, mul64(cres, xd));
+            d = sub64((it << 1) == last ? Lk : X.r, mul64(cres, X.D));
         }
         const float df = narrow(d);
         LF[0] = __shfl_sync(all, df, 0);
@@ -549,8 +673,12 @@ __device__ __forceinline__ void sweep_items_mixed(const SweepArgs& a, RingM& R, 
         if (last == a.skip_code) {  // test hook: this item publishes nothing and hands nothing on
             last = -1;
         } else {
+            if (lane == 0) {
+                box.rec[bslot][0] = make_double2(pack2(LF[0], LF[1]), pack2(LF[2], LF[3]));
+                st_release(&box.seq[bslot], idx);
+            }
             publish_mixed(lane, a.outf + slotr, reinterpret_cast<double2*>(a.outd + slotr), LF, L0, L1, L2, L3);
-            if (pass == 1 && lane < 4) reinterpret_cast<double*>(&a.qc[it])[lane] = add64(xo, d);
+            if (pass == 1 && lane < 4) reinterpret_cast<double*>(&a.qc[it])[lane] = add64(X.o, d);
         }
     }
 }
@@ -561,28 +689,36 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, const int* __res
     extern __shared__ __align__(16) unsigned char sweep_smem[];
     __shared__ __align__(16) double wxs[kSweepPairs][32];  // per sweep warp: exchange of lane values
     typedef typename std::conditional<kMixed, RingM, RingD>::type Ring;
+    typedef typename std::conditional<kMixed, BoxM, BoxD>::type Box;
     Ring* rings = reinterpret_cast<Ring*>(sweep_smem);
+    Box* boxes = reinterpret_cast<Box*>(sweep_smem + kSweepPairs * sizeof(Ring));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wib = warp % kSweepPairs, role = warp / kSweepPairs;
-    if (threadIdx.x < kSweepPairs) ring_init(rings[threadIdx.x]);
+    if (threadIdx.x < kSweepPairs) { ring_init(rings[threadIdx.x]); box_init(boxes[threadIdx.x]); }
     __syncthreads();
     const int gw = blockIdx.x * kSweepPairs + wib;
     const int kbeg = woff[gw], kend = woff[gw + 1];
     if (kbeg >= kend) return;
     Ring& R = rings[wib];
     if constexpr (kMixed) {
-        if (role == 0) sweep_items_mixed<kCC>(a, R, kbeg, kend, lane);
+        if (role == 0) sweep_items_mixed<kCC>(a, R, boxes[wib], kbeg, kend, lane);
         else if (role == 1) sweep_feed_mixed<kCC>(a, R, kbeg, kend, lane);
-        else sweep_poll_mixed(a, R, kbeg, kend, lane);
+        else sweep_poll_mixed(a, R, boxes, kbeg, kend, lane);
     } else {
-        if (role == 0) sweep_items<kCC>(a, R, wxs[wib], kbeg, kend, lane);
+        if (role == 0) sweep_items<kCC>(a, R, boxes[wib], wxs[wib], kbeg, kend, lane);
         else if (role == 1) sweep_feed(a, R, kbeg, kend, lane);
-        else sweep_poll(a, R, kbeg, kend, lane);
+        else sweep_poll(a, R, boxes, kbeg, kend, lane);
     }
 }
 
 template <bool kMixed>
 constexpr int sweep_smem_bytes() {
-    return kSweepPairs * (int)(kMixed ? sizeof(RingM) : sizeof(RingD));
+    return kSweepPairs * (int)(kMixed ? sizeof(RingM) + sizeof(BoxM) : sizeof(RingD) + sizeof(BoxD));
+}
+
+// Lets a sweep kernel take its dynamic shared memory (over 48 KB).
+template <bool kMixed, class K>
+cudaError_t sweep_allow_smem(K kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sweep_smem_bytes<kMixed>());
 }
 
 }  // namespace uns

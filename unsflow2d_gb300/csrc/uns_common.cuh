@@ -107,31 +107,6 @@ __device__ __forceinline__ bool set_f4(const float w[4]) {
     return !is_unset(w[0]) && !is_unset(w[1]) && !is_unset(w[2]) && !is_unset(w[3]);
 }
 
-// LU-SGS normal flux change F(q + dq) - F(q) along (nx, ny), component k, in
-// FP32 and in delta form: from dq and q's state and primitives (fields rho,
-// ru, rv, E, u, v, p, un = u.n, nx, ny of `e`), never as the difference of
-// two O(1) fluxes, so its rounding error is relative to the change itself.
-// F = ((E + p) u.n, rho u.n, rho u.n u + p nx, rho u.n v + p ny).
-template <class Rec>
-__device__ __forceinline__ float dflux_k(const Rec& e, float gm1, const float dq[4], int k) {
-    const float dE = dq[0], dr = dq[1], dru = dq[2], drv = dq[3];
-    const float rn = e.rho + dr;
-    const float du = (dru - e.u * dr) / rn, dv = (drv - e.v * dr) / rn;
-    const float u2 = e.u + du, v2 = e.v + dv;
-    const float dp = gm1 * (dE - 0.5f * (dru * u2 + e.ru * du + drv * v2 + e.rv * dv));
-    const float dun = du * e.nx + dv * e.ny;
-    const float un2 = e.un + dun;
-    const float df1 = dr * un2 + e.rho * dun;  // change of rho u.n
-    const float run = e.rho * e.un;
-    // the four components as one pass of selected operands (a warp's lanes
-    // hold all four): k = 0 (dE + dp) un2 + (E + p) dun, k = 1 df1, k = 2 and
-    // 3 df1 (u2 or v2) + run (du or dv) + dp (nx or ny)
-    const float x = k == 0 ? dE + dp : df1, y = k == 0 ? un2 : (k == 2 ? u2 : v2);
-    const float z = k == 0 ? e.E + e.p : run, w = k == 0 ? dun : (k == 2 ? du : dv);
-    const float s = x * y + z * w;
-    return k == 1 ? df1 : (k == 0 ? s : s + dp * (k == 2 ? e.nx : e.ny));
-}
-
 // Publishes a mixed-form sweep record: lane 0 the FP32 dq (one float4
 // slot), lane 1 the FP64 dq (two double2), as predicated stores of one
 // instruction sequence; lane-divergent branches around the stores cost a

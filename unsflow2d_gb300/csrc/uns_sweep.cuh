@@ -14,13 +14,13 @@
 // so an addition's result waits for a load in flight (NCFVM 1024x512: 9.56 ms;
 // 7.00 with one helper for loads and polls; %POLL% with two).
 //
-// An entry is handed over through mbarriers: `full` (the feeder has written
-// the inputs and set the neighbours' fields to kUnset) and `empty` (the sweep
-// warp has read the entry and the poller has finished with it).  The poller
-// then writes each neighbour's values as they come, and the sweep warp reads
-// its fields until none holds kUnset, as the poller does the records.  Every
-// wait is bounded; a warp that gives up raises `abort`, on which its partners
-// return.
+// An entry passes from the feeder to the poller through the mbarrier `full`
+// (the inputs are there, the neighbours' fields that must be polled hold
+// kUnset), from the poller to the sweep warp through the count `ready` (a load
+// of shared memory is all that a sweep warp spends where the entry is there;
+// an mbarrier wait took 200 cycles of each item) and back to the feeder
+// through the mbarrier `empty`.  Every wait is bounded; a warp that gives up
+// raises `abort`, on which its partners return.
 //
 // Lanes of an item: lane = 4 * slot + k, slot = the taken face or edge (up to
 // 8 per entry), k = the variable.  An FP64 instruction holds the sub-partition's
@@ -68,8 +68,9 @@ struct __align__(16) SweepRing {
     unsigned long long full[kSweepStages], empty[kSweepStages];
     double f[kSweepStages][NF][32];
     int4 item[kSweepStages];
+    int ready;  // entries that the sweep warp may read
     int abort;
-    int pad[3];
+    int pad[2];
 };
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -78,8 +79,9 @@ template <int NF>
 __device__ __forceinline__ void ring_init(SweepRing<NF>& R) {
     for (int s = 0; s < kSweepStages; ++s) {
         asm volatile("mbarrier.init.shared.b64 [%0], 1;" : : "r"(smem_addr(&R.full[s])) : "memory");
-        asm volatile("mbarrier.init.shared.b64 [%0], 2;" : : "r"(smem_addr(&R.empty[s])) : "memory");
+        asm volatile("mbarrier.init.shared.b64 [%0], 1;" : : "r"(smem_addr(&R.empty[s])) : "memory");
     }
+    R.ready = 0;
     R.abort = 0;
 }
 
@@ -87,6 +89,14 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long* b) {
     asm volatile("mbarrier.arrive.release.cta.shared.b64 _, [%0];" : : "r"(smem_addr(b)) : "memory");
 }
 
+__device__ __forceinline__ int ld_acquire(const int* p) {
+    int x;
+    asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(x) : "r"(smem_addr(p)) : "memory");
+    return x;
+}
+__device__ __forceinline__ void st_release(int* p, int x) {
+    asm volatile("st.release.cta.shared.s32 [%0], %1;" : : "r"(smem_addr(p)), "r"(x) : "memory");
+}
 // A wait inside the ring (all lanes) outlasts the poller's own for a record;
 // it ends early when a partner has aborted.  False: the caller returns.
 struct RingWait {
@@ -120,6 +130,13 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity
     }
 }
 
+// The sweep warp's wait (all lanes) for the ring's entry of that number.
+__device__ __forceinline__ bool entry_wait(const int* ready, int entry, RingWait w) {
+    for (int spins = 0; ld_acquire(ready) < entry; ++spins)
+        if (!w.go_on(spins)) return false;
+    return true;
+}
+
 // The last kBox records of a sweep warp, for the warps of its block: a record
 // that a neighbouring warp needs is read here a few hundred cycles after its
 // item ends, against 1 500-2 900 through L2 (store, poll, the two dies).
@@ -136,14 +153,6 @@ struct __align__(16) SweepBox {
 template <int NP>
 __device__ __forceinline__ void box_init(SweepBox<NP>& b) {
     for (int i = 0; i < kBox; ++i) b.seq[i] = ~0;
-}
-__device__ __forceinline__ int ld_acquire(const int* p) {
-    int x;
-    asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(x) : "r"(smem_addr(p)) : "memory");
-    return x;
-}
-__device__ __forceinline__ void st_release(int* p, int x) {
-    asm volatile("st.release.cta.shared.s32 [%0], %1;" : : "r"(smem_addr(p)), "r"(x) : "memory");
 }
 // Marks the slot of list index idx as being written (lane 0, early in the item).
 template <int NP>
@@ -250,6 +259,7 @@ __device__ __forceinline__ void sweep_feed(const SweepArgs& a, RingD& R, int kbe
 __device__ __forceinline__ void sweep_poll(const SweepArgs& a, RingD& R, const BoxD* boxes, int kbeg, int kend, int lane) {
     const int k = lane & 3;
     RingPos pos;
+    int entries = 0;
     for (int kk = kbeg; kk < kend; ++kk) {
         int ntake = 0, base = 0;
         do {
@@ -301,7 +311,7 @@ __device__ __forceinline__ void sweep_poll(const SweepArgs& a, RingD& R, const B
             }
             if (__any_sync(0xffffffffu, nb || own)) return;  // a wait gave up; the error is recorded
             __syncwarp();
-            if (lane == 0) mbar_arrive(&R.empty[pos.stage]);
+            if (lane == 0) st_release(&R.ready, ++entries);
             pos.next();
             base += 8;
         } while (base < ntake);
@@ -322,28 +332,36 @@ __device__ __forceinline__ void sweep_poll(const SweepArgs& a, RingD& R, const B
 //
 // Sums and products are register FMAs (64 cycles each); the two divisions (590
 // cycles each on the FP64 unit) run on the integer pipe (240).  %PERF%
+// Per-lane selection by a mask (all ones: a) that the compiler does not know
+// to be a comparison of k: as a plain conditional it became branches around
+// the FMA that takes the value, one copy of it per value (64 cycles each).
+__device__ __forceinline__ unsigned lane_mask(bool on) {
+    unsigned m = on ? 0xffffffffu : 0u;
+    asm volatile("" : "+r"(m));
+    return m;
+}
+__device__ __forceinline__ double pick(unsigned m, double a, double b) {
+    return dmake((dhi(a) & m) | (dhi(b) & ~m), (dlo(a) & m) | (dlo(b) & ~m));
+}
+__device__ __forceinline__ float pick(unsigned m, float a, float b) {
+    return __uint_as_float((__float_as_uint(a) & m) | (__float_as_uint(b) & ~m));
+}
+
 // An entry of the ring in registers.
 struct SweepEntry {
     double f1, nx, ny, ds, ol, u, v, p, et, rho, dq, D2, o, r;
     long long code;
     int4 item;
-    __device__ __forceinline__ void neighbour(const double (*f)[32], int lane) {
-        u = ld_field(&f[SF_U][lane]); v = ld_field(&f[SF_V][lane]); p = ld_field(&f[SF_P][lane]);
-        et = ld_field(&f[SF_ET][lane]); rho = ld_field(&f[SF_RHO][lane]); dq = ld_field(&f[SF_DQ][lane]);
-    }
     __device__ __forceinline__ void load(const RingD& R, int stage, int lane, bool first) {
         const double(*f)[32] = R.f[stage];
-        f1 = f[SF_F1][lane]; nx = f[SF_NX][lane]; ny = f[SF_NY][lane]; ds = f[SF_DS][lane]; ol = f[SF_OL][lane];
-        code = __double_as_longlong(f[SF_CODE][lane]);
-        neighbour(f, lane);
         if (first) {
             item = R.item[stage];
-            D2 = f[SF_D2][lane]; o = f[SF_O][lane];
-            r = ld_field(&f[SF_R][lane]);
+            D2 = f[SF_D2][lane]; o = f[SF_O][lane]; r = f[SF_R][lane];
         }
-    }
-    __device__ __forceinline__ bool waits() const {
-        return is_unset(u) || is_unset(v) || is_unset(p) || is_unset(et) || is_unset(rho) || is_unset(dq) || is_unset(r);
+        code = __double_as_longlong(f[SF_CODE][lane]);
+        u = f[SF_U][lane]; v = f[SF_V][lane]; p = f[SF_P][lane];
+        et = f[SF_ET][lane]; rho = f[SF_RHO][lane]; dq = f[SF_DQ][lane];
+        f1 = f[SF_F1][lane]; nx = f[SF_NX][lane]; ny = f[SF_NY][lane]; ds = f[SF_DS][lane]; ol = f[SF_OL][lane];
     }
 };
 
@@ -352,11 +370,14 @@ __device__ __forceinline__ void sweep_items(const SweepArgs& a, RingD& R, BoxD& 
     const unsigned all = 0xffffffffu;
     const int k = lane & 3;
     const double gm1 = in_register(a.gm1), one = opaque_one(), mzero = opaque_mzero();
+    const unsigned m0 = lane_mask(k == 0), m2 = lane_mask(k == 2), m01 = lane_mask(k < 2);
+    const unsigned ml1 = lane_mask(lane == 1), ml01 = lane_mask(lane < 2);
     RingPos pos;
     int last = -1;  // code of the warp's previous item; its values below, in every lane
     double Lu = 0.0, Lv = 0.0, Lp = 0.0, Let = 0.0, Lrho = 0.0, Ldq = 0.0;
     SweepEntry X;
     X.r = 0.0;
+    int entries = 0;
     for (int kk = kbeg; kk < kend; ++kk) {
         double cres = 0.0;  // lanes 0..3: sum over the terms of component k
         unsigned Y = 0;     // the diagonal's reciprocal digits, off the chain
@@ -364,17 +385,8 @@ __device__ __forceinline__ void sweep_items(const SweepArgs& a, RingD& R, BoxD& 
         if (lane == 0) box_open(box, idx);
         int it = 0, pass = 0, ntake = 0, base = 0;
         do {
-            if (!mbar_wait(&R.full[pos.stage], pos.phase, RingWait(&R.abort, a))) return;
+            if (!entry_wait(&R.ready, ++entries, RingWait(&R.abort, a))) return;
             X.load(R, pos.stage, lane, base == 0);
-            if (__any_sync(all, X.waits())) {
-                RingWait w(&R.abort, a);
-                for (int spins = 0;; ++spins) {
-                    X.neighbour(R.f[pos.stage], lane);
-                    if (base == 0) X.r = ld_field(&R.f[pos.stage][SF_R][lane]);
-                    if (!__any_sync(all, X.waits())) break;
-                    if (__any_sync(all, !w.go_on(spins))) return;
-                }
-            }
             __syncwarp();
             if (lane == 0) mbar_arrive(&R.empty[pos.stage]);
             pos.next();
@@ -389,12 +401,13 @@ __device__ __forceinline__ void sweep_items(const SweepArgs& a, RingD& R, BoxD& 
             // component k, then the term; idle slots compute on zeros.  Lane k
             // = 0 forms (et + p)*un, k = 1 rho*un, k = 2 and 3 rho*un*(u or v)
             // + p*(nx or ny): one FMA with per-lane operands does an addition
-            // in some lanes and a product in others (x*1 + y, x*y + -0).
+            // in some lanes and a product in others (x*1 + y, x*y + -0; B + -0
+            // is B).
             const double un = add64(mul64(X.u, X.nx), mul64(X.v, X.ny));
-            const double hp = __fma_rn(k == 0 ? X.et : X.p, k == 0 ? one : (k == 2 ? X.nx : X.ny), k == 0 ? X.p : mzero);
-            const double A = mul64(k == 0 ? hp : X.rho, un);
-            const double B = __fma_rn(A, k < 2 ? one : (k == 2 ? X.u : X.v), mzero);
-            const double o = k < 2 ? B : add64(B, hp);
+            const double hp = __fma_rn(pick(m0, X.et, X.p), pick(m0, one, pick(m2, X.nx, X.ny)), pick(m0, X.p, mzero));
+            const double A = mul64(pick(m0, hp, X.rho), un);
+            const double B = __fma_rn(A, pick(m01, one, pick(m2, X.u, X.v)), mzero);
+            const double o = __fma_rn(B, one, pick(m01, mzero, hp));
             const double df = kCC ? mul64(X.ds, sub64(o, X.f1)) : flip64(sub64(mul64(o, X.ds), X.f1), X.code < 0);
             const double t = sub64(df, mul64(X.ol, X.dq));
             // the terms in order, from 0.0 (the first addition is exact)
@@ -425,7 +438,7 @@ __device__ __forceinline__ void sweep_items(const SweepArgs& a, RingD& R, BoxD& 
         const double quo = div_digits(q, rn);
         // the four products of the pressure and the record as one
         // multiplication: lane 0 e*rho, lane 1 0.5*rho, lane 2 u*u, lane 3 v*v
-        const double pr = mul64(lane == 1 ? 0.5 : quo, lane < 2 ? rn : quo);
+        const double pr = mul64(pick(ml1, 0.5, quo), pick(ml01, rn, quo));
         if (lane < 4) { wx[10 + lane] = quo; wx[14 + lane] = pr; }
         if (lane == 1) wx[4] = rn;
         __syncwarp();
@@ -467,6 +480,28 @@ struct SweepRecM {
     float rho, ru, rv, E, u, v, p, un, nx, ny;  // the slot's record, as dflux_k reads it
 };
 
+// LU-SGS normal flux change F(q + dq) - F(q) along (nx, ny), component k (the
+// lane's masks), in FP32 and in delta form: from dq and q's state and
+// primitives, never as the difference of two O(1) fluxes, so its rounding
+// error is relative to the change itself.
+// F = ((E + p) u.n, rho u.n, rho u.n u + p nx, rho u.n v + p ny).
+__device__ __forceinline__ float dflux_k(const SweepRecM& e, float gm1, const float dq[4], unsigned m0, unsigned m1,
+                                         unsigned m2) {
+    const float dE = dq[0], dr = dq[1], dru = dq[2], drv = dq[3];
+    const float rn = e.rho + dr;
+    const float du = (dru - e.u * dr) / rn, dv = (drv - e.v * dr) / rn;
+    const float u2 = e.u + du, v2 = e.v + dv;
+    const float dp = gm1 * (dE - 0.5f * (dru * u2 + e.ru * du + drv * v2 + e.rv * dv));
+    const float dun = du * e.nx + dv * e.ny;
+    const float un2 = e.un + dun;
+    const float df1 = dr * un2 + e.rho * dun;  // change of rho u.n
+    const float run = e.rho * e.un;
+    // k = 0 (dE + dp) un2 + (E + p) dun, k = 1 df1, k = 2 and 3 df1 (u2 or v2)
+    // + run (du or dv) + dp (nx or ny)
+    const float s = pick(m0, dE + dp, df1) * pick(m0, un2, pick(m2, u2, v2)) + pick(m0, e.E + e.p, run) * pick(m0, dun, pick(m2, du, dv));
+    return pick(m1, df1, pick(m0, s, s + dp * pick(m2, e.nx, e.ny)));
+}
+
 // Fields of an entry: two floats to a field.
 enum { MF_R01, MF_R23, MF_UV, MF_PUN, MF_N, MF_DSOL, MF_DQ01, MF_DQ23, MF_D, MF_O, MF_R, MF_CODE, MF_COUNT };
 typedef SweepRing<MF_COUNT> RingM;
@@ -507,7 +542,9 @@ __device__ __forceinline__ void sweep_feed_mixed(const SweepArgs& a, RingM& R, i
             f[MF_UV][lane] = pack2(b.x, b.y); f[MF_PUN][lane] = pack2(b.z, b.w);
             f[MF_N][lane] = pack2(c.x, c.y); f[MF_DSOL][lane] = pack2(c.z, c.w);
             f[MF_CODE][lane] = dmake((d.x < 0.f ? 0x80000000u : 0u) | (unsigned)(src + 1), (unsigned)code);
-            const double none = nb ? unset() : 0.0;
+            // (an idle slot computes on ones: a zero numerator takes the FP32
+            // division's slow path, some 300 cycles of every item)
+            const double none = nb ? unset() : pack2(1.f, 1.f);
             f[MF_DQ01][lane] = none; f[MF_DQ23][lane] = none;
             if (base == 0) {
                 f[MF_D][lane] = kCC ? dhalf(D) : D;
@@ -528,6 +565,7 @@ __device__ __forceinline__ void sweep_feed_mixed(const SweepArgs& a, RingM& R, i
 
 __device__ __forceinline__ void sweep_poll_mixed(const SweepArgs& a, RingM& R, const BoxM* boxes, int kbeg, int kend, int lane) {
     RingPos pos;
+    int entries = 0;
     for (int kk = kbeg; kk < kend; ++kk) {
         int ntake = 0, base = 0;
         do {
@@ -575,7 +613,7 @@ __device__ __forceinline__ void sweep_poll_mixed(const SweepArgs& a, RingM& R, c
             }
             if (__any_sync(0xffffffffu, nb || own)) return;
             __syncwarp();
-            if (lane == 0) mbar_arrive(&R.empty[pos.stage]);
+            if (lane == 0) st_release(&R.ready, ++entries);
             pos.next();
             base += 8;
         } while (base < ntake);
@@ -586,22 +624,17 @@ struct SweepEntryM {
     double r01, r23, uv, pun, nn, dsol, q01, q23, D, o, r;
     long long code;
     int4 item;
-    __device__ __forceinline__ void neighbour(const double (*f)[32], int lane) {
-        q01 = ld_field(&f[MF_DQ01][lane]); q23 = ld_field(&f[MF_DQ23][lane]);
-    }
     __device__ __forceinline__ void load(const RingM& R, int stage, int lane, bool first) {
         const double(*f)[32] = R.f[stage];
-        r01 = f[MF_R01][lane]; r23 = f[MF_R23][lane]; uv = f[MF_UV][lane]; pun = f[MF_PUN][lane];
-        nn = f[MF_N][lane]; dsol = f[MF_DSOL][lane];
-        code = __double_as_longlong(f[MF_CODE][lane]);
-        neighbour(f, lane);
         if (first) {
             item = R.item[stage];
-            D = f[MF_D][lane]; o = f[MF_O][lane];
-            r = ld_field(&f[MF_R][lane]);
+            D = f[MF_D][lane]; o = f[MF_O][lane]; r = f[MF_R][lane];
         }
+        code = __double_as_longlong(f[MF_CODE][lane]);
+        q01 = f[MF_DQ01][lane]; q23 = f[MF_DQ23][lane];
+        r01 = f[MF_R01][lane]; r23 = f[MF_R23][lane]; uv = f[MF_UV][lane]; pun = f[MF_PUN][lane];
+        nn = f[MF_N][lane]; dsol = f[MF_DSOL][lane];
     }
-    __device__ __forceinline__ bool waits() const { return is_unset(q01) || is_unset(q23) || is_unset(r); }
 };
 
 template <bool kCC>
@@ -609,29 +642,22 @@ __device__ __forceinline__ void sweep_items_mixed(const SweepArgs& a, RingM& R, 
     const unsigned all = 0xffffffffu;
     const int k = lane & 3;
     const float gm1 = (float)a.gm1;
+    const unsigned m0 = lane_mask(k == 0), m1 = lane_mask(k == 1), m2 = lane_mask(k == 2);
     RingPos pos;
     int last = -1;
     float LF[4] = {0.f, 0.f, 0.f, 0.f};  // previous item's dq (FP32)
     double Lk = 0.0;                     // and in FP64, component k
     SweepEntryM X;
     X.r = 0.0;
+    int entries = 0;
     for (int kk = kbeg; kk < kend; ++kk) {
         double cres = 0.0;
         const int idx = kk - kbeg, bslot = idx % kBox;
         if (lane == 0) box_open(box, idx);
         int it = 0, pass = 0, ntake = 0, base = 0;
         do {
-            if (!mbar_wait(&R.full[pos.stage], pos.phase, RingWait(&R.abort, a))) return;
+            if (!entry_wait(&R.ready, ++entries, RingWait(&R.abort, a))) return;
             X.load(R, pos.stage, lane, base == 0);
-            if (__any_sync(all, X.waits())) {
-                RingWait w(&R.abort, a);
-                for (int spins = 0;; ++spins) {
-                    X.neighbour(R.f[pos.stage], lane);
-                    if (base == 0) X.r = ld_field(&R.f[pos.stage][MF_R][lane]);
-                    if (!__any_sync(all, X.waits())) break;
-                    if (__any_sync(all, !w.go_on(spins))) return;
-                }
-            }
             __syncwarp();
             if (lane == 0) mbar_arrive(&R.empty[pos.stage]);
             pos.next();
@@ -644,7 +670,7 @@ __device__ __forceinline__ void sweep_items_mixed(const SweepArgs& a, RingM& R, 
                                  mine ? LF[3] : high_f(X.q23)};
             const SweepRecM E = {low_f(X.r01), high_f(X.r01), low_f(X.r23), high_f(X.r23), low_f(X.uv), high_f(X.uv),
                                  low_f(X.pun), high_f(X.pun), low_f(X.nn), high_f(X.nn)};
-            const float df = dflux_k(E, gm1, dq, k);
+            const float df = dflux_k(E, gm1, dq, m0, m1, m2);
             const float dqk = k == 0 ? dq[0] : (k == 1 ? dq[1] : (k == 2 ? dq[2] : dq[3]));
             const double t = widen(kCC ? low_f(X.dsol) * df - high_f(X.dsol) * dqk
                                        : 0.5f * ((X.code < 0 ? -df : df) * low_f(X.dsol) - high_f(X.dsol) * dqk));

@@ -74,6 +74,7 @@ __device__ __forceinline__ unsigned long long grp_max_u64(unsigned grp, unsigned
     return ((unsigned long long)mh << 32) | ml;
 }
 
+static __device__ __noinline__ double pow_rare(double a, double b) { return pow(a, b); }
 static __device__ __noinline__ double mean_rare(double a, double b) { return 0.5 * (a + b); }
 __device__ __forceinline__ void d4get(const double4& q, double o[4]) { o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w; }
 __device__ __forceinline__ double4 d4(const double o[4]) { return make_double4(o[0], o[1], o[2], o[3]); }
@@ -267,64 +268,60 @@ __global__ void __launch_bounds__(kBlock) k_face_prim_spec(CCView v) {
 }
 
 // Diamond-path face gradient (gradient.F90:183-261, gradtrixy :281-321).
-__device__ __forceinline__ bool gradtri(const double* pr0, const double* pr1, const double* pr2, double x0, double y0,
-                                        double x1, double y1, double x2, double y2, double gxo[5], double gyo[5],
-                                        double& tarea) {
-    const double xs[3] = {x0, x1, x2}, ys[3] = {y0, y1, y2};
-    const double* prs[3] = {pr0, pr1, pr2};
-    tarea = 0.0;
+__device__ __forceinline__ bool gradtri(const F64I* pr0, const F64I* pr1, const F64I* pr2, F64I x0, F64I y0,
+                                        F64I x1, F64I y1, F64I x2, F64I y2, F64I gxo[5], F64I gyo[5], F64I& tarea) {
+    const F64I xs[3] = {x0, x1, x2}, ys[3] = {y0, y1, y2};
+    const F64I* prs[3] = {pr0, pr1, pr2};
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        int ip1 = (i == 2) ? 0 : i + 1;
-        double dx = 0.5 * (xs[ip1] + xs[i]);
-        double dy = ys[ip1] - ys[i];
-        tarea = tarea + dx * dy;
+        const int ip1 = (i == 2) ? 0 : i + 1;
+        const F64I dx = half(xs[ip1] + xs[i]), dy = ys[ip1] - ys[i];
+        tarea = i == 0 ? F64I(zero_plus((dx * dy).v)) : tarea + dx * dy;
     }
 #pragma unroll
-    for (int k = 0; k < 5; ++k) { gxo[k] = 0.0; gyo[k] = 0.0; }
-#pragma unroll
     for (int i = 0; i < 3; ++i) {
-        int ip1 = (i == 2) ? 0 : i + 1;
-        double dx = ys[ip1] - ys[i];
-        double dy = -(xs[ip1] - xs[i]);
+        const int ip1 = (i == 2) ? 0 : i + 1;
+        const F64I dx = ys[ip1] - ys[i], dy = -(xs[ip1] - xs[i]);
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
-            double var = 0.5 * (prs[i][k] + prs[ip1][k]);
-            gxo[k] = gxo[k] + var * dx;
-            gyo[k] = gyo[k] + var * dy;
+            const F64I var = half(prs[i][k] + prs[ip1][k]);
+            gxo[k] = i == 0 ? F64I(zero_plus((var * dx).v)) : gxo[k] + var * dx;
+            gyo[k] = i == 0 ? F64I(zero_plus((var * dy).v)) : gyo[k] + var * dy;
         }
     }
 #pragma unroll
     for (int k = 0; k < 5; ++k) { gxo[k] = gxo[k] / tarea; gyo[k] = gyo[k] / tarea; }
-    return tarea > 0.0;
+    return dpos(tarea.v);
 }
 
+// FP64 unit-bound as plain doubles (477 instructions per face, thirty
+// divisions among them): 373 -> 143 us at 262 k cells.
 __global__ void __launch_bounds__(kBlock) k_face_ggfc(CCView v) {
     int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= v.nof || stopped(v, face_inst(v, f))) return;
     int2 nb = v.fnb[f];
     int2 p = v.fpt[f];
-    double2 X1 = v.pxy[p.x], X2 = v.pxy[p.y], Ci = v.cen[nb.x], Co = v.cen[nb.y];
-    double4 a = v.pp[p.x], b = v.pp[p.y], qi = v.qp[nb.x], qo = v.qp[nb.y];
-    double P1[5] = {a.x, a.y, a.z, a.w, v.ppT[p.x]};
-    double P2[5] = {b.x, b.y, b.z, b.w, v.ppT[p.y]};
-    double QI[5] = {qi.x, qi.y, qi.z, qi.w, v.qT[nb.x]};
-    double QO[5] = {qo.x, qo.y, qo.z, qo.w, v.qT[nb.y]};
-    double g1x[5], g1y[5], g2x[5], g2y[5], a1, a2;
-    bool ok1 = gradtri(P1, QO, P2, X1.x, X1.y, Co.x, Co.y, X2.x, X2.y, g1x, g1y, a1);
-    bool ok2 = gradtri(P1, P2, QI, X1.x, X1.y, X2.x, X2.y, Ci.x, Ci.y, g2x, g2y, a2);
+    const double2 X1 = v.pxy[p.x], X2 = v.pxy[p.y], Ci = v.cen[nb.x], Co = v.cen[nb.y];
+    F64I P1[5], P2[5], QI[5], QO[5];
+    f4get(v.pp[p.x], P1); P1[4] = v.ppT[p.x];
+    f4get(v.pp[p.y], P2); P2[4] = v.ppT[p.y];
+    f4get(v.qp[nb.x], QI); QI[4] = v.qT[nb.x];
+    f4get(v.qp[nb.y], QO); QO[4] = v.qT[nb.y];
+    F64I g1x[5], g1y[5], g2x[5], g2y[5], a1, a2;
+    const bool ok1 = gradtri(P1, QO, P2, X1.x, X1.y, Co.x, Co.y, X2.x, X2.y, g1x, g1y, a1);
+    const bool ok2 = gradtri(P1, P2, QI, X1.x, X1.y, X2.x, X2.y, Ci.x, Ci.y, g2x, g2y, a2);
     if (!(ok1 && ok2)) set_err(v.err, UNS_ERR_MESH, f);
-    double s = a1 + a2;
-    double gx[5], gy[5];
+    const F64I s = a1 + a2;
+    F64I gx[5], gy[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
         gx[k] = (a1 * g1x[k] + a2 * g2x[k]) / s;
         gy[k] = (a1 * g1y[k] + a2 * g2y[k]) / s;
     }
-    v.fgx[f] = make_double4(gx[0], gx[1], gx[2], gx[3]);
-    v.fgy[f] = make_double4(gy[0], gy[1], gy[2], gy[3]);
-    v.fgT[f] = make_double2(gx[4], gy[4]);
-    v.fasum[f] = s;
+    v.fgx[f] = f4(gx);
+    v.fgy[f] = f4(gy);
+    v.fgT[f] = make_double2(gx[4].v, gy[4].v);
+    v.fasum[f] = s.v;
 }
 
 // Per-cell gather over the index-sorted face list: spectral radius + dt
@@ -867,18 +864,43 @@ __global__ void __launch_bounds__(std::is_same<R, float>::value ? 512 : kBlock, 
     }
 }
 
-// Sutherland viscosity of every interior cell (viscous_flux.F90:20-22,127-141).
-__global__ void __launch_bounds__(kBlock) k_cell_mul(CCView v) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Sutherland viscosity of an interior cell (viscous_flux.F90:20-22,127-141).
+__device__ __forceinline__ void cell_mul(const CCView& v, int i) {
     if (i >= v.noc) return;
     const int inst = cell_inst(v, i);
     if (inst < 0 || stopped(v, inst)) return;
     const Gas& g = gas_of(v, inst);
     double4 c = v.qc[i];
-    Prim P = con2prim(g, c.x, c.y, c.z, c.w);
-    double num = 1.0 + g.T_infd / g.SCONST;
-    double den = P.t + g.T_infd / g.SCONST;
-    v.mul[i] = (num / den) * pow(P.t, 1.5);
+    const PrimT<F64I> P = con2prim_t<F64I>(g, c.x, c.y, c.z, c.w);
+    const F64I s0 = F64I(g.T_infd) / g.SCONST;
+    const F64I num = F64I(1.0) + s0, den = P.t + s0;
+    // t^1.5 as t sqrt(t): within one unit in the last place (two correctly
+    // rounded operations; pow's bound is two), without pow's 100 instructions
+    // on the FP64 unit (262 k cells: 73 -> 13 us).  What pow makes of t <= 0
+    // stays pow's.
+    const F64I t15 = dpos(P.t.v) ? P.t * sqrt(P.t) : F64I(pow_rare(P.t.v, 1.5));
+    v.mul[i] = ((num / den) * t15).v;
+}
+__global__ void __launch_bounds__(kBlock) k_cell_mul(CCView v) { cell_mul(v, blockIdx.x * blockDim.x + threadIdx.x); }
+
+// The wall faces' convective fluxes and ghosts, and beside them (with_mul)
+// every cell's viscosity: the wall faces' long chains take the first one-warp
+// blocks, the cells run under them (laminar 512x256: 31 + 13 -> 29 us).
+template <class R>
+__global__ void __launch_bounds__(32) k_wall_faces(CCView v, int with_mul) {
+    const int nwb = (v.nbf + 31) / 32;
+    if ((int)blockIdx.x >= nwb) {
+        if (with_mul) cell_mul(v, (blockIdx.x - nwb) * 32 + threadIdx.x);
+        return;
+    }
+    const int f = v.nfi + blockIdx.x * 32 + threadIdx.x;
+    if (f >= v.nof || v.fbc[f] != 1001) return;
+    const int inst = face_inst(v, f);
+    if (stopped(v, inst)) return;
+    const int in = v.fnb[f].x;
+    double cin[4];
+    d4get(v.qc[in], cin);
+    bnd_face_flux<R>(v, gas_of(v, inst), f, in, cin);
 }
 
 // Laminar viscous face flux (viscous_flux.F90:30-76), stored as flux*area.
@@ -891,25 +913,27 @@ __global__ void __launch_bounds__(kBlock) k_face_visc(CCView v) {
     int2 nb = v.fnb[f];
     double2 n = v.fn[f];
     double area = v.farea[f];
-    double mu = (nb.y < v.noc) ? 0.5 * (v.mul[nb.x] + v.mul[nb.y]) : v.mul[nb.x];
-    v.fmu[f] = mu;
-    double4 q = v.fq[f];
-    double4 a = v.fgx[f], b = v.fgy[f];
-    double2 t = v.fgT[f];
-    double uvel = q.y, vvel = q.z;
-    double ux = a.y, uy = b.y, vx = a.z, vy = b.z, tx = t.x, ty = t.y;
-    const double two = 2.0, two_third = two / 3.0;
-    double tauxx = two_third * (two * ux - vy);
-    double tauxy = (uy + vx);
-    double tauyy = two_third * (two * vy - ux);
-    double factor = (g.gamma - 1.0) * g.m_inf * g.m_inf * g.prandtl;
-    double qx = -(tx / factor), qy = -(ty / factor);
-    double mr = mu / g.rey;
-    double f1 = mr * ((uvel * tauxx + vvel * tauxy - qx) * n.x + (uvel * tauxy + vvel * tauyy - qy) * n.y);
-    double f3 = mr * (tauxx * n.x + tauxy * n.y);
-    double f4 = mr * (tauxy * n.x + tauyy * n.y);
-    v.fV[f] = make_double4(f1 * area, 0.0 * area, f3 * area, f4 * area);
-    if (f >= v.nfi) v.fwallv[f - v.nfi] = (v.fbc[f] == 1001) ? make_double2(f3 * area, f4 * area) : make_double2(0.0, 0.0);
+    typedef F64I S;
+    const S mu = (nb.y < v.noc) ? half(S(v.mul[nb.x]) + v.mul[nb.y]) : S(v.mul[nb.x]);
+    v.fmu[f] = mu.v;
+    const double4 q = v.fq[f];
+    const double4 a = v.fgx[f], b = v.fgy[f];
+    const double2 t = v.fgT[f];
+    const S uvel = q.y, vvel = q.z;
+    const S ux = a.y, uy = b.y, vx = a.z, vy = b.z;
+    const S two_third = 2.0 / 3.0;
+    const S tauxx = two_third * (twice(ux) - vy);
+    const S tauxy = uy + vx;
+    const S tauyy = two_third * (twice(vy) - ux);
+    const S factor = (S(g.gamma) - 1.0) * g.m_inf * g.m_inf * g.prandtl;
+    const S qx = -(S(t.x) / factor), qy = -(S(t.y) / factor);
+    const S mr = mu / g.rey;
+    const S f1 = mr * ((uvel * tauxx + vvel * tauxy - qx) * n.x + (uvel * tauxy + vvel * tauyy - qy) * n.y);
+    const S f3 = mr * (tauxx * n.x + tauxy * n.y);
+    const S f4_ = mr * (tauxy * n.x + tauyy * n.y);
+    const double V2 = (f3 * area).v, V3 = (f4_ * area).v;
+    v.fV[f] = make_double4((f1 * area).v, 0.0, V2, V3);
+    if (f >= v.nfi) v.fwallv[f - v.nfi] = (v.fbc[f] == 1001) ? make_double2(V2, V3) : make_double2(0.0, 0.0);
 }
 
 // Residual gather in the reference's accumulation order, optionally fused
@@ -1654,18 +1678,25 @@ bool grad_by_sides(const uns_cc_handle* h, const CCView& v) {
     return v.mixed && v.sideg != nullptr && h->P.time_mode == UNS_TIME_RK3;
 }
 
+// The wall faces' convective fluxes and ghosts, with_mul the cells' viscosity
+// too.  (A farfield face's flux and ghost follow from the reconstructed state.)
+int enqueue_wall_faces(uns_cc_handle* h, CCView& v, bool with_mul) {
+    const int nb = (v.nbf + 31) / 32 + (with_mul ? (v.noc + 31) / 32 : 0);
+    if (nb == 0) return UNS_OK;
+    if (v.mixed) k_wall_faces<float><<<nb, 32, 0, h->stream>>>(v, with_mul ? 1 : 0);
+    else k_wall_faces<double><<<nb, 32, 0, h->stream>>>(v, with_mul ? 1 : 0);
+    UNS_CUDA(cudaGetLastError());
+    return UNS_OK;
+}
+
 // uns_cc_fvresidual when only the wall ghosts can have changed since the last
 // call that computed every face (same primitives, gradient and limiter; the
 // reference main loop's RK stages 2 and 3): the boundary faces' fluxes and
 // the wall cells' residuals; every other cell keeps the residual it has.
 int enqueue_wall_res(uns_cc_handle* h, CCView& v) {
-    const int bs = v.mixed ? face_bs<float>(h, v) : face_bs<double>(h, v);
-    const int nbb = (v.nbf + bs - 1) / bs;  // k_face_conv's boundary blocks come first
-    if (nbb == 0) return UNS_OK;
-    if (v.mixed) k_face_conv<float><<<nbb, bs, 0, h->stream>>>(v);
-    else k_face_conv<double><<<nbb, bs, 0, h->stream>>>(v);
-    UNS_CUDA(cudaGetLastError());
-    if (v.nwcell > 0) {
+    int rc = enqueue_wall_faces(h, v, false);
+    if (rc) return rc;
+    if (v.nbf > 0 && v.nwcell > 0) {
         const int nb = (v.nwcell + 31) / 32;
         if (v.mixed) k_wall_res<float><<<nb, 32, 0, h->stream>>>(v);
         else k_wall_res<double><<<nb, 32, 0, h->stream>>>(v);
@@ -1714,11 +1745,16 @@ int enqueue_rk23(uns_cc_handle* h, CCView& v) {
 
 // fvresidual as a kernel sequence; irk > 0 fuses that RK stage into the
 // residual gather (only when no smoothing sweep sits in between).
-int enqueue_fvresidual(uns_cc_handle* h, CCView& v, double cfl, int irk, int partial, bool* fused) {
-    if (h->P.precision == UNS_PREC_MIXED) LAUNCH_FACE_CONV(float, v);
+// walls_only: the other faces' convective fluxes of the step's first stage
+// still hold (same primitives, gradient and limiter).
+int enqueue_fvresidual(uns_cc_handle* h, CCView& v, double cfl, int irk, int partial, bool* fused, bool walls_only = false) {
+    if (walls_only) {
+        int rc = enqueue_wall_faces(h, v, v.laminar != 0);
+        if (rc) return rc;
+    } else if (h->P.precision == UNS_PREC_MIXED) LAUNCH_FACE_CONV(float, v);
     else LAUNCH_FACE_CONV(double, v);
     if (v.laminar) {
-        LAUNCH(k_cell_mul, v.noc, v);
+        if (!walls_only) LAUNCH(k_cell_mul, v.noc, v);
         if (v.grad_type != UNS_GRAD_GGFC) {
             CCView w = v;
             w.grad_type = UNS_GRAD_GGFC;
@@ -1813,9 +1849,16 @@ int enqueue_iteration(uns_cc_handle* h, CCView& v, double cfl_for_eps) {
         UNS_CUDA(cudaGetLastError());
         return UNS_OK;
     } else if (h->P.time_mode == UNS_TIME_RK3) {
+        // A viscous stage with the GG-FC gradient, and a smoothing sweep, keep
+        // the primitives, gradient and limiter that the interior and farfield
+        // fluxes read (above): stages 2 and 3 recompute the wall faces alone
+        // (laminar 512x256: three times 157 us of fluxes and viscosities ->
+        // 157 + 2 x 29).
+        // With another gradient a viscous stage replaces the cell gradient.
+        const bool keep = !v.laminar || v.grad_type == UNS_GRAD_GGFC;
         for (int irk = 1; irk <= 3; ++irk) {
             bool fused = false;
-            if ((rc = enqueue_fvresidual(h, v, cfl_for_eps, irk, irk == 3, &fused))) return rc;
+            if ((rc = enqueue_fvresidual(h, v, cfl_for_eps, irk, irk == 3, &fused, keep && irk > 1))) return rc;
             if (!fused) LAUNCH(k_rk_stage, v.noc, v, irk);
         }
     } else {
@@ -2857,6 +2900,7 @@ int uns_cc_profile(uns_cc_handle* h, double cfl, int reps, double* ms, const cha
         const bool one_pass = rk23_in_one_pass(h, v, cfl);
         for (int irk = 1; irk <= (rk3 && !one_pass ? 3 : 1) && !rc; ++irk) {
             rc = timed(5, [&]() -> int {
+                if (irk > 1 && (!v.laminar || v.grad_type == UNS_GRAD_GGFC)) return enqueue_wall_faces(h, v, false);
                 if (h->P.precision == UNS_PREC_MIXED) LAUNCH_FACE_CONV(float, v);
                 else LAUNCH_FACE_CONV(double, v);
                 return UNS_OK;

@@ -99,25 +99,28 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
 
     std::vector<int> preds;
     auto place = [&](int code) {
-        // ready time of the item on warp w
-        auto start_on = [&](int w) {
-            double s = wfree[w];
-            for (int p : preds) {
-                const int v = wof[p];
-                s = std::max(s, fin[p] + (v == w ? 0.0 : (v / kSchedGroup == w / kSchedGroup ? kNear : kSync)));
-            }
-            return s;
-        };
+        // The item's start on warp c, and the candidates: a warp that is not
+        // free before the best start so far cannot improve on it.
         int w = -1;
         double s = 0.0;
         auto consider = [&](int c) {
-            const double t = start_on(c);
+            double t = wfree[c];
+            if (w >= 0 && t >= s - 1e-12) return;
+            for (int p : preds) {
+                const int v = wof[p];
+                t = std::max(t, fin[p] + (v == c ? 0.0 : (v / kSchedGroup == c / kSchedGroup ? kNear : kSync)));
+            }
             if (w < 0 || t < s - 1e-12) { w = c; s = t; }
         };
         for (int p : preds)
             if (wlast[wof[p]] == p) consider(wof[p]);
+        int seen[8], nseen = 0;
         for (int p : preds) {
             const int g = wof[p] / kSchedGroup * kSchedGroup;
+            bool again = false;
+            for (int q = 0; q < nseen; ++q) again = again || seen[q] == g;
+            if (again) continue;
+            if (nseen < 8) seen[nseen++] = g;
             for (int c = g; c < g + kSchedGroup && c < nwarps; ++c) consider(c);
         }
         while (heap.top().first != wfree[heap.top().second]) heap.pop();  // drop stale entries

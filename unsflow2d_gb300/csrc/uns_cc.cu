@@ -2174,6 +2174,7 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
         std::vector<int> src;
         std::vector<int4> sched(ws.items.size());
         std::vector<int> rf, rn, rl;
+        rf.reserve(2 * (size_t)nfi); rn.reserve(2 * (size_t)nfi); rl.reserve(2 * (size_t)nfi); src.reserve(2 * (size_t)nfi);
         for (size_t pos = 0; pos < ws.items.size(); ++pos) {
             const int it = ws.items[pos] >> 1, pass = ws.items[pos] & 1;
             const int first = (int)rf.size();

@@ -46,7 +46,7 @@ struct AdjView {
     const double4* JF;   // [3][8][nfi]: dF/d(ql[j]) (j < 4), dF/d(qr[j-4]) of interior faces
     const double* BJ;    // [3][nbf][9 in][9 out]: d(F[4], ghost prim[4], ghost T)/d(qcl[4], qc_in[4], alpha)
     const double4* DM;   // [3][noc]: d mul / d qc
-    const double* VI;    // [3][nof][9]: mu_f, u, v, ux, uy, vx, vy, Tx, Ty at the viscous flux
+    const double* VI;    // [3][9][nof]: mu_f, u, v, ux, uy, vx, vy, Tx, Ty at the viscous flux (a warp reads each in one run)
     const double* Dv;    // [noc]: dt / cv
     const double4* q0;   // [noc]: conserved state at the start of the recorded iteration
     // transposed connectivity
@@ -113,10 +113,18 @@ namespace {
 constexpr int V2F_P2 = 1 << 30;
 
 __device__ __forceinline__ double4 z4() { return make_double4(0.0, 0.0, 0.0, 0.0); }
-__device__ __forceinline__ double4 add(double4 a, double4 b) { return make_double4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
-__device__ __forceinline__ double4 sub(double4 a, double4 b) { return make_double4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w); }
-__device__ __forceinline__ double4 scl(double s, double4 a) { return make_double4(s * a.x, s * a.y, s * a.z, s * a.w); }
-__device__ __forceinline__ double dot(double4 a, double4 b) { return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
+// The transposed kernels are linear maps bound by the FP64 unit (80-87 % busy
+// as plain doubles); N leaves it their sums.  The values are the same bits.
+// At 262 k cells (laminar): k_adj_visc 109 -> 56 us, k_adj_recon 110 -> 74,
+// k_adj_conv 62 -> 42, k_adj_ggfc 157 -> 59, k_adj_final 150 -> 60,
+// k_adj_start_grad 43 -> 25, k_adj_init 30 -> 23.
+typedef F64I N;
+__device__ __forceinline__ double4 add(double4 a, double4 b) { return make_double4(add64(a.x, b.x), add64(a.y, b.y), add64(a.z, b.z), add64(a.w, b.w)); }
+__device__ __forceinline__ double4 sub(double4 a, double4 b) { return make_double4(sub64(a.x, b.x), sub64(a.y, b.y), sub64(a.z, b.z), sub64(a.w, b.w)); }
+__device__ __forceinline__ double4 scl(double s, double4 a) { return make_double4((N(s) * a.x).v, (N(s) * a.y).v, (N(s) * a.z).v, (N(s) * a.w).v); }
+__device__ __forceinline__ double4 scl(N s, double4 a) { return scl(s.v, a); }
+__device__ __forceinline__ double dot(double4 a, double4 b) { return (N(a.x) * b.x + N(a.y) * b.y + N(a.z) * b.z + N(a.w) * b.w).v; }
+__device__ __forceinline__ double2 sum2(double2 a, N x, N y) { return make_double2((N(a.x) + x).v, (N(a.y) + y).v); }
 __device__ __forceinline__ double at(const double4& a, int j) { return j == 0 ? a.x : j == 1 ? a.y : j == 2 ? a.z : a.w; }
 __device__ __forceinline__ void put(double4& a, int j, double x) {
     if (j == 0) a.x = x; else if (j == 1) a.y = x; else if (j == 2) a.z = x; else a.w = x;
@@ -250,9 +258,10 @@ __global__ void k_rec_visc(CCView v, AdjView a, int s) {
     if (f >= v.nof) return;
     const double4 q = v.fq[f], gx = v.fgx[f], gy = v.fgy[f];
     const double2 t = v.fgT[f];
-    double* o = (double*)a.VI + ((size_t)s * v.nof + f) * 9;
-    o[0] = v.fmu[f]; o[1] = q.y; o[2] = q.z;
-    o[3] = gx.y; o[4] = gy.y; o[5] = gx.z; o[6] = gy.z; o[7] = t.x; o[8] = t.y;
+    double* o = (double*)a.VI + (size_t)s * 9 * v.nof + f;
+    const double x[9] = {v.fmu[f], q.y, q.z, gx.y, gy.y, gx.z, gy.z, t.x, t.y};
+#pragma unroll
+    for (int k = 0; k < 9; ++k) o[(size_t)k * v.nof] = x[k];
 }
 
 // ------------------------------------------------------- transposed pass
@@ -267,7 +276,9 @@ __global__ void k_adj_init(CCView v, AdjView a) {
     }
     if (i < v.nof) {
         a.fq[i] = z4(); a.fgx[i] = z4(); a.fgy[i] = z4(); a.fgT[i] = make_double2(0.0, 0.0);
-        a.sgx[i] = z4(); a.sgy[i] = z4(); a.sgT[i] = make_double2(0.0, 0.0);
+        if (v.laminar && v.grad_type != UNS_GRAD_GGFC) {  // read by a stage gradient alone
+            a.sgx[i] = z4(); a.sgy[i] = z4(); a.sgT[i] = make_double2(0.0, 0.0);
+        }
     }
     if (i < v.nbf) a.falpha[i] = 0.0;
     if (a.geo && i < v.nof) {
@@ -284,7 +295,7 @@ __global__ void k_adj_stage(CCView v, AdjView a, int irk) {
     if (i >= v.noc) return;
     const double4 l = a.qc[i];
     const double ak = rk_a(irk), bk = rk_b(irk);
-    a.res[i] = scl(-bk * a.Dv[i], l);
+    a.res[i] = scl(N(-bk) * a.Dv[i], l);
     a.qold[i] = add(a.qold[i], scl(ak, l));
     a.qc[i] = scl(bk, l);
 }
@@ -292,54 +303,54 @@ __global__ void k_adj_stage(CCView v, AdjView a, int irk) {
 // Viscous face flux transposed: the face-viscosity adjoint per face, the
 // face-velocity adjoint into fq, the face-gradient adjoint into fg (the
 // gradients of the start of the iteration) or sg (this stage's).
-__global__ void k_adj_visc(CCView v, AdjView a, int s, int last, int stage_grad) {
+__global__ void __launch_bounds__(kBlock, 3) k_adj_visc(CCView v, AdjView a, int s, int last, int stage_grad) {
     int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= v.nof) return;
     const int2 nb = v.fnb[f];
-    double4 b = f < v.nfi ? sub(a.res[nb.y], a.res[nb.x]) : scl(-1.0, a.res[nb.x]);
-    if (last && f >= v.nfi && v.fbc[f] == 1001) { b.z = b.z - a.jx; b.w = b.w - a.jy; }
-    const double* o = a.VI + ((size_t)s * v.nof + f) * 9;
-    const double mu = o[0], u = o[1], vv = o[2], ux = o[3], uy = o[4], vx = o[5], vy = o[6];
+    const double4 bi = a.res[nb.x];
+    double4 b = f < v.nfi ? sub(a.res[nb.y], bi) : make_double4(neg64(bi.x), neg64(bi.y), neg64(bi.z), neg64(bi.w));
+    if (last && f >= v.nfi && v.fbc[f] == 1001) { b.z = add_rare(b.z, -a.jx); b.w = add_rare(b.w, -a.jy); }
+    double o[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) o[k] = a.VI[((size_t)s * 9 + k) * v.nof + f];
+    const N mu = o[0], u = o[1], vv = o[2], ux = o[3], uy = o[4], vx = o[5], vy = o[6];
     const double2 n = v.fn[f];
-    const double area = v.farea[f];
-    const double two_third = 2.0 / 3.0;
-    const double txx = two_third * (2.0 * ux - vy), txy = uy + vx, tyy = two_third * (2.0 * vy - ux);
-    const double factor = (v.g.gamma - 1.0) * v.g.m_inf * v.g.m_inf * v.g.prandtl;
-    const double qx = -(o[7] / factor), qy = -(o[8] / factor);
-    const double mr = mu / v.g.rey;
-    const double S1 = (u * txx + vv * txy - qx) * n.x + (u * txy + vv * tyy - qy) * n.y;
-    const double f1b = b.x * area, f3b = b.z * area, f4b = b.w * area;
-    const double mrb = f1b * S1 + f3b * (txx * n.x + txy * n.y) + f4b * (txy * n.x + tyy * n.y);
-    a.fmu[f] = mrb / v.g.rey;
-    const double S1b = mr * f1b;
-    const double ub = S1b * (txx * n.x + txy * n.y), vb = S1b * (txy * n.x + tyy * n.y);
-    const double qxb = -S1b * n.x, qyb = -S1b * n.y;
-    const double txxb = S1b * u * n.x + mr * f3b * n.x;
-    const double txyb = S1b * (vv * n.x + u * n.y) + mr * f3b * n.y + mr * f4b * n.x;
-    const double tyyb = S1b * vv * n.y + mr * f4b * n.y;
-    const double uxb = two_third * 2.0 * txxb - two_third * tyyb;
-    const double vyb = -two_third * txxb + two_third * 2.0 * tyyb;
-    const double uyb = txyb, vxb = txyb;
-    const double txb = -qxb / factor, tyb = -qyb / factor;
+    const N area = v.farea[f], bx = b.x, bz = b.z, bw = b.w;
+    const N two_third = 2.0 / 3.0, four_third = 2.0 / 3.0 * 2.0;
+    const N txx = two_third * (twice(ux) - vy), txy = uy + vx, tyy = two_third * (twice(vy) - ux);
+    const N factor = (N(v.g.gamma) - 1.0) * v.g.m_inf * v.g.m_inf * v.g.prandtl;
+    const N qx = -(N(o[7]) / factor), qy = -(N(o[8]) / factor);
+    const N mr = mu / v.g.rey;
+    const N A = u * txx + vv * txy - qx, B = u * txy + vv * tyy - qy;
+    const N t1 = txx * n.x + txy * n.y, t2 = txy * n.x + tyy * n.y;
+    const N S1 = A * n.x + B * n.y;
+    const N f1b = bx * area, f3b = bz * area, f4b = bw * area;
+    const N mrb = f1b * S1 + f3b * t1 + f4b * t2;
+    a.fmu[f] = (mrb / v.g.rey).v;
+    const N S1b = mr * f1b;
+    const N ub = S1b * t1, vb = S1b * t2;
+    const N qxb = -S1b * n.x, qyb = -S1b * n.y;
+    const N m3 = mr * f3b, m4 = mr * f4b;
+    const N txxb = S1b * u * n.x + m3 * n.x;
+    const N txyb = S1b * (vv * n.x + u * n.y) + m3 * n.y + m4 * n.x;
+    const N tyyb = S1b * vv * n.y + m4 * n.y;
+    const N uxb = four_third * txxb - two_third * tyyb;
+    const N vyb = -two_third * txxb + four_third * tyyb;
+    const N txb = -qxb / factor, tyb = -qyb / factor;
     double4 q = a.fq[f];
-    q.y = q.y + ub; q.z = q.z + vb;
+    q.y = (N(q.y) + ub).v; q.z = (N(q.z) + vb).v;
     a.fq[f] = q;
     double4* GX = stage_grad ? a.sgx : a.fgx;
     double4* GY = stage_grad ? a.sgy : a.fgy;
     double2* GT = stage_grad ? a.sgT : a.fgT;
     double4 gx = GX[f], gy = GY[f];
-    gx.y = gx.y + uxb; gx.z = gx.z + vxb;
-    gy.y = gy.y + uyb; gy.z = gy.z + vyb;
+    gx.y = (N(gx.y) + uxb).v; gx.z = (N(gx.z) + txyb).v;
+    gy.y = (N(gy.y) + txyb).v; gy.z = (N(gy.z) + vyb).v;
     GX[f] = gx; GY[f] = gy;
-    double2 t = GT[f];
-    GT[f] = make_double2(t.x + txb, t.y + tyb);
+    GT[f] = sum2(GT[f], txb, tyb);
     if (a.geo) {  // flux*area = area*mr*(S1, 0, txx nx + txy ny, txy nx + tyy ny): its normal and length
-        const double A = u * txx + vv * txy - qx, B = u * txy + vv * tyy - qy;
-        const double t1 = txx * n.x + txy * n.y, t2 = txy * n.x + tyy * n.y;
-        a.garea[f] = a.garea[f] + mr * (b.x * S1 + b.z * t1 + b.w * t2);
-        const double2 gn = a.gfn[f];
-        a.gfn[f] = make_double2(gn.x + area * mr * (b.x * A + b.z * txx + b.w * txy),
-                                gn.y + area * mr * (b.x * B + b.z * txy + b.w * tyy));
+        a.garea[f] = (N(a.garea[f]) + mr * (bx * S1 + bz * t1 + bw * t2)).v;
+        a.gfn[f] = sum2(a.gfn[f], area * mr * (bx * A + bz * txx + bw * txy), area * mr * (bx * B + bz * txy + bw * tyy));
     }
 }
 
@@ -347,10 +358,11 @@ __global__ void k_adj_visc(CCView v, AdjView a, int s, int last, int stage_grad)
 __global__ void k_adj_mul(CCView v, AdjView a, int s) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= v.noc) return;
-    double m = 0.0;
+    N m = 0.0;
     for (int k = v.cf_off[i]; k < v.cf_off[i + 1]; ++k) {
         int f = v.cf[k] & FACE_MASK;
-        m = m + (v.fnb[f].y < v.noc ? 0.5 * a.fmu[f] : a.fmu[f]);
+        const N x = a.fmu[f];
+        m = m + (v.fnb[f].y < v.noc ? half(x) : x);
     }
     a.qc[i] = add(a.qc[i], scl(m, a.DM[(size_t)s * v.noc + i]));
 }
@@ -359,27 +371,29 @@ __global__ void k_adj_mul(CCView v, AdjView a, int s) {
 // derivative of (gx, gy) of the face with respect to the value at each of its
 // four points, per unit gradient adjoint (gb_x, gb_y), as
 // w = 0.5 (edge terms of the two edges at the point) / (a1 + a2).
-struct GgfcW { double p1x, p1y, p2x, p2y, ix, iy, ox, oy; };
+struct GgfcW { N p1x, p1y, p2x, p2y, ix, iy, ox, oy; };
 __device__ __forceinline__ GgfcW ggfc_weights(const CCView& v, int f) {
     const int2 nb = v.fnb[f], p = v.fpt[f];
     const double2 X1 = v.pxy[p.x], X2 = v.pxy[p.y], Ci = v.cen[nb.x], Co = v.cen[nb.y];
-    const double s = v.fasum[f];
+    const N s = v.fasum[f];
     // triangle 1: (P1, QO, P2) at (X1, Co, X2); triangle 2: (P1, P2, QI) at (X1, X2, Ci)
-    auto tri = [&](double2 A, double2 B, double2 C, double wx[3], double wy[3]) {
-        const double xs[3] = {A.x, B.x, C.x}, ys[3] = {A.y, B.y, C.y};
-        double ex[3], ey[3];
+    auto tri = [&](double2 A, double2 B, double2 C, N wx[3], N wy[3]) {
+        const N xs[3] = {A.x, B.x, C.x}, ys[3] = {A.y, B.y, C.y};
+        N ex[3], ey[3];
+#pragma unroll
         for (int i = 0; i < 3; ++i) {
-            int ip1 = (i == 2) ? 0 : i + 1;
+            const int ip1 = (i == 2) ? 0 : i + 1;
             ex[i] = ys[ip1] - ys[i];
             ey[i] = -(xs[ip1] - xs[i]);
         }
+#pragma unroll
         for (int m = 0; m < 3; ++m) {
-            int mm1 = (m == 0) ? 2 : m - 1;
-            wx[m] = 0.5 * (ex[m] + ex[mm1]) / s;
-            wy[m] = 0.5 * (ey[m] + ey[mm1]) / s;
+            const int mm1 = (m == 0) ? 2 : m - 1;
+            wx[m] = half(ex[m] + ex[mm1]) / s;
+            wy[m] = half(ey[m] + ey[mm1]) / s;
         }
     };
-    double w1x[3], w1y[3], w2x[3], w2y[3];
+    N w1x[3], w1y[3], w2x[3], w2y[3];
     tri(X1, Co, X2, w1x, w1y);
     tri(X1, X2, Ci, w2x, w2y);
     GgfcW w;
@@ -400,23 +414,24 @@ __global__ void k_adj_stage_ggfc(CCView v, AdjView a) {
     int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= v.nof) return;
     const int2 nb = v.fnb[f];
-    const double s = v.fasum[f];
-    double4 gx = add(a.sgx[f], scl(s / v.cov[nb.x], a.gx[nb.x]));
-    double4 gy = add(a.sgy[f], scl(s / v.cov[nb.x], a.gy[nb.x]));
+    const N s = v.fasum[f];
+    const N si = s / v.cov[nb.x];
+    double4 gx = add(a.sgx[f], scl(si, a.gx[nb.x]));
+    double4 gy = add(a.sgy[f], scl(si, a.gy[nb.x]));
     if (f < v.nfi) {
-        gx = add(gx, scl(s / v.cov[nb.y], a.gx[nb.y]));
-        gy = add(gy, scl(s / v.cov[nb.y], a.gy[nb.y]));
+        const N so = s / v.cov[nb.y];
+        gx = add(gx, scl(so, a.gx[nb.y]));
+        gy = add(gy, scl(so, a.gy[nb.y]));
     }
     const double2 gt = a.sgT[f];
     if (f >= v.nfi) {
         GgfcW w = ggfc_weights(v, f);
         a.qp[nb.y] = add(a.qp[nb.y], add(scl(w.ox, gx), scl(w.oy, gy)));
-        a.qT[nb.y] = a.qT[nb.y] + w.ox * gt.x + w.oy * gt.y;
+        a.qT[nb.y] = (N(a.qT[nb.y]) + w.ox * gt.x + w.oy * gt.y).v;
     }
     a.fgx[f] = add(a.fgx[f], gx);
     a.fgy[f] = add(a.fgy[f], gy);
-    double2 t = a.fgT[f];
-    a.fgT[f] = make_double2(t.x + gt.x, t.y + gt.y);
+    a.fgT[f] = sum2(a.fgT[f], gt.x, gt.y);
     a.sgx[f] = z4(); a.sgy[f] = z4(); a.sgT[f] = make_double2(0.0, 0.0);
 }
 
@@ -430,14 +445,14 @@ __global__ void k_adj_conv(CCView v, AdjView a, int s, int last) {
     if (f < v.nfi) {
         const double4 Fb = sub(a.res[nb.x], a.res[nb.y]);
         double l[8];
+#pragma unroll
         for (int dir = 0; dir < 8; ++dir) l[dir] = dot(a.JF[((size_t)s * 8 + dir) * v.nfi + f], Fb);
         a.fl[f] = make_double4(l[0], l[1], l[2], l[3]);
         a.fr[f] = make_double4(l[4], l[5], l[6], l[7]);
         if (a.geo) {
-            const double2 gn = a.gfn[f];
-            a.gfn[f] = make_double2(gn.x + dot(a.JG[((size_t)s * 3 + 0) * v.nfi + f], Fb),
-                                    gn.y + dot(a.JG[((size_t)s * 3 + 1) * v.nfi + f], Fb));
-            a.garea[f] = a.garea[f] + dot(a.JG[((size_t)s * 3 + 2) * v.nfi + f], Fb);
+            a.gfn[f] = sum2(a.gfn[f], dot(a.JG[((size_t)s * 3 + 0) * v.nfi + f], Fb),
+                            dot(a.JG[((size_t)s * 3 + 1) * v.nfi + f], Fb));
+            a.garea[f] = add64(a.garea[f], dot(a.JG[((size_t)s * 3 + 2) * v.nfi + f], Fb));
             a.fls[f] = add(a.fls[f], a.fl[f]);
             a.frs[f] = add(a.frs[f], a.fr[f]);
         }
@@ -475,37 +490,46 @@ __global__ void k_adj_conv(CCView v, AdjView a, int s, int last) {
 // cell over its faces: primitive adjoint (start of the iteration), gradient
 // adjoint (the gradient this stage read; reset first when a viscous stage
 // had recomputed it), and the wall closure's current-state adjoint.
-__global__ void k_adj_recon(CCView v, AdjView a, int reset_g) {
+__global__ void __launch_bounds__(kBlock, 3) k_adj_recon(CCView v, AdjView a, int reset_g) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= v.noc) return;
-    const double zhi = 1.0 / 3.0;
+    const N zhi = 1.0 / 3.0, zlo = 1.0 - 1.0 / 3.0;
     const double4 ph = v.phi[i];
     const double2 c = v.cen[i];
     double4 aq = z4(), ac = z4();
     double4 gx = reset_g ? z4() : a.gx[i], gy = reset_g ? z4() : a.gy[i];
+    N own_w[4], own_e[4], hp[4];  // per variable: 1 - phi/2 zhi, phi/2 (1 - zhi)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        hp[j] = half(N(at(ph, j)));
+        own_w[j] = N(1.0) - hp[j] * zhi;
+        own_e[j] = hp[j] * zlo;
+    }
     for (int k = v.cf_off[i]; k < v.cf_off[i + 1]; ++k) {
         const int e = v.cf[k], f = e & FACE_MASK;
         const double2 fc = v.fcen[f];
-        const double d0 = fc.x - c.x, d1 = fc.y - c.y;
+        const N d0 = N(fc.x) - c.x, d1 = N(fc.y) - c.y;
         if (f < v.nfi) {
             const bool is_out = (e & SIDE_BIT) != 0;
             const int2 nb = v.fnb[f];
             const double4 po = v.phi[is_out ? nb.x : nb.y];
             const double4 own = is_out ? a.fr[f] : a.fl[f], oth = is_out ? a.fl[f] : a.fr[f];
+#pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const double pj = at(ph, j), oj = at(po, j);
-                put(aq, j, at(aq, j) + (1.0 - 0.5 * pj * zhi) * at(own, j) + 0.5 * oj * zhi * at(oth, j));
-                const double ej = 0.5 * pj * (1.0 - zhi) * at(own, j);
-                put(gx, j, at(gx, j) + ej * d0);
-                put(gy, j, at(gy, j) + ej * d1);
+                const N oj = at(po, j), w = at(own, j);
+                put(aq, j, (N(at(aq, j)) + own_w[j] * w + half(oj) * zhi * at(oth, j)).v);
+                const N ej = own_e[j] * w;
+                put(gx, j, (N(at(gx, j)) + ej * d0).v);
+                put(gy, j, (N(at(gy, j)) + ej * d1).v);
             }
         } else {
             const double4 l = a.fl[f];
             aq = add(aq, l);
+#pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const double ej = at(ph, j) * at(l, j);
-                put(gx, j, at(gx, j) + ej * d0);
-                put(gy, j, at(gy, j) + ej * d1);
+                const N ej = N(at(ph, j)) * at(l, j);
+                put(gx, j, (N(at(gx, j)) + ej * d0).v);
+                put(gy, j, (N(at(gy, j)) + ej * d1).v);
             }
             ac = add(ac, a.fr[f]);
         }
@@ -526,17 +550,18 @@ __global__ void k_adj_start_grad(CCView v, AdjView a) {
     if (v.grad_type == UNS_GRAD_GG) {
         const double2 n = v.fn[f];
         const double area = v.farea[f];
-        const double dx = n.x * area, dy = n.y * area;
-        const double si = interior ? 1.0 : -1.0;
-        double4 t = add(scl(si * dx / v.cv[nb.x], a.gx[nb.x]), scl(si * dy / v.cv[nb.x], a.gy[nb.x]));
+        const N dx = N(n.x) * area, dy = N(n.y) * area;
+        double4 t = add(scl(N(flip64(dx.v, !interior)) / v.cv[nb.x], a.gx[nb.x]),
+                        scl(N(flip64(dy.v, !interior)) / v.cv[nb.x], a.gy[nb.x]));
         if (interior) t = sub(t, add(scl(dx / v.cv[nb.y], a.gx[nb.y]), scl(dy / v.cv[nb.y], a.gy[nb.y])));
         a.fq[f] = add(a.fq[f], t);
     } else if (v.grad_type == UNS_GRAD_GGFC) {
-        const double s = v.fasum[f];
-        double4 gx = scl(s / v.cov[nb.x], a.gx[nb.x]), gy = scl(s / v.cov[nb.x], a.gy[nb.x]);
+        const N s = v.fasum[f], si = s / v.cov[nb.x];
+        double4 gx = scl(si, a.gx[nb.x]), gy = scl(si, a.gy[nb.x]);
         if (interior) {
-            gx = add(gx, scl(s / v.cov[nb.y], a.gx[nb.y]));
-            gy = add(gy, scl(s / v.cov[nb.y], a.gy[nb.y]));
+            const N so = s / v.cov[nb.y];
+            gx = add(gx, scl(so, a.gx[nb.y]));
+            gy = add(gy, scl(so, a.gy[nb.y]));
         }
         a.fgx[f] = add(a.fgx[f], gx);
         a.fgy[f] = add(a.fgy[f], gy);
@@ -549,16 +574,16 @@ __global__ void k_adj_start_grad(CCView v, AdjView a) {
 }
 
 // Diamond-path face gradient transposed onto its four points.
-__global__ void k_adj_ggfc(CCView v, AdjView a) {
+__global__ void __launch_bounds__(kBlock, 3) k_adj_ggfc(CCView v, AdjView a) {
     int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= v.nof) return;
     GgfcW w = ggfc_weights(v, f);
     const double4 gx = a.fgx[f], gy = a.fgy[f];
     const double2 gt = a.fgT[f];
-    a.cp1[f] = add(scl(w.p1x, gx), scl(w.p1y, gy)); a.cp1T[f] = w.p1x * gt.x + w.p1y * gt.y;
-    a.cp2[f] = add(scl(w.p2x, gx), scl(w.p2y, gy)); a.cp2T[f] = w.p2x * gt.x + w.p2y * gt.y;
-    a.cpi[f] = add(scl(w.ix, gx), scl(w.iy, gy)); a.cpiT[f] = w.ix * gt.x + w.iy * gt.y;
-    a.cpo[f] = add(scl(w.ox, gx), scl(w.oy, gy)); a.cpoT[f] = w.ox * gt.x + w.oy * gt.y;
+    a.cp1[f] = add(scl(w.p1x, gx), scl(w.p1y, gy)); a.cp1T[f] = (w.p1x * gt.x + w.p1y * gt.y).v;
+    a.cp2[f] = add(scl(w.p2x, gx), scl(w.p2y, gy)); a.cp2T[f] = (w.p2x * gt.x + w.p2y * gt.y).v;
+    a.cpi[f] = add(scl(w.ix, gx), scl(w.iy, gy)); a.cpiT[f] = (w.ix * gt.x + w.iy * gt.y).v;
+    a.cpo[f] = add(scl(w.ox, gx), scl(w.oy, gy)); a.cpoT[f] = (w.ox * gt.x + w.oy * gt.y).v;
 }
 
 // avg_c2v face part (face value = mean of its two vertices) and the
@@ -570,10 +595,12 @@ __global__ void k_adj_vertex(CCView v, AdjView a, int use_ggfc) {
     double pT = 0.0;
     for (int e = a.v2f_off[k]; e < a.v2f_off[k + 1]; ++e) {
         const int x = a.v2f[e], f = x & ~V2F_P2;
-        p = add(p, scl(0.5, a.fq[f]));
+        const double4 q = a.fq[f];
+        p = add(p, make_double4(dhalf(q.x), dhalf(q.y), dhalf(q.z), dhalf(q.w)));
         if (use_ggfc) {
-            if (x & V2F_P2) { p = add(p, a.cp2[f]); pT = pT + a.cp2T[f]; }
-            else { p = add(p, a.cp1[f]); pT = pT + a.cp1T[f]; }
+            const bool second = (x & V2F_P2) != 0;
+            p = add(p, second ? a.cp2[f] : a.cp1[f]);
+            pT = add64(pT, second ? a.cp2T[f] : a.cp1T[f]);
         }
     }
     a.pp[k] = p;
@@ -583,7 +610,7 @@ __global__ void k_adj_vertex(CCView v, AdjView a, int use_ggfc) {
 // Per cell (ghosts included): vertex average transposed, diamond-path and
 // LSQ cell terms, then con2prim transposed onto the state at the start of the
 // iteration.  Writes the new adjoint vector in place and the squared change.
-__global__ void k_adj_final(CCView v, AdjView a, int use_ggfc, int use_lsq) {
+__global__ void __launch_bounds__(kBlock, 3) k_adj_final(CCView v, AdjView a, int use_ggfc, int use_lsq) {
     // Ghost values of the start of the iteration reach a diamond-path
     // gradient only through Gradient_GG_FC of the start (grad_type GGFC); the
     // in-stage recomputation read each stage's own ghosts (already applied).
@@ -597,15 +624,18 @@ __global__ void k_adj_final(CCView v, AdjView a, int use_ggfc, int use_lsq) {
             const int k = a.c2v[e];
             const double w = a.c2v_w[e];
             q = add(q, scl(w, a.pp[k]));
-            T = T + w * a.ppT[k];
+            T = (N(T) + N(w) * a.ppT[k]).v;
         }
         if (use_ggfc || use_lsq) {
             auto face_terms = [&](int f, bool is_out) {
                 if (use_ggfc) {
-                    if (is_out) { q = add(q, a.cpo[f]); T = T + a.cpoT[f]; }
-                    else { q = add(q, a.cpi[f]); T = T + a.cpiT[f]; }
+                    q = add(q, is_out ? a.cpo[f] : a.cpi[f]);
+                    T = add64(T, is_out ? a.cpoT[f] : a.cpiT[f]);
                 }
-                if (use_lsq) q = is_out ? add(q, a.lsq[f]) : sub(q, a.lsq[f]);
+                if (use_lsq) {
+                    const double4 l = a.lsq[f];
+                    q = add(q, make_double4(flip64(l.x, !is_out), flip64(l.y, !is_out), flip64(l.z, !is_out), flip64(l.w, !is_out)));
+                }
             };
             if (i < v.noc) {
                 for (int k = v.cf_off[i]; k < v.cf_off[i + 1]; ++k) {
@@ -620,13 +650,20 @@ __global__ void k_adj_final(CCView v, AdjView a, int use_ggfc, int use_lsq) {
         }
         if (i < v.noc) {
             const double4 c = a.q0[i];
-            double r[4];
-            for (int dir = 0; dir < 4; ++dir) {
-                Tan E(c.x, dir == 0), rr(c.y, dir == 1), ru(c.z, dir == 2), rv(c.w, dir == 3);
-                PrimT<Tan> P = con2prim_t<Tan>(v.g, E, rr, ru, rv);
-                r[dir] = q.x * P.rho.d + q.y * P.u.d + q.z * P.v.d + q.w * P.p.d + T * P.t.d;
-            }
-            const double4 n = add(add(a.qc[i], a.qold[i]), make_double4(r[0], r[1], r[2], r[3]));
+            // con2prim's derivatives by the quotient rule, as the tangent type
+            // forms them, without the products by its zero seeds
+            const PrimT<N> P = con2prim_t<N>(v.g, c.x, c.y, c.z, c.w);
+            const N rho = c.y, ru = N(1.0) / rho, rz = rho * v.g.znd, gm1 = v.g.gamma - 1.0;
+            const N uu = P.u, vv = P.v, q2 = uu * uu + vv * vv, hr = half(rho);
+            const N ur = -uu / rho, vr = -vv / rho;  // du/drho, dv/drho
+            const N pr = -(gm1 * (half(q2) + hr * (twice(uu * ur) + twice(vv * vr))));
+            const N pu = -(gm1 * (hr * twice(uu * ru))), pv = -(gm1 * (hr * twice(vv * ru)));
+            const N qw = q.w, qT = T;
+            const N rE = qw * gm1 + qT * (gm1 / rz);
+            const N rr = N(q.x) + N(q.y) * ur + N(q.z) * vr + qw * pr + qT * ((pr - P.t * v.g.znd) / rz);
+            const N rru = N(q.y) * ru + qw * pu + qT * (pu / rz);
+            const N rrv = N(q.z) * ru + qw * pv + qT * (pv / rz);
+            const double4 n = add(add(a.qc[i], a.qold[i]), make_double4(rE.v, rr.v, rru.v, rrv.v));
             const double4 o = a.lq[i];
             const double4 dl = sub(n, o);
             dd = dot(dl, dl);

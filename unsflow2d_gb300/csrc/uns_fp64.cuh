@@ -80,8 +80,16 @@ __device__ __forceinline__ double flip64(double a, bool minus) { return dmake(dh
 // The native operations where they are rarely needed, as calls: branched
 // around (predicated off, they would hold the FP64 unit all the same), and
 // once in a kernel's code.
+static __device__ __noinline__ double native_mul(double a, double b) { return a * b; }
 static __device__ __noinline__ double add_rare(double a, double b) { return a + b; }
-static __device__ __noinline__ double mul_rare(double a, double b) { return a * b; }
+static __device__ __noinline__ double mul_rare(double a, double b) {
+    // zeros (uniform flow, the first steps of a solve) without the unit
+    const unsigned ha = dhi(a), hb = dhi(b);
+    const bool za = ((ha << 1) | dlo(a)) == 0, zb = ((hb << 1) | dlo(b)) == 0;
+    const bool fa = (ha & 0x7ff00000u) != 0x7ff00000u, fb = (hb & 0x7ff00000u) != 0x7ff00000u;
+    if ((za && fb) || (zb && fa)) return dmake((ha ^ hb) & 0x80000000u, 0u);
+    return native_mul(a, b);
+}
 static __device__ __noinline__ double div_rare(double a, double b) { return a / b; }
 static __device__ __noinline__ double sqrt_rare(double a) { return sqrt(a); }
 static __device__ __noinline__ double widen_rare(float a) { return (double)a; }

@@ -1078,6 +1078,7 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
         std::vector<int> src;
         std::vector<int4> sched(ws.items.size());
         std::vector<int> re, rn, rs;
+        re.reserve(2 * (size_t)nof); rn.reserve(2 * (size_t)nof); rs.reserve(2 * (size_t)nof); src.reserve(2 * (size_t)nof);
         for (size_t pos = 0; pos < ws.items.size(); ++pos) {
             const int it = ws.items[pos] >> 1, pass = ws.items[pos] & 1;
             const int first = (int)re.size();

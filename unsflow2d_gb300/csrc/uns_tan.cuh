@@ -11,6 +11,8 @@
 
 #include <cmath>
 
+#include "uns_fp64.cuh"
+
 namespace uns {
 // A namespace of its own, so that sqrt/fabs/pow of Tan are found only by
 // argument-dependent lookup and never hide ::sqrt for doubles in namespace uns.
@@ -23,39 +25,45 @@ struct Tan {
     __host__ __device__ Tan(double x, double dx) : v(x), d(dx) {}
 };
 
-__host__ __device__ __forceinline__ Tan operator+(Tan a, Tan b) { return Tan(a.v + b.v, a.d + b.d); }
-__host__ __device__ __forceinline__ Tan operator-(Tan a, Tan b) { return Tan(a.v - b.v, a.d - b.d); }
-__host__ __device__ __forceinline__ Tan operator-(Tan a) { return Tan(-a.v, -a.d); }
-__host__ __device__ __forceinline__ Tan operator*(Tan a, Tan b) { return Tan(a.v * b.v, a.d * b.v + a.v * b.d); }
-__host__ __device__ __forceinline__ Tan operator/(Tan a, Tan b) {
-    double q = a.v / b.v;
-    return Tan(q, (a.d - q * b.d) / b.v);
+// (Register FMAs and divisions on the integer pipe: the IEEE results,
+// uns_fp64.cuh.  Not its products: a seed's derivatives are mostly zero, which
+// the integer route hands to a call.)
+typedef F64 N;
+__device__ __forceinline__ Tan operator+(Tan a, Tan b) { return Tan((N(a.v) + b.v).v, (N(a.d) + b.d).v); }
+__device__ __forceinline__ Tan operator-(Tan a, Tan b) { return Tan((N(a.v) - b.v).v, (N(a.d) - b.d).v); }
+__device__ __forceinline__ Tan operator-(Tan a) { return Tan(neg64(a.v), neg64(a.d)); }
+__device__ __forceinline__ Tan operator*(Tan a, Tan b) {
+    return Tan((N(a.v) * b.v).v, (N(a.d) * b.v + N(a.v) * b.d).v);
 }
-__host__ __device__ __forceinline__ Tan operator+(Tan a, double b) { return Tan(a.v + b, a.d); }
-__host__ __device__ __forceinline__ Tan operator+(double a, Tan b) { return Tan(a + b.v, b.d); }
-__host__ __device__ __forceinline__ Tan operator-(Tan a, double b) { return Tan(a.v - b, a.d); }
-__host__ __device__ __forceinline__ Tan operator-(double a, Tan b) { return Tan(a - b.v, -b.d); }
-__host__ __device__ __forceinline__ Tan operator*(Tan a, double b) { return Tan(a.v * b, a.d * b); }
-__host__ __device__ __forceinline__ Tan operator*(double a, Tan b) { return Tan(a * b.v, a * b.d); }
-__host__ __device__ __forceinline__ Tan operator/(Tan a, double b) { return Tan(a.v / b, a.d / b); }
-__host__ __device__ __forceinline__ Tan operator/(double a, Tan b) {
-    double q = a / b.v;
-    return Tan(q, -q * b.d / b.v);
+__device__ __forceinline__ Tan operator/(Tan a, Tan b) {
+    const N q = N(a.v) / b.v;
+    return Tan(q.v, ((N(a.d) - q * b.d) / b.v).v);
 }
-__host__ __device__ __forceinline__ Tan& operator+=(Tan& a, Tan b) { a = a + b; return a; }
-__host__ __device__ __forceinline__ Tan& operator-=(Tan& a, Tan b) { a = a - b; return a; }
-__host__ __device__ __forceinline__ Tan& operator*=(Tan& a, Tan b) { a = a * b; return a; }
+__device__ __forceinline__ Tan operator+(Tan a, double b) { return Tan((N(a.v) + b).v, a.d); }
+__device__ __forceinline__ Tan operator+(double a, Tan b) { return Tan((N(a) + b.v).v, b.d); }
+__device__ __forceinline__ Tan operator-(Tan a, double b) { return Tan((N(a.v) - b).v, a.d); }
+__device__ __forceinline__ Tan operator-(double a, Tan b) { return Tan((N(a) - b.v).v, neg64(b.d)); }
+__device__ __forceinline__ Tan operator*(Tan a, double b) { return Tan((N(a.v) * b).v, (N(a.d) * b).v); }
+__device__ __forceinline__ Tan operator*(double a, Tan b) { return Tan((N(a) * b.v).v, (N(a) * b.d).v); }
+__device__ __forceinline__ Tan operator/(Tan a, double b) { return Tan((N(a.v) / b).v, (N(a.d) / b).v); }
+__device__ __forceinline__ Tan operator/(double a, Tan b) {
+    const N q = N(a) / b.v;
+    return Tan(q.v, (-q * b.d / b.v).v);
+}
+__device__ __forceinline__ Tan& operator+=(Tan& a, Tan b) { a = a + b; return a; }
+__device__ __forceinline__ Tan& operator-=(Tan& a, Tan b) { a = a - b; return a; }
+__device__ __forceinline__ Tan& operator*=(Tan& a, Tan b) { a = a * b; return a; }
 
 __host__ __device__ __forceinline__ bool operator<(Tan a, Tan b) { return a.v < b.v; }
 __host__ __device__ __forceinline__ bool operator>(Tan a, Tan b) { return a.v > b.v; }
 __host__ __device__ __forceinline__ bool operator<=(Tan a, Tan b) { return a.v <= b.v; }
 __host__ __device__ __forceinline__ bool operator>=(Tan a, Tan b) { return a.v >= b.v; }
 
-__host__ __device__ __forceinline__ Tan sqrt(Tan a) {
-    double r = ::sqrt(a.v);
-    return Tan(r, a.d / (2.0 * r));
+__device__ __forceinline__ Tan sqrt(Tan a) {
+    const double r = sqrt_digits(a.v);
+    return Tan(r, (N(a.d) / (N(2.0) * r)).v);
 }
-__host__ __device__ __forceinline__ Tan fabs(Tan a) { return a.v < 0.0 ? Tan(-a.v, -a.d) : a; }
+__device__ __forceinline__ Tan fabs(Tan a) { return a.v < 0.0 ? -a : a; }
 // a^b for a > 0: d(a^b) = a^b (b' ln a + b a'/a).
 __host__ __device__ __forceinline__ Tan pow(Tan a, Tan b) {
     double p = ::pow(a.v, b.v);

@@ -87,6 +87,10 @@ __device__ __forceinline__ double4 f4(const F64 o[4]) { return make_double4(o[0]
 // con2prim (main.F90:62-67) + save_old (solution.F90:118-132) + the global
 // min/max of every cell's primitives incl. ghosts (limiter.F90:146-149) +
 // the positivity check of main.F90:384-411, fused over one pass of the cells.
+// The eight ranges reduce over a warp by its integer reductions, on the high
+// and then the low word (4.2 M cells: 133 -> 107 us, mixed form 96 -> 81,
+// against five exchanges of both words each); an atomic skipped where the
+// stored range already covers a block's gained nothing.
 enum { BEGIN_PRIM = 1, BEGIN_OLD = 2, BEGIN_MINMAX = 4, BEGIN_POS = 8 };
 
 __global__ void __launch_bounds__(kBlock) k_begin(CCView v, int flags) {
@@ -102,12 +106,12 @@ __global__ void __launch_bounds__(kBlock) k_begin(CCView v, int flags) {
         const Gas& gi = gas_of(v, inst);
         double4 q = v.qc[i];
         if ((flags & BEGIN_PRIM) && v.mixed) {  // con2prim in FP32 from the rounded state
-            const float E = (float)q.x, r = (float)q.y, ru = (float)q.z, rv = (float)q.w;
+            const float E = narrow(q.x), r = narrow(q.y), ru = narrow(q.z), rv = narrow(q.w);
             const float u = ru / r, w = rv / r;
-            const float p = (float)gi.gamma1 * (E - 0.5f * r * (u * u + w * w));
+            const float p = narrow(gi.gamma1) * (E - 0.5f * r * (u * u + w * w));
             v.qpf[i] = make_float4(r, u, w, p);
-            v.qp[i] = make_double4(r, u, w, p);
-            pr[0] = r; pr[1] = u; pr[2] = w; pr[3] = p;
+            pr[0] = widen(r); pr[1] = widen(u); pr[2] = widen(w); pr[3] = widen(p);
+            v.qp[i] = make_double4(pr[0], pr[1], pr[2], pr[3]);
             have = true;
             if (v.laminar || v.grad_type == UNS_GRAD_GGFC) v.qT[i] = (double)(p / (r * (float)gi.znd));
             if ((flags & BEGIN_POS) && (r <= 0.f || p <= 0.f)) set_err(v.err, UNS_ERR_NONPOSITIVE, i);
@@ -143,15 +147,7 @@ __global__ void __launch_bounds__(kBlock) k_begin(CCView v, int flags) {
             return;
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                unsigned long long t = __shfl_xor_sync(0xffffffffu, emx[j], o);
-                emx[j] = t > emx[j] ? t : emx[j];
-                t = __shfl_xor_sync(0xffffffffu, emn[j], o);
-                emn[j] = t < emn[j] ? t : emn[j];
-            }
-        }
+        for (int j = 0; j < 4; ++j) { emx[j] = grp_max_u64(0xffffffffu, emx[j]); emn[j] = grp_min_u64(0xffffffffu, emn[j]); }
         __shared__ unsigned long long smx[kBlock / 32][4], smn[kBlock / 32][4];
         int w = threadIdx.x >> 5, l = threadIdx.x & 31;
         if (l == 0)
@@ -660,7 +656,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_cell_grad_side(CCView v, int flag
     const int inst = cell_inst(v, i);
     if (inst < 0 || stopped(v, inst)) return;
     const Gas& g = gas_of(v, inst);
-    const float gam = (float)g.gamma;
+    const float gam = (float)(g.gamma);
     const int k0 = v.cf_off[i], k1 = v.cf_off[i + 1];
     const float4 q4 = v.qpf[i];
     const float qi[4] = {q4.x, q4.y, q4.z, q4.w};
@@ -685,17 +681,18 @@ __global__ void __launch_bounds__(kBlock, 4) k_cell_grad_side(CCView v, int flag
         umax[2] = rmax(umax[2], w.z); umin[2] = rmin(umin[2], w.z);
         umax[3] = rmax(umax[3], w.w); umin[3] = rmin(umin[3], w.w);
     }
-    const float cvf = (float)v.cv[i];
+    const float cvf = (float)(v.cv[i]);
     if (flags & CG_DT) {
-        const float dt = (float)cur_cfl(v, inst, cfl_in) * cvf / la;
-        v.la[i] = (double)la;
-        v.dt[i] = (double)dt;
+        const float dt = (float)(cur_cfl(v, inst, cfl_in)) * cvf / la;
+        const double dtd = (double)(dt);
+        v.la[i] = (double)(la);
+        v.dt[i] = dtd;
         v.dcv[i] = (double)(dt / cvf);
         if (flags & CG_DIAG) {
             v.diag[i] = (double)(cvf / dt + 0.75f * la);
             v.diaginv[i] = 1.0 / v.diag[i];
         }
-        warp_atomic_min_u64(v, inst, enc_ord((double)dt));
+        warp_atomic_min_u64(v, inst, enc_ord(dtd));
     }
     {
         const float r = 1.f / cvf;
@@ -775,10 +772,13 @@ __device__ __forceinline__ double4 bnd_face_flux(const CCView& v, const Gas& g, 
         v.qc[out] = make_double4(b.gq[0].v, b.gq[1].v, b.gq[2].v, b.gq[3].v);
         v.qp[out] = make_double4(b.gp[0].v, b.gp[1].v, b.gp[2].v, b.gp[3].v);
         v.qT[out] = b.gT.v;
-        v.qpf[out] = make_float4((float)b.gp[0], (float)b.gp[1], (float)b.gp[2], (float)b.gp[3]);
+        v.qpf[out] = make_float4(narrow(b.gp[0].v), narrow(b.gp[1].v), narrow(b.gp[2].v), narrow(b.gp[3].v));
         if (bc == 1001) v.fwall[f - v.nfi] = make_double2(Fd.z, Fd.w);
     }
-    v.fF[f] = Fd;
+    if constexpr (std::is_same<R, float>::value)  // values of FP32 arithmetic
+        v.fFf()[f] = make_float4(narrow(Fd.x), narrow(Fd.y), narrow(Fd.z), narrow(Fd.w));
+    else
+        v.fF[f] = Fd;
     return Fd;
 }
 
@@ -830,7 +830,7 @@ __global__ void __launch_bounds__(std::is_same<R, float>::value ? 512 : kBlock, 
         }
         bool ok = flux_dispatch<float>(g, na.x, na.y, na.z, ql, qr, F);
         if (!ok) set_err(v.err, UNS_ERR_NEG_SOUND_SPEED, f);
-        v.fF[f] = make_double4((double)F[0], (double)F[1], (double)F[2], (double)F[3]);
+        v.fFf()[f] = make_float4(F[0], F[1], F[2], F[3]);
     } else {
         const int in = nb.x, out = nb.y;
         const double2 n = v.fn[f];
@@ -936,6 +936,16 @@ __global__ void __launch_bounds__(kBlock) k_face_visc(CCView v) {
     if (f >= v.nfi) v.fwallv[f - v.nfi] = (v.fbc[f] == 1001) ? make_double2(V2, V3) : make_double2(0.0, 0.0);
 }
 
+// A face's stored flux: FP64, or in the mixed form the FP32 values that its
+// arithmetic gave (half the bytes of writing them as FP64, and the conversion
+// on the integer pipe of the reader instead of the FP64 unit of the writer).
+__device__ __forceinline__ double4 widen4(const float4& F) { return make_double4(widen(F.x), widen(F.y), widen(F.z), widen(F.w)); }
+template <class R>
+__device__ __forceinline__ double4 stored_flux(const CCView& v, int f) {
+    if constexpr (std::is_same<R, float>::value) return widen4(v.fFf()[f]);
+    else return v.fF[f];
+}
+
 // Residual gather in the reference's accumulation order, optionally fused
 // with one RK3 stage (main.F90:92-101) and the block partials of the norm.
 // FP64 form, 4.2 M cells: 0.48 -> 0.20 ms (60 FP64 instructions per cell -> 25:
@@ -1030,6 +1040,10 @@ __global__ void __launch_bounds__(kBlock) k_cell_res(CCView v, int irk, int part
 // this kernel on GB300).  walls_done: the mixed form's one-pass step, where
 // k_cell_rk23_wall has already advanced the wall cells through all three
 // stages; they only contribute their residual to the norm here.
+// The fluxes are read as the FP32 values they are, 16 bytes a face instead of
+// 32, and widened here.  4.2 M cells: 153 -> 144 us, of which the 17 FP64
+// instructions per cell hold the unit 117 and the memory traffic takes 90; with
+// fewer than seven blocks per SM it is slower (six: 162, five: 177).
 __global__ void __launch_bounds__(kBlock, 8) k_cell_res_mixed(CCView v, int irk, int partial, int walls_done) {
     if (stopped(v, block_inst(v))) return;  // blocks of cells are instance-pure
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1040,30 +1054,28 @@ __global__ void __launch_bounds__(kBlock, 8) k_cell_res_mixed(CCView v, int irk,
             d4get(v.res[i], r);  // a wall cell: its last-stage residual (k_cell_rk23_wall)
         } else {
             const int k0 = v.cf_off[i], k1 = v.cf_off[i + 1];
-            auto add = [&](int k, int e, const double4& F) {
-                const int f = e & FACE_MASK;
-                const bool neg = f < v.nfi && (e & SIDE_BIT);
-                if (k == k0) {  // sign flip on the bits: no FP64 instruction
-                    const long long m = neg ? (long long)0x8000000000000000ULL : 0LL;
-                    r[0] = __longlong_as_double(__double_as_longlong(F.x) ^ m);
-                    r[1] = __longlong_as_double(__double_as_longlong(F.y) ^ m);
-                    r[2] = __longlong_as_double(__double_as_longlong(F.z) ^ m);
-                    r[3] = __longlong_as_double(__double_as_longlong(F.w) ^ m);
+            const float4* fF = v.fFf();
+            auto add = [&](int k, int e, float4 F) {
+                const unsigned m = (e & FACE_MASK) < v.nfi && (e & SIDE_BIT) ? 0x80000000u : 0u;
+                F.x = __uint_as_float(__float_as_uint(F.x) ^ m); F.y = __uint_as_float(__float_as_uint(F.y) ^ m);
+                F.z = __uint_as_float(__float_as_uint(F.z) ^ m); F.w = __uint_as_float(__float_as_uint(F.w) ^ m);
+                const double4 D = widen4(F);
+                if (k == k0) {
+                    r[0] = D.x; r[1] = D.y; r[2] = D.z; r[3] = D.w;
                 } else {
-                    const double s = neg ? -1.0 : 1.0;
-                    r[0] = __fma_rn(s, F.x, r[0]); r[1] = __fma_rn(s, F.y, r[1]); r[2] = __fma_rn(s, F.z, r[2]); r[3] = __fma_rn(s, F.w, r[3]);
+                    r[0] = add64(r[0], D.x); r[1] = add64(r[1], D.y); r[2] = add64(r[2], D.z); r[3] = add64(r[3], D.w);
                 }
             };
             if (k1 - k0 == 3) {  // a triangle: the three fluxes' gathers in flight together, summed in order
                 const int e0 = v.cf[k0], e1 = v.cf[k0 + 1], e2 = v.cf[k0 + 2];
-                const double4 F0 = v.fF[e0 & FACE_MASK], F1 = v.fF[e1 & FACE_MASK], F2 = v.fF[e2 & FACE_MASK];
+                const float4 F0 = fF[e0 & FACE_MASK], F1 = fF[e1 & FACE_MASK], F2 = fF[e2 & FACE_MASK];
                 add(k0, e0, F0);
                 add(k0 + 1, e1, F1);
                 add(k0 + 2, e2, F2);
             } else {
                 for (int k = k0; k < k1; ++k) {
                     const int e = v.cf[k];
-                    add(k, e, v.fF[e & FACE_MASK]);
+                    add(k, e, fF[e & FACE_MASK]);
                 }
             }
             if (v.laminar) {
@@ -1080,18 +1092,18 @@ __global__ void __launch_bounds__(kBlock, 8) k_cell_res_mixed(CCView v, int irk,
                 double c[4], q[4];
                 d4get(v.qc[i], c);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) q[j] = __fma_rn(-D, r[j], c[j]);
+                for (int j = 0; j < 4; ++j) q[j] = __fma_rn(neg64(D), r[j], c[j]);
                 if (irk > 1) {
                     const double a = rk3_a(irk), b = rk3_b(irk);
                     double o[4];
                     d4get(v.qold[i], o);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) q[j] = __fma_rn(a, o[j], b * q[j]);
+                    for (int j = 0; j < 4; ++j) q[j] = __fma_rn(a, o[j], mul64(b, q[j]));
                 }
                 v.qc[i] = d4(q);
             }
         }
-        if (partial) rr = __fma_rn(r[3], r[3], __fma_rn(r[2], r[2], __fma_rn(r[1], r[1], r[0] * r[0])));
+        if (partial) rr = __fma_rn(r[3], r[3], __fma_rn(r[2], r[2], __fma_rn(r[1], r[1], mul64(r[0], r[0]))));
     }
     if (partial) {
         __shared__ double sh[kBlock];
@@ -1099,7 +1111,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_cell_res_mixed(CCView v, int irk,
         __syncthreads();
         if (threadIdx.x < 32) {
             double t = sh[threadIdx.x];
-            for (int k = threadIdx.x + 32; k < kBlock; k += 32) t = t + sh[k];
+            for (int k = threadIdx.x + 32; k < kBlock; k += 32) t = add64(t, sh[k]);
             t = warp_sum(t);
             if (threadIdx.x == 0) v.partial[blockIdx.x] = t;
         }
@@ -1123,7 +1135,7 @@ __device__ __forceinline__ void rk_update(int irk, double D, const double o[4], 
     const double a = rk3_a(irk), b = rk3_b(irk);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        if (kMixed) q[j] = __fma_rn(a, o[j], b * __fma_rn(-D, r[j], q[j]));
+        if (kMixed) q[j] = __fma_rn(a, o[j], mul64(b, __fma_rn(neg64(D), r[j], q[j])));
         else if (irk == 2) q[j] = (F64I(a) * F64I(o[j]) + quarter(F64I(q[j]) - F64I(D) * F64I(r[j]))).v;  // b = 1/4
         else q[j] = (F64I(a) * F64I(o[j]) + F64I(b) * (F64I(q[j]) - F64I(D) * F64I(r[j]))).v;
     }
@@ -1140,7 +1152,7 @@ __device__ __forceinline__ void wall_cell_res(const CCView& v, const Gas& g, int
                                               bool recompute = true) {
     const int k0 = v.cf_off[i], k1 = v.cf_off[i + 1];
     auto flux = [&](int f) -> double4 {
-        return (recompute && f >= v.nfi && v.fbc[f] == 1001) ? bnd_face_flux<R>(v, g, f, i, q) : v.fF[f];
+        return (recompute && f >= v.nfi && v.fbc[f] == 1001) ? bnd_face_flux<R>(v, g, f, i, q) : stored_flux<R>(v, f);
     };
     if constexpr (std::is_same<R, float>::value) {  // k_cell_res_mixed's order
         for (int k = k0; k < k1; ++k) {

@@ -64,7 +64,8 @@ struct CCView {
     double* fqT;
     double* fla;
     double* fmu;
-    double4* fF;   // convective face flux (boundary: flux into `in`)
+    double4* fF;   // convective face flux (boundary: flux into `in`); the mixed form stores its FP32 values (fFf)
+    __device__ __forceinline__ float4* fFf() const { return reinterpret_cast<float4*>(fF); }
     double4* fV;   // viscous flux * area
     double4* fgx;  // diamond-path face gradient, rho,u,v,p
     double4* fgy;

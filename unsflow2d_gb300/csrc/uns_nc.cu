@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kBlock) k_nc_save_old(NCView v) {
     double4 q = v.qc[i];
     const PrimT<F64I> P = con2prim_t<F64I>(v.g, q.x, q.y, q.z, q.w);
     v.qp[i] = make_double4(q.y, P.u.v, P.v.v, P.p.v);
-    v.qpf[i] = make_float4((float)q.y, (float)P.u, (float)P.v, (float)P.p);
+    v.qpf[i] = make_float4(narrow(q.y), narrow(P.u.v), narrow(P.v.v), narrow(P.p.v));
     v.qold[i] = q;
 }
 
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kBlock) k_nc_grad_lim_mixed(NCView v) {
     }
     v.gx[i] = make_double4(gx[0], gx[1], gx[2], gx[3]);
     v.gy[i] = make_double4(gy[0], gy[1], gy[2], gy[3]);
-    const float eps = (float)v.eps;
+    const float eps = narrow(v.eps);
     float dmx[4], dmn[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) { dmn[k] = eps; dmx[k] = -eps; }
@@ -166,7 +166,9 @@ __global__ void __launch_bounds__(kBlock) k_nc_grad_lim_mixed(NCView v) {
     }
     double ph[4];
     g4(v.phi[i], ph);
-    const float sq = sqrtf((float)v.cv[i]);
+    const float sq = sqrtf(narrow(v.cv[i]));
+    const float kap = narrow(v.kappa);
+    float mn[4] = {INFINITY, INFINITY, INFINITY, INFINITY};  // a NaN is passed over here as in the chain of minima
     const bool vkn = v.limiter == UNS_LIM_VKN, corrected = v.limiter == UNS_LIM_BARTH_CORRECTED;
     for (int k = k0; k < k1; ++k) {
         const int e = v.v2f[k], f = e & EDGE_MASK;
@@ -177,7 +179,7 @@ __global__ void __launch_bounds__(kBlock) k_nc_grad_lim_mixed(NCView v) {
             float phj;
             if (vkn) {
                 const float D_L = (e & P2_BIT) ? -(0.5f * s) : 0.5f * s;
-                const float kk = (float)v.kappa * sq;
+                const float kk = kap * sq;
                 const float TOL = kk * kk * kk;
                 float alfa = D_L > 0.f ? dmx[j] : dmn[j];
                 if (fabsf(alfa) < eps) alfa = 0.f;
@@ -192,14 +194,19 @@ __global__ void __launch_bounds__(kBlock) k_nc_grad_lim_mixed(NCView v) {
                 else phj = 1.f;
                 if (corrected) phj = rmax(0.f, phj);
             }
-            ph[j] = rmin(ph[j], (double)phj);
+            mn[j] = rmin(mn[j], phj);
         }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const double pd = widen(mn[j]);
+        if (dlt(pd, ph[j])) ph[j] = pd;
     }
     v.phi[i] = m4(ph);
     float4* pk = v.packn + 3 * (size_t)i;
     pk[0] = make_float4(gx[0], gx[1], gx[2], gx[3]);
     pk[1] = make_float4(gy[0], gy[1], gy[2], gy[3]);
-    pk[2] = make_float4((float)ph[0], (float)ph[1], (float)ph[2], (float)ph[3]);
+    pk[2] = make_float4(narrow(ph[0]), narrow(ph[1]), narrow(ph[2]), narrow(ph[3]));
 }
 
 // The FP64 form.  S = F64I (sums on the FP64 unit, products, divisions and
@@ -390,20 +397,21 @@ __global__ void __launch_bounds__(kBlock, std::is_same<R, float>::value ? 1 : 3)
                 Rt[k] = q2[k] - 0.5f * g * f2[k];
             }
             const double2 n = v.fn[f];
-            const float area = (float)v.farea[f];
-            const float G = (float)v.g.gamma, G1 = (float)v.g.gamma1;
+            const float area = narrow(v.farea[f]);
+            const float G = narrow(v.g.gamma), G1 = narrow(v.g.gamma1);
+            const float nx = narrow(n.x), ny = narrow(n.y);
             float hl, hr;
-            if (v.g.flux == UNS_FLUX_AUSM) ausm_core<float>(G, G1, (float)n.x, (float)n.y, (float)v.g.mref, L, Rt, F, hl, hr);
-            else vanleer_core<float>(G, G1, (float)n.x, (float)n.y, L, Rt, F, hl, hr);
-            v.fF[f] = make_double4(F[0] * area, F[1] * area, F[2] * area, F[3] * area);
+            if (v.g.flux == UNS_FLUX_AUSM) ausm_core<float>(G, G1, nx, ny, narrow(v.g.mref), L, Rt, F, hl, hr);
+            else vanleer_core<float>(G, G1, nx, ny, L, Rt, F, hl, hr);
+            v.fF[f] = make_double4(widen(F[0] * area), widen(F[1] * area), widen(F[2] * area), widen(F[3] * area));
             // Roe-averaged spectral radius (vanleer_flux.f90:102-115)
             const float RT = sqrtf(Rt[0] / L[0]);
             const float u = (L[1] + RT * Rt[1]) / (1.f + RT);
             const float vv = (L[2] + RT * Rt[2]) / (1.f + RT);
             const float H = (hl + RT * hr) / (1.f + RT);
             const float aa = sqrtf(G1 * (H - 0.5f * (u * u + vv * vv)));
-            const float un = fabsf(u * (float)n.x + vv * (float)n.y);
-            v.fla[f] = (double)((un + aa) * area);
+            const float un = fabsf(u * nx + vv * ny);
+            v.fla[f] = widen((un + aa) * area);
             return;
         }
     }

@@ -337,17 +337,25 @@ struct Cvt<T, T> {
 };
 template <>
 struct Cvt<F64I, float> {
-    __device__ __forceinline__ static F64I f(float x) { return F64I((double)x); }
+    __device__ __forceinline__ static F64I f(float x) { return F64I(widen(x)); }
 };
 template <>
 struct Cvt<F64, float> {
-    __device__ __forceinline__ static F64 f(float x) { return F64((double)x); }
+    __device__ __forceinline__ static F64 f(float x) { return F64(widen(x)); }
+};
+template <>
+struct Cvt<float, double> {
+    __device__ __forceinline__ static float f(double x) { return narrow(x); }
+};
+template <>
+struct Cvt<float, F64> {
+    __device__ __forceinline__ static float f(F64 x) { return narrow(x.v); }
 };
 
 // Convective flux of the selected scheme (fvresidual.F90 flux selection).
 template <class R>
 __device__ __forceinline__ bool face_flux(const Gas& g, R nx, R ny, R area, V4<R>& ql, V4<R>& qr, V4<R>& F) {
-    const R G = (R)g.gamma, G1 = (R)g.gamma1;
+    const R G = Cvt<R, double>::f(g.gamma), G1 = Cvt<R, double>::f(g.gamma1);
     bool ok = true;
     R hl, hr;
     switch (g.flux) {
@@ -358,7 +366,7 @@ __device__ __forceinline__ bool face_flux(const Gas& g, R nx, R ny, R area, V4<R
             for (int k = 0; k < 4; ++k) F[k] = F[k] * area;
             break;
         default: {  // AUSM+-up: the reference scales by |n| of the unit normal
-            ausm_core<R>(G, G1, nx, ny, (R)g.mref, ql, qr, F, hl, hr);
+            ausm_core<R>(G, G1, nx, ny, Cvt<R, double>::f(g.mref), ql, qr, F, hl, hr);
             R an = sqrt(nx * nx + ny * ny);
             for (int k = 0; k < 4; ++k) F[k] = F[k] * an;
         }

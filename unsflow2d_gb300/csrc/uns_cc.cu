@@ -2182,7 +2182,6 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
                 nbr[k] = other(i, m->c2f[k], &fl);
             }
         WarpSchedule ws = list_schedule(noc, m->c2f_off, nbr.data(), h->coop_blocks * kSweepPairs);
-        const std::vector<int> at = record_places(ws);
         std::vector<int> src;
         std::vector<int4> sched(ws.items.size());
         std::vector<int> rf, rn, rl;
@@ -2191,11 +2190,11 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
             const int it = ws.items[pos] >> 1, pass = ws.items[pos] & 1;
             const int first = (int)rf.size();
             for (int k = m->c2f_off[it]; k < m->c2f_off[it + 1]; ++k) {
-                int fl, nb = other(it, m->c2f[k], &fl);
-                bool take = nb >= 0 && nb < noc && (pass == 0 ? nb < it : nb > it);
-                if (take) { rf.push_back(m->c2f[k]); rn.push_back(nb); rl.push_back(fl);
-                    const int from = (nb << 1) | pass;
-                    src.push_back(ws.warp[from] / kSchedGroup == ws.warp[ws.items[pos]] / kSchedGroup ? at[from] : -1); }
+                const int nb = nbr[k];
+                const bool take = nb >= 0 && nb < noc && (pass == 0 ? nb < it : nb > it);
+                if (!take) continue;
+                rf.push_back(m->c2f[k]); rn.push_back(nb); rl.push_back(m->fout[m->c2f[k]] == it ? 1 : 0);
+                src.push_back(record_source(ws, (nb << 1) | pass, ws.items[pos]));
             }
             sched[pos] = make_int4(it, pass, first, (int)rf.size() - first);
         }

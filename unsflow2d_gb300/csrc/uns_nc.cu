@@ -1082,7 +1082,6 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
         WarpSchedule ws = list_schedule(nop, m->v2f_off, nbr.data(), h->coop_blocks * kSweepPairs);
         h->lev_fwd = ws.nlev_fwd;
         h->lev_bwd = ws.nlev_bwd;
-        const std::vector<int> at = record_places(ws);
         std::vector<int> src;
         std::vector<int4> sched(ws.items.size());
         std::vector<int> re, rn, rs;
@@ -1091,11 +1090,13 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
             const int it = ws.items[pos] >> 1, pass = ws.items[pos] & 1;
             const int first = (int)re.size();
             for (int k = m->v2f_off[it]; k < m->v2f_off[it + 1]; ++k) {
-                int sg, nb = other(it, m->v2f[k], &sg);
-                bool take = nb >= 0 && nb < nop && (pass == 0 ? nb < it : nb > it);
-                if (take) { re.push_back(m->v2f[k]); rn.push_back(nb); rs.push_back(sg);
-                    const int from = (nb << 1) | pass;
-                    src.push_back(ws.warp[from] / kSchedGroup == ws.warp[ws.items[pos]] / kSchedGroup ? at[from] : -1); }
+                const int nb = nbr[k];
+                const bool take = nb >= 0 && nb < nop && (pass == 0 ? nb < it : nb > it);
+                if (!take) continue;
+                int sg;
+                other(it, m->v2f[k], &sg);
+                re.push_back(m->v2f[k]); rn.push_back(nb); rs.push_back(sg);
+                src.push_back(record_source(ws, (nb << 1) | pass, ws.items[pos]));
             }
             sched[pos] = make_int4(it, pass, first, (int)re.size() - first);
         }

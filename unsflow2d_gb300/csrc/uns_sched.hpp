@@ -29,10 +29,6 @@
 // always proceed: the sweep cannot deadlock.
 #pragma once
 #include <algorithm>
-#include <cstdlib>
-#include <functional>
-#include <queue>
-#include <utility>
 #include <vector>
 
 namespace uns {
@@ -40,7 +36,10 @@ namespace uns {
 struct WarpSchedule {
     std::vector<int> off;    // nwarps + 1 offsets into items
     std::vector<int> items;  // (entity << 1) | pass, pass 0 = forward, 1 = backward
-    std::vector<int> warp;   // item code -> its warp
+    struct Place {
+        int warp, index;
+    };
+    std::vector<Place> place;  // item code -> its warp and where in the warp's list
     double makespan = 0.0;   // simulated length in units of one item's compute
     int nlev_fwd = 0, nlev_bwd = 0;
 };
@@ -88,48 +87,57 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
         for (int i = n - 1; i >= 0; --i) bwd[cb[levb[i]]++] = i;
     }
 
-    std::vector<double> fin(2 * (size_t)n, 0.0);  // item code -> simulated finish
-    std::vector<int> wof(2 * (size_t)n, -1);      // item code -> warp
+    struct Item {  // a placed item: its simulated finish, warp and place in the warp's list
+        double fin;
+        int warp, index;
+    };
+    std::vector<Item> done(2 * (size_t)n);
     std::vector<double> wfree(nwarps, 0.0);
     std::vector<int> wlast(nwarps, -1);
     std::vector<std::vector<int>> lists(nwarps);
-    using E = std::pair<double, int>;
-    std::priority_queue<E, std::vector<E>, std::greater<E>> heap;
-    for (int w = 0; w < nwarps; ++w) heap.push({0.0, w});
+    // The warp that frees up first (of several, the lowest): a tournament.  A
+    // heap with an entry per placement outgrows the caches on a large mesh
+    // (4.2 M cells).
+    int leaves = 1;
+    while (leaves < nwarps) leaves *= 2;
+    std::vector<int> first(2 * (size_t)leaves, -1);
+    auto earlier = [&](int a, int b) { return b < 0 || (a >= 0 && wfree[a] <= wfree[b]) ? a : b; };
+    for (int w = 0; w < nwarps; ++w) first[leaves + w] = w;
+    for (int k = leaves - 1; k > 0; --k) first[k] = earlier(first[2 * k], first[2 * k + 1]);
 
     std::vector<int> preds;
+    std::vector<Item> pr;  // the predecessors' items
+    double makespan = 0.0;
     auto place = [&](int code) {
+        pr.clear();
+        double last = 0.0;
+        for (int p : preds) { pr.push_back(done[p]); last = std::max(last, done[p].fin); }
         // The item's start on warp c, and the candidates: a warp that is not
         // free before the best start so far cannot improve on it.
         int w = -1;
         double s = 0.0;
         auto consider = [&](int c) {
             double t = wfree[c];
-            if (w >= 0 && t >= s - 1e-12) return;
-            for (int p : preds) {
-                const int v = wof[p];
-                t = std::max(t, fin[p] + (v == c ? 0.0 : (v / kSchedGroup == c / kSchedGroup ? kNear : kSync)));
-            }
+            if (w >= 0 && std::max(t, last) >= s - 1e-12) return;
+            for (const Item& p : pr)
+                t = std::max(t, p.fin + (p.warp == c ? 0.0 : (p.warp / kSchedGroup == c / kSchedGroup ? kNear : kSync)));
             if (w < 0 || t < s - 1e-12) { w = c; s = t; }
         };
-        for (int p : preds)
-            if (wlast[wof[p]] == p) consider(wof[p]);
-        int seen[8], nseen = 0;
-        for (int p : preds) {
-            const int g = wof[p] / kSchedGroup * kSchedGroup;
+        for (size_t k = 0; k < pr.size(); ++k)
+            if (wlast[pr[k].warp] == preds[k]) consider(pr[k].warp);
+        for (size_t k = 0; k < pr.size(); ++k) {
+            const int g = pr[k].warp / kSchedGroup;
             bool again = false;
-            for (int q = 0; q < nseen; ++q) again = again || seen[q] == g;
+            for (size_t q = 0; q < k; ++q) again = again || pr[q].warp / kSchedGroup == g;
             if (again) continue;
-            if (nseen < 8) seen[nseen++] = g;
-            for (int c = g; c < g + kSchedGroup && c < nwarps; ++c) consider(c);
+            for (int c = g * kSchedGroup; c < (g + 1) * kSchedGroup && c < nwarps; ++c) consider(c);
         }
-        while (heap.top().first != wfree[heap.top().second]) heap.pop();  // drop stale entries
-        consider(heap.top().second);
-        fin[code] = s + kCompute;
-        wof[code] = w;
-        wfree[w] = fin[code];
+        consider(first[1]);
+        done[code] = {s + kCompute, w, (int)lists[w].size()};
+        makespan = std::max(makespan, s + kCompute);
+        wfree[w] = s + kCompute;
         wlast[w] = code;
-        heap.push({wfree[w], w});
+        for (int k = (leaves + w) / 2; k > 0; k /= 2) first[k] = earlier(first[2 * k], first[2 * k + 1]);
         lists[w].push_back(code);
     };
     for (int i : fwd) {
@@ -150,25 +158,23 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
         place(2 * i + 1);
     }
     WarpSchedule out;
-    out.makespan = fin.empty() ? 0.0 : *std::max_element(fin.begin(), fin.end());
+    out.makespan = makespan;
     out.nlev_fwd = nlev;
     out.nlev_bwd = nlevb;
     out.off.assign(nwarps + 1, 0);
     for (int w = 0; w < nwarps; ++w) out.off[w + 1] = out.off[w] + (int)lists[w].size();
-    out.warp = wof;
+    out.place.resize(done.size());
+    for (size_t k = 0; k < done.size(); ++k) out.place[k] = {done[k].warp, done[k].index};
     out.items.reserve(2 * (size_t)n);
     for (int w = 0; w < nwarps; ++w) out.items.insert(out.items.end(), lists[w].begin(), lists[w].end());
     return out;
 }
 
-// Per item code: where the sweep warps of its block find its record, (warp of
-// the block << 28) | list index.
-inline std::vector<int> record_places(const WarpSchedule& ws) {
-    std::vector<int> at(ws.items.size());
-    for (size_t w = 0; w + 1 < ws.off.size(); ++w)
-        for (int k = ws.off[w]; k < ws.off[w + 1]; ++k)
-            at[ws.items[k]] = (int)(w % kSchedGroup) << 28 | (k - ws.off[w]);
-    return at;
+// Where item `to`'s sweep warp finds the record of the item `from`: for one
+// of its block (warp of the block << 28) | list index, else -1 (in L2).
+inline int record_source(const WarpSchedule& ws, int from, int to) {
+    const WarpSchedule::Place f = ws.place[from];
+    return f.warp / kSchedGroup == ws.place[to].warp / kSchedGroup ? (f.warp % kSchedGroup) << 28 | f.index : -1;
 }
 
 }  // namespace uns

@@ -2176,31 +2176,32 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
             return m->fout[f];
         };
         std::vector<int> nbr(m->c2f_off[noc]);
+        std::vector<signed char> flip(m->c2f_off[noc]);
         for (int i = 0; i < noc; ++i)
             for (int k = m->c2f_off[i]; k < m->c2f_off[i + 1]; ++k) {
                 int fl;
                 nbr[k] = other(i, m->c2f[k], &fl);
+                flip[k] = (signed char)fl;
             }
         WarpSchedule ws = list_schedule(noc, m->c2f_off, nbr.data(), h->coop_blocks * kSweepPairs);
-        std::vector<int> src;
         std::vector<int4> sched(ws.items.size());
         std::vector<int> rf, rn, rl;
-        rf.reserve(2 * (size_t)nfi); rn.reserve(2 * (size_t)nfi); rl.reserve(2 * (size_t)nfi); src.reserve(2 * (size_t)nfi);
+        rf.reserve(2 * (size_t)nfi); rn.reserve(2 * (size_t)nfi); rl.reserve(2 * (size_t)nfi);
         for (size_t pos = 0; pos < ws.items.size(); ++pos) {
             const int it = ws.items[pos] >> 1, pass = ws.items[pos] & 1;
             const int first = (int)rf.size();
+            ask_ahead(ws, pos, m->c2f_off, nbr.data(), m->c2f, flip.data());
             for (int k = m->c2f_off[it]; k < m->c2f_off[it + 1]; ++k) {
                 const int nb = nbr[k];
                 const bool take = nb >= 0 && nb < noc && (pass == 0 ? nb < it : nb > it);
                 if (!take) continue;
-                rf.push_back(m->c2f[k]); rn.push_back(nb); rl.push_back(m->fout[m->c2f[k]] == it ? 1 : 0);
-                src.push_back(record_source(ws, (nb << 1) | pass, ws.items[pos]));
+                rf.push_back(m->c2f[k]); rn.push_back(nb); rl.push_back(flip[k]);
             }
             sched[pos] = make_int4(it, pass, first, (int)rf.size() - first);
         }
         v.nrec = (int)rf.size();
         if ((rc = h->upload(h->woff, ws.off.data(), ws.off.size()))) return fail(rc);
-        UP(sched, sched); UP(rec_face, rf); UP(rec_nb, rn); UP(rec_flip, rl); UP(rec_src, src);
+        UP(sched, sched); UP(rec_face, rf); UP(rec_nb, rn); UP(rec_flip, rl); UP(rec_src, ws.src);
         AL(rec, 3 * rf.size());
         AL(srec, 10 * (size_t)noc);
     }

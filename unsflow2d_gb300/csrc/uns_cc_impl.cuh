@@ -83,7 +83,7 @@ struct CCView {
     const int* rec_face;
     const int* rec_nb;
     const int* rec_flip;
-    const int* rec_src;  // producer in the same block (record_places), or -1
+    const int* rec_src;  // producer in the same block (WarpSchedule::src), or -1
     int nrec;
     double4* rec;     // per record, per LU-SGS call: 3 x double4 (k_cc_sweep_prep) or 4 x float4 (k_cc_sweep_prep_mixed)
     double2* srec;    // sweep records (sweep_args): 10 per cell

@@ -76,7 +76,7 @@ struct NCView {
     const int* rec_edge;
     const int* rec_nb;
     const int* rec_sign;
-    const int* rec_src;  // producer in the same block (record_places), or -1
+    const int* rec_src;  // producer in the same block (WarpSchedule::src), or -1
     int nrec;
     double4* rec;    // per record, per LU-SGS call: 3 x double4 (k_nc_sweep_prep) or 4 x float4 (k_nc_sweep_prep_mixed)
     double* diag;    // LU-SGS diagonal cv/dt + 0.5*omega*la (lusgs.f90:36)
@@ -1074,35 +1074,34 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
             return m->fp2[e];
         };
         std::vector<int> nbr(m->v2f_off[nop]);
+        std::vector<signed char> sgn(m->v2f_off[nop]);
         for (int i = 0; i < nop; ++i)
             for (int k = m->v2f_off[i]; k < m->v2f_off[i + 1]; ++k) {
                 int sg;
                 nbr[k] = other(i, m->v2f[k], &sg);
+                sgn[k] = (signed char)sg;
             }
         WarpSchedule ws = list_schedule(nop, m->v2f_off, nbr.data(), h->coop_blocks * kSweepPairs);
         h->lev_fwd = ws.nlev_fwd;
         h->lev_bwd = ws.nlev_bwd;
-        std::vector<int> src;
         std::vector<int4> sched(ws.items.size());
         std::vector<int> re, rn, rs;
-        re.reserve(2 * (size_t)nof); rn.reserve(2 * (size_t)nof); rs.reserve(2 * (size_t)nof); src.reserve(2 * (size_t)nof);
+        re.reserve(2 * (size_t)nof); rn.reserve(2 * (size_t)nof); rs.reserve(2 * (size_t)nof);
         for (size_t pos = 0; pos < ws.items.size(); ++pos) {
             const int it = ws.items[pos] >> 1, pass = ws.items[pos] & 1;
             const int first = (int)re.size();
+            ask_ahead(ws, pos, m->v2f_off, nbr.data(), m->v2f, sgn.data());
             for (int k = m->v2f_off[it]; k < m->v2f_off[it + 1]; ++k) {
                 const int nb = nbr[k];
                 const bool take = nb >= 0 && nb < nop && (pass == 0 ? nb < it : nb > it);
                 if (!take) continue;
-                int sg;
-                other(it, m->v2f[k], &sg);
-                re.push_back(m->v2f[k]); rn.push_back(nb); rs.push_back(sg);
-                src.push_back(record_source(ws, (nb << 1) | pass, ws.items[pos]));
+                re.push_back(m->v2f[k]); rn.push_back(nb); rs.push_back(sgn[k]);
             }
             sched[pos] = make_int4(it, pass, first, (int)re.size() - first);
         }
         h->v.nrec = (int)re.size();
         if ((rc = h->upload(h->woff, ws.off.data(), ws.off.size()))) return fail(rc);
-        UPN(sched, sched); UPN(rec_edge, re); UPN(rec_nb, rn); UPN(rec_sign, rs); UPN(rec_src, src);
+        UPN(sched, sched); UPN(rec_edge, re); UPN(rec_nb, rn); UPN(rec_sign, rs); UPN(rec_src, ws.src);
         ALN(rec, 3 * re.size());
     }
 #undef UPN

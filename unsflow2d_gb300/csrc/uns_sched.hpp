@@ -36,10 +36,10 @@ namespace uns {
 struct WarpSchedule {
     std::vector<int> off;    // nwarps + 1 offsets into items
     std::vector<int> items;  // (entity << 1) | pass, pass 0 = forward, 1 = backward
-    struct Place {
-        int warp, index;
-    };
-    std::vector<Place> place;  // item code -> its warp and where in the warp's list
+    // Item by item, for each neighbour that the item waits for (in the order of
+    // its CSR list): where its sweep warp finds the neighbour's record, (warp of
+    // the block << 28) | list index, or -1 for one of another block, in L2.
+    std::vector<int> src;
     double makespan = 0.0;   // simulated length in units of one item's compute
     int nlev_fwd = 0, nlev_bwd = 0;
 };
@@ -94,7 +94,11 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
     std::vector<Item> done(2 * (size_t)n);
     std::vector<double> wfree(nwarps, 0.0);
     std::vector<int> wlast(nwarps, -1);
-    std::vector<std::vector<int>> lists(nwarps);
+    std::vector<std::vector<int>> lists(nwarps), srcs(nwarps);
+    for (int w = 0; w < nwarps; ++w) {
+        lists[w].reserve(2 * (size_t)n / nwarps + 64);
+        srcs[w].reserve((size_t)(nbr_off[n] - nbr_off[0]) / nwarps + 64);
+    }
     // The warp that frees up first (of several, the lowest): a tournament.  A
     // heap with an entry per placement outgrows the caches on a large mesh
     // (4.2 M cells).
@@ -137,8 +141,11 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
         makespan = std::max(makespan, s + kCompute);
         wfree[w] = s + kCompute;
         wlast[w] = code;
-        for (int k = (leaves + w) / 2; k > 0; k /= 2) first[k] = earlier(first[2 * k], first[2 * k + 1]);
+        // w frees up later than before: only the rounds that it had won change
+        for (int k = (leaves + w) / 2; k > 0 && first[k] == w; k /= 2) first[k] = earlier(first[2 * k], first[2 * k + 1]);
         lists[w].push_back(code);
+        for (size_t k = code & 1; k < pr.size(); ++k)  // not a backward item's own forward value
+            srcs[w].push_back(pr[k].warp / kSchedGroup == w / kSchedGroup ? (pr[k].warp % kSchedGroup) << 28 | pr[k].index : -1);
     };
     for (int i : fwd) {
         preds.clear();
@@ -163,18 +170,22 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
     out.nlev_bwd = nlevb;
     out.off.assign(nwarps + 1, 0);
     for (int w = 0; w < nwarps; ++w) out.off[w + 1] = out.off[w] + (int)lists[w].size();
-    out.place.resize(done.size());
-    for (size_t k = 0; k < done.size(); ++k) out.place[k] = {done[k].warp, done[k].index};
     out.items.reserve(2 * (size_t)n);
     for (int w = 0; w < nwarps; ++w) out.items.insert(out.items.end(), lists[w].begin(), lists[w].end());
+    for (const auto& l : srcs) out.src.insert(out.src.end(), l.begin(), l.end());
     return out;
 }
 
-// Where item `to`'s sweep warp finds the record of the item `from`: for one
-// of its block (warp of the block << 28) | list index, else -1 (in L2).
-inline int record_source(const WarpSchedule& ws, int from, int to) {
-    const WarpSchedule::Place f = ws.place[from];
-    return f.warp / kSchedGroup == ws.place[to].warp / kSchedGroup ? (f.warp % kSchedGroup) << 28 | f.index : -1;
+// Asks for what the records of some later item are made of: a warp's list jumps
+// over the whole mesh (CCFVM, 4.2 M cells: the records 1.1 -> 0.64 s).
+inline void ask_ahead(const WarpSchedule& ws, size_t pos, const int* off, const int* nbr, const int* edge, const signed char* side) {
+    if (pos + 32 < ws.items.size()) __builtin_prefetch(off + (ws.items[pos + 32] >> 1));
+    if (pos + 16 < ws.items.size()) {
+        const int k = off[ws.items[pos + 16] >> 1];
+        __builtin_prefetch(nbr + k);
+        __builtin_prefetch(edge + k);
+        __builtin_prefetch(side + k);
+    }
 }
 
 }  // namespace uns

@@ -89,9 +89,12 @@ WORKLOADS = {
 
 # Kernels launched per iteration (our own; memsets excluded).
 # CCFVM inviscid RK3 in FP64: reset_minmax, begin, vertex_avg, face_prim_spec, cell_grad,
-# face_conv, cell_res (stage 1), cell_rk23_wall + cell_rk23 (stages 2-3), res_final.
+# face_conv, wall_rk3 (wall cells, stages 1-3), cell_rk3 (the others; one launch where the
+# stages apart were two, which cc_kernels takes off), res_final.
 # Mixed GG form: reset_minmax, begin, vertex_avg, cell_grad_side, face_conv,
-# cell_rk23_wall (wall cells, stages 1-3), cell_res_mixed, res_final.
+# wall_rk3, cell_res_mixed, res_final.
+# LU-SGS: reset_minmax, begin, vertex_avg, face_prim_spec, cell_grad, face_conv, cell_res,
+# sweep_prep, one fill of the records (two in the FP32 form), sweeps, res_final.
 LAUNCHES = {("nc", "lusgs"): 9, ("nc", "rk3"): 5, ("cc", "rk3"): 10, ("cc", "lusgs"): 12, ("cc", "rk3_mixed_gg"): 8}
 
 
@@ -110,6 +113,16 @@ def cc_launches(p) -> int:
     # 3 x (face_conv, cell_mul, [face_ggfc, (reset_minmax, begin), cell_grad], face_visc, cell_res), res_final
     per_stage = 4 + (0 if ggfc else 2 + (2 if p.ilimit else 0))
     return 5 + (1 if ggfc else 0) + 3 * per_stage + 1
+
+
+def cc_kernels(p) -> int:
+    """cc_launches less the launches that one iteration no longer makes of that sequence."""
+    n = cc_launches(p)
+    if p.time_mode != abi.TIME["rk3"]:
+        return n - (1 if p.precision == abi.PREC["fp64"] else 0)  # one fill of the sweeps' records
+    if p.flow_type == abi.FLOW["laminar"]:
+        return n - (2 if p.grad_type == abi.GRAD["ggfc"] else 0)  # stages 2-3: cell_mul with the wall faces
+    return n - (1 if p.precision != abi.PREC["mixed"] else 0)  # cell_rk3
 
 
 def adjoint_cost(solver, w: dict, cfl: float, prof: dict) -> dict:
@@ -199,9 +212,9 @@ def algorithmic_bytes(kind: str, m: dict, mixed: bool = False, sides: bool = Fal
             # offsets, 32-byte cell-side records, vertex values, FP32 primitives (own and across), cv;
             # la, dt, dt/cv written; pack (phi read, 64 B written)
             "cell_grad": 4 * N + 32 * nside + 16 * P + 16 * N + 8 * N + 24 * N + 16 * N + 64 * N,
-            "face_conv": 8 * F + 32 * F + 64 * N + 32 * F + 72 * G,
-            # face lists, FP64 fluxes, qc read+write, res written, dt/cv, wall bits
-            "cell_res": 16 * N + 32 * F + 64 * N + 32 * N + 8 * N + N // 8,
+            "face_conv": 8 * F + 32 * F + 64 * N + 16 * F + 72 * G,
+            # face lists, FP32 fluxes, qc read+write, res written, dt/cv, wall bits
+            "cell_res": 16 * N + 16 * F + 64 * N + 32 * N + 8 * N + N // 8,
             # wall cells, stages 1-3: per wall face its neighbours, geometry, the pack of its cell, ghost
             # writes, wall force and flux; its cell's face lists, stored fluxes, state and residual
             "cell_rk23": (300 + 148 + 80) * W,
@@ -219,15 +232,13 @@ def algorithmic_bytes(kind: str, m: dict, mixed: bool = False, sides: bool = Fal
             # face lists, FP32 radii / normals / face values / offsets, neighbours, cv; la, dt, dt/cv, diag;
             # FP32 primitives; pack (phi read, 64 B written)
             "cell_grad": 4 * N + 8 * F + 4 * F + 16 * F + 16 * F + 16 * F + 8 * F + 8 * N + 32 * N + 16 * N + 16 * N + 64 * N,
-            # neighbours, FP32 offsets + normal/length, two 64-byte packs (each cell once), FP64 flux written;
+            # neighbours, FP32 offsets + normal/length, two 64-byte packs (each cell once), FP32 flux written;
             # boundary: ghost writes and wall force
-            "face_conv": 8 * F + 32 * F + 64 * N + 32 * F + 72 * G,
-            # face lists, FP64 fluxes, qc read+write, qold, res, dt/cv
-            "cell_res": 16 * N + 32 * F + 32 * N * 4 + 8 * N,
-            # RK stages 2-3 in one pass: per cell the stored residual, qc read+write, qold, dt/cv and
-            # its wall bit; per wall face its neighbours, geometry, the 64-byte pack of its cell, ghost
-            # writes, wall force and flux, and its cell's face lists, stored fluxes and residual write
-            "cell_rk23": 136 * N + N // 8 + (300 + 148) * W,
+            "face_conv": 8 * F + 32 * F + 64 * N + 16 * F + 72 * G,
+            # face lists, FP32 fluxes, qc read+write, res written, dt/cv, wall bits
+            "cell_res": 16 * N + 16 * F + 96 * N + 8 * N + N // 8,
+            # wall cells, stages 1-3, as above
+            "cell_rk23": (300 + 148 + 80) * W,
             "residue": 8 * ((N + 255) // 256),
         }
     return {
@@ -237,8 +248,10 @@ def algorithmic_bytes(kind: str, m: dict, mixed: bool = False, sides: bool = Fal
         "face_ggfc": 8 * F * 2 + 16 * P + 16 * (N + G) + 40 * P + 40 * (N + G) + 88 * F,
         "cell_grad": 4 * N + 12 * N + 8 * F + 40 * F + 24 * F + 16 * N + 64 * N + 32 * N + 40 * P + 16 * F + 32 * N * 2,
         "face_conv": 8 * F + 24 * F + 16 * F + 4 * G + 16 * (N + G) + 32 * (N + G) + 64 * N + 32 * N + 32 * F + 72 * G,
-        "cell_res": 16 * N + 32 * F + 32 * N * 4 + 16 * N,
-        "cell_rk23": 136 * N + N // 8 + (364 + 148) * W,
+        # face lists, fluxes, qc read+write, res written, dt/cv, wall bits
+        "cell_res": 16 * N + 32 * F + 96 * N + 8 * N + N // 8,
+        # wall cells, stages 1-3
+        "cell_rk23": (364 + 148 + 112) * W,
         "residue": 8 * ((N + 255) // 256),
     }
 
@@ -287,9 +300,9 @@ SWEEP_ITEM_FLOOR_CYCLES = 9 * FP64_ADD + FP64_ADD + FP64_ADD + FP64_DIV + FP64_A
 def launches_per_iter(kind: str, rk3: bool, laminar: bool, irs: bool = False, sides: bool = False) -> dict:
     """How many launches of each profiled phase one iteration makes.  An
     inviscid CCFVM RK3 step without smoothing computes its face fluxes once
-    (stage 1) and runs stages 2 and 3 as one pass over the cells (cell_rk23),
-    recomputing only the wall faces' fluxes; the mixed Green-Gauss step
-    (sides) has no face pass and runs its wall cells as the cell_rk23 phase."""
+    and runs its wall cells through all three stages (the cell_rk23 phase,
+    recomputing only their wall faces' fluxes), then the other cells in one pass
+    (the cell_res phase); the mixed Green-Gauss step (sides) has no face pass."""
     if kind == "nc":  # RK3: the stages share one residual
         return {"grad_lim": 1, "edge": 1, "node_res": 1}
     n = 3 if rk3 else 1
@@ -805,7 +818,7 @@ def run_ours(args, w, dist, rank, local_rank) -> dict | None:
                    "l2": f"inputs larger than L2: ~{ws_mb:.0f} MB of per-iteration arrays vs 129 MB L2, no flush",
                    "setup_s": round(setup_s, 2), "block_sizes": blocks},
         "e2e": e2e,
-        "gpu_launches": (cc_launches(p) if kind == "cc" else
+        "gpu_launches": (cc_kernels(p) if kind == "cc" else
                          LAUNCHES[(kind, "lusgs" if p.time_mode == abi.TIME["lusgs"] else "rk3")]
                          + (1 if (kind, p.time_mode, p.precision) == ("nc", abi.TIME["lusgs"], abi.PREC["fp64"]) else 0))
                         * args.steps,

@@ -950,7 +950,7 @@ __device__ __forceinline__ double4 stored_flux(const CCView& v, int f) {
 // with one RK3 stage (main.F90:92-101) and the block partials of the norm.
 // FP64 form, 4.2 M cells: 0.48 -> 0.20 ms (60 FP64 instructions per cell -> 25:
 // products on the integer pipe, the sum's first term and stage 1's weights 0
-// and 1 dropped); k_cell_rk23 0.45 -> 0.25 ms and k_begin 0.32 -> 0.13 ms alike.
+// and 1 dropped); k_begin 0.32 -> 0.13 ms alike.
 __device__ __forceinline__ void add4(double r[4], const double4& a) { r[0] = r[0] + a.x; r[1] = r[1] + a.y; r[2] = r[2] + a.z; r[3] = r[3] + a.w; }
 __device__ __forceinline__ void sub4(double r[4], const double4& a) { r[0] = r[0] - a.x; r[1] = r[1] - a.y; r[2] = r[2] - a.z; r[3] = r[3] - a.w; }
 
@@ -1038,7 +1038,7 @@ __global__ void __launch_bounds__(kBlock) k_cell_res(CCView v, int irk, int part
 // RK stage with fused multiply-adds, and the FP64 norm partial reduced with
 // one FP64 add per cell before the warp stage (FP64 issue, not bytes, bounds
 // this kernel on GB300).  walls_done: the mixed form's one-pass step, where
-// k_cell_rk23_wall has already advanced the wall cells through all three
+// k_wall_rk3 has already advanced the wall cells through all three
 // stages; they only contribute their residual to the norm here.
 // The fluxes are read as the FP32 values they are, 16 bytes a face instead of
 // 32, and widened here.  4.2 M cells: 153 -> 144 us, of which the 17 FP64
@@ -1051,7 +1051,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_cell_res_mixed(CCView v, int irk,
     if (i < v.noc && cell_inst(v, i) >= 0) {
         double r[4] = {0.0, 0.0, 0.0, 0.0};
         if (walls_done && ((__ldg(v.bcell + (i >> 5)) >> (i & 31)) & 1u)) {
-            d4get(v.res[i], r);  // a wall cell: its last-stage residual (k_cell_rk23_wall)
+            d4get(v.res[i], r);  // a wall cell: its last-stage residual (k_wall_rk3)
         } else {
             const int k0 = v.cf_off[i], k1 = v.cf_off[i + 1];
             const float4* fF = v.fFf();
@@ -1118,8 +1118,8 @@ __global__ void __launch_bounds__(kBlock, 8) k_cell_res_mixed(CCView v, int irk,
     }
 }
 
-// RK stages 2 and 3 of an inviscid step in one pass over the cells.  Those
-// stages' interior and farfield face fluxes equal the first stage's: their
+// The RK stages of an inviscid step in one pass over the cells.  Stage 2's and
+// 3's interior and farfield face fluxes equal the first stage's: their
 // inputs -- the cells' primitives, gradient and limiter -- are formed once
 // per time step (main.F90:62-84) and the farfield ghost is built from them
 // alone; only a wall ghost reads the stage's conserved state (slip_wall /
@@ -1176,49 +1176,39 @@ __device__ __forceinline__ void wall_cell_res(const CCView& v, const Gas& g, int
     }
 }
 
-// Stages 2 and 3 of cell i (instance inst): the stage updates and, for a
-// wall cell, its residual in each stage; returns the squared residual that
-// the last stage's norm takes.  kFrom1 (a wall cell of the mixed form): the
-// first stage too, from the stored face fluxes (k_cell_res_mixed's sum and
-// update).
-template <class R, bool kWall, bool kFrom1 = false>
-__device__ __forceinline__ double rk23_cell(const CCView& v, int i, int inst) {
+// The three stages of wall cell i (instance inst), from the stored face fluxes
+// (k_face_conv's) in the first and its own wall faces' recomputed ones in the
+// other two.
+template <class R>
+__device__ __forceinline__ void wall_cell_rk3(const CCView& v, int i, int inst) {
     constexpr bool kMixed = std::is_same<R, float>::value;
-    constexpr int kRkUnroll = kWall ? 1 : 2;  // one copy of a wall cell's long body
     double r[4], q[4], o[4];
     d4get(v.qc[i], q);
     d4get(v.qold[i], o);
     const double D = v.dcv[i];
-    if constexpr (kFrom1) {
-        static_assert(kMixed && kWall, "the first stage here is the mixed form's");
-        wall_cell_res<R>(v, gas_of(v, inst), i, q, r, false);
+    wall_cell_res<R>(v, gas_of(v, inst), i, q, r, false);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) q[j] = __fma_rn(-D, r[j], q[j]);
-    } else {
-        d4get(v.res[i], r);
-    }
-#pragma unroll kRkUnroll
+    for (int j = 0; j < 4; ++j) q[j] = kMixed ? __fma_rn(-D, r[j], q[j]) : (F64(q[j]) - F64(D) * F64(r[j])).v;
+#pragma unroll 1  // one copy of the long body
     for (int irk = 2; irk <= 3; ++irk) {
-        if (kWall) wall_cell_res<R>(v, gas_of(v, inst), i, q, r);
+        wall_cell_res<R>(v, gas_of(v, inst), i, q, r);
         rk_update<kMixed>(irk, D, o, r, q);
     }
-    if (kWall) v.res[i] = d4(r);
+    v.res[i] = d4(r);
     v.qc[i] = d4(q);
-    if (kMixed) return __fma_rn(r[3], r[3], __fma_rn(r[2], r[2], __fma_rn(r[1], r[1], r[0] * r[0])));
-    return norm2(r);
 }
 
 // The wall cells (v.wcell), one per thread in one-warp blocks so that their
-// long FP64 chains spread over the SMs; they run before k_cell_rk23 (FP64
-// form, stages 2-3) or k_cell_res_mixed (mixed form, all three stages).
-template <class R, bool kFrom1>
-__global__ void __launch_bounds__(32) k_cell_rk23_wall(CCView v) {
+// long FP64 chains spread over the SMs; they run before k_cell_rk3 or
+// k_cell_res_mixed, which advance the other cells.
+template <class R>
+__global__ void __launch_bounds__(32) k_wall_rk3(CCView v) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= v.nwcell) return;
     const int i = v.wcell[t];
     const int inst = cell_inst(v, i);
     if (inst < 0 || stopped(v, inst)) return;
-    rk23_cell<R, true, kFrom1>(v, i, inst);
+    wall_cell_rk3<R>(v, i, inst);
 }
 
 // The residual of every wall cell (v.wcell) from the stored face fluxes, in
@@ -1236,37 +1226,41 @@ __global__ void __launch_bounds__(32) k_wall_res(CCView v) {
     v.res[i] = d4(r);
 }
 
-// Every other cell: a stream over the stored residual and states; the wall
-// cells contribute the last-stage residual k_cell_rk23_wall stored.  The norm
-// partial is reduced as the stage-by-stage kernels reduce it.
-template <class R>
-__global__ void __launch_bounds__(kBlock) k_cell_rk23(CCView v) {
-    constexpr bool kMixed = std::is_same<R, float>::value;
+// Every other cell's three stages and the norm in the FP64 form; the wall cells
+// contribute the last-stage residual that k_wall_rk3 stored.  A stage's state
+// is the next one's in registers, and the state that began the step is the one
+// read (k_begin copied it to qold), so a cell reads its state once and its
+// fluxes once: 4.2 M cells 316 us against 150 for the first stage with the
+// residual and 204 for the other two, which read residual and both states
+// again; 16 384 cells 12.6 us against 10.0 + 4.8 and a launch.
+__global__ void __launch_bounds__(kBlock) k_cell_rk3(CCView v) {
     if (stopped(v, block_inst(v))) return;  // blocks of cells are instance-pure
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int inst = i < v.noc ? cell_inst(v, i) : -1;
     double rr = 0.0;
     if (inst >= 0) {
+        double r[4];
         if ((__ldg(v.bcell + (i >> 5)) >> (i & 31)) & 1u) {
-            double r[4];
             d4get(v.res[i], r);
-            if (kMixed) rr = __fma_rn(r[3], r[3], __fma_rn(r[2], r[2], __fma_rn(r[1], r[1], r[0] * r[0])));
-            else rr = norm2(r);
         } else {
-            rr = rk23_cell<R, false>(v, i, inst);
+            F64I R[4];
+            gather_res(v, v.cf_off[i], v.cf_off[i + 1], R);
+            v.res[i] = f4(R);
+            double o[4], q[4];
+            d4get(v.qc[i], o);
+            const double D = v.dcv[i];  // dt / cv, formed once per time step
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                r[j] = R[j].v;
+                q[j] = (F64I(o[j]) - F64I(D) * R[j]).v;  // stage 1: a = 0, b = 1
+            }
+            rk_update<false>(2, D, o, r, q);
+            rk_update<false>(3, D, o, r, q);
+            v.qc[i] = d4(q);
         }
+        rr = norm2(r);
     }
-    if (kMixed) {  // k_cell_res_mixed's block reduction
-        __shared__ double sh[kBlock];
-        sh[threadIdx.x] = rr;
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            double t = sh[threadIdx.x];
-            for (int k = threadIdx.x + 32; k < kBlock; k += 32) t = t + sh[k];
-            t = warp_sum(t);
-            if (threadIdx.x == 0) v.partial[blockIdx.x] = t;
-        }
-    } else if (v.wpart) {  // one partial per warp (v.ninst == 0)
+    if (v.wpart) {  // one partial per warp (v.ninst == 0)
         rr = warp_sum(rr);
         if ((threadIdx.x & 31) == 0) v.partial[i >> 5] = rr;
     } else {  // k_cell_res's
@@ -1673,11 +1667,11 @@ double epsirs_of(const uns_cc_handle* h, double cfl) {
     return std::max(0.25 * (r * r - 1.0), 0.0);
 }
 
-// Whether the main loop's RK3 step runs stages 2 and 3 as one pass over the
-// cells (k_cell_rk23): an inviscid flow without a smoothing sweep (a viscous
+// Whether the main loop's RK3 step runs its three stages as one pass over the
+// cells (k_cell_rk3): an inviscid flow without a smoothing sweep (a viscous
 // stage recomputes the cell gradient and viscosity from the stage's state; a
 // smoothing sweep replaces the residual that the pass reuses).
-bool rk23_in_one_pass(const uns_cc_handle* h, const CCView& v, double cfl) {
+bool rk3_in_one_pass(const uns_cc_handle* h, const CCView& v, double cfl) {
     const double eps = v.irs ? epsirs_of(h, cfl) : 0.0;
     return h->P.time_mode == UNS_TIME_RK3 && !v.laminar && !(v.irs && eps > 0.0);
 }
@@ -1717,40 +1711,39 @@ int enqueue_wall_res(uns_cc_handle* h, CCView& v) {
     return UNS_OK;
 }
 
-// The wall cells' stages: 2-3 in the FP64 form, 1-3 in the mixed form.
-// Whether the FP64 k_cell_rk23 of this handle runs spread over the SMs with
+// Whether k_cell_rk3 of this handle runs spread over the SMs with
 // per-warp norm partials: one case (no packed instances) on a small mesh.
-inline bool rk23_warp_partials(const uns_cc_handle* h, const CCView& v) {
+inline bool rk3_warp_partials(const uns_cc_handle* h, const CCView& v) {
     return v.ninst == 0 && spread_bs(h, v.noc) < kBlock;
 }
 
 // k_res_final's view after the FP64 one-pass RK stages.
 inline CCView final_view(const uns_cc_handle* h, const CCView& v) {
     CCView w = v;
-    w.wpart = rk23_warp_partials(h, v) ? 1 : 0;
+    w.wpart = rk3_warp_partials(h, v) ? 1 : 0;
     return w;
 }
 
+// The wall cells' three stages.
 int enqueue_wall_rk(uns_cc_handle* h, CCView& v) {
     if (v.nwcell == 0) return UNS_OK;
     const int nb = (v.nwcell + 31) / 32;
-    if (v.mixed) k_cell_rk23_wall<float, true><<<nb, 32, 0, h->stream>>>(v);
-    else k_cell_rk23_wall<double, false><<<nb, 32, 0, h->stream>>>(v);
+    if (v.mixed) k_wall_rk3<float><<<nb, 32, 0, h->stream>>>(v);
+    else k_wall_rk3<double><<<nb, 32, 0, h->stream>>>(v);
     UNS_CUDA(cudaGetLastError());
     return UNS_OK;
 }
 
-// RK stages 2 and 3 of the FP64 form in one pass over the cells: the wall
-// cells first.
-int enqueue_rk23(uns_cc_handle* h, CCView& v) {
-    int rc = enqueue_wall_rk(h, v);
-    if (rc) return rc;
-    if (rk23_warp_partials(h, v)) {
+// The other cells' three stages and the norm's partials.
+int enqueue_cell_rk(uns_cc_handle* h, CCView& v) {
+    if (v.mixed) {
+        LAUNCH(k_cell_res_mixed, v.noc, v, 1, 1, 1);
+    } else if (rk3_warp_partials(h, v)) {
         CCView w = v;
         w.wpart = 1;
-        LAUNCH_SPREAD(k_cell_rk23<double>, v.noc, w);
+        LAUNCH_SPREAD(k_cell_rk3, v.noc, w);
     } else {
-        LAUNCH(k_cell_rk23<double>, v.noc, v);
+        LAUNCH(k_cell_rk3, v.noc, v);
     }
     return UNS_OK;
 }
@@ -1839,27 +1832,25 @@ int enqueue_iteration(uns_cc_handle* h, CCView& v, double cfl_for_eps) {
         if (v.grad_type == UNS_GRAD_GGFC) LAUNCH(k_face_ggfc, v.nof, v);
         LAUNCH_CELL_GRAD(v, gflags, 0.0);
     }
-    if (rk23_in_one_pass(h, v, cfl_for_eps) && v.mixed) {
-        // Mixed form: the wall cells through all three stages, then every other
-        // cell's update and the norm.  A cell without a wall face has the same
-        // residual r in all three stages, and then the RK3 stages (main.F90:
-        // 92-101, a = 0, 3/4, 1/3; b = 1, 1/4, 2/3) give, with D = dt/cv,
+    if (rk3_in_one_pass(h, v, cfl_for_eps)) {
+        // The wall cells through all three stages, then every other cell and the
+        // norm.  A cell without a wall face has the same residual r in all three
+        // stages, and then the RK3 stages (main.F90:92-101, a = 0, 3/4, 1/3;
+        // b = 1, 1/4, 2/3) give, with D = dt/cv,
         //   q1 = qold - D r,  q2 = 3/4 qold + 1/4 (q1 - D r) = qold - D r / 2,
         //   q3 = 1/3 qold + 2/3 (q2 - D r) = qold - D r = q1
-        // in exact arithmetic; this form keeps the FP64 q1 (it differs from the
-        // three rounded stage updates in the last bits, far below the FP32 face
-        // arithmetic).  The FP64 form evaluates both stage updates in the
-        // reference's operation order (k_cell_rk23).
-        LAUNCH_FACE_CONV(float, v);
-        if ((rc = enqueue_wall_rk(h, v))) return rc;
-        LAUNCH(k_cell_res_mixed, v.noc, v, 1, 1, 1);
-    } else if (rk23_in_one_pass(h, v, cfl_for_eps)) {
-        bool fused = false;
-        if ((rc = enqueue_fvresidual(h, v, cfl_for_eps, 1, 0, &fused))) return rc;
-        if ((rc = enqueue_rk23(h, v))) return rc;
-        k_res_final<<<std::max(1, v.ninst), kBlock, 0, h->stream>>>(final_view(h, v), h->nparts, nullptr);
-        UNS_CUDA(cudaGetLastError());
-        return UNS_OK;
+        // in exact arithmetic; the mixed form keeps the FP64 q1 (it differs from
+        // the three rounded stage updates in the last bits, far below the FP32
+        // face arithmetic).  The FP64 form evaluates every stage's update in the
+        // reference's operation order (k_cell_rk3).
+        if (v.mixed) LAUNCH_FACE_CONV(float, v);
+        else LAUNCH_FACE_CONV(double, v);
+        if ((rc = enqueue_wall_rk(h, v)) || (rc = enqueue_cell_rk(h, v))) return rc;
+        if (!v.mixed) {
+            k_res_final<<<std::max(1, v.ninst), kBlock, 0, h->stream>>>(final_view(h, v), h->nparts, nullptr);
+            UNS_CUDA(cudaGetLastError());
+            return UNS_OK;
+        }
     } else if (h->P.time_mode == UNS_TIME_RK3) {
         // A viscous stage with the GG-FC gradient, and a smoothing sweep, keep
         // the primitives, gradient and limiter that the interior and farfield
@@ -2910,7 +2901,7 @@ int uns_cc_profile(uns_cc_handle* h, double cfl, int reps, double* ms, const cha
             else LAUNCH_CELL_GRAD(v, gflags, cfl);
             return UNS_OK;
         });
-        const bool one_pass = rk23_in_one_pass(h, v, cfl);
+        const bool one_pass = rk3_in_one_pass(h, v, cfl);
         for (int irk = 1; irk <= (rk3 && !one_pass ? 3 : 1) && !rc; ++irk) {
             rc = timed(5, [&]() -> int {
                 if (irk > 1 && (!v.laminar || v.grad_type == UNS_GRAD_GGFC)) return enqueue_wall_faces(h, v, false);
@@ -2930,10 +2921,11 @@ int uns_cc_profile(uns_cc_handle* h, double cfl, int reps, double* ms, const cha
                 return UNS_OK;
             });
             int fuse = (rk3 && !smooth) ? irk : 0;
-            if (!rc && one_pass && v.mixed) rc = timed(11, [&]() -> int { return enqueue_wall_rk(h, v); });
+            if (!rc && one_pass) rc = timed(11, [&]() -> int { return enqueue_wall_rk(h, v); });
             if (!rc) rc = timed(7, [&]() -> int {
-                if (v.mixed) LAUNCH(k_cell_res_mixed, v.noc, v, fuse, smooth ? 0 : 1, one_pass ? 1 : 0);
-                else if (!(smooth || one_pass) || v.ninst) LAUNCH(k_cell_res, v.noc, v, fuse, (smooth || one_pass) ? 0 : 1);
+                if (one_pass) return enqueue_cell_rk(h, v);
+                if (v.mixed) LAUNCH(k_cell_res_mixed, v.noc, v, fuse, smooth ? 0 : 1, 0);
+                else if (!smooth || v.ninst) LAUNCH(k_cell_res, v.noc, v, fuse, smooth ? 0 : 1);
                 else LAUNCH_SPREAD(k_cell_res, v.noc, v, fuse, 0);  // as the iteration launches it
                 return UNS_OK;
             });
@@ -2946,7 +2938,6 @@ int uns_cc_profile(uns_cc_handle* h, double cfl, int reps, double* ms, const cha
                 return UNS_OK;
             });
         }
-        if (!rc && one_pass && !v.mixed) rc = timed(11, [&]() -> int { return enqueue_rk23(h, v); });
         if (!rc && !rk3) rc = timed(9, [&]() -> int { return enqueue_lusgs(h, v); });
         if (!rc) rc = timed(10, [&]() -> int {
             k_res_final<<<1, kBlock, 0, h->stream>>>(one_pass && !v.mixed ? final_view(h, v) : v, h->nparts, h->d_scalar);

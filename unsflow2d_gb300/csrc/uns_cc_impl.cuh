@@ -120,7 +120,7 @@ struct CCView {
     // every block of cells belongs to one instance.
     int ninst, cfl_stride;
     // 1 when `partial` holds one sum per warp of 32 cells (a small mesh's
-    // spread k_cell_rk23): k_res_final adds each 8 of them in warp order,
+    // spread k_cell_rk3): k_res_final adds each 8 of them in warp order,
     // which is the 256-cell block partial bit for bit.
     int wpart;
     const int* cinst;       // [ntot] instance of each cell, ghosts included

@@ -1556,10 +1556,15 @@ __global__ void __launch_bounds__(kSweepBlock, 1) k_lusgs_mixed(SweepArgs a, con
 
 namespace {
 
-int check_dev_err(uns_cc_handle* h) {
-    DevErr e;
-    UNS_CUDA(cudaMemcpyAsync(&e, h->v.err, sizeof(DevErr), cudaMemcpyDeviceToHost, h->stream));
+// The handle's report (h->v.err leads it), after all that the stream holds.
+int read_report(uns_cc_handle* h, DevReport* r) {
+    UNS_CUDA(cudaMemcpyAsync(r, h->v.err, sizeof(DevReport), cudaMemcpyDeviceToHost, h->stream));
     UNS_CUDA(cudaStreamSynchronize(h->stream));
+    return UNS_OK;
+}
+
+// The device error e, if it is one: its message set, the device's cleared.
+int take_dev_err(uns_cc_handle* h, const DevErr& e) {
     if (e.code != 0) {
         const char* what = e.code == UNS_ERR_NEG_SOUND_SPEED ? "Roe scheme: sonic speed is negative at face "
                            : e.code == UNS_ERR_NONPOSITIVE  ? "Density/pressure is negative at cell "
@@ -1574,6 +1579,12 @@ int check_dev_err(uns_cc_handle* h) {
         return code;
     }
     return UNS_OK;
+}
+
+int check_dev_err(uns_cc_handle* h) {
+    DevReport r;
+    const int rc = read_report(h, &r);
+    return rc ? rc : take_dev_err(h, r.err);
 }
 
 // Build the forward/backward level schedules of the lusgs2 sweeps: a cell
@@ -2136,12 +2147,15 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
     UP(fgeof, fgeof); UP(fnaf, fnaf); UP(lswf, lswf);
     AL(qpf, ntot); AL(fqf, nof); AL(flaf, nof); AL(packf, 4 * (size_t)noc); AL(ppf, nop); AL(dcv, noc);
     { std::vector<float> t(m->v2c_wt, m->v2c_wt + m->v2c_off[nop]); UP(v2c_wtf, t); }
-    AL(minmax, 8); AL(dtmin, 1); AL(err, 1);
+    AL(minmax, 8); AL(dtmin, 1);
     h->v.wait_cycles = kWaitCycles;
     h->v.skip_code = -1;
     h->nparts = nblocks(noc);
     AL(partial, 8 * (size_t)h->nparts);  // per-warp partials of a small mesh's spread RK pass
-    if ((rc = h->alloc(h->d_scalar, 4))) return fail(rc);
+    DevReport* report = nullptr;
+    if ((rc = h->alloc(report, 1))) return fail(rc);
+    v.err = &report->err;
+    h->d_scalar = report->scalar;
     if ((rc = h->alloc(h->d_iter, 1))) return fail(rc);
     if ((rc = h->alloc(h->d_done, 1))) return fail(rc);
     if ((rc = h->alloc(h->d_fres1, 1))) return fail(rc);
@@ -2448,14 +2462,15 @@ int uns_cc_lusgs(uns_cc_handle* h) {
 int uns_cc_check_positivity(uns_cc_handle* h, int* bad) {
     if (!h) return UNS_ERR_ARG;
     CCView v = h->v;
-    int rc = check_dev_err(h);
-    if (rc) { if (bad) *bad = -1; return rc; }
+    // An error that is there already is reported in place of the check's (the
+    // first error stays, set_err).
+    UNS_CUDA(cudaMemcpyAsync(v.err + 1, v.err, sizeof(DevErr), cudaMemcpyDeviceToDevice, h->stream));
     LAUNCH(k_check_pos, v.noc, v);
-    DevErr e;
-    UNS_CUDA(cudaMemcpyAsync(&e, v.err, sizeof(DevErr), cudaMemcpyDeviceToHost, h->stream));
-    UNS_CUDA(cudaStreamSynchronize(h->stream));
-    if (bad) *bad = e.code == UNS_ERR_NONPOSITIVE ? e.index : -1;
-    return check_dev_err(h);
+    DevReport r;
+    const int rc = read_report(h, &r);
+    if (rc) { if (bad) *bad = -1; return rc; }
+    if (bad) *bad = r.before.code == 0 && r.err.code == UNS_ERR_NONPOSITIVE ? r.err.index : -1;
+    return take_dev_err(h, r.err);
 }
 
 int uns_cc_residue(uns_cc_handle* h, double* fres) {
@@ -2464,9 +2479,11 @@ int uns_cc_residue(uns_cc_handle* h, double* fres) {
     LAUNCH(k_res_partial, v.noc, v);
     k_res_final<<<1, kBlock, 0, h->stream>>>(v, h->nparts, h->d_scalar);
     UNS_CUDA(cudaGetLastError());
-    UNS_CUDA(cudaMemcpyAsync(fres, h->d_scalar, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    UNS_CUDA(cudaStreamSynchronize(h->stream));
-    return check_dev_err(h);
+    DevReport r;
+    const int rc = read_report(h, &r);
+    if (rc) return rc;
+    *fres = r.scalar[0];
+    return take_dev_err(h, r.err);
 }
 
 int uns_cc_forces(uns_cc_handle* h, double* fx, double* fy) {

@@ -30,6 +30,13 @@ struct DevErr {
     int code, index, iter, spare;
 };
 
+// What a call's host side reads at its end, side by side on the device so that
+// one copy (each waits for the stream) brings all of it.
+struct DevReport {
+    DevErr err, before;  // before: err as it was when uns_cc_check_positivity began
+    double scalar[4];
+};
+
 __device__ __forceinline__ void set_err(DevErr* e, int code, int index) {
     if (atomicCAS(&e->code, 0, code) == 0) e->index = index;
 }

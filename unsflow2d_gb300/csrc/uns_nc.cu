@@ -834,10 +834,15 @@ struct uns_nc_handle {
 
 namespace {
 
-int check_err_nc(uns_nc_handle* h) {
-    DevErr e;
-    UNS_CUDA(cudaMemcpyAsync(&e, h->v.err, sizeof(DevErr), cudaMemcpyDeviceToHost, h->stream));
+// The handle's report (h->v.err leads it), after all that the stream holds.
+int read_report(uns_nc_handle* h, DevReport* r) {
+    UNS_CUDA(cudaMemcpyAsync(r, h->v.err, sizeof(DevReport), cudaMemcpyDeviceToHost, h->stream));
     UNS_CUDA(cudaStreamSynchronize(h->stream));
+    return UNS_OK;
+}
+
+// The device error e, if it is one: its message set, the device's cleared.
+int take_err_nc(uns_nc_handle* h, const DevErr& e) {
     if (e.code != 0) {
         set_last_error(std::string(e.code == UNS_ERR_TIMEOUT ? "bounded device wait timed out in block " : "device error at ") +
                        std::to_string(e.index));
@@ -848,6 +853,12 @@ int check_err_nc(uns_nc_handle* h) {
         return code;
     }
     return UNS_OK;
+}
+
+int check_err_nc(uns_nc_handle* h) {
+    DevReport r;
+    const int rc = read_report(h, &r);
+    return rc ? rc : take_err_nc(h, r.err);
 }
 
 #define NLAUNCH(kern, n, ...)                                                        \
@@ -1042,13 +1053,15 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
     ALN(qc, nop); ALN(qp, nop); ALN(qpf, nop); ALN(packn, 3 * (size_t)nop); ALN(qold, nop); ALN(qoldp, nop); ALN(res, nop); ALN(gx, nop); ALN(gy, nop); ALN(phi, nop);
     ALN(dt, nop); ALN(la, nop); ALN(fla, nof); ALN(fF, nof); ALN(bres1, nbnd); ALN(bres2, nbnd); ALN(bla, nbnd);
     ALN(diag, nop); ALN(diaginv, nop); ALN(srec, 10 * (size_t)nop);
-    ALN(err, 1);
     h->v.wait_cycles = kWaitCycles;
     h->v.skip_code = -1;
     h->nparts = nblocks(nop);
     ALN(partial, 2 * h->nparts);
     ALN(partial_i, h->nparts);
-    if ((rc = h->alloc(h->d_scalar, 4))) return fail(rc);
+    DevReport* report = nullptr;
+    if ((rc = h->alloc(report, 1))) return fail(rc);
+    h->v.err = &report->err;
+    h->d_scalar = report->scalar;
     if ((rc = h->alloc(h->d_iter, 1))) return fail(rc);
     if ((rc = h->alloc(h->d_done, 1))) return fail(rc);
     if ((rc = h->alloc(h->d_fres1, 1))) return fail(rc);
@@ -1211,13 +1224,13 @@ int uns_nc_residue(uns_nc_handle* h, double* fres, double* fresi, int* iresi) {
     NLAUNCH(k_nc_res_partial, v.nop, v);
     k_nc_res_final<<<1, kBlock, 0, h->stream>>>(v, h->nparts, h->d_scalar);
     UNS_CUDA(cudaGetLastError());
-    double r[3];
-    UNS_CUDA(cudaMemcpyAsync(r, h->d_scalar, 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    UNS_CUDA(cudaStreamSynchronize(h->stream));
-    if (fres) *fres = r[0];
-    if (fresi) *fresi = r[1];
-    if (iresi) *iresi = (int)r[2];
-    return check_err_nc(h);
+    DevReport r;
+    const int rc = read_report(h, &r);
+    if (rc) return rc;
+    if (fres) *fres = r.scalar[0];
+    if (fresi) *fresi = r.scalar[1];
+    if (iresi) *iresi = (int)r.scalar[2];
+    return take_err_nc(h, r.err);
 }
 
 int uns_nc_iterate(uns_nc_handle* h, int niter, const double* cfl, int first_iter, double* fres_raw, double* fresi,

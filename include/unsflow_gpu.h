@@ -28,9 +28,12 @@ const char* uns_version(void);
 /* Test hooks (no reference counterpart), n host values each:
  * out[i] = a[i] / b[i] by the kernels' division through the reciprocal
  * (must equal IEEE division), and lt[i] = whether a[i]/b[i] < c[i]/d[i]
- * by the kernels' exact ratio comparison (-1 where it does not apply). */
+ * by the kernels' exact ratio comparison (-1 where it does not apply);
+ * uns_selftest_fp64 applies operation op of the FP64 arithmetic off the FP64
+ * unit (k_selftest_fp64 in csrc/uns_api.cu lists them) to a[i], b[i]. */
 int uns_selftest_div(const double* a, const double* b, double* out, int n);
 int uns_selftest_ratio(const double* a, const double* b, const double* c, const double* d, int* lt, int n);
+int uns_selftest_fp64(int op, const double* a, const double* b, double* out, int n);
 
 /* ============================================================ CCFVM =====*/
 typedef struct uns_cc_handle uns_cc_handle;

@@ -95,7 +95,7 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
     std::vector<double> wfree(nwarps, 0.0);
     std::vector<int> wlast(nwarps, -1);
     std::vector<std::vector<int>> lists(nwarps), srcs(nwarps);
-    for (int w = 0; w < nwarps; ++w) {
+    for (int w = 0; w < nwarps && n / nwarps >= 64; ++w) {
         lists[w].reserve(2 * (size_t)n / nwarps + 64);
         srcs[w].reserve((size_t)(nbr_off[n] - nbr_off[0]) / nwarps + 64);
     }

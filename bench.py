@@ -263,24 +263,24 @@ def algorithmic_bytes(kind: str, m: dict, mixed: bool = False, sides: bool = Fal
 # summaries under profiles/): scaled here to the benchmark's size.
 TRAFFIC_PER_UNIT = {
     ("nc", "lusgs_sweeps", False): ((457.42e6 + 75.82e6) / 525312, "nodes", "profiles/nc_lusgs_1024x512_launches.md"),
-    ("cc", "face_conv", False): (58.58e6 / 393728, "faces", "profiles/cc_fp64_512x256_full.md"),
-    ("cc", "face_conv", True): (156.96e6 / 1573888, "faces", "profiles/cc_mixed_1024x512_full.md"),
-    ("cc", "cell_res", True): (138.34e6 / 1048576, "cells", "profiles/cc_mixed_1024x512_full.md"),
-    ("cc", "cell_grad", True): (261.72e6 / 1048576, "cells", "profiles/cc_mixed_1024x512_full.md"),
-    ("cc", "cell_grad", False): (68.84e6 / 262144, "cells", "profiles/cc_fp64_512x256_full.md"),
+    ("cc", "face_conv", False): (58.19e6 / 393728, "faces", "profiles/cc_fp64_512x256_full.md"),
+    ("cc", "face_conv", True): (142.2e6 / 1573888, "faces", "profiles/cc_mixed_1024x512_full.md"),
+    ("cc", "cell_res", True): (104.6e6 / 1048576, "cells", "profiles/cc_mixed_1024x512_full.md"),
+    ("cc", "cell_grad", True): (259.9e6 / 1048576, "cells", "profiles/cc_mixed_1024x512_full.md"),
+    ("cc", "cell_grad", False): (70.67e6 / 262144, "cells", "profiles/cc_fp64_512x256_full.md"),
 }
 
 # FP64-pipe utilisation (sm__pipe_fp64_cycles_active, fraction of peak while
 # active) of the same kernels from the same captures: the second roofline
-# fraction, the one that bounds the FP64 kernels.
+# fraction.
 FP64_PIPE = {
-    ("nc", "lusgs_sweeps", False): (0.123, "profiles/nc_lusgs_512x256_full.md"),
-    ("cc", "cell_grad", False): (0.845, "profiles/cc_fp64_512x256_full.md"),
-    ("cc", "face_conv", False): (0.847, "profiles/cc_fp64_512x256_full.md"),
-    ("cc", "cell_res", False): (0.799, "profiles/cc_fp64_512x256_full.md"),
-    ("cc", "cell_grad", True): (0.198, "profiles/cc_mixed_1024x512_full.md"),
-    ("cc", "face_conv", True): (0.354, "profiles/cc_mixed_1024x512_full.md"),
-    ("cc", "cell_res", True): (0.755, "profiles/cc_mixed_1024x512_full.md"),
+    ("nc", "lusgs_sweeps", False): (0.115, "profiles/nc_lusgs_512x256_full.md"),
+    ("cc", "cell_grad", False): (0.539, "profiles/cc_fp64_512x256_full.md"),
+    ("cc", "face_conv", False): (0.389, "profiles/cc_fp64_512x256_full.md"),
+    ("cc", "cell_res", False): (0.586, "profiles/cc_fp64_512x256_full.md"),
+    ("cc", "cell_grad", True): (0.18, "profiles/cc_mixed_1024x512_full.md"),
+    ("cc", "face_conv", True): (0.013, "profiles/cc_mixed_1024x512_full.md"),
+    ("cc", "cell_res", True): (0.769, "profiles/cc_mixed_1024x512_full.md"),
 }
 
 

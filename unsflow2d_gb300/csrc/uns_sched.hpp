@@ -94,11 +94,10 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
     std::vector<Item> done(2 * (size_t)n);
     std::vector<double> wfree(nwarps, 0.0);
     std::vector<int> wlast(nwarps, -1);
-    std::vector<std::vector<int>> lists(nwarps), srcs(nwarps);
-    for (int w = 0; w < nwarps && n / nwarps >= 64; ++w) {
-        lists[w].reserve(2 * (size_t)n / nwarps + 64);
-        srcs[w].reserve((size_t)(nbr_off[n] - nbr_off[0]) / nwarps + 64);
-    }
+    std::vector<int> count(nwarps, 0), codes, srcs;  // items per warp; every item and its sources as they are placed
+    std::vector<int> nsrc(nwarps, 0);
+    codes.reserve(2 * (size_t)n);
+    srcs.reserve(nbr_off[n] - nbr_off[0]);
     // The warp that frees up first (of several, the lowest): a tournament.  A
     // heap with an entry per placement outgrows the caches on a large mesh
     // (4.2 M cells).
@@ -137,15 +136,16 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
             for (int c = g * kSchedGroup; c < (g + 1) * kSchedGroup && c < nwarps; ++c) consider(c);
         }
         consider(first[1]);
-        done[code] = {s + kCompute, w, (int)lists[w].size()};
+        done[code] = {s + kCompute, w, count[w]++};
         makespan = std::max(makespan, s + kCompute);
         wfree[w] = s + kCompute;
         wlast[w] = code;
         // w frees up later than before: only the rounds that it had won change
         for (int k = (leaves + w) / 2; k > 0 && first[k] == w; k /= 2) first[k] = earlier(first[2 * k], first[2 * k + 1]);
-        lists[w].push_back(code);
+        codes.push_back(code);
         for (size_t k = code & 1; k < pr.size(); ++k)  // not a backward item's own forward value
-            srcs[w].push_back(pr[k].warp / kSchedGroup == w / kSchedGroup ? (pr[k].warp % kSchedGroup) << 28 | pr[k].index : -1);
+            srcs.push_back(pr[k].warp / kSchedGroup == w / kSchedGroup ? (pr[k].warp % kSchedGroup) << 28 | pr[k].index : -1);
+        nsrc[w] += (int)pr.size() - (code & 1);
     };
     for (int i : fwd) {
         preds.clear();
@@ -169,10 +169,23 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
     out.nlev_fwd = nlev;
     out.nlev_bwd = nlevb;
     out.off.assign(nwarps + 1, 0);
-    for (int w = 0; w < nwarps; ++w) out.off[w + 1] = out.off[w] + (int)lists[w].size();
-    out.items.reserve(2 * (size_t)n);
-    for (int w = 0; w < nwarps; ++w) out.items.insert(out.items.end(), lists[w].begin(), lists[w].end());
-    for (const auto& l : srcs) out.src.insert(out.src.end(), l.begin(), l.end());
+    std::vector<int> at(nwarps + 1, 0);  // where each warp's sources go
+    for (int w = 0; w < nwarps; ++w) {
+        out.off[w + 1] = out.off[w] + count[w];
+        at[w + 1] = at[w] + nsrc[w];
+    }
+    out.items.resize(codes.size());
+    out.src.resize(srcs.size());
+    size_t from = 0;
+    for (int code : codes) {
+        const Item& d = done[code];
+        out.items[out.off[d.warp] + d.index] = code;
+        const int i = code >> 1, pass = code & 1;
+        for (int k = nbr_off[i]; k < nbr_off[i + 1]; ++k) {
+            const int j = nbr[k];
+            if (j >= 0 && j < n && (pass == 0 ? j < i : j > i)) out.src[at[d.warp]++] = srcs[from++];
+        }
+    }
     return out;
 }
 

@@ -117,7 +117,8 @@ __device__ __forceinline__ double4 z4() { return make_double4(0.0, 0.0, 0.0, 0.0
 // as plain doubles); N leaves it their sums.  The values are the same bits.
 // At 262 k cells (laminar): k_adj_visc 109 -> 56 us, k_adj_recon 110 -> 74,
 // k_adj_conv 62 -> 42, k_adj_ggfc 157 -> 59, k_adj_final 150 -> 60,
-// k_adj_start_grad 43 -> 25, k_adj_init 30 -> 23.
+// k_adj_start_grad 43 -> 25; with the sums not cleared first and k_adj_reduce by
+// warps, one transposed product 1 170 -> 1 130 us.
 typedef F64I N;
 __device__ __forceinline__ double4 add(double4 a, double4 b) { return make_double4(add64(a.x, b.x), add64(a.y, b.y), add64(a.z, b.z), add64(a.w, b.w)); }
 __device__ __forceinline__ double4 sub(double4 a, double4 b) { return make_double4(sub64(a.x, b.x), sub64(a.y, b.y), sub64(a.z, b.z), sub64(a.w, b.w)); }
@@ -265,20 +266,21 @@ __global__ void k_rec_visc(CCView v, AdjView a, int s) {
 }
 
 // ------------------------------------------------------- transposed pass
-__global__ void k_adj_init(CCView v, AdjView a) {
+// What the last stage's kernels (the first to run) do not start afresh
+// themselves: they write where the other stages add, so that the cells' and
+// faces' sums are neither cleared nor read back first.
+__global__ void k_adj_init(CCView v, AdjView a, int stage_grad) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < v.noc) {
-        a.qc[i] = a.lq[i];
-        a.qold[i] = z4(); a.qp[i] = z4(); a.qT[i] = 0.0; a.gx[i] = z4(); a.gy[i] = z4();
+        a.qT[i] = 0.0;
+        if (stage_grad) { a.gx[i] = z4(); a.gy[i] = z4(); }  // read by the first stage gradient
     } else if (i < v.ntot) {
         a.qp[i] = a.lg[i - v.noc];
         a.qT[i] = a.lgT[i - v.noc];
     }
     if (i < v.nof) {
-        a.fq[i] = z4(); a.fgx[i] = z4(); a.fgy[i] = z4(); a.fgT[i] = make_double2(0.0, 0.0);
-        if (v.laminar && v.grad_type != UNS_GRAD_GGFC) {  // read by a stage gradient alone
-            a.sgx[i] = z4(); a.sgy[i] = z4(); a.sgT[i] = make_double2(0.0, 0.0);
-        }
+        if (!v.laminar) a.fq[i] = z4();
+        if (!v.laminar || stage_grad) { a.fgx[i] = z4(); a.fgy[i] = z4(); a.fgT[i] = make_double2(0.0, 0.0); }
     }
     if (i < v.nbf) a.falpha[i] = 0.0;
     if (a.geo && i < v.nof) {
@@ -289,14 +291,16 @@ __global__ void k_adj_init(CCView v, AdjView a) {
     }
 }
 
-// RK update q = a*qold + b*(q - dt/cv * res) of stage irk, transposed.
-__global__ void k_adj_stage(CCView v, AdjView a, int irk) {
+// RK update q = a*qold + b*(q - dt/cv * res) of stage irk, transposed; last:
+// from the iteration's adjoint.
+__global__ void k_adj_stage(CCView v, AdjView a, int irk, int last) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= v.noc) return;
-    const double4 l = a.qc[i];
+    const double4 l = last ? a.lq[i] : a.qc[i];
     const double ak = rk_a(irk), bk = rk_b(irk);
     a.res[i] = scl(N(-bk) * a.Dv[i], l);
-    a.qold[i] = add(a.qold[i], scl(ak, l));
+    const double4 o = scl(ak, l);
+    a.qold[i] = last ? o : add(a.qold[i], o);
     a.qc[i] = scl(bk, l);
 }
 
@@ -337,17 +341,17 @@ __global__ void __launch_bounds__(kBlock, 3) k_adj_visc(CCView v, AdjView a, int
     const N uxb = four_third * txxb - two_third * tyyb;
     const N vyb = -two_third * txxb + four_third * tyyb;
     const N txb = -qxb / factor, tyb = -qyb / factor;
-    double4 q = a.fq[f];
+    double4 q = last ? z4() : a.fq[f];
     q.y = (N(q.y) + ub).v; q.z = (N(q.z) + vb).v;
     a.fq[f] = q;
     double4* GX = stage_grad ? a.sgx : a.fgx;
     double4* GY = stage_grad ? a.sgy : a.fgy;
     double2* GT = stage_grad ? a.sgT : a.fgT;
-    double4 gx = GX[f], gy = GY[f];
+    double4 gx = last ? z4() : GX[f], gy = last ? z4() : GY[f];
     gx.y = (N(gx.y) + uxb).v; gx.z = (N(gx.z) + txyb).v;
     gy.y = (N(gy.y) + txyb).v; gy.z = (N(gy.z) + vyb).v;
     GX[f] = gx; GY[f] = gy;
-    GT[f] = sum2(GT[f], txb, tyb);
+    GT[f] = last ? make_double2(txb.v, tyb.v) : sum2(GT[f], txb, tyb);
     if (a.geo) {  // flux*area = area*mr*(S1, 0, txx nx + txy ny, txy nx + tyy ny): its normal and length
         a.garea[f] = (N(a.garea[f]) + mr * (bx * S1 + bz * t1 + bw * t2)).v;
         a.gfn[f] = sum2(a.gfn[f], area * mr * (bx * A + bz * txx + bw * txy), area * mr * (bx * B + bz * txy + bw * tyy));
@@ -490,14 +494,14 @@ __global__ void k_adj_conv(CCView v, AdjView a, int s, int last) {
 // cell over its faces: primitive adjoint (start of the iteration), gradient
 // adjoint (the gradient this stage read; reset first when a viscous stage
 // had recomputed it), and the wall closure's current-state adjoint.
-__global__ void __launch_bounds__(kBlock, 3) k_adj_recon(CCView v, AdjView a, int reset_g) {
+__global__ void __launch_bounds__(kBlock, 3) k_adj_recon(CCView v, AdjView a, int reset_g, int last) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= v.noc) return;
     const N zhi = 1.0 / 3.0, zlo = 1.0 - 1.0 / 3.0;
     const double4 ph = v.phi[i];
     const double2 c = v.cen[i];
     double4 aq = z4(), ac = z4();
-    double4 gx = reset_g ? z4() : a.gx[i], gy = reset_g ? z4() : a.gy[i];
+    double4 gx = reset_g || last ? z4() : a.gx[i], gy = reset_g || last ? z4() : a.gy[i];
     N own_w[4], own_e[4], hp[4];  // per variable: 1 - phi/2 zhi, phi/2 (1 - zhi)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -534,7 +538,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_adj_recon(CCView v, AdjView a, in
             ac = add(ac, a.fr[f]);
         }
     }
-    a.qp[i] = add(a.qp[i], aq);
+    a.qp[i] = last ? aq : add(a.qp[i], aq);
     a.gx[i] = gx;
     a.gy[i] = gy;
     a.qc[i] = add(a.qc[i], ac);
@@ -689,18 +693,21 @@ __global__ void __launch_bounds__(kBlock, 3) k_adj_final(CCView v, AdjView a, in
 }
 
 // d/dalpha (boundary terms in face order + the explicit term) and the norm of
-// the change, in a fixed order; hist (may be null) receives sqrt(change).
+// the change, in a fixed order; hist (may be null) receives sqrt(change).  The
+// threads' sums add up warp by warp: by one thread they were 512 dependent
+// additions (22 of the kernel's 24 us).
 __global__ void k_adj_reduce(CCView v, AdjView a, int nparts, double* hist, int k) {
-    __shared__ double sa[kBlock], sd[kBlock];
+    __shared__ double sa[kBlock / 32], sd[kBlock / 32];
     double ta = 0.0, td = 0.0;
     for (int b = threadIdx.x; b < v.nbf; b += kBlock) ta = ta + a.falpha[b];
     for (int b = threadIdx.x; b < nparts; b += kBlock) td = td + a.part[b];
-    sa[threadIdx.x] = ta;
-    sd[threadIdx.x] = td;
+    ta = warp_sum(ta);
+    td = warp_sum(td);
+    if ((threadIdx.x & 31) == 0) { sa[threadIdx.x >> 5] = ta; sd[threadIdx.x >> 5] = td; }
     __syncthreads();
     if (threadIdx.x == 0) {
         double x = 0.0, y = 0.0;
-        for (int t = 0; t < kBlock; ++t) { x = x + sa[t]; y = y + sd[t]; }
+        for (int t = 0; t < kBlock / 32; ++t) { x = x + sa[t]; y = y + sd[t]; }
         a.out[0] = x + a.jalpha;
         a.out[1] = y;
         if (hist) hist[k] = sqrt(y);
@@ -869,17 +876,17 @@ int enqueue_vjp(uns_cc_handle* h, double* hist, int k) {
     const AdjView& a = h->adj->a;
     const bool lam = v.laminar != 0;
     const bool stage_grad = lam && v.grad_type != UNS_GRAD_GGFC;
-    LAUNCH(k_adj_init, std::max(v.ntot, v.nof), v, a);
+    LAUNCH(k_adj_init, std::max(v.ntot, v.nof), v, a, stage_grad ? 1 : 0);
     for (int s = 2; s >= 0; --s) {
         const int last = s == 2;
-        LAUNCH(k_adj_stage, v.noc, v, a, s + 1);
+        LAUNCH(k_adj_stage, v.noc, v, a, s + 1, last);
         if (lam) {
             LAUNCH(k_adj_visc, v.nof, v, a, s, last, stage_grad ? 1 : 0);
             LAUNCH(k_adj_mul, v.noc, v, a, s);
             if (stage_grad) LAUNCH(k_adj_stage_ggfc, v.nof, v, a);
         }
         LAUNCH(k_adj_conv, v.nof, v, a, s, last);
-        LAUNCH(k_adj_recon, v.noc, v, a, stage_grad ? 1 : 0);
+        LAUNCH(k_adj_recon, v.noc, v, a, stage_grad ? 1 : 0, last);
     }
     LAUNCH(k_adj_start_grad, v.nof, v, a);
     const bool use_ggfc = lam || v.grad_type == UNS_GRAD_GGFC;

@@ -1199,8 +1199,8 @@ __device__ __forceinline__ void wall_cell_rk3(const CCView& v, int i, int inst) 
 }
 
 // The wall cells (v.wcell), one per thread in one-warp blocks so that their
-// long FP64 chains spread over the SMs; they run before k_cell_rk3 or
-// k_cell_res_mixed, which advance the other cells.
+// long FP64 chains spread over the SMs; before k_cell_rk3 or k_cell_res_mixed,
+// which advance the other cells, or beside the first (enqueue_rk3).
 template <class R>
 __global__ void __launch_bounds__(32) k_wall_rk3(CCView v) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1239,9 +1239,9 @@ __global__ void __launch_bounds__(kBlock) k_cell_rk3(CCView v) {
     const int inst = i < v.noc ? cell_inst(v, i) : -1;
     double rr = 0.0;
     if (inst >= 0) {
-        double r[4];
+        double r[4] = {0.0, 0.0, 0.0, 0.0};
         if ((__ldg(v.bcell + (i >> 5)) >> (i & 31)) & 1u) {
-            d4get(v.res[i], r);
+            if (!v.wpart) d4get(v.res[i], r);  // else k_wall_parts, when both kernels are done
         } else {
             F64I R[4];
             gather_res(v, v.cf_off[i], v.cf_off[i + 1], R);
@@ -1274,6 +1274,22 @@ __global__ void __launch_bounds__(kBlock) k_cell_rk3(CCView v) {
             v.partial[blockIdx.x] = t;
         }
     }
+}
+
+// The norm's per-warp partials of the blocks of cells that hold wall cells
+// (v.wblk), from the stored last-stage residuals of all their cells, once
+// k_wall_rk3 and the k_cell_rk3 that ran beside it are both done.
+__global__ void __launch_bounds__(kBlock) k_wall_parts(CCView v) {
+    if (stopped(v)) return;
+    const int i = v.wblk[blockIdx.x] * kBlock + threadIdx.x;
+    double rr = 0.0;
+    if (i < v.noc) {
+        double r[4];
+        d4get(v.res[i], r);
+        rr = norm2(r);
+    }
+    rr = warp_sum(rr);
+    if ((threadIdx.x & 31) == 0) v.partial[i >> 5] = rr;
 }
 
 // One Jacobi sweep of cirs (ImpResiSmoothening.F90:27-44).
@@ -1736,27 +1752,52 @@ inline CCView final_view(const uns_cc_handle* h, const CCView& v) {
 }
 
 // The wall cells' three stages.
-int enqueue_wall_rk(uns_cc_handle* h, CCView& v) {
+int enqueue_wall_rk(uns_cc_handle* h, CCView& v, cudaStream_t stream) {
     if (v.nwcell == 0) return UNS_OK;
     const int nb = (v.nwcell + 31) / 32;
-    if (v.mixed) k_wall_rk3<float><<<nb, 32, 0, h->stream>>>(v);
-    else k_wall_rk3<double><<<nb, 32, 0, h->stream>>>(v);
+    if (v.mixed) k_wall_rk3<float><<<nb, 32, 0, stream>>>(v);
+    else k_wall_rk3<double><<<nb, 32, 0, stream>>>(v);
     UNS_CUDA(cudaGetLastError());
     return UNS_OK;
 }
 
-// The other cells' three stages and the norm's partials.
-int enqueue_cell_rk(uns_cc_handle* h, CCView& v) {
+// The other cells' three stages and the norm's partials; beside the wall cells'
+// where walls is their event (or null, behind them) and the pass is spread.
+int enqueue_cell_rk(uns_cc_handle* h, CCView& v, cudaEvent_t walls) {
     if (v.mixed) {
         LAUNCH(k_cell_res_mixed, v.noc, v, 1, 1, 1);
     } else if (rk3_warp_partials(h, v)) {
         CCView w = v;
         w.wpart = 1;
         LAUNCH_SPREAD(k_cell_rk3, v.noc, w);
+        if (v.nwcell == 0) return UNS_OK;
+        if (walls) UNS_CUDA(cudaStreamWaitEvent(h->stream, walls, 0));
+        k_wall_parts<<<v.nwblk, kBlock, 0, h->stream>>>(w);
+        UNS_CUDA(cudaGetLastError());
     } else {
         LAUNCH(k_cell_rk3, v.noc, v);
     }
     return UNS_OK;
+}
+
+// Both.  The wall cells' chain (a thread per cell, 27-40 us at any size) runs on
+// a stream of its own beside the other cells' where these leave it room, on the
+// meshes that spread their launches: 16 384 cells 114 -> 109 us per iteration.
+// On larger ones they fill the chip, the chain gets its turn behind them and the
+// partials' launch comes on top (a mixed packed study: 503 -> 510 us).
+int enqueue_rk3(uns_cc_handle* h, CCView& v) {
+    if (v.nwcell > 0 && !v.mixed && rk3_warp_partials(h, v)) {
+        UNS_CUDA(cudaEventRecord(h->fork, h->stream));
+        UNS_CUDA(cudaStreamWaitEvent(h->side, h->fork, 0));
+        int rc = enqueue_wall_rk(h, v, h->side);
+        const cudaError_t e = cudaEventRecord(h->join, h->side);  // joined on an error too
+        if (rc == UNS_OK) rc = enqueue_cell_rk(h, v, h->join);
+        else cudaStreamWaitEvent(h->stream, h->join, 0);
+        UNS_CUDA(e);
+        return rc;
+    }
+    int rc = enqueue_wall_rk(h, v, h->stream);
+    return rc ? rc : enqueue_cell_rk(h, v, nullptr);
 }
 
 // fvresidual as a kernel sequence; irk > 0 fuses that RK stage into the
@@ -1856,7 +1897,7 @@ int enqueue_iteration(uns_cc_handle* h, CCView& v, double cfl_for_eps) {
         // reference's operation order (k_cell_rk3).
         if (v.mixed) LAUNCH_FACE_CONV(float, v);
         else LAUNCH_FACE_CONV(double, v);
-        if ((rc = enqueue_wall_rk(h, v)) || (rc = enqueue_cell_rk(h, v))) return rc;
+        if ((rc = enqueue_rk3(h, v))) return rc;
         if (!v.mixed) {
             k_res_final<<<std::max(1, v.ninst), kBlock, 0, h->stream>>>(final_view(h, v), h->nparts, nullptr);
             UNS_CUDA(cudaGetLastError());
@@ -2004,7 +2045,12 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
     h->P = *p;
     int rc = UNS_OK;
     auto fail = [&](int code) { uns_cc_destroy(h); return code; };
-    if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
+    int lowest = 0, highest = 0;
+    if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaDeviceGetStreamPriorityRange(&lowest, &highest) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&h->side, cudaStreamNonBlocking, highest) != cudaSuccess ||
+        cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming) != cudaSuccess) {
         set_last_error("uns_cc_create: cudaStreamCreate failed (no usable GPU?)");
         delete h;
         return UNS_ERR_CUDA;
@@ -2131,8 +2177,12 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
         }
         for (int c = 0; c < noc; ++c)
             if ((t[c >> 5] >> (c & 31)) & 1u) wc.push_back(c);
-        UP(bcell, t); UP(wcell, wc);
+        std::vector<int> wb;
+        for (int c : wc)
+            if (wb.empty() || wb.back() != c / kBlock) wb.push_back(c / kBlock);
+        UP(bcell, t); UP(wcell, wc); UP(wblk, wb);
         v.nwcell = (int)wc.size();
+        v.nwblk = (int)wb.size();
     }
     UP(rc2f_off, rc2f_off); UP(rc2f, rc2f);
     { std::vector<int> t(m->v2c_off, m->v2c_off + nop + 1); UP(v2c_off, t); }
@@ -2229,6 +2279,9 @@ int uns_cc_destroy(uns_cc_handle* h) {
     for (void* p : h->allocs) cudaFree(p);
     if (h->d_cfl) cudaFree(h->d_cfl);
     if (h->d_hist) cudaFree(h->d_hist);
+    if (h->fork) cudaEventDestroy(h->fork);
+    if (h->join) cudaEventDestroy(h->join);
+    if (h->side) cudaStreamDestroy(h->side);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return UNS_OK;
@@ -2938,9 +2991,9 @@ int uns_cc_profile(uns_cc_handle* h, double cfl, int reps, double* ms, const cha
                 return UNS_OK;
             });
             int fuse = (rk3 && !smooth) ? irk : 0;
-            if (!rc && one_pass) rc = timed(11, [&]() -> int { return enqueue_wall_rk(h, v); });
+            if (!rc && one_pass) rc = timed(11, [&]() -> int { return enqueue_wall_rk(h, v, h->stream); });
             if (!rc) rc = timed(7, [&]() -> int {
-                if (one_pass) return enqueue_cell_rk(h, v);
+                if (one_pass) return enqueue_cell_rk(h, v, nullptr);
                 if (v.mixed) LAUNCH(k_cell_res_mixed, v.noc, v, fuse, smooth ? 0 : 1, 0);
                 else if (!smooth || v.ninst) LAUNCH(k_cell_res, v.noc, v, fuse, smooth ? 0 : 1);
                 else LAUNCH_SPREAD(k_cell_res, v.noc, v, fuse, 0);  // as the iteration launches it

@@ -39,6 +39,8 @@ struct CCView {
     const unsigned* bcell;  // bit i: interior cell i has a wall face
     const int* wcell;       // those cells in increasing order
     int nwcell;
+    const int* wblk;        // the blocks of kBlock cells that hold them
+    int nwblk;
     const int* rc2f_off;  // reference c2f order (LU-SGS)
     const int* rc2f;
     const int* v2c_off;
@@ -162,6 +164,8 @@ struct uns_cc_handle {
     int* d_done = nullptr;
     double* d_hist = nullptr;
     double* d_fres1 = nullptr;
+    cudaStream_t side = nullptr;  // the wall cells' stages, between fork and join
+    cudaEvent_t fork = nullptr, join = nullptr;
     double* d_scalar = nullptr;  // [4] scratch for host-visible scalars
     int graph_first = -1;
     int gen = 0;           // bumped whenever the captured iteration changes (precision, capacity)

@@ -883,18 +883,19 @@ __device__ __forceinline__ void cell_mul(const CCView& v, int i) {
 }
 __global__ void __launch_bounds__(kBlock) k_cell_mul(CCView v) { cell_mul(v, blockIdx.x * blockDim.x + threadIdx.x); }
 
-// The wall faces' convective fluxes and ghosts, and beside them (with_mul)
-// every cell's viscosity: the wall faces' long chains take the first one-warp
-// blocks, the cells run under them (laminar 512x256: 31 + 13 -> 29 us).
+// The wall faces' convective fluxes and ghosts (all: every boundary face's),
+// and beside them (with_mul) every cell's viscosity: the wall faces' long
+// chains take the first one-warp blocks, the cells run under them (laminar
+// 512x256: 31 + 13 -> 29 us).
 template <class R>
-__global__ void __launch_bounds__(32) k_wall_faces(CCView v, int with_mul) {
+__global__ void __launch_bounds__(32) k_wall_faces(CCView v, int with_mul, int all) {
     const int nwb = (v.nbf + 31) / 32;
     if ((int)blockIdx.x >= nwb) {
         if (with_mul) cell_mul(v, (blockIdx.x - nwb) * 32 + threadIdx.x);
         return;
     }
     const int f = v.nfi + blockIdx.x * 32 + threadIdx.x;
-    if (f >= v.nof || v.fbc[f] != 1001) return;
+    if (f >= v.nof || (!all && v.fbc[f] != 1001)) return;
     const int inst = face_inst(v, f);
     if (stopped(v, inst)) return;
     const int in = v.fnb[f].x;
@@ -1590,6 +1591,7 @@ int take_dev_err(uns_cc_handle* h, const DevErr& e) {
         set_last_error(std::string(what) + std::to_string(e.index));
         int code = e.code;
         DevErr z = {0, 0, 0, 0};
+        h->ghosts_set = true;  // a boundary face that raised it raises it again in the next call
         UNS_CUDA(cudaMemcpyAsync(h->v.err, &z, sizeof(DevErr), cudaMemcpyHostToDevice, h->stream));
         UNS_CUDA(cudaStreamSynchronize(h->stream));
         return code;
@@ -1712,22 +1714,25 @@ bool grad_by_sides(const uns_cc_handle* h, const CCView& v) {
 }
 
 // The wall faces' convective fluxes and ghosts, with_mul the cells' viscosity
-// too.  (A farfield face's flux and ghost follow from the reconstructed state.)
-int enqueue_wall_faces(uns_cc_handle* h, CCView& v, bool with_mul) {
+// too.  (A farfield face's flux and ghost follow from the reconstructed state;
+// all: they are formed again all the same.)
+int enqueue_wall_faces(uns_cc_handle* h, CCView& v, bool with_mul, bool all = false) {
     const int nb = (v.nbf + 31) / 32 + (with_mul ? (v.noc + 31) / 32 : 0);
     if (nb == 0) return UNS_OK;
-    if (v.mixed) k_wall_faces<float><<<nb, 32, 0, h->stream>>>(v, with_mul ? 1 : 0);
-    else k_wall_faces<double><<<nb, 32, 0, h->stream>>>(v, with_mul ? 1 : 0);
+    if (v.mixed) k_wall_faces<float><<<nb, 32, 0, h->stream>>>(v, with_mul, all);
+    else k_wall_faces<double><<<nb, 32, 0, h->stream>>>(v, with_mul, all);
     UNS_CUDA(cudaGetLastError());
     return UNS_OK;
 }
 
-// uns_cc_fvresidual when only the wall ghosts can have changed since the last
-// call that computed every face (same primitives, gradient and limiter; the
-// reference main loop's RK stages 2 and 3): the boundary faces' fluxes and
-// the wall cells' residuals; every other cell keeps the residual it has.
+// uns_cc_fvresidual when only the wall faces' fluxes can have changed since
+// the last call that computed every face (same primitives, gradient and
+// limiter; the reference main loop's RK stages 2 and 3): those fluxes and the
+// wall cells' residuals; every other cell keeps the residual it has.  The
+// other boundary faces give what they gave, which their ghost rows still hold
+// unless set_state wrote them (ghosts_set): then they run too.
 int enqueue_wall_res(uns_cc_handle* h, CCView& v) {
-    int rc = enqueue_wall_faces(h, v, false);
+    int rc = enqueue_wall_faces(h, v, false, h->ghosts_set);
     if (rc) return rc;
     if (v.nbf > 0 && v.nwcell > 0) {
         const int nb = (v.nwcell + 31) / 32;
@@ -2301,6 +2306,7 @@ int uns_cc_initialize(uns_cc_handle* h) {
 
 int uns_cc_set_state(uns_cc_handle* h, const double* qc) {
     if (!h || !qc) return UNS_ERR_ARG;
+    h->ghosts_set = true;
     UNS_CUDA(cudaMemcpyAsync(h->v.qc, qc, sizeof(double4) * h->v.ntot, cudaMemcpyHostToDevice, h->stream));
     UNS_CUDA(cudaStreamSynchronize(h->stream));
     return UNS_OK;
@@ -2487,13 +2493,14 @@ int uns_cc_fvresidual(uns_cc_handle* h) {
     // Since the last call that computed every face, only the conserved state
     // has changed (rk_stage, set_state): the interior and farfield fluxes read
     // the primitives, gradient and limiter alone, so only the wall faces and
-    // their cells' residuals are recomputed (bit-identical to a full call).
+    // their cells' residuals are recomputed, and after set_state every
+    // boundary face and ghost row (bit-identical to a full call).
     // Viscous fluxes read the state, and a smoothing sweep replaces the stored
     // residual: those calls compute everything.
     const bool smooth = v.irs && epsirs_of(h, h->cfl_cur) > 0.0;
-    if (!v.laminar && !smooth && h->res_gen == h->flux_gen) return enqueue_wall_res(h, v);
-    const int rc = enqueue_fvresidual(h, v, h->cfl_cur, 0, 0, &fused);
-    if (!rc) h->res_gen = h->flux_gen;
+    const bool walls = !v.laminar && !smooth && h->res_gen == h->flux_gen;
+    const int rc = walls ? enqueue_wall_res(h, v) : enqueue_fvresidual(h, v, h->cfl_cur, 0, 0, &fused);
+    if (!rc) { h->res_gen = h->flux_gen; h->ghosts_set = false; }
     return rc;
 }
 

@@ -173,9 +173,11 @@ struct uns_cc_handle {
     // uns_cc_fvresidual's flux cache: flux_gen is bumped by every call that may
     // change the inputs of the interior and farfield face fluxes (primitives,
     // gradient, limiter, precision, the whole step); res_gen is the flux_gen
-    // of the last fvresidual that computed every face.
+    // of the last fvresidual that computed every face.  ghosts_set: since
+    // then the caller has written the state, ghost rows included.
     long long flux_gen = 0;
     long long res_gen = -1;
+    bool ghosts_set = false;
     uns::CCAdj* adj = nullptr;  // discrete-adjoint state, created by uns_cc_adjoint_prepare
     double* d_post = nullptr;   // post-processing scratch (uns_cc_post.cu), created on first use
     double* d_tec = nullptr;    // tecplt vertex table (uns_cc_post.cu), created on first use

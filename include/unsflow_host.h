@@ -81,6 +81,13 @@ void uns_host_nc_free(uns_host_nc* m);
 int uns_host_sweep_schedule(int n, const int32_t* nbr_off, const int32_t* nbr, int nwarps, int32_t* off, int32_t* items,
                             int32_t* levels);
 
+/* Test hook (no reference counterpart): how uns_cc_create_packed lays out n
+ * cases of cells[i] interior cells: first[n+1] = where each case's cells
+ * begin, and for every block of `threads` threads (one per cell)
+ * block_cell[first[n] / threads] = the cell by which the kernels look up the
+ * block's case. */
+int uns_host_packed_layout(int n, const int32_t* cells, int threads, int32_t* first, int32_t* block_cell);
+
 /* flo.inp readers.  `grid` receives the GridFile value (up to gridlen-1
  * characters). */
 int uns_host_read_flo_cc(const char* path, uns_params* p, char* grid, int gridlen);

@@ -8,6 +8,7 @@
 #include <string>
 #include <vector>
 
+#include "../uns_packed.hpp"
 #include "../uns_sched.hpp"
 #include "host_mesh.hpp"
 #include "unsflow_host.h"
@@ -288,6 +289,15 @@ int uns_host_sweep_schedule(int n, const int32_t* nbr_off, const int32_t* nbr, i
     std::copy(ws.items.begin(), ws.items.end(), items);
     levels[0] = ws.nlev_fwd;
     levels[1] = ws.nlev_bwd;
+    return UNS_OK;
+}
+
+int uns_host_packed_layout(int n, const int32_t* cells, int threads, int32_t* first, int32_t* block_cell) {
+    if (n < 1 || !cells || threads < 1 || threads > uns::kCasePad || (threads & (threads - 1)) || !first || !block_cell)
+        return fail(UNS_ERR_ARG, "uns_host_packed_layout: bad argument");
+    first[0] = 0;
+    for (int i = 0; i < n; ++i) first[i + 1] = first[i] + (int32_t)uns::padded_cells(cells[i]);
+    for (int b = 0; b < first[n] / threads; ++b) block_cell[b] = uns::block_case_cell(b, threads);
     return UNS_OK;
 }
 

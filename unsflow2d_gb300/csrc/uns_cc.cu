@@ -33,6 +33,7 @@
 
 #include "uns_cc_impl.cuh"
 #include "uns_common.cuh"
+#include "uns_packed.hpp"
 #include "uns_phys.cuh"
 #include "uns_sched.hpp"
 #include "uns_sweep.cuh"
@@ -54,8 +55,12 @@ __device__ __forceinline__ double cur_cfl(const CCView& v, int inst, double cfl)
 __device__ __forceinline__ int cell_inst(const CCView& v, int i) { return v.ninst ? v.cinst[i] : 0; }
 __device__ __forceinline__ int face_inst(const CCView& v, int f) { return v.ninst ? v.finst[f] : 0; }
 __device__ __forceinline__ int vert_inst(const CCView& v, int k) { return v.ninst ? v.pinst[k] : 0; }
-// Instance of a block of interior cells: its first cell is a real one.
-__device__ __forceinline__ int block_inst(const CCView& v) { return v.ninst ? v.cinst[blockIdx.x * blockDim.x] : 0; }
+// Instance of a block of interior cells, of any width up to kBlock (every
+// case has cells, so never -1).
+static_assert(kBlock == kCasePad, "the norm's blocks are a case's own");
+__device__ __forceinline__ int block_inst(const CCView& v) {
+    return v.ninst ? v.cinst[block_case_cell(blockIdx.x, blockDim.x)] : 0;
+}
 __device__ __forceinline__ const Gas& gas_of(const CCView& v, int inst) { return v.ninst ? v.gas[inst] : v.g; }
 
 // Minimum / maximum of a 64-bit key over a group of lanes (all of which call
@@ -3062,7 +3067,7 @@ int uns_cc_create_packed(const uns_cc_mesh* meshes, const uns_params* params, in
     std::vector<long long> C(n + 1, 0), F(n + 1, 0), B(n + 1, 0), P(n + 1, 0);
     for (int i = 0; i < n; ++i) {
         const uns_cc_mesh& m = meshes[i];
-        C[i + 1] = C[i] + ((long long)m.noc + kBlock - 1) / kBlock * kBlock;
+        C[i + 1] = C[i] + padded_cells(m.noc);
         F[i + 1] = F[i] + m.nfi;
         B[i + 1] = B[i] + m.nbf;
         P[i + 1] = P[i] + m.nop;

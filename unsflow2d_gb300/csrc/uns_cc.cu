@@ -2518,6 +2518,10 @@ int uns_cc_rk_stage(uns_cc_handle* h, int irk) {
 
 int uns_cc_lusgs(uns_cc_handle* h) {
     if (!h) return UNS_ERR_ARG;
+    if (!h->v.srec) {  // packed cases are explicit: no sweep schedule, no records
+        set_last_error("uns_cc_lusgs: the handle has no sweep schedule (packed cases)");
+        return UNS_ERR_ARG;
+    }
     int rc = uns_cc_fvresidual(h);
     if (rc) return rc;
     CCView v = h->v;

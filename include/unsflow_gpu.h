@@ -155,7 +155,12 @@ int uns_nc_iterate(uns_nc_handle* h, int niter, const double* cfl, int first_ite
  * their own state, CFL schedule, residual history and stop test (an
  * instance whose residual has dropped to its min_res skips its kernels).
  * The handles stay owned by the caller, must outlive the batch and must not
- * be used on their own while a batch call runs. */
+ * be used on their own while a batch call runs.
+ * Implicit (LU-SGS) instances: a sweep is one block per SM at most, on a
+ * narrow mesh fewer, and sweeps that fit on the GPU's SMs together run beside
+ * each other, in a batch or from streams and threads of their own.  A batch
+ * whose sweeps do not fit so takes a form of which an SM holds two, a few per
+ * cent slower alone; handles on threads of their own then take turns. */
 typedef struct uns_cc_batch uns_cc_batch;
 int uns_cc_batch_create(uns_cc_handle* const* handles, int n, uns_cc_batch** out);
 int uns_cc_batch_destroy(uns_cc_batch* b);

@@ -1562,8 +1562,12 @@ SweepArgs sweep_args(const CCView& v, bool mixed) {
     return a;
 }
 
-// The sweeps (uns_sweep.cuh) over the interior cells.
-__global__ void __launch_bounds__(kSweepBlock, 1) k_lusgs(SweepArgs a, const int* done, const int* __restrict__ woff) {
+// The sweeps (uns_sweep.cuh) over the interior cells.  kPerSM: blocks that an
+// SM must have room for.  The FP64 sweep takes 91 registers where it has them
+// (one block), and 80 where sweeps of several handles are to share the SMs
+// (two; 3 to 5 % longer alone).  The FP32 one takes 76 either way.
+template <int kPerSM>
+__global__ void __launch_bounds__(kSweepBlock, kPerSM) k_lusgs(SweepArgs a, const int* done, const int* __restrict__ woff) {
     if (done && *((volatile const int*)done) != 0) return;
     sweep_block<true, false>(a, woff);
 }
@@ -1863,7 +1867,7 @@ int enqueue_lusgs(uns_cc_handle* h, CCView& v) {
     }
     UNS_CUDA(cudaGetLastError());
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(h->coop_blocks);
+    cfg.gridDim = dim3(h->sweep_blocks);
     cfg.blockDim = dim3(kSweepBlock);
     cfg.dynamicSmemBytes = mixed ? sweep_smem_bytes<true>() : sweep_smem_bytes<false>();
     cfg.stream = h->stream;
@@ -1873,8 +1877,8 @@ int enqueue_lusgs(uns_cc_handle* h, CCView& v) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const SweepArgs a = sweep_args(v, mixed);
-    if (mixed) UNS_CUDA(cudaLaunchKernelEx(&cfg, k_lusgs_mixed, a, (const int*)v.done, (const int*)h->woff));
-    else UNS_CUDA(cudaLaunchKernelEx(&cfg, k_lusgs, a, (const int*)v.done, (const int*)h->woff));
+    auto kern = mixed ? k_lusgs_mixed : h->share_sms ? k_lusgs<2> : k_lusgs<1>;
+    UNS_CUDA(cudaLaunchKernelEx(&cfg, kern, a, (const int*)v.done, (const int*)h->woff));
     return UNS_OK;
 }
 
@@ -2226,13 +2230,14 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
         if (maxdeg > 32) { set_last_error("uns_cc_create: a cell has more than 32 faces"); return fail(UNS_ERR_MESH); }
         if (noc >= (1 << 30)) { set_last_error("uns_cc_create: too many cells"); return fail(UNS_ERR_MESH); }
         int dev = 0, nsm = 0, per = 0;
-        if (sweep_allow_smem<false>(k_lusgs) != cudaSuccess || sweep_allow_smem<true>(k_lusgs_mixed) != cudaSuccess ||
+        if (sweep_allow_smem<false>(k_lusgs<1>) != cudaSuccess || sweep_allow_smem<false>(k_lusgs<2>) != cudaSuccess ||
+            sweep_allow_smem<true>(k_lusgs_mixed) != cudaSuccess ||
             cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_lusgs, kSweepBlock, sweep_smem_bytes<false>()) != cudaSuccess || per < 1) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_lusgs<1>, kSweepBlock, sweep_smem_bytes<false>()) != cudaSuccess || per < 1) {
             set_last_error("uns_cc_create: cannot size the cooperative LU-SGS launch");
             return fail(UNS_ERR_CUDA);
         }
-        h->coop_blocks = nsm * std::min(per, kSweepBlocksPerSM);
+        const int blocks = nsm * std::min(per, kSweepBlocksPerSM);
         // the cell across each c2f face (ghosts >= noc), and whether the face
         // normal points into the cell
         auto other = [&](int i, int f, int* flip) {
@@ -2248,7 +2253,8 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
                 nbr[k] = other(i, m->c2f[k], &fl);
                 flip[k] = (signed char)fl;
             }
-        WarpSchedule ws = list_schedule(noc, m->c2f_off, nbr.data(), h->coop_blocks * kSweepPairs);
+        WarpSchedule ws = list_schedule(noc, m->c2f_off, nbr.data(), blocks * kSweepPairs);
+        h->sweep_blocks = ws.blocks();
         std::vector<int4> sched(ws.items.size());
         std::vector<int> rf, rn, rl;
         rf.reserve(2 * (size_t)nfi); rn.reserve(2 * (size_t)nfi); rl.reserve(2 * (size_t)nfi);
@@ -2798,11 +2804,20 @@ int uns_cc_batch_iterate(uns_cc_batch* b, int niter, const double* cfl, int firs
     for (int i = 0; i < n && !rebuild; ++i) rebuild = b->gens[i] != b->hs[i]->gen;
     if (rebuild) {
         if (b->exec) { cudaGraphExecDestroy(b->exec); b->exec = nullptr; }
+        // Sweeps that do not fit beside each other, one block per SM, take the
+        // form of which an SM holds two (102 400 cells each: two handles 3.17
+        // -> 2.02 ms per iteration, three 4.72 -> 3.29, eight 12.6 -> 7.6).
+        int sweeps = 0, blocks = 0;
+        for (const uns_cc_handle* h : b->hs)
+            if (h->P.time_mode == UNS_TIME_LUSGS) { ++sweeps; blocks += h->sweep_blocks; }
+        const bool share = sweeps > 1 && blocks > b->hs[0]->nsm;
         cudaGraph_t parent;
         UNS_CUDA(cudaGraphCreate(&parent, 0));
         for (int i = 0; i < n; ++i) {
             cudaGraph_t child;
+            b->hs[i]->share_sms = share;
             int rc = capture_iteration(b->hs[i], first_iter, &child);
+            b->hs[i]->share_sms = false;
             if (rc) { cudaGraphDestroy(parent); return rc; }
             cudaGraphNode_t node;
             cudaError_t ce = cudaGraphAddChildGraphNode(&node, parent, nullptr, 0, child);

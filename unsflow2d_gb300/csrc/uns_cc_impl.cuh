@@ -152,7 +152,8 @@ struct uns_cc_handle {
     int nparts = 0;
     // LU-SGS levels
     int* woff = nullptr;   // LU-SGS warp schedule: per-warp ranges of v.sched
-    int coop_blocks = 0;
+    int sweep_blocks = 0;  // blocks of the sweeps' launch: those whose lists have items
+    bool share_sms = false;  // the sweeps being captured run beside other handles' (uns_cc_batch_iterate)
     bool blk_face_set = false;  // v.blk_face was chosen (environment, autotuner), not the default
     int nsm = 1;           // SMs of the device (launch widths of small meshes)
     double4 qinf;

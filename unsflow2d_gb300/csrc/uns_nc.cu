@@ -796,7 +796,7 @@ struct uns_nc_handle {
     std::vector<void*> allocs;
     int nparts = 0;
     int* woff = nullptr;    // LU-SGS warp schedule: per-warp ranges of v.sched
-    int coop_blocks = 0;
+    int sweep_blocks = 0;   // blocks of the sweeps' launch: those whose lists have items
     int nsm = 1;            // SMs of the device
     int lev_fwd = 0, lev_bwd = 0;  // dependency levels of the two sweeps (their critical path)
     double4 qinf;
@@ -905,7 +905,7 @@ int launch_sweeps_nc(uns_nc_handle* h, NCView& v) {
     }
     UNS_CUDA(cudaGetLastError());
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(h->coop_blocks);
+    cfg.gridDim = dim3(h->sweep_blocks);
     cfg.blockDim = dim3(kSweepBlock);
     cfg.dynamicSmemBytes = mixed ? sweep_smem_bytes<true>() : sweep_smem_bytes<false>();
     cfg.stream = h->stream;
@@ -1079,7 +1079,7 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
             return fail(UNS_ERR_CUDA);
         }
         h->nsm = nsm;
-        h->coop_blocks = nsm * std::min(per, kSweepBlocksPerSM);
+        const int blocks = nsm * std::min(per, kSweepBlocksPerSM);
         // other end of each v2f edge, and the reference's orientation sign
         auto other = [&](int i, int e, int* sign) {
             if (m->fp2[e] == i) { *sign = -1; return m->fp1[e]; }
@@ -1094,7 +1094,8 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
                 nbr[k] = other(i, m->v2f[k], &sg);
                 sgn[k] = (signed char)sg;
             }
-        WarpSchedule ws = list_schedule(nop, m->v2f_off, nbr.data(), h->coop_blocks * kSweepPairs);
+        WarpSchedule ws = list_schedule(nop, m->v2f_off, nbr.data(), blocks * kSweepPairs);
+        h->sweep_blocks = ws.blocks();
         h->lev_fwd = ws.nlev_fwd;
         h->lev_bwd = ws.nlev_bwd;
         std::vector<int4> sched(ws.items.size());

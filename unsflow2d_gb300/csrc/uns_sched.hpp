@@ -42,14 +42,31 @@ struct WarpSchedule {
     std::vector<int> src;
     double makespan = 0.0;   // simulated length in units of one item's compute
     int nlev_fwd = 0, nlev_bwd = 0;
+
+    // The blocks that have items: the launch needs no others.
+    int blocks() const;
 };
 
 constexpr int kSchedGroup = 4;  // consecutive warps of a block
+constexpr int kSideBySide = 3;  // sweeps of separate handles that should fit beside each other
+
+// How many of nwarps warps the lists of 2 n items in `levels` dependency levels
+// are spread over.  Two warps per item of an average level keep the chain
+// within 3 % of what all the warps give it (NCFVM sweeps, 92 items per level:
+// 1.83 ms on 608 warps, 1.87 on 200; 147 items: 2.99 and, on 304, 3.01), so a
+// graph narrow enough takes a half or a third of the blocks and leaves the
+// other SMs to other handles' sweeps: three solves of the first mesh in three
+// threads 5.49 -> 2.18 ms per iteration.
+inline int sweep_warps(int n, int levels, int nwarps) {
+    const long long side = n > 0 ? std::min<long long>(kSideBySide, (long long)nwarps * levels / (4LL * n)) : 1;
+    if (side < 2) return nwarps;
+    return std::min(nwarps, std::max(1, nwarps / kSchedGroup / (int)side) * kSchedGroup);
+}
 
 // nbr_off / nbr: CSR neighbour lists of the n entities (any order, entries
 // outside [0, n) ignored).  nwarps: warps of the cooperative launch.  kNear,
 // kSync: the extra delay of a dependency on another warp of the block and of
-// another block, in units of one item's compute.
+// another block, in units of one item's compute.  sweep_warps of them get items.
 inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int nwarps, double kNear = 0.05,
                                   double kSync = 0.30) {
     constexpr double kCompute = 1.0;
@@ -92,6 +109,7 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
         int warp, index;
     };
     std::vector<Item> done(2 * (size_t)n);
+    const int used = sweep_warps(n, nlev + nlevb, nwarps);
     std::vector<double> wfree(nwarps, 0.0);
     std::vector<int> wlast(nwarps, -1);
     std::vector<int> count(nwarps, 0), codes, srcs;  // items per warp; every item and its sources as they are placed
@@ -102,10 +120,10 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
     // heap with an entry per placement outgrows the caches on a large mesh
     // (4.2 M cells).
     int leaves = 1;
-    while (leaves < nwarps) leaves *= 2;
+    while (leaves < used) leaves *= 2;
     std::vector<int> first(2 * (size_t)leaves, -1);
     auto earlier = [&](int a, int b) { return b < 0 || (a >= 0 && wfree[a] <= wfree[b]) ? a : b; };
-    for (int w = 0; w < nwarps; ++w) first[leaves + w] = w;
+    for (int w = 0; w < used; ++w) first[leaves + w] = w;
     for (int k = leaves - 1; k > 0; --k) first[k] = earlier(first[2 * k], first[2 * k + 1]);
 
     std::vector<int> preds;
@@ -133,7 +151,7 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
             bool again = false;
             for (size_t q = 0; q < k; ++q) again = again || pr[q].warp / kSchedGroup == g;
             if (again) continue;
-            for (int c = g * kSchedGroup; c < (g + 1) * kSchedGroup && c < nwarps; ++c) consider(c);
+            for (int c = g * kSchedGroup; c < (g + 1) * kSchedGroup && c < used; ++c) consider(c);
         }
         consider(first[1]);
         done[code] = {s + kCompute, w, count[w]++};
@@ -187,6 +205,12 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
         }
     }
     return out;
+}
+
+inline int WarpSchedule::blocks() const {
+    int w = (int)off.size() - 1;
+    while (w > 0 && off[w] == off[w - 1]) --w;
+    return std::max(1, (w + kSchedGroup - 1) / kSchedGroup);
 }
 
 // Asks for what the records of some later item are made of: a warp's list jumps

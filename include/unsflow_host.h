@@ -81,6 +81,11 @@ void uns_host_nc_free(uns_host_nc* m);
 int uns_host_sweep_schedule(int n, const int32_t* nbr_off, const int32_t* nbr, int nwarps, int32_t* off, int32_t* items,
                             int32_t* levels);
 
+/* Test hook (no reference counterpart): the bound, in cycles, that the sweep
+ * kernels put on the waits between a block's own warps when
+ * uns_*_set_wait_limit is given `cycles`. */
+int64_t uns_host_ring_wait_limit(int64_t cycles);
+
 /* Test hook (no reference counterpart): how uns_cc_create_packed lays out n
  * cases of cells[i] interior cells: first[n+1] = where each case's cells
  * begin, and for every block of `threads` threads (one per cell)

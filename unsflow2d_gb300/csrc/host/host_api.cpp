@@ -292,6 +292,8 @@ int uns_host_sweep_schedule(int n, const int32_t* nbr_off, const int32_t* nbr, i
     return UNS_OK;
 }
 
+int64_t uns_host_ring_wait_limit(int64_t cycles) { return uns::ring_wait_limit(cycles); }
+
 int uns_host_packed_layout(int n, const int32_t* cells, int threads, int32_t* first, int32_t* block_cell) {
     if (n < 1 || !cells || threads < 1 || threads > uns::kCasePad || (threads & (threads - 1)) || !first || !block_cell)
         return fail(UNS_ERR_ARG, "uns_host_packed_layout: bad argument");

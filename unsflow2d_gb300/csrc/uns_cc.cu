@@ -1557,7 +1557,7 @@ SweepArgs sweep_args(const CCView& v, bool mixed) {
     a.qold = v.qold; a.res = v.res; a.qc = v.qc;
     a.out = v.srec; a.outf = reinterpret_cast<float4*>(v.srec);
     a.outd = reinterpret_cast<double4*>(v.srec + 2 * (size_t)v.noc);
-    a.err = v.err; a.wait_cycles = v.wait_cycles; a.skip_code = v.skip_code;
+    a.err = v.err; a.wait_cycles = v.wait_cycles; a.ring_cycles = ring_wait_limit(v.wait_cycles); a.skip_code = v.skip_code;
     a.gm1 = v.g.gamma - 1.0;
     return a;
 }

@@ -207,6 +207,14 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
     return out;
 }
 
+// The bound of a wait inside a sweep block for a wait limit of `wait` cycles on
+// another block's record: longer than that wait, so that the warp whose record
+// does not come is the one to report it.  (A limit of any size: no overflow.)
+constexpr long long ring_wait_limit(long long wait) {
+    constexpr long long kMost = 0x7fffffffffffffffLL, kExtra = 100000000LL;
+    return wait > (kMost - kExtra) / 4 ? kMost : 4 * wait + kExtra;
+}
+
 inline int WarpSchedule::blocks() const {
     int w = (int)off.size() - 1;
     while (w > 0 && off[w] == off[w - 1]) --w;

@@ -58,6 +58,7 @@ struct SweepArgs {
     double4* outd;         //   and in FP64 (the entity's own backward step)
     DevErr* err;
     long long wait_cycles; // bound of a wait for a record
+    long long ring_cycles; // and of a wait for a partner (ring_wait_limit)
     int skip_code;         // test hook: the item (entity << 1 | pass) that publishes nothing, or -1
     double gm1;
 };
@@ -104,7 +105,7 @@ struct RingWait {
     DevErr* err;
     long long limit, t0;
     __device__ __forceinline__ RingWait(const int* a, const SweepArgs& s)
-        : abort(a), err(s.err), limit(4 * s.wait_cycles + 100000000LL), t0(0) {}
+        : abort(a), err(s.err), limit(s.ring_cycles), t0(0) {}
     __device__ __forceinline__ bool go_on(int spins) {
         if (spins == 0) t0 = clock64();
         if ((spins & 15) != 15) return true;

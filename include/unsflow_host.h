@@ -81,6 +81,13 @@ void uns_host_nc_free(uns_host_nc* m);
 int uns_host_sweep_schedule(int n, const int32_t* nbr_off, const int32_t* nbr, int nwarps, int32_t* off, int32_t* items,
                             int32_t* levels);
 
+/* Test hook (no reference counterpart): where the sweep warps of that schedule
+ * find their neighbours' records: for each item in the order of `items`, for
+ * each neighbour it waits for in the order of its list, (warp of the block <<
+ * 28) | index in that warp's list, or -1 where another block of four warps
+ * computes it.  src holds nbr_off[n] values at most; *nsrc receives how many. */
+int uns_host_sweep_sources(int n, const int32_t* nbr_off, const int32_t* nbr, int nwarps, int32_t* src, int32_t* nsrc);
+
 /* Test hook (no reference counterpart): the bound, in cycles, that the sweep
  * kernels put on the waits between a block's own warps when
  * uns_*_set_wait_limit is given `cycles`. */

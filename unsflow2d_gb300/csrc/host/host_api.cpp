@@ -292,6 +292,18 @@ int uns_host_sweep_schedule(int n, const int32_t* nbr_off, const int32_t* nbr, i
     return UNS_OK;
 }
 
+int uns_host_sweep_sources(int n, const int32_t* nbr_off, const int32_t* nbr, int nwarps, int32_t* src, int32_t* nsrc) {
+    std::vector<int32_t> off(nwarps > 0 ? nwarps + 1 : 0), items(n > 0 ? 2 * (size_t)n : 0);
+    int32_t lev[2];
+    const int rc = uns_host_sweep_schedule(n, nbr_off, nbr, nwarps, off.data(), items.data(), lev);
+    if (rc) return rc;
+    if (!src || !nsrc) return fail(UNS_ERR_ARG, "uns_host_sweep_sources: bad argument");
+    const uns::WarpSchedule ws = uns::list_schedule(n, nbr_off, nbr, nwarps);
+    std::copy(ws.src.begin(), ws.src.end(), src);
+    *nsrc = (int32_t)ws.src.size();
+    return UNS_OK;
+}
+
 int64_t uns_host_ring_wait_limit(int64_t cycles) { return uns::ring_wait_limit(cycles); }
 
 int uns_host_packed_layout(int n, const int32_t* cells, int threads, int32_t* first, int32_t* block_cell) {

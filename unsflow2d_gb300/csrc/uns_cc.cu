@@ -2254,6 +2254,7 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
                 flip[k] = (signed char)fl;
             }
         WarpSchedule ws = list_schedule(noc, m->c2f_off, nbr.data(), blocks * kSweepPairs);
+        if (!ws.indexable()) { set_last_error("uns_cc_create: too many cells"); return fail(UNS_ERR_MESH); }
         h->sweep_blocks = ws.blocks();
         std::vector<int4> sched(ws.items.size());
         std::vector<int> rf, rn, rl;

@@ -1095,6 +1095,7 @@ int uns_nc_create(const uns_nc_mesh* m, const uns_params* p, uns_nc_handle** out
                 sgn[k] = (signed char)sg;
             }
         WarpSchedule ws = list_schedule(nop, m->v2f_off, nbr.data(), blocks * kSweepPairs);
+        if (!ws.indexable()) { set_last_error("uns_nc_create: too many nodes"); return fail(UNS_ERR_MESH); }
         h->sweep_blocks = ws.blocks();
         h->lev_fwd = ws.nlev_fwd;
         h->lev_bwd = ws.nlev_bwd;

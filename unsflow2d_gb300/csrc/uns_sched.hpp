@@ -33,21 +33,26 @@
 
 namespace uns {
 
+constexpr int kSrcBits = 28;  // of WarpSchedule::src: the list index, under the warp of the block
+
 struct WarpSchedule {
     std::vector<int> off;    // nwarps + 1 offsets into items
     std::vector<int> items;  // (entity << 1) | pass, pass 0 = forward, 1 = backward
     // Item by item, for each neighbour that the item waits for (in the order of
     // its CSR list): where its sweep warp finds the neighbour's record, (warp of
-    // the block << 28) | list index, or -1 for one of another block, in L2.
+    // the block << kSrcBits) | list index, or -1 for one of another block, in L2.
     std::vector<int> src;
     double makespan = 0.0;   // simulated length in units of one item's compute
     int nlev_fwd = 0, nlev_bwd = 0;
 
     // The blocks that have items: the launch needs no others.
     int blocks() const;
+    // Whether every list index fits in src.
+    bool indexable() const;
 };
 
 constexpr int kSchedGroup = 4;  // consecutive warps of a block
+static_assert(kSchedGroup <= 4, "WarpSchedule::src has two bits for the warp");
 constexpr int kSideBySide = 3;  // sweeps of separate handles that should fit beside each other
 
 // How many of nwarps warps the lists of 2 n items in `levels` dependency levels
@@ -162,7 +167,7 @@ inline WarpSchedule list_schedule(int n, const int* nbr_off, const int* nbr, int
         for (int k = (leaves + w) / 2; k > 0 && first[k] == w; k /= 2) first[k] = earlier(first[2 * k], first[2 * k + 1]);
         codes.push_back(code);
         for (size_t k = code & 1; k < pr.size(); ++k)  // not a backward item's own forward value
-            srcs.push_back(pr[k].warp / kSchedGroup == w / kSchedGroup ? (pr[k].warp % kSchedGroup) << 28 | pr[k].index : -1);
+            srcs.push_back(pr[k].warp / kSchedGroup == w / kSchedGroup ? (pr[k].warp % kSchedGroup) << kSrcBits | pr[k].index : -1);
         nsrc[w] += (int)pr.size() - (code & 1);
     };
     for (int i : fwd) {
@@ -219,6 +224,12 @@ inline int WarpSchedule::blocks() const {
     int w = (int)off.size() - 1;
     while (w > 0 && off[w] == off[w - 1]) --w;
     return std::max(1, (w + kSchedGroup - 1) / kSchedGroup);
+}
+
+inline bool WarpSchedule::indexable() const {
+    for (size_t w = 0; w + 1 < off.size(); ++w)
+        if (off[w + 1] - off[w] > 1 << kSrcBits) return false;
+    return true;
 }
 
 // Asks for what the records of some later item are made of: a warp's list jumps

@@ -31,12 +31,14 @@
 #pragma once
 #include "uns_common.cuh"
 #include "uns_fp64.cuh"
+#include "uns_sched.hpp"
 
 #include <type_traits>
 
 namespace uns {
 
 constexpr int kSweepPairs = 4;                   // sweep warps per block: one per SM sub-partition
+static_assert(kSweepPairs == kSchedGroup, "WarpSchedule::src names a warp of a block");
 constexpr int kSweepBlock = 3 * 32 * kSweepPairs;  // sweep warps, feeders, pollers
 // One sweep block per SM, so that concurrently active items never share an FP64 unit.
 constexpr int kSweepBlocksPerSM = 1;
@@ -47,7 +49,7 @@ constexpr double kOmega = 1.5;                   // CCFVM/lusgs.F90:229, NCFVM/l
 struct SweepArgs {
     int n;                 // entities
     const int4* sched;     // (entity, pass, first record, records) per list position
-    const int* rec_src;    // per record: its producer in this block (warp << 28 | list index), or -1
+    const int* rec_src;    // per record: its producer in this block (WarpSchedule::src), or -1
     const double4* rec;    // inputs per record (k_*_sweep_prep): 3 x double4, or 4 x float4 in the mixed form
     const double* diag;    // the diagonal, or its reciprocal in the mixed form
     const double4* qold;
@@ -163,7 +165,7 @@ __device__ __forceinline__ void box_open(SweepBox<NP>& b, int idx) {
 }
 
 // Where a record comes from, in the upper word of an entry's code field: bits
-// 0..30 one more than (warp of the block << 28 | list index), 0 for another
+// 0..30 one more than WarpSchedule::src, 0 for another
 // block's; bit 31 the orientation's sign.
 __device__ __forceinline__ int src_of(long long code) { return (int)((unsigned long long)code >> 32 & 0x7fffffffu) - 1; }
 
@@ -281,8 +283,8 @@ __device__ __forceinline__ void sweep_poll(const SweepArgs& a, RingD& R, const B
                     double2 x0, x1;
                     double rho, dq;
                     if (src >= 0) {
-                        const BoxD& b = boxes[src >> 28];
-                        const int idx = src & 0xfffffff, seq = ld_acquire(&b.seq[idx % kBox]);
+                        const BoxD& b = boxes[src >> kSrcBits];
+                        const int idx = src & ((1 << kSrcBits) - 1), seq = ld_acquire(&b.seq[idx % kBox]);
                         const volatile double* q = reinterpret_cast<const volatile double*>(b.rec[idx % kBox]);
                         x0.x = q[0]; x0.y = q[1]; x1.x = q[2]; x1.y = q[3];
                         rho = q[4]; dq = q[5 + k];
@@ -589,8 +591,8 @@ __device__ __forceinline__ void sweep_poll_mixed(const SweepArgs& a, RingM& R, c
                 if (nb) {
                     float w[4];
                     if (src >= 0) {
-                        const BoxM& b = boxes[src >> 28];
-                        const int idx = src & 0xfffffff, seq = ld_acquire(&b.seq[idx % kBox]);
+                        const BoxM& b = boxes[src >> kSrcBits];
+                        const int idx = src & ((1 << kSrcBits) - 1), seq = ld_acquire(&b.seq[idx % kBox]);
                         const volatile float* q = reinterpret_cast<const volatile float*>(b.rec[idx % kBox]);
                         w[0] = q[0]; w[1] = q[1]; w[2] = q[2]; w[3] = q[3];
                         __threadfence_block();

@@ -1775,22 +1775,26 @@ int enqueue_wall_rk(uns_cc_handle* h, CCView& v, cudaStream_t stream) {
     return UNS_OK;
 }
 
-// The other cells' three stages and the norm's partials; beside the wall cells'
-// where walls is their event (or null, behind them) and the pass is spread.
-int enqueue_cell_rk(uns_cc_handle* h, CCView& v, cudaEvent_t walls) {
+// The other cells' three stages and the norm's partials, but for those of the
+// wall cells' blocks where the pass is spread (enqueue_wall_parts).
+int enqueue_cell_rk(uns_cc_handle* h, CCView& v) {
     if (v.mixed) {
         LAUNCH(k_cell_res_mixed, v.noc, v, 1, 1, 1);
     } else if (rk3_warp_partials(h, v)) {
         CCView w = v;
         w.wpart = 1;
         LAUNCH_SPREAD(k_cell_rk3, v.noc, w);
-        if (v.nwcell == 0) return UNS_OK;
-        if (walls) UNS_CUDA(cudaStreamWaitEvent(h->stream, walls, 0));
-        k_wall_parts<<<v.nwblk, kBlock, 0, h->stream>>>(w);
-        UNS_CUDA(cudaGetLastError());
     } else {
         LAUNCH(k_cell_rk3, v.noc, v);
     }
+    return UNS_OK;
+}
+
+// Those partials, after both kernels.
+int enqueue_wall_parts(uns_cc_handle* h, CCView& v) {
+    if (v.mixed || v.nwcell == 0 || !rk3_warp_partials(h, v)) return UNS_OK;
+    k_wall_parts<<<v.nwblk, kBlock, 0, h->stream>>>(v);
+    UNS_CUDA(cudaGetLastError());
     return UNS_OK;
 }
 
@@ -1800,18 +1804,21 @@ int enqueue_cell_rk(uns_cc_handle* h, CCView& v, cudaEvent_t walls) {
 // On larger ones they fill the chip, the chain gets its turn behind them and the
 // partials' launch comes on top (a mixed packed study: 503 -> 510 us).
 int enqueue_rk3(uns_cc_handle* h, CCView& v) {
-    if (v.nwcell > 0 && !v.mixed && rk3_warp_partials(h, v)) {
-        UNS_CUDA(cudaEventRecord(h->fork, h->stream));
-        UNS_CUDA(cudaStreamWaitEvent(h->side, h->fork, 0));
-        int rc = enqueue_wall_rk(h, v, h->side);
-        const cudaError_t e = cudaEventRecord(h->join, h->side);  // joined on an error too
-        if (rc == UNS_OK) rc = enqueue_cell_rk(h, v, h->join);
-        else cudaStreamWaitEvent(h->stream, h->join, 0);
-        UNS_CUDA(e);
-        return rc;
+    const bool beside = v.nwcell > 0 && !v.mixed && rk3_warp_partials(h, v);
+    if (!beside) {
+        const int rc = enqueue_wall_rk(h, v, h->stream);
+        return rc ? rc : enqueue_cell_rk(h, v);
     }
-    int rc = enqueue_wall_rk(h, v, h->stream);
-    return rc ? rc : enqueue_cell_rk(h, v, nullptr);
+    UNS_CUDA(cudaEventRecord(h->fork, h->stream));
+    UNS_CUDA(cudaStreamWaitEvent(h->side, h->fork, 0));
+    int rc = enqueue_wall_rk(h, v, h->side);
+    if (!rc) rc = enqueue_cell_rk(h, v);
+    // joined whichever of the two launches failed, so that no capture is left open
+    cudaError_t e = cudaEventRecord(h->join, h->side);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(h->stream, h->join, 0);
+    if (rc) return rc;
+    UNS_CUDA(e);
+    return enqueue_wall_parts(h, v);
 }
 
 // fvresidual as a kernel sequence; irk > 0 fuses that RK stage into the
@@ -3025,7 +3032,10 @@ int uns_cc_profile(uns_cc_handle* h, double cfl, int reps, double* ms, const cha
             int fuse = (rk3 && !smooth) ? irk : 0;
             if (!rc && one_pass) rc = timed(11, [&]() -> int { return enqueue_wall_rk(h, v, h->stream); });
             if (!rc) rc = timed(7, [&]() -> int {
-                if (one_pass) return enqueue_cell_rk(h, v, nullptr);
+                if (one_pass) {
+                    const int rc1 = enqueue_cell_rk(h, v);
+                    return rc1 ? rc1 : enqueue_wall_parts(h, v);
+                }
                 if (v.mixed) LAUNCH(k_cell_res_mixed, v.noc, v, fuse, smooth ? 0 : 1, 0);
                 else if (!smooth || v.ninst) LAUNCH(k_cell_res, v.noc, v, fuse, smooth ? 0 : 1);
                 else LAUNCH_SPREAD(k_cell_res, v.noc, v, fuse, 0);  // as the iteration launches it

@@ -2073,8 +2073,7 @@ static int create_impl(const uns_cc_mesh* m, const uns_params* p, bool lusgs_sch
         cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming) != cudaSuccess) {
         set_last_error("uns_cc_create: cudaStreamCreate failed (no usable GPU?)");
-        delete h;
-        return UNS_ERR_CUDA;
+        return fail(UNS_ERR_CUDA);  // with the streams and events that were created
     }
     {
         int dev = 0, nsm = 0;

@@ -26,8 +26,8 @@ const char* uns_last_error(void);
 /* Library version string. */
 const char* uns_version(void);
 /* Test hooks (no reference counterpart), n host values each:
- * out[i] = a[i] / b[i] by the kernels' division through the reciprocal
- * (must equal IEEE division), and lt[i] = whether a[i]/b[i] < c[i]/d[i]
+ * out[i] = a[i] / b[i] by the kernels' division (must equal IEEE division),
+ * and lt[i] = whether a[i]/b[i] < c[i]/d[i]
  * by the kernels' exact ratio comparison (-1 where it does not apply);
  * uns_selftest_fp64 applies operation op of the FP64 arithmetic off the FP64
  * unit (k_selftest_fp64 in csrc/uns_api.cu lists them) to a[i], b[i]. */

@@ -11,12 +11,12 @@
 namespace {
 __global__ void k_selftest_div(const double* a, const double* b, double* out, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = uns::div_rn_recip(a[i], b[i], 1.0 / b[i]);
+    if (i < n) out[i] = uns::div_digits(a[i], b[i]);
 }
 __global__ void k_selftest_ratio(const double* a, const double* b, const double* c, const double* d, int* lt, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    lt[i] = (uns::ratio_ok(a[i], b[i]) && uns::ratio_ok(c[i], d[i])) ? (uns::ratio_less(a[i], b[i], c[i], d[i]) ? 1 : 0) : -1;
+    lt[i] = (uns::ratio_ok(a[i], b[i]) && uns::ratio_ok(c[i], d[i])) ? (uns::ratio_less<uns::F64I>(a[i], b[i], c[i], d[i]) ? 1 : 0) : -1;
 }
 // The operations of uns_fp64.cuh by number, in the order of uns_selftest_fp64.
 __global__ void k_selftest_fp64(int op, const double* a, const double* b, double* out, int n) {

@@ -879,10 +879,11 @@ __device__ __forceinline__ void cell_mul(const CCView& v, int i) {
     const PrimT<F64I> P = con2prim_t<F64I>(g, c.x, c.y, c.z, c.w);
     const F64I s0 = F64I(g.T_infd) / g.SCONST;
     const F64I num = F64I(1.0) + s0, den = P.t + s0;
-    // t^1.5 as t sqrt(t): within one unit in the last place (two correctly
-    // rounded operations; pow's bound is two), without pow's 100 instructions
-    // on the FP64 unit (262 k cells: 73 -> 13 us).  What pow makes of t <= 0
-    // stays pow's.
+    // t^1.5 as t sqrt(t): two correctly rounded operations, each half a unit
+    // in the last place of its own result, together below 1.3 of t^1.5's
+    // (1.2845 at t = 0x1.945ff5c063268p+0; pow's bound is two), without pow's
+    // 100 instructions on the FP64 unit (262 k cells: 73 -> 13 us).  What pow
+    // makes of t <= 0 stays pow's.
     const F64I t15 = dpos(P.t.v) ? P.t * sqrt(P.t) : F64I(pow_rare(P.t.v, 1.5));
     v.mul[i] = ((num / den) * t15).v;
 }
@@ -958,7 +959,6 @@ __device__ __forceinline__ double4 stored_flux(const CCView& v, int f) {
 // products on the integer pipe, the sum's first term and stage 1's weights 0
 // and 1 dropped); k_begin 0.32 -> 0.13 ms alike.
 __device__ __forceinline__ void add4(double r[4], const double4& a) { r[0] = r[0] + a.x; r[1] = r[1] + a.y; r[2] = r[2] + a.z; r[3] = r[3] + a.w; }
-__device__ __forceinline__ void sub4(double r[4], const double4& a) { r[0] = r[0] - a.x; r[1] = r[1] - a.y; r[2] = r[2] - a.z; r[3] = r[3] - a.w; }
 
 // The same on F64 or F64I, the sign by a flip of the operand's sign bit.
 template <class S>
@@ -1614,9 +1614,6 @@ int check_dev_err(uns_cc_handle* h) {
     return rc ? rc : take_dev_err(h, r.err);
 }
 
-// Build the forward/backward level schedules of the lusgs2 sweeps: a cell
-// waits for every interior neighbour that precedes it in sweep order.
-
 void launch_cfg(int n, dim3& g, dim3& b) { b = dim3(kBlock); g = dim3(std::max(1, nblocks(n))); }
 
 #define LAUNCH(kern, n, ...)                                                         \
@@ -1634,7 +1631,6 @@ int enqueue_minmax(uns_cc_handle* h, CCView& v) {
     return UNS_OK;
 }
 
-// k_cell_grad, or its FP32 form for a handle in the mixed form.
 // k_face_conv's grid: the boundary faces' blocks, then the interior faces'.
 #define LAUNCH_FACE_CONV(R, v)                                                                     \
     do {                                                                                           \
@@ -1681,6 +1677,8 @@ inline int face_bs(const uns_cc_handle* h, const CCView& v) {
 
 #define LAUNCH_SPREAD(kern, n, ...) LAUNCH_BS(kern, (n), spread_bs(h, (n)), __VA_ARGS__)
 
+// k_cell_grad by the size of the launch; LAUNCH_CELL_GRAD: or its FP32 form for
+// a handle in the mixed form.
 #define LAUNCH_FP64_GRAD(v, flags, cfl)                                                          \
     do {                                                                                       \
         if (spread_bs(h, (v).noc) < kBlock) LAUNCH_SPREAD(k_cell_grad<F64>, (v).noc, (v), (int)(flags), (cfl)); \

@@ -459,51 +459,23 @@ __device__ __forceinline__ double vk_limit(double a, double b, double tol) {
 // Exponent field of a double (integer pipe).
 __device__ __forceinline__ int dexp_field(double x) { return (int)((__double_as_longlong(x) >> 52) & 0x7ff); }
 
-// RN(a / b) given y = RN(1 / b), by Markstein's correction (P. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000
-// processor", IBM J. Res. Develop. 34(1), 1990): with q0 = RN(a y) (within
-// one ulp of a/b) the remainder r = a - b q0 is exact in one FMA, and
-// RN(q0 + r y) is the correctly rounded quotient.  The theorem assumes no
-// overflow or underflow, so operands and results outside a margin of the
-// normal range (and subnormals) take the IEEE division instead; for a zero
-// numerator the quotient is q0 itself (the corrected sum would turn -0 into
-// +0).  One IEEE division per distinct divisor, then three FP64 operations
-// per quotient.
-__device__ __forceinline__ double div_rn_recip(double a, double b, double y) {
-    const double q0 = a * y;
-    const bool zero = (__double_as_longlong(a) & 0x7fffffffffffffffLL) == 0;
-    if (zero) return q0;
-    const double r = __fma_rn(-q0, b, a);
-    const double q1 = __fma_rn(r, y, q0);
-    const int ea = dexp_field(a), eq = dexp_field(q1);
-    if (ea < 128 || ea > 1920 || eq < 128 || eq > 1920) return a / b;
-    return q1;
-}
-
 // Whether n1/d1 < n2/d2 exactly (d1, d2 > 0, all finite and normal, the
 // cross products inside the normal range): n1 d2 and n2 d1 as exact
 // double-double values (product and its FMA error term) compared.  The
 // minimum of correctly rounded quotients is the correctly rounded quotient
 // of the exact minimum (rounding is monotonic), so one division of the
-// selected pair gives min_k RN(n_k / d_k).
-__device__ __forceinline__ bool ratio_less(double n1, double d1, double n2, double d2) {
-    const double p1 = n1 * d2, p2 = n2 * d1;
-    if (p1 != p2) return p1 < p2;
-    return __fma_rn(n1, d2, -p1) < __fma_rn(n2, d1, -p2);
-}
-
-// The same on F64 or F64I (their products and comparison are the same bits);
-// equal products, which are rare, in a call (see uns_fp64.cuh's rare paths).
+// selected pair gives min_k RN(n_k / d_k).  S = F64 or F64I; equal products,
+// which are rare, in a call (see uns_fp64.cuh's rare paths).
 static __device__ __noinline__ bool ratio_less_tie(double n1, double d1, double n2, double d2, double p) {
     return __fma_rn(n1, d2, -p) < __fma_rn(n2, d1, -p);
 }
-static __device__ __noinline__ double vk_limit_rare(double a, double b, double tol) { return vk_limit(a, b, tol); }
 template <class S>
 __device__ __forceinline__ bool ratio_less(S n1, S d1, S n2, S d2) {
     const S p1 = n1 * d2, p2 = n2 * d1;
     if (__double_as_longlong(p1.v) != __double_as_longlong(p2.v)) return p1 < p2;
     return ratio_less_tie(n1.v, d1.v, n2.v, d2.v, p1.v);
 }
+static __device__ __noinline__ double vk_limit_rare(double a, double b, double tol) { return vk_limit(a, b, tol); }
 
 // Whether the ratio test above is exact for these operands: d positive,
 // both with binary exponents within [-463, 457] (n may be zero), so that

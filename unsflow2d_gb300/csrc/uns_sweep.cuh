@@ -373,7 +373,6 @@ struct SweepEntry {
 
 template <bool kCC>
 __device__ __forceinline__ void sweep_items(const SweepArgs& a, RingD& R, BoxD& box, double* wx, int kbeg, int kend, int lane) {
-    const unsigned all = 0xffffffffu;
     const int k = lane & 3;
     const double gm1 = in_register(a.gm1), one = opaque_one(), mzero = opaque_mzero();
     const unsigned m0 = lane_mask(k == 0), m2 = lane_mask(k == 2), m01 = lane_mask(k < 2);

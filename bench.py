@@ -95,6 +95,8 @@ WORKLOADS = {
 # cell_res_mixed, res_final.
 # LU-SGS: reset_minmax, begin, vertex_avg, face_prim_spec, cell_grad, face_conv, cell_res,
 # sweep_prep, one fill of the records (two in the FP32 form), sweeps, res_final.
+# NCFVM LU-SGS: save_old, grad_lim, edge, node_res, then in FP64 qold_prim, sweep_prep and one
+# fill of the records, in the FP32 form sweep_prep and two; sweeps, res_final.
 LAUNCHES = {("nc", "lusgs"): 9, ("nc", "rk3"): 5, ("cc", "rk3"): 10, ("cc", "lusgs"): 12, ("cc", "rk3_mixed_gg"): 8}
 
 
@@ -115,14 +117,20 @@ def cc_launches(p) -> int:
     return 5 + (1 if ggfc else 0) + 3 * per_stage + 1
 
 
-def cc_kernels(p, cells: int) -> int:
-    """cc_launches less what one iteration on that many cells does not launch of that sequence."""
+def cc_kernels(p, cells: int, sms: int) -> int:
+    """cc_launches less what one iteration on that many cells, on a GPU of that many SMs, does not launch
+    of that sequence."""
     n = cc_launches(p)
     if p.time_mode != abi.TIME["rk3"]:
         return n - (1 if p.precision == abi.PREC["fp64"] else 0)  # one fill of the sweeps' records
     if p.flow_type == abi.FLOW["laminar"]:
         return n - (2 if p.grad_type == abi.GRAD["ggfc"] else 0)  # stages 2-3: cell_mul with the wall faces
-    return n - (1 if p.precision != abi.PREC["mixed"] and cells > 2 * 256 * 152 - 256 else 0)  # wall_parts
+    return n - (1 if p.precision != abi.PREC["mixed"] and cells > (2 * sms - 1) * 256 else 0)  # wall_parts
+
+
+def nc_kernels(p) -> int:
+    """Kernels one NCFVM iteration launches (enqueue_iteration_nc)."""
+    return LAUNCHES[("nc", "lusgs" if p.time_mode == abi.TIME["lusgs"] else "rk3")]
 
 
 def adjoint_cost(solver, w: dict, cfl: float, prof: dict) -> dict:
@@ -818,10 +826,8 @@ def run_ours(args, w, dist, rank, local_rank) -> dict | None:
                    "l2": f"inputs larger than L2: ~{ws_mb:.0f} MB of per-iteration arrays vs 129 MB L2, no flush",
                    "setup_s": round(setup_s, 2), "block_sizes": blocks},
         "e2e": e2e,
-        "gpu_launches": (cc_kernels(p, units) if kind == "cc" else
-                         LAUNCHES[(kind, "lusgs" if p.time_mode == abi.TIME["lusgs"] else "rk3")]
-                         + (1 if (kind, p.time_mode, p.precision) == ("nc", abi.TIME["lusgs"], abi.PREC["fp64"]) else 0))
-                        * args.steps,
+        "gpu_launches": (nc_kernels(p) if kind == "nc" else
+                         cc_kernels(p, units, torch.cuda.get_device_properties(dev).multi_processor_count)) * args.steps,
         "clocks": clocks,
         "roofline": {"bound": "hbm", "kernel": rl_kernel, "achieved": round(achieved, 1), "peak": peak,
                      "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": traffic,

@@ -993,7 +993,7 @@ def run_configs(args, dist, rank, local_rank) -> dict:
         r = subprocess.run(cmd, capture_output=True, text=True, env=dict(os.environ, UNSFLOW_FP64_FMA="1"),
                            timeout=1200)
         try:
-            d = json.loads(r.stdout.strip().splitlines()[-1])
+            d = json.loads(next(x for x in r.stderr.splitlines() if x.startswith(DETAILS))[len(DETAILS):])
             fma[key] = {"workload": d["config"]["workload"], "gpu_library": d.get("gpu_library"), "value": d["value"],
                         "ms_per_step": d["ms_per_step"], "clocks": d["clocks"],
                         "kernels_ms_per_iter": {k: v["ms_per_iter"] for k, v in d["kernels"].items()}}
@@ -1010,6 +1010,32 @@ def run_configs(args, dist, rank, local_rank) -> dict:
                 out[key]["speedup_vs_plain_fp64"] = round(out[key]["value"] / plain, 3)
                 out[key]["plain_fp64_reference"] = "configuration 3's 2048x1024 mesh in the plain FP64 form (key 3_fp64)"
     return out
+
+
+DETAILS = "bench: details "  # how the line of all details begins, on stderr
+
+
+def headline(out: dict) -> dict:
+    """The one line for stdout: the contract's keys and one figure per
+    configuration, short enough to be read whole from the tail of a log."""
+    pick = lambda d, *ks: {k: d[k] for k in ks if d.get(k) is not None}  # noqa: E731
+    line = {k: v for k, v in out.items() if not isinstance(v, dict)}
+    line["config"] = pick(out["config"], "workload", "instances", "units", "global_batch", "seq_len", "parallelism", "l2",
+                          "block_sizes")
+    line["e2e"] = {k: round(v, 3) if isinstance(v, float) else v
+                   for k, v in pick(out["e2e"], "value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step").items()}
+    line["clocks"] = out["clocks"]
+    line["roofline"] = pick(out["roofline"], "bound", "kernel", "achieved", "peak", "unit", "frac", "traffic", "duration_ms")
+    if "cpu_baseline" in out:
+        line["cpu_baseline"] = pick(out["cpu_baseline"], "value", "unit", "cores", "kind")
+    if "parity" in out:
+        line["parity"] = pick(out["parity"], "pass", "iterations", "state_bit_identical")
+    if "time_to_1e-8" in out:
+        line["time_to_1e-8_s"] = {k: v["seconds"] for k, v in out["time_to_1e-8"].items() if isinstance(v, dict)}
+    if "configs" in out:
+        line["configs"] = {k: v.get("value") for k, v in out["configs"].items() if k != "fp64_fma"}
+        line["fp64_fma"] = {k: v.get("value") for k, v in out["configs"].get("fp64_fma", {}).items()}
+    return line
 
 
 def main():
@@ -1062,7 +1088,8 @@ def main():
             if fma2.get("value"):
                 fma2["speedup_vs_bit_exact"] = round(fma2["value"] / out["value"], 3)
     if out is not None:
-        print(json.dumps(out))
+        print(DETAILS + json.dumps(out), file=sys.stderr, flush=True)
+        print(json.dumps(headline(out)))
     if dist is not None:
         dist.destroy_process_group()
     return 0

@@ -1062,13 +1062,15 @@ __global__ void __launch_bounds__(kBlock, 8) k_cell_res_mixed(CCView v, int irk,
             const int k0 = v.cf_off[i], k1 = v.cf_off[i + 1];
             const float4* fF = v.fFf();
             auto add = [&](int k, int e, float4 F) {
-                const unsigned m = (e & FACE_MASK) < v.nfi && (e & SIDE_BIT) ? 0x80000000u : 0u;
-                F.x = __uint_as_float(__float_as_uint(F.x) ^ m); F.y = __uint_as_float(__float_as_uint(F.y) ^ m);
-                F.z = __uint_as_float(__float_as_uint(F.z) ^ m); F.w = __uint_as_float(__float_as_uint(F.w) ^ m);
-                const double4 D = widen4(F);
+                const bool minus = (e & FACE_MASK) < v.nfi && (e & SIDE_BIT);
+                const unsigned m = minus ? 0x80000000u : 0u;
                 if (k == k0) {
-                    r[0] = D.x; r[1] = D.y; r[2] = D.z; r[3] = D.w;
+                    const double4 D = widen4(F);
+                    r[0] = flip64(D.x, minus); r[1] = flip64(D.y, minus); r[2] = flip64(D.z, minus); r[3] = flip64(D.w, minus);
                 } else {
+                    F.x = __uint_as_float(__float_as_uint(F.x) ^ m); F.y = __uint_as_float(__float_as_uint(F.y) ^ m);
+                    F.z = __uint_as_float(__float_as_uint(F.z) ^ m); F.w = __uint_as_float(__float_as_uint(F.w) ^ m);
+                    const double4 D = widen4(F);
                     r[0] = add64(r[0], D.x); r[1] = add64(r[1], D.y); r[2] = add64(r[2], D.z); r[3] = add64(r[3], D.w);
                 }
             };
@@ -1098,7 +1100,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_cell_res_mixed(CCView v, int irk,
                 double c[4], q[4];
                 d4get(v.qc[i], c);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) q[j] = __fma_rn(neg64(D), r[j], c[j]);
+                for (int j = 0; j < 4; ++j) q[j] = __fma_rn(-D, r[j], c[j]);
                 if (irk > 1) {
                     const double a = rk3_a(irk), b = rk3_b(irk);
                     double o[4];
@@ -1141,7 +1143,7 @@ __device__ __forceinline__ void rk_update(int irk, double D, const double o[4], 
     const double a = rk3_a(irk), b = rk3_b(irk);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        if (kMixed) q[j] = __fma_rn(a, o[j], mul64(b, __fma_rn(neg64(D), r[j], q[j])));
+        if (kMixed) q[j] = __fma_rn(a, o[j], mul64(b, __fma_rn(-D, r[j], q[j])));
         else if (irk == 2) q[j] = (F64I(a) * F64I(o[j]) + quarter(F64I(q[j]) - F64I(D) * F64I(r[j]))).v;  // b = 1/4
         else q[j] = (F64I(a) * F64I(o[j]) + F64I(b) * (F64I(q[j]) - F64I(D) * F64I(r[j]))).v;
     }

@@ -92,7 +92,9 @@ static __device__ __noinline__ double mul_rare(double a, double b) {
 }
 static __device__ __noinline__ double div_rare(double a, double b) { return a / b; }
 static __device__ __noinline__ double sqrt_rare(double a) { return sqrt(a); }
-static __device__ __noinline__ double widen_rare(float a) { return (double)a; }
+static __device__ __noinline__ double widen_rare(float a) {  // a NaN as FP32 arithmetic gives it, whatever sign a flip left on it
+    return a != a ? dmake(0x7fffffffu, 0xe0000000u) : (double)a;
+}
 static __device__ __noinline__ float narrow_rare(double a) { return (float)a; }
 
 // (double)a and (float)a on the integer pipe (the conversions hold the FP64

@@ -486,10 +486,16 @@ __device__ __forceinline__ bool ratio_ok(double n, double d) {
     return (nz || (en >= 560 && en <= 1480)) && ed >= 560 && ed <= 1480 && __double_as_longlong(d) > 0;
 }
 
-// Order-preserving 64-bit encoding of a double for atomicMax/atomicMin.
+// Order-preserving 64-bit encoding of a double for atomicMax/atomicMin.  A
+// positive NaN, what FP32 arithmetic gives, reads as a number just below zero
+// (so that a non-finite cell leaves the limiter range of the others finite), a
+// negative one as the lowest.  (On 32-bit words: the compiler makes a 64-bit
+// "b | sign" a floating-point -|x|, whose NaN is its own.)
 __device__ __forceinline__ unsigned long long enc_ord(double x) {
-    unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    return (b & 0x8000000000000000ULL) ? ~b : (b | 0x8000000000000000ULL);
+    const unsigned h = dhi(x), l = dlo(x);
+    if (h & 0x80000000u) return u64(~h, ~l);
+    const bool nan = h > 0x7ff00000u || (h == 0x7ff00000u && l != 0u);
+    return u64(nan ? h : h | 0x80000000u, l);
 }
 __host__ __device__ __forceinline__ double dec_ord(unsigned long long e) {
     unsigned long long b = (e & 0x8000000000000000ULL) ? (e & 0x7FFFFFFFFFFFFFFFULL) : ~e;

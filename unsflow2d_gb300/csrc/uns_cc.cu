@@ -2966,6 +2966,8 @@ int uns_cc_autotune(uns_cc_handle* h, int reps, int* blocks) {
     return check_dev_err(h);
 }
 
+// cell_rk23 is the wall cells' three stages (k_wall_rk3); where they run,
+// cell_res is the other cells' pass (k_cell_rk3 or k_cell_res_mixed).
 int uns_cc_profile(uns_cc_handle* h, double cfl, int reps, double* ms, const char** names, int nphase) {
     static const char* kNames[] = {"begin", "vertex_avg", "face_prim_spec", "face_ggfc", "cell_grad", "face_conv",
                                    "viscous", "cell_res", "cirs", "lusgs_sweeps", "residue", "cell_rk23"};

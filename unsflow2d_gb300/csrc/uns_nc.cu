@@ -236,9 +236,9 @@ __global__ void __launch_bounds__(kBlock, std::is_same<S, F64I>::value ? 3 : 1) 
     v.gx[i] = m4s(gx);
     v.gy[i] = m4s(gy);
     // DUmax/DUmin over the node's edges (limiter.f90:24-39), as order keys
-    // (of two zeros they prefer the positive, rmax / rmin the first; a zero
-    // extreme has magnitude below eps or is the ratio's numerator, where its
-    // sign drops out).
+    // (of two zeros they prefer the positive, rmax / rmin the first: a zero
+    // extreme has magnitude below eps or is a Barth ratio's numerator, and then
+    // phi is a zero, whose sign alone may differ).
     long long dmx[4], dmn[4];
     S ph[4];
 #pragma unroll
